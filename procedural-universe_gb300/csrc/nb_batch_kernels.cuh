@@ -38,7 +38,7 @@ namespace nb {
 constexpr int kGWarps = 4;              // warps per traversal block
 constexpr int kGroupMax = 64;           // bodies per traversal group (two per lane)
 constexpr int kGroupMinDepth = 4;       // a group cell lies >= 4 levels below its galaxy root
-constexpr int kBoxChunk = 8192;         // bodies per block of the bounding-box pass
+constexpr int kBoxChunk = 2048;         // bodies per block of the bounding-box pass (8 a thread)
 constexpr int kGStack = 512;            // cells waiting to be opened, per warp (<= 32 pushed per step)
 constexpr int kStackCellLimit = 1 << 27;   // a stack entry packs a first-child index below this with 4 bits
 constexpr int kGMultiTop = kGStack - 155 - 32;   // stack height up to which a walk step takes several cells
@@ -90,7 +90,8 @@ __device__ __forceinline__ void box_flush(unsigned* bits, int slot, const float 
     }
 }
 
-// block b reduces bodies [b*kBoxChunk, (b+1)*kBoxChunk) of the Barnes-Hut range
+// block b reduces bodies [b*kBoxChunk, (b+1)*kBoxChunk) of the Barnes-Hut range.
+// Latency-bound: eight dependent loads a thread instead of 32, four times the blocks.
 __global__ void __launch_bounds__(256) k_gal_box_chunks(const float4* __restrict__ pos,
                                                         const int32_t* __restrict__ body_slot, int n, int nslot,
                                                         unsigned* __restrict__ bits) {
@@ -111,18 +112,40 @@ __global__ void __launch_bounds__(256) k_gal_box_chunks(const float4* __restrict
         lo[0] = fminf(lo[0], p.x); lo[1] = fminf(lo[1], p.y); lo[2] = fminf(lo[2], p.z);
         hi[0] = fmaxf(hi[0], p.x); hi[1] = fmaxf(hi[1], p.y); hi[2] = fmaxf(hi[2], p.z);
     }
-    // common case: the whole warp ended in one galaxy -> one set of atomics per warp
-    const int lane = threadIdx.x & 31;
-    const int c0 = __shfl_sync(0xffffffffu, cur, 0);
-    if (__all_sync(0xffffffffu, cur == c0)) {
+    // a warp that ended in one galaxy reduces its bounds; a block that did adds one set of atomics
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ int sh_gal;
+    __shared__ float sh_box[8][6];
+    if (threadIdx.x == 0) sh_gal = cur;
+    __syncthreads();
+    const int c0 = sh_gal;
+    const bool one = __syncthreads_and(cur == c0 || cur < 0) != 0;   // no body: neutral bounds
+    const int w0 = __shfl_sync(0xffffffffu, cur, 0);
+    if (__all_sync(0xffffffffu, cur == w0 || cur < 0)) {
         for (int a = 0; a < 3; ++a)
             for (int o = 16; o > 0; o >>= 1) {
                 lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
                 hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
             }
-        if (lane == 0 && c0 >= 0) box_flush(bits, c0, lo, hi);
+        if (lane == 0 && w0 >= 0 && !one) box_flush(bits, w0, lo, hi);
+        if (lane == 0 && one)
+            for (int a = 0; a < 3; ++a) {
+                sh_box[warp][a] = lo[a];
+                sh_box[warp][3 + a] = hi[a];
+            }
     } else if (cur >= 0) {
         box_flush(bits, cur, lo, hi);
+    }
+    if (one) {   // block-uniform
+        __syncthreads();
+        if (threadIdx.x == 0 && c0 >= 0) {
+            for (int w = 1; w < 8; ++w)
+                for (int a = 0; a < 3; ++a) {
+                    lo[a] = fminf(lo[a], sh_box[w][a]);
+                    hi[a] = fmaxf(hi[a], sh_box[w][3 + a]);
+                }
+            box_flush(bits, c0, lo, hi);
+        }
     }
 }
 

@@ -69,33 +69,31 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
 
 // ---------------------------------------------------------------- K2 keys --
 // The octant path of body p (Octree::Add's descent) and its length; gap: the
-// path met a gap between float child bounds and was cut short.
+// path met a gap between float child bounds and was cut short.  A body that a
+// cell holds is never below the cell's lower bound, so an axis takes the upper
+// half when p >= middle and only there can it miss (p beyond middle + size, the
+// float sum the upper child ends at).  No branch a level: the three axes of 32
+// bodies go eight ways.
 __device__ __forceinline__ uint64_t body_key(const float4 p, float half, int D, bool& inside, bool& gap, int& d) {
-    float lo0 = -half, lo1 = -half, lo2 = -half, hi0 = half, hi1 = half, hi2 = half;
-    inside = p.x >= lo0 && p.y >= lo1 && p.z >= lo2 && p.x < hi0 && p.y < hi1 && p.z < hi2;
+    float lo0 = -half, lo1 = -half, lo2 = -half;
+    const float hi = half;
+    inside = p.x >= lo0 && p.y >= lo1 && p.z >= lo2 && p.x < hi && p.y < hi && p.z < hi;
     gap = false;
     d = 0;
     if (!inside) return ~0ull;
     uint64_t key = 0;
-    float size = __fsub_rn(hi0, lo0);
+    float size = __fsub_rn(hi, lo0);
     for (int l = 0; l < D; ++l) {
         const float s = __fmul_rn(size, 0.5f);   // Size / 2: exact halving, the same value as a division
         const float m0 = __fadd_rn(lo0, s), m1 = __fadd_rn(lo1, s), m2 = __fadd_rn(lo2, s);
         const float t0 = __fadd_rn(m0, s), t1 = __fadd_rn(m1, s), t2 = __fadd_rn(m2, s);
-        int oct = 0;
-        bool ok = true;
-        if (p.x >= m0 && p.x < t0) { oct |= 1; lo0 = m0; hi0 = t0; }
-        else if (p.x >= lo0 && p.x < m0) { hi0 = m0; }
-        else ok = false;
-        if (p.y >= m1 && p.y < t1) { oct |= 2; lo1 = m1; hi1 = t1; }
-        else if (p.y >= lo1 && p.y < m1) { hi1 = m1; }
-        else ok = false;
-        if (p.z >= m2 && p.z < t2) { oct |= 4; lo2 = m2; hi2 = t2; }
-        else if (p.z >= lo2 && p.z < m2) { hi2 = m2; }
-        else ok = false;
-        if (!ok) break;
-        size = __fsub_rn(hi0, lo0);
-        key = (key << 3) | (uint64_t)oct;
+        const bool u0 = p.x >= m0, u1 = p.y >= m1, u2 = p.z >= m2;
+        if ((u0 && !(p.x < t0)) || (u1 && !(p.y < t1)) || (u2 && !(p.z < t2))) break;
+        size = u0 ? __fsub_rn(t0, m0) : __fsub_rn(m0, lo0);   // the child's extent along x
+        lo0 = u0 ? m0 : lo0;
+        lo1 = u1 ? m1 : lo1;
+        lo2 = u2 ? m2 : lo2;
+        key = (key << 3) | (uint64_t)((u0 ? 1u : 0u) | (u1 ? 2u : 0u) | (u2 ? 4u : 0u));
         ++d;
     }
     if (d < D) {   // a gap between float child bounds: left-align the path
@@ -105,13 +103,24 @@ __device__ __forceinline__ uint64_t body_key(const float4 p, float half, int D, 
     return key;
 }
 
-// Zeroes this tile's look-back status words: every radix pass's, and the
-// positions scan's.
+// Keys per thread of the keys kernels.  A key is a chain of ~21 dependent float
+// steps, so a block of few keys a thread hides it behind other blocks: a whole
+// 4096-key tile a block left 25 blocks at 100,000 bodies and one at 4,000
+// (64 us either way).  More keys a thread only pays once every SM holds its
+// eight blocks, by fewer histogram flushes.
+inline int keys_per_thread(size_t nk, int sm_count) {
+    int items = 1;
+    while (items < 4 && nk / (size_t)(kSortThreads * items * 2) >= (size_t)(8 * sm_count)) items *= 2;
+    return items;
+}
+
+// Zeroes the look-back status words of every radix pass and of the positions
+// scan, spread over the grid.
 __device__ __forceinline__ void zero_tile_status(unsigned long long* sort_status, int ntiles,
-                                                 unsigned long long* pos_status) {
-    for (int p = 0; p < kPasses; ++p)
-        sort_status[((size_t)p * ntiles + blockIdx.x) * 256 + threadIdx.x] = 0ull;
-    if (threadIdx.x == 0) pos_status[blockIdx.x] = 0ull;
+                                                 unsigned long long* pos_status, int blocks) {
+    const int words = kPasses * ntiles * 256;
+    for (int i = blockIdx.x * kSortThreads + threadIdx.x; i < words; i += blocks * kSortThreads) sort_status[i] = 0ull;
+    for (int i = blockIdx.x * kSortThreads + threadIdx.x; i < ntiles; i += blocks * kSortThreads) pos_status[i] = 0ull;
 }
 
 // Radix passes that the top bits make redundant.  Keys are grouped by their
@@ -130,21 +139,32 @@ __device__ __forceinline__ unsigned long long* group_bits(uint32_t* ghist) {
     return reinterpret_cast<unsigned long long*>(ghist + kPasses * 256);
 }
 
-// Adds a key to its group's bits in shared memory: one atomic pair per warp
-// when the warp's keys share a group (the common case once keys are in
-// galaxy or octant order), else one per lane.
-__device__ __forceinline__ void note_group(uint64_t key, unsigned long long* sh) {
+// Counts a warp's keys into the digit histograms and the group bits in shared
+// memory.  A digit that the whole warp shares (the upper levels of a galaxy
+// that fills a small part of the root cube) is added once for the warp: 32
+// atomics on one word would be done one after the other.
+__device__ __forceinline__ void count_key(uint64_t key, uint32_t (*h)[256], unsigned long long* sh) {
+    const uint32_t full = 0xffffffffu;
+    const uint32_t lo = (uint32_t)key, hi = (uint32_t)(key >> 32);
+    const uint32_t olo = __reduce_or_sync(full, lo), ohi = __reduce_or_sync(full, hi);
+    const uint32_t zlo = __reduce_or_sync(full, ~lo), zhi = __reduce_or_sync(full, ~hi);
+    const uint64_t o = ((uint64_t)ohi << 32) | olo, z = ((uint64_t)zhi << 32) | zlo;
+    const uint64_t varies = o & z;   // bits that differ within the warp
+    const bool first = (threadIdx.x & 31) == 0;
+#pragma unroll
+    for (int p = 0; p < kPasses; ++p) {
+        const uint32_t d = (uint32_t)(key >> (8 * p)) & 255u;
+        if (((varies >> (8 * p)) & 255ull) == 0ull) {
+            if (first) atomicAdd(&h[p][d], 32u);
+        } else {
+            atomicAdd(&h[p][d], 1u);
+        }
+    }
     const uint32_t g = (uint32_t)(key >> 60);
-    const uint32_t g0 = __shfl_sync(0xffffffffu, g, 0);
-    if (__all_sync(0xffffffffu, g == g0)) {
-        const uint32_t lo = (uint32_t)key, hi = (uint32_t)(key >> 32);
-        const unsigned long long o =
-            ((unsigned long long)__reduce_or_sync(0xffffffffu, hi) << 32) | __reduce_or_sync(0xffffffffu, lo);
-        const unsigned long long z =
-            ((unsigned long long)__reduce_or_sync(0xffffffffu, ~hi) << 32) | __reduce_or_sync(0xffffffffu, ~lo);
-        if ((threadIdx.x & 31) == 0) {
-            atomicOr(&sh[g0], o);
-            atomicOr(&sh[kKeyGroups + g0], z);
+    if ((varies >> 60) == 0ull) {
+        if (first) {
+            atomicOr(&sh[g], (unsigned long long)o);
+            atomicOr(&sh[kKeyGroups + g], (unsigned long long)z);
         }
     } else {
         atomicOr(&sh[g], (unsigned long long)key);
@@ -152,8 +172,8 @@ __device__ __forceinline__ void note_group(uint64_t key, unsigned long long* sh)
     }
 }
 
-// Adds a tile's digit histograms of every pass into ghist (bins that are
-// zero in this tile cost nothing), and its group bits after them.
+// Adds a block's digit histograms of every pass into ghist (bins that are
+// zero in this block cost nothing), and its group bits after them.
 __device__ __forceinline__ void flush_hist(uint32_t (*h)[256], const unsigned long long* sh_groups, uint32_t* ghist) {
     __syncthreads();
     for (int i = threadIdx.x; i < kPasses * 256; i += kSortThreads) {
@@ -164,22 +184,28 @@ __device__ __forceinline__ void flush_hist(uint32_t (*h)[256], const unsigned lo
         atomicOr(&group_bits(ghist)[threadIdx.x], sh_groups[threadIdx.x]);
 }
 
-// K2 + the radix sort's global histograms: one block per tile of kSortTile
-// keys (key ~0 past n); counts bodies inside the root and paths cut by gaps.
+// K2 + the radix sort's global histograms: kSortThreads * items keys a block
+// (key ~0 past n); counts bodies inside the root and paths cut by gaps.
+// Bound by the descent's arithmetic (~21 levels a key) once there are enough
+// blocks; before, by one long chain a thread and, at 1M, by 32,768 atomics on
+// the body count.  GB300, events: 4,000 bodies 62 -> 10 us, 100,003 64 -> 12 us,
+// 1,048,576 74 -> 41 us.
 __global__ void __launch_bounds__(kSortThreads) k_keys_hist(const float4* __restrict__ pos, int n, float half, int D,
                                                             uint64_t* __restrict__ keys, int32_t* __restrict__ vals,
                                                             int32_t* __restrict__ depth,
                                                             int32_t* __restrict__ counters, uint32_t* __restrict__ ghist,
                                                             unsigned long long* __restrict__ sort_status, int ntiles,
-                                                            unsigned long long* __restrict__ pos_status) {
+                                                            unsigned long long* __restrict__ pos_status, int items) {
     __shared__ uint32_t h[kPasses][256];
     __shared__ unsigned long long sh_groups[2 * kKeyGroups];
+    __shared__ int sh_in, sh_gaps;   // one global atomic a block: one a warp queued 32,768 on one word at 1M
     for (int i = threadIdx.x; i < kPasses * 256; i += kSortThreads) (&h[0][0])[i] = 0;
     if (threadIdx.x < 2 * kKeyGroups) sh_groups[threadIdx.x] = 0ull;
-    zero_tile_status(sort_status, ntiles, pos_status);
+    if (threadIdx.x == 0) sh_in = sh_gaps = 0;
+    zero_tile_status(sort_status, ntiles, pos_status, gridDim.x);
     __syncthreads();
-    for (int it = 0; it < kSortItems; ++it) {
-        const int i = blockIdx.x * kSortTile + it * kSortThreads + threadIdx.x;
+    for (int it = 0; it < items; ++it) {
+        const int i = (blockIdx.x * items + it) * kSortThreads + threadIdx.x;
         vals[i] = i;
         bool inside = false, gap = false;
         uint64_t key = ~0ull;
@@ -189,51 +215,69 @@ __global__ void __launch_bounds__(kSortThreads) k_keys_hist(const float4* __rest
             depth[i] = d;
         }
         keys[i] = key;
-#pragma unroll
-        for (int p = 0; p < kPasses; ++p) atomicAdd(&h[p][(key >> (8 * p)) & 255], 1u);
-        note_group(key, sh_groups);
+        count_key(key, h, sh_groups);
         const uint32_t in_b = __ballot_sync(0xffffffffu, inside);
         const uint32_t gap_b = __ballot_sync(0xffffffffu, gap);
         if ((threadIdx.x & 31) == 0) {
-            if (in_b) atomicAdd(&counters[TC_NIN], __popc(in_b));
-            if (gap_b) atomicAdd(&counters[TC_GAPS], __popc(gap_b));
+            if (in_b) atomicAdd(&sh_in, __popc(in_b));
+            if (gap_b) atomicAdd(&sh_gaps, __popc(gap_b));
         }
     }
     flush_hist(h, sh_groups, ghist);
+    if (threadIdx.x == 0) {
+        if (sh_in) atomicAdd(&counters[TC_NIN], sh_in);
+        if (sh_gaps) atomicAdd(&counters[TC_GAPS], sh_gaps);
+    }
 }
 
 // ------------------------------------------------------------ K3 radix sort --
 // plan[p] = 1 when pass p is skipped: every key has the same digit, or (below
-// the top pass) every key of each top group has (note_group); plan[8+p] =
+// the top pass) every key of each top group has (count_key); plan[8+p] =
 // buffer the pass reads; plan[16] = buffer holding the result.  dig_off[p][d] = keys
 // with a smaller digit than d in pass p (where digit d's keys start).
-__global__ void k_sort_plan(const uint32_t* __restrict__ ghist, int nk, int32_t* __restrict__ plan,
-                            int32_t* __restrict__ dig_off) {
+// One warp per pass, eight digits a lane: 8.3 -> 4 us against eight block scans
+// one after the other (ncu).
+static_assert(kPasses * 32 == 256, "one warp per pass");
+__global__ void __launch_bounds__(256) k_sort_plan(const uint32_t* __restrict__ ghist, int nk,
+                                                   int32_t* __restrict__ plan, int32_t* __restrict__ dig_off) {
     __shared__ int triv[kPasses];
-    __shared__ int sh_warp[33];
+    const int p = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint4* bins = reinterpret_cast<const uint4*>(ghist + p * 256) + 2 * lane;
+    const uint4 a = bins[0], b = bins[1];
     // bits that vary within some top group
-    __shared__ unsigned long long sh_var;
-    if (threadIdx.x == 0) {
-        const unsigned long long* gb = group_bits(const_cast<uint32_t*>(ghist));
-        unsigned long long var = 0ull;
-        for (int g = 0; g < kKeyGroups; ++g) var |= gb[g] & gb[kKeyGroups + g];
-        sh_var = var;
+    const unsigned long long* gb = group_bits(const_cast<uint32_t*>(ghist));
+    const unsigned long long v = lane < kKeyGroups ? gb[lane] & gb[kKeyGroups + lane] : 0ull;
+    const uint32_t vlo = __reduce_or_sync(0xffffffffu, (uint32_t)v);
+    const uint32_t vhi = __reduce_or_sync(0xffffffffu, (uint32_t)(v >> 32));
+    const unsigned long long var = ((unsigned long long)vhi << 32) | vlo;
+    const int c[8] = {(int)a.x, (int)a.y, (int)a.z, (int)a.w, (int)b.x, (int)b.y, (int)b.z, (int)b.w};
+    int sum = 0;
+    bool all = false;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        sum += c[k];
+        all |= c[k] == nk;
     }
-    __syncthreads();
-    for (int p = 0; p < kPasses; ++p) {
-        const int c = (int)ghist[p * 256 + threadIdx.x];
-        const int t = __syncthreads_or(c == nk);
-        if (threadIdx.x == 0) triv[p] = t || (p < kPasses - 1 && ((sh_var >> (8 * p)) & 255ull) == 0ull);
-        int total;
-        dig_off[p * 256 + threadIdx.x] = block_excl_scan(c, sh_warp, &total);
+    int run = warp_incl_scan(sum) - sum;
+    int4 o[2];
+    int* of = reinterpret_cast<int*>(o);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        of[k] = run;
+        run += c[k];
     }
+    int4* out = reinterpret_cast<int4*>(dig_off + p * 256) + 2 * lane;
+    out[0] = o[0];
+    out[1] = o[1];
+    const bool one = __any_sync(0xffffffffu, all);
+    if (lane == 0) triv[p] = one || (p < kPasses - 1 && ((var >> (8 * p)) & 255ull) == 0ull);
     __syncthreads();
     if (threadIdx.x == 0) {
         int cur = 0;
-        for (int p = 0; p < kPasses; ++p) {
-            plan[p] = triv[p];
-            plan[8 + p] = cur;
-            if (!triv[p]) cur ^= 1;
+        for (int q = 0; q < kPasses; ++q) {
+            plan[q] = triv[q];
+            plan[8 + q] = cur;
+            if (!triv[q]) cur ^= 1;
         }
         plan[16] = cur;
     }
@@ -803,25 +847,25 @@ __global__ void k_mass(int n_int, const int32_t* __restrict__ n_int_dev, const i
 
 // ------------------------------------------------- batched forest keys ----
 // Keys of the batched form's Barnes-Hut bodies [0, n) (nb_morton.cuh), with
-// the radix sort's histograms and the look-back status cleared, one block per
-// sort tile; the first threads also write each galaxy's cube for the
+// the radix sort's histograms and the look-back status cleared,
+// kSortThreads * items keys a block; the first threads also write each galaxy's cube for the
 // traversal.  Pad entries [n, tiles * kSortTile) get key ~0.
 __global__ void __launch_bounds__(kSortThreads) k_batch_keys_hist(
     const float4* __restrict__ pos, const int32_t* __restrict__ body_slot, int n, const unsigned* __restrict__ box_bits,
     int nslot, float4* __restrict__ gal_box, uint64_t* __restrict__ keys, int32_t* __restrict__ vals,
     int32_t* __restrict__ depth, uint32_t* __restrict__ ghist, unsigned long long* __restrict__ sort_status,
-    int ntiles, unsigned long long* __restrict__ pos_status) {
+    int ntiles, unsigned long long* __restrict__ pos_status, int items, int key_blocks) {
     __shared__ uint32_t h[kPasses][256];
     __shared__ unsigned long long sh_groups[2 * kKeyGroups];
     const int g = blockIdx.x * kSortThreads + threadIdx.x;
     if (g < nslot) gal_box[g] = gal_cube(box_bits, g);
-    if ((int)blockIdx.x >= ntiles) return;   // blocks past the keys only write galaxy cubes (block-uniform)
+    if ((int)blockIdx.x >= key_blocks) return;   // blocks past the keys only write galaxy cubes (block-uniform)
     for (int i = threadIdx.x; i < kPasses * 256; i += kSortThreads) (&h[0][0])[i] = 0;
     if (threadIdx.x < 2 * kKeyGroups) sh_groups[threadIdx.x] = 0ull;
-    zero_tile_status(sort_status, ntiles, pos_status);
+    zero_tile_status(sort_status, ntiles, pos_status, key_blocks);
     __syncthreads();
-    for (int it = 0; it < kSortItems; ++it) {
-        const int i = blockIdx.x * kSortTile + it * kSortThreads + threadIdx.x;
+    for (int it = 0; it < items; ++it) {
+        const int i = (blockIdx.x * items + it) * kSortThreads + threadIdx.x;
         vals[i] = i;
         uint64_t key = ~0ull;
         if (i < n) {
@@ -830,9 +874,7 @@ __global__ void __launch_bounds__(kSortThreads) k_batch_keys_hist(
             depth[i] = kBatchDepth;
         }
         keys[i] = key;
-#pragma unroll
-        for (int p = 0; p < kPasses; ++p) atomicAdd(&h[p][(key >> (8 * p)) & 255], 1u);
-        note_group(key, sh_groups);
+        count_key(key, h, sh_groups);
     }
     flush_hist(h, sh_groups, ghist);
 }
@@ -962,9 +1004,10 @@ static cudaError_t launch_keys(nb_sim* sim, size_t nk) {
     const int ntiles = (int)(nk / kSortTile);
     NB_TRY(cudaMemsetAsync(t.counters, 0, (kCounterWords + kPasses * 256 + 4 * kKeyGroups) * 4, sim->stream));
     PhaseScope ps(sim, NB_PHASE_KEYS);
-    k_keys_hist<<<ntiles, kSortThreads, 0, sim->stream>>>(sim->pos, (int)sim->n, sim->prm.bounds_half,
-                                                          sim->prm.max_depth, t.keys[0], t.vals[0], t.depth,
-                                                          t.counters, t.ghist, t.sort_status, ntiles, t.pos_status);
+    const int items = keys_per_thread(nk, sim->sm_count);
+    k_keys_hist<<<(unsigned)(nk / (size_t)(kSortThreads * items)), kSortThreads, 0, sim->stream>>>(
+        sim->pos, (int)sim->n, sim->prm.bounds_half, sim->prm.max_depth, t.keys[0], t.vals[0], t.depth, t.counters,
+        t.ghist, t.sort_status, ntiles, t.pos_status, items);
     return cudaGetLastError();
 }
 
@@ -1084,12 +1127,16 @@ int tree_counter_words() { return kCounterWords + kPasses * 256 + 4 * kKeyGroups
 cudaError_t tree_batch_keys(nb_sim* sim, const float4* pos, const int32_t* body_slot, int n,
                             const unsigned* box_bits, int nslot, float4* gal_box) {
     TreeBuffers& t = sim->tree;
-    const int ntiles = (int)(pad_up(std::max<size_t>((size_t)n, 1), kSortTile) / kSortTile);
-    const int blocks = std::max(ntiles, (nslot + kSortThreads - 1) / kSortThreads);
+    const size_t nk = pad_up(std::max<size_t>((size_t)n, 1), kSortTile);
+    const int ntiles = (int)(nk / kSortTile);
+    const int items = keys_per_thread(nk, sim->sm_count);
+    const int key_blocks = (int)(nk / (size_t)(kSortThreads * items));
+    const int blocks = std::max(key_blocks, (nslot + kSortThreads - 1) / kSortThreads);
     PhaseScope ps(sim, NB_PHASE_KEYS);
     k_batch_keys_hist<<<blocks, kSortThreads, 0, sim->stream>>>(pos, body_slot, n, box_bits, nslot, gal_box,
                                                                 t.keys[0], t.vals[0], t.depth, t.ghist,
-                                                                t.sort_status, ntiles, t.pos_status);
+                                                                t.sort_status, ntiles, t.pos_status, items,
+                                                                key_blocks);
     return cudaGetLastError();
 }
 
