@@ -372,11 +372,18 @@ struct TopoView {
     const int32_t* depth;     // per body (input order)
     int n_in, n_total, D;
     int int_cap, cell_cap;    // capacities of the internal-node and cell arrays
+    bool cut;                 // some path met a gap: depths differ from D
+    // Bodies' depths are all D unless a path met a gap between float child
+    // bounds (never in the batched form): only then are they gathered, two
+    // random reads for every delta.
+    __device__ void read_gaps(const int32_t* counters) { cut = counters[TC_GAPS] != 0; }
     __device__ int delta(int s) const {   // common levels of sorted bodies s and s+1; -1 past the end
         if (s < 0 || s + 1 >= n_in) return -1;
         int l = lcp_levels(keys[s], keys[s + 1], D);
-        l = min(l, depth[vals[s]]);
-        l = min(l, depth[vals[s + 1]]);
+        if (cut) {
+            l = min(l, depth[vals[s]]);
+            l = min(l, depth[vals[s + 1]]);
+        }
         return l;
     }
     // Nodes starting at sorted position s: internal levels lo..hi and a leaf at
@@ -489,57 +496,71 @@ __device__ __forceinline__ void position_nodes(const TopoView& tv, const float4*
     }
 }
 
-// Per tile of kSortTile sorted positions (kSortItems consecutive ones per
-// thread): the nodes starting there, and the exclusive prefix of their
-// internal-node counts by single-pass scan (pos_nint; the total goes to
-// counters[TC_NINT]).  With hk_zero, the threads also clear the internal-node
-// hash table for the emission that follows.
-__global__ void __launch_bounds__(kSortThreads) k_positions_scan(TopoView tv, const float4* __restrict__ spos,
-                                                                 int32_t* __restrict__ pos_nint,
-                                                                 int32_t* __restrict__ leaf_level,
-                                                                 int32_t* __restrict__ leaf_count,
-                                                                 int32_t* __restrict__ counters,
-                                                                 unsigned long long* __restrict__ status, int ntiles,
-                                                                 uint64_t* __restrict__ hk_zero, int hk_n,
-                                                                 int* __restrict__ err) {
-    __shared__ int sh_warp[33], sh_off, sh_tile;
+// Per tile of kSortTile sorted positions: the nodes starting there, and the
+// exclusive prefix of their internal-node counts by single-pass scan (pos_nint;
+// the total goes to counters[TC_NINT]).  With hk_zero, the threads also clear
+// the internal-node hash table for the emission that follows.
+//
+// A thread takes every kPosThreads-th position (neighbouring threads read and
+// write neighbouring words), and the counts go through shared memory to the
+// scan, which wants consecutive ones.  Sixteen consecutive positions a thread and
+// a depth gather for each delta took 81 us cold at 1M bodies; the whole topology
+// phase went from 258 to 194 us there, from 98 to 73 us at 100,003 (events).
+constexpr int kPosThreads = 1024;
+constexpr int kPosItems = kSortTile / kPosThreads;
+static_assert(kPosItems == 4, "the scan's counts are read as one int4 a thread");
+__global__ void __launch_bounds__(kPosThreads) k_positions_scan(TopoView tv, const float4* __restrict__ spos,
+                                                                int32_t* __restrict__ pos_nint,
+                                                                int32_t* __restrict__ leaf_level,
+                                                                int32_t* __restrict__ leaf_count,
+                                                                int32_t* __restrict__ counters,
+                                                                unsigned long long* __restrict__ status, int ntiles,
+                                                                uint64_t* __restrict__ hk_zero, int hk_n,
+                                                                int* __restrict__ err) {
+    __shared__ int sh_warp[33], sh_off, sh_tile, sh_leaf, sh_deeper;
+    __shared__ __align__(16) int sh_nint[kSortTile];
     if (hk_zero)
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < hk_n; i += gridDim.x * blockDim.x) hk_zero[i] = 0ull;
+    if (threadIdx.x == 0) sh_leaf = sh_deeper = 0;
     const int tile = lb_tile_index(&counters[TC_TILE_POS], &sh_tile);
     tv.n_in = counters[TC_NIN];
-    const int s0 = tile * kSortTile + threadIdx.x * kSortItems;
-    int nint[kSortItems];
-    int sum = 0;
+    tv.read_gaps(counters);
     unsigned nleaf = 0, ndeeper = 0;
 #pragma unroll
-    for (int k = 0; k < kSortItems; ++k) {
-        const int s = s0 + k;
-        nint[k] = 0;
+    for (int k = 0; k < kPosItems; ++k) {
+        const int j = k * kPosThreads + threadIdx.x, s = tile * kSortTile + j;
+        int nint = 0;
         if (s < tv.n_total) {
             int lf, count;
             bool deeper;
-            position_nodes(tv, spos, s, nint[k], lf, count, deeper);
+            position_nodes(tv, spos, s, nint, lf, count, deeper);
             leaf_level[s] = lf;
             leaf_count[s] = count;
             nleaf += lf >= 0 ? 1u : 0u;
             ndeeper += deeper ? 1u : 0u;
         }
-        sum += nint[k];
+        sh_nint[j] = nint;
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        nleaf += __shfl_xor_sync(0xffffffffu, nleaf, o);
-        ndeeper += __shfl_xor_sync(0xffffffffu, ndeeper, o);
-    }
+    nleaf = __reduce_add_sync(0xffffffffu, nleaf);
+    ndeeper = __reduce_add_sync(0xffffffffu, ndeeper);
     if ((threadIdx.x & 31) == 0) {
-        if (nleaf) atomicAdd(&counters[TC_NLEAF], (int)nleaf);
-        if (ndeeper) atomicAdd(&counters[TC_DEEPER], (int)ndeeper);
+        if (nleaf) atomicAdd(&sh_leaf, (int)nleaf);
+        if (ndeeper) atomicAdd(&sh_deeper, (int)ndeeper);
     }
-    int run = lb_scan_tile(sum, tile, ntiles, status, counters + TC_NINT, sh_warp, &sh_off, err);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (sh_leaf) atomicAdd(&counters[TC_NLEAF], sh_leaf);
+        if (sh_deeper) atomicAdd(&counters[TC_DEEPER], sh_deeper);
+    }
+    int4* mine = reinterpret_cast<int4*>(sh_nint) + threadIdx.x;
+    const int4 c = *mine;
+    const int run = lb_scan_tile(c.x + c.y + c.z + c.w, tile, ntiles, status, counters + TC_NINT, sh_warp, &sh_off, err);
+    *mine = make_int4(run, run + c.x, run + c.x + c.y, run + c.x + c.y + c.z);
+    __syncthreads();
 #pragma unroll
-    for (int k = 0; k < kSortItems; ++k) {
-        const int s = s0 + k;
-        if (s < tv.n_total) pos_nint[s] = run;
-        run += nint[k];
+    for (int k = 0; k < kPosItems; ++k) {
+        const int j = k * kPosThreads + threadIdx.x, s = tile * kSortTile + j;
+        if (s < tv.n_total) pos_nint[s] = sh_nint[j];
     }
 }
 
@@ -555,6 +576,7 @@ __global__ void k_emit(TopoView tv, const int32_t* __restrict__ int_base, int32_
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     for (int i = s; i < popc_tiles; i += gridDim.x * blockDim.x) popc_status[i] = 0ull;   // for k_popc_scan
     if (s >= tv.n_in) return;
+    tv.read_gaps(counters);
     int lo, hi, nint, lf, cur;
     tv.info(s, lo, hi, nint, lf, cur);
     const uint64_t key = tv.keys[s];
@@ -628,6 +650,7 @@ __global__ void k_link(const int32_t* __restrict__ int_level, const int32_t* __r
                        const int32_t* __restrict__ hv, uint32_t hmask, int32_t* __restrict__ int_parent,
                        int32_t* __restrict__ leaf_parent, uint32_t* __restrict__ int_mask,
                        int32_t* __restrict__ int_nint, int32_t* __restrict__ counters) {
+    tv.read_gaps(counters);
     if ((int)blockIdx.x < int_blocks) {
         const int k = blockIdx.x * blockDim.x + threadIdx.x;
         const int ni = n_int_dev ? min(*n_int_dev, n_int) : n_int;
@@ -640,8 +663,9 @@ __global__ void k_link(const int32_t* __restrict__ int_level, const int32_t* __r
 }
 
 // int_block[k] = non-empty children of internal nodes before k (their first
-// child cell, less one), by single-pass scan over tiles of kSortTile nodes.
-__global__ void __launch_bounds__(kSortThreads) k_popc_scan(const uint32_t* __restrict__ mask, int n_int,
+// child cell, less one), by single-pass scan over tiles of kSortTile nodes
+// (the layout of k_positions_scan).
+__global__ void __launch_bounds__(kPosThreads) k_popc_scan(const uint32_t* __restrict__ mask, int n_int,
                                                             const int32_t* __restrict__ n_int_dev,
                                                             int32_t* __restrict__ out, int32_t* __restrict__ counters,
                                                             unsigned long long* __restrict__ status, int ntiles,
@@ -649,17 +673,22 @@ __global__ void __launch_bounds__(kSortThreads) k_popc_scan(const uint32_t* __re
     __shared__ int sh_warp[33], sh_off, sh_tile;
     const int tile = lb_tile_index(&counters[TC_TILE_POPC], &sh_tile);
     const int ni = n_int_dev ? min(*n_int_dev, n_int) : n_int;
-    const int k0 = tile * kSortTile + threadIdx.x * kSortItems;
-    int c[kSortItems];
-    int sum = 0;
-    for (int k = 0; k < kSortItems; ++k) {
-        c[k] = (k0 + k < ni) ? __popc(mask[k0 + k]) : 0;
-        sum += c[k];
+    __shared__ __align__(16) int sh_cnt[kSortTile];
+#pragma unroll
+    for (int k = 0; k < kPosItems; ++k) {
+        const int j = k * kPosThreads + threadIdx.x, q = tile * kSortTile + j;
+        sh_cnt[j] = q < ni ? __popc(mask[q]) : 0;
     }
-    int run = lb_scan_tile(sum, tile, ntiles, status, nullptr, sh_warp, &sh_off, err);
-    for (int k = 0; k < kSortItems; ++k) {
-        if (k0 + k < n_int) out[k0 + k] = run;
-        run += c[k];
+    __syncthreads();
+    int4* mine = reinterpret_cast<int4*>(sh_cnt) + threadIdx.x;
+    const int4 c = *mine;
+    const int run = lb_scan_tile(c.x + c.y + c.z + c.w, tile, ntiles, status, nullptr, sh_warp, &sh_off, err);
+    *mine = make_int4(run, run + c.x, run + c.x + c.y, run + c.x + c.y + c.z);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kPosItems; ++k) {
+        const int j = k * kPosThreads + threadIdx.x, q = tile * kSortTile + j;
+        if (q < n_int) out[q] = sh_cnt[j];
     }
 }
 
@@ -994,6 +1023,7 @@ static TopoView topo_view(nb_sim* sim) {
     tv.D = sim->prm.max_depth;
     tv.int_cap = (int)t.int_cap;
     tv.cell_cap = (int)t.cell_cap;
+    tv.cut = true;   // read_gaps in the kernels
     return tv;
 }
 
@@ -1044,7 +1074,7 @@ cudaError_t tree_build(nb_sim* sim) {
                                                         t.plan, t.spos);
         t.final_buf = 0;
         TopoView tv = topo_view(sim);
-        k_positions_scan<<<ntiles, kSortThreads, 0, st>>>(tv, t.spos, t.pos_nint, t.leaf_level, t.leaf_count,
+        k_positions_scan<<<ntiles, kPosThreads, 0, st>>>(tv, t.spos, t.pos_nint, t.leaf_level, t.leaf_count,
                                                           t.counters, t.pos_status, ntiles, nullptr, 0, sim->d_err);
         NB_TRY(cudaMemcpyAsync(t.h_counters, t.counters, TC_COUNT * 4, cudaMemcpyDeviceToHost, st));
         NB_TRY(cudaStreamSynchronize(st));
@@ -1071,7 +1101,7 @@ cudaError_t tree_build(nb_sim* sim) {
         k_link<<<ib + nbk, kEmitBlock, 0, st>>>(t.int_level, t.int_first, t.int_code, tv, ni, nullptr, ib, t.pos_nint,
                                                t.leaf_level, t.hkeys, t.hvals, hmask, t.int_parent, t.leaf_parent,
                                                t.int_mask, t.int_nint, t.counters);
-        k_popc_scan<<<ptiles, kSortThreads, 0, st>>>(t.int_mask, ni, nullptr, t.int_block, t.counters,
+        k_popc_scan<<<ptiles, kPosThreads, 0, st>>>(t.int_mask, ni, nullptr, t.int_block, t.counters,
                                                      t.popc_status, ptiles, sim->d_err);
         k_place<<<ib + nbk, kEmitBlock, 0, st>>>(t.int_level, t.int_code, t.int_parent, t.int_mask, t.int_block, ni,
                                                 nullptr, ib, tv, t.leaf_level, t.leaf_count, t.leaf_parent, t.spos,
@@ -1157,6 +1187,7 @@ cudaError_t tree_build_graph(nb_sim* sim, const float4* pos, int n, int D, bool 
     tv.D = D;
     tv.int_cap = (int)t.int_cap;
     tv.cell_cap = (int)t.cell_cap;
+    tv.cut = true;   // read_gaps in the kernels
     const int icap = (int)t.int_cap;
     const uint32_t hmask = (uint32_t)(t.hash_cap - 1);
     const int nbk = (n + kEmitBlock - 1) / kEmitBlock;
@@ -1166,7 +1197,7 @@ cudaError_t tree_build_graph(nb_sim* sim, const float4* pos, int n, int D, bool 
     k_gather_final<<<(n + 255) / 256, 256, 0, st>>>(pos, t.keys[0], t.keys[1], t.vals[0], t.vals[1], n, t.plan,
                                                     t.spos);
     // this scan also clears the internal-node hash table for the emission
-    k_positions_scan<<<ntiles, kSortThreads, 0, st>>>(tv, t.spos, t.pos_nint, t.leaf_level, t.leaf_count, t.counters,
+    k_positions_scan<<<ntiles, kPosThreads, 0, st>>>(tv, t.spos, t.pos_nint, t.leaf_level, t.leaf_count, t.counters,
                                                       t.pos_status, ntiles, counts_only ? nullptr : t.hkeys,
                                                       (int)t.hash_cap, sim->d_err);
     if (counts_only) return cudaGetLastError();   // the node counts are in counters[TC_NINT], [TC_NLEAF]
@@ -1175,7 +1206,7 @@ cudaError_t tree_build_graph(nb_sim* sim, const float4* pos, int n, int D, bool 
     k_link<<<ib + nbk, kEmitBlock, 0, st>>>(t.int_level, t.int_first, t.int_code, tv, icap, t.counters + TC_NINT, ib,
                                            t.pos_nint, t.leaf_level, t.hkeys, t.hvals, hmask, t.int_parent,
                                            t.leaf_parent, t.int_mask, t.int_nint, t.counters);
-    k_popc_scan<<<ptiles, kSortThreads, 0, st>>>(t.int_mask, icap, t.counters + TC_NINT, t.int_block, t.counters,
+    k_popc_scan<<<ptiles, kPosThreads, 0, st>>>(t.int_mask, icap, t.counters + TC_NINT, t.int_block, t.counters,
                                                  t.popc_status, ptiles, sim->d_err);
     k_place<<<ib + nbk, kEmitBlock, 0, st>>>(t.int_level, t.int_code, t.int_parent, t.int_mask, t.int_block, icap,
                                             t.counters + TC_NINT, ib, tv, t.leaf_level, t.leaf_count, t.leaf_parent,
