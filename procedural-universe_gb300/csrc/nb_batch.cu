@@ -194,7 +194,7 @@ int enqueue_step(nb_batch* b, float dt, bool update, bool tree_only = false) {
         if (tree_only) return NB_OK;
         {
             PhaseScope ps(c, NB_PHASE_MASS, 3);
-            k_batch_moments<<<(unsigned)((t.int_cap + 255) / 256), 256, 0, st>>>(
+            k_batch_moments<<<(unsigned)((t.int_cap + 127) / 128), 128, 0, st>>>(
                 (int)t.int_cap, t.counters, t.int_parent, t.int_nint, t.int_pending, t.int_cell, t.int_block,
                 t.int_mask, t.int_first, t.int_level, b->cell_rec, (int)t.cell_cap, c->d_err);
             k_batch_roots<<<(b->nslot + 127) / 128, 128, 0, st>>>(b->slot_start, b->nslot, t.keys[0], t.pos_nint,

