@@ -160,6 +160,197 @@ __global__ void __launch_bounds__(BLOCK) k_direct_force(const float4* __restrict
     }
 }
 
+// K1 for large states: every unordered pair once (Newton's third law).
+//
+// The force kernel is bound by the FP32 pipe: 13 operations an interaction in
+// k_direct_force.  A pair's separation and its reciprocal root serve both of
+// its bodies, so doing the pair once costs 17 operations for two interactions.
+//
+// A row is a block of kPairRow = 1024 target bodies, eight a thread in
+// registers (four packed FP32x2 pairs); a unit of work is a row against a run
+// of source tiles at or after the row's own first tile.  Lane l of a warp
+// takes source (l + r) mod 32 of a 32-body chunk at step r, read from the
+// shared tile without bank conflicts, and the sources' own sums travel with
+// them: six shuffles a step move them to the lane that takes that source
+// next.  The four warps take the
+// tile's four chunks in turn (a barrier between turns), adding the chunk's
+// sums into the tile's shared totals in a fixed order, so results are
+// deterministic.  Tiles of the row's own block take part as sources only: all
+// their ordered pairs are evaluated from the target side.
+//
+// Targets are folded into compensated totals every 32 sources as in
+// k_direct_force (the totals live in shared memory, registers hold the running
+// sums), sources every kPairGroup = 4 steps (16 terms in each packed half) into
+// a second running sum and once a chunk into the totals.  A unit
+// writes its targets' totals, and for each tile behind the row the sources':
+// part holds [units][n_pad] target partials, then for each row of the launch
+// one entry per body behind it.
+// Bound by the FP32 pipe (77-79% of its cycles; three-operand packed
+// instructions leave the rest).  Three blocks an SM at 156 registers: four
+// (128) and five (102) measured 1% and 4% slower.  A step, GB300: 262,144
+// bodies 28.5 -> 19.7 ms, 100,003 4.27 -> 2.97 ms, 20,001 217 -> 156 us; the
+// force error against FP64 is k_direct_force's (2.8e-8 and 2.8e-8 at 262,144
+// bodies of the Plummer sphere, 3.5e-8 and 3.5e-8 at 20,001).
+constexpr int kPairThreads = 128, kPairIpt = 8, kPairGroup = 4;
+constexpr int kPairRow = kPairThreads * kPairIpt;
+constexpr int kPairRowTiles = kPairRow / kTileJ;
+static_assert(kPairThreads == kTileJ, "one thread per source of a tile");
+static_assert(kPad % kPairRow == 0, "padded states hold whole rows");
+
+// Tiles per unit of a row that has `tiles` source tiles, cut into at most `units`.
+__host__ __device__ __forceinline__ int pair_unit_tiles(int tiles, int units) { return (tiles + units - 1) / units; }
+
+// Source entries of the rows before `row` in a launch that starts at row0.
+__host__ __device__ __forceinline__ size_t pair_source_base(int row, int row0, int n_pad) {
+    const size_t r = (size_t)(row - row0), first = (size_t)n_pad - (size_t)(row0 + 1) * kPairRow;
+    return r * first - (size_t)kPairRow * (r * (r - (r > 0 ? 1 : 0)) / 2);
+}
+
+template <int LAW, bool HEAVY>
+__global__ void __launch_bounds__(kPairThreads, 3) k_direct_pairs(const float4* __restrict__ pos, int n_pad, int row0,
+                                                                  int units, float S, float4* __restrict__ part,
+                                                                  int* __restrict__ err, uint32_t polls,
+                                                                  const unsigned* __restrict__ mmax) {
+    __shared__ __align__(128) float4 tile[2][kTileJ];
+    __shared__ float tot[2][3 * kPairIpt][kPairThreads];   // targets: sums, compensations
+    __shared__ float src[2][3][kTileJ];                    // the tile's sources: sums, compensations
+    __shared__ __align__(8) uint64_t bar[2];
+    const int row = row0 + blockIdx.y, ntiles = n_pad / kTileJ;
+    const int per = pair_unit_tiles(ntiles - row * kPairRowTiles, units);
+    const int t_begin = row * kPairRowTiles + blockIdx.x * per;
+    const int nt = min(ntiles, t_begin + per) - t_begin;
+    if (nt <= 0) return;   // the whole block
+    const float tiny = HEAVY ? self_pair_tiny(mmax) : kTiny;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int P = kPairIpt / 2;
+    constexpr int kTurns = kTileJ / 32;
+    constexpr uint32_t kBytes = kTileJ * sizeof(float4);
+    const float2 S2 = make_float2(S, S), T2 = make_float2(tiny, tiny), z2 = make_float2(0.f, 0.f);
+
+    float2 nx[P], ny[P], nz[P], mi[P];   // negated target coordinates, masses
+#pragma unroll
+    for (int q = 0; q < P; ++q) {
+        const float4 a = pos[row * kPairRow + (2 * q) * kPairThreads + tid];
+        const float4 b = pos[row * kPairRow + (2 * q + 1) * kPairThreads + tid];
+        nx[q] = make_float2(-a.x, -b.x);
+        ny[q] = make_float2(-a.y, -b.y);
+        nz[q] = make_float2(-a.z, -b.z);
+        mi[q] = make_float2(a.w, b.w);
+    }
+#pragma unroll
+    for (int k = 0; k < 3 * kPairIpt; ++k) tot[0][k][tid] = tot[1][k][tid] = 0.f;
+    if (tid == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        fence_mbar_init();
+    }
+    __syncthreads();
+    if (tid == 0) {
+        for (int q = 0; q < 2 && q < nt; ++q) {
+            mbar_arrive_expect_tx(&bar[q], kBytes);
+            bulk_g2s(tile[q], pos + (size_t)(t_begin + q) * kTileJ, kBytes, &bar[q]);
+        }
+    }
+    float4* sources = part + (size_t)units * n_pad + pair_source_base(row, row0, n_pad);
+    auto fold_target = [&](int k, float x) {
+        float s = tot[0][k][tid], c = tot[1][k][tid];
+        kahan_add(s, c, x);
+        tot[0][k][tid] = s;
+        tot[1][k][tid] = c;
+    };
+    int t = 0;
+    bool abandoned = false;
+    for (; t < nt; ++t) {
+        const float4* tj = tile[t & 1];
+        const bool ok = mbar_wait_bounded(&bar[t & 1], (uint32_t)((t >> 1) & 1), polls);
+        if (__syncthreads_or(!ok)) { abandoned = true; break; }
+#pragma unroll 1
+        for (int turn = 0; turn < kTurns; ++turn) {
+            const int chunk = ((warp + turn) & (kTurns - 1)) * 32;
+            float2 ax[P], ay[P], az[P];
+            float sx = 0.f, sy = 0.f, sz = 0.f;   // the travelling source's sums over whole groups of steps
+#pragma unroll
+            for (int q = 0; q < P; ++q) ax[q] = ay[q] = az[q] = z2;
+#pragma unroll 1
+            for (int g = 0; g < 32; g += kPairGroup) {
+                float2 bx = z2, by = z2, bz = z2;
+#pragma unroll
+                for (int u = 0; u < kPairGroup; ++u) {
+                    const float4 pj = tj[chunk + ((lane + g + u) & 31)];
+                    const float2 jx = make_float2(pj.x, pj.x), jy = make_float2(pj.y, pj.y);
+                    const float2 jz = make_float2(pj.z, pj.z), jm = make_float2(pj.w, pj.w);
+#pragma unroll
+                    for (int q = 0; q < P; ++q) {
+                        const float2 dx = __fadd2_rn(jx, nx[q]), dy = __fadd2_rn(jy, ny[q]), dz = __fadd2_rn(jz, nz[q]);
+                        const float2 w = pair_factor_x2<LAW>(dx, dy, dz, S2, T2);
+                        const float2 wi = __fmul2_rn(jm, w), wj = __fmul2_rn(mi[q], w);
+                        ax[q] = __ffma2_rn(wi, dx, ax[q]);
+                        ay[q] = __ffma2_rn(wi, dy, ay[q]);
+                        az[q] = __ffma2_rn(wi, dz, az[q]);
+                        bx = __ffma2_rn(wj, dx, bx);
+                        by = __ffma2_rn(wj, dy, by);
+                        bz = __ffma2_rn(wj, dz, bz);
+                    }
+                    if (u + 1 < kPairGroup) {
+                        const int next = (lane + 1) & 31;
+                        bx.x = __shfl_sync(0xffffffffu, bx.x, next); bx.y = __shfl_sync(0xffffffffu, bx.y, next);
+                        by.x = __shfl_sync(0xffffffffu, by.x, next); by.y = __shfl_sync(0xffffffffu, by.y, next);
+                        bz.x = __shfl_sync(0xffffffffu, bz.x, next); bz.y = __shfl_sync(0xffffffffu, bz.y, next);
+                    }
+                }
+                // this lane holds source (lane + g + kPairGroup - 1): its earlier groups' sums were left
+                // kPairGroup lanes on
+                const int from = (lane + kPairGroup) & 31;
+                sx = __shfl_sync(0xffffffffu, sx, from) + (bx.x + bx.y);
+                sy = __shfl_sync(0xffffffffu, sy, from) + (by.x + by.y);
+                sz = __shfl_sync(0xffffffffu, sz, from) + (bz.x + bz.y);
+            }
+            // lane l now holds source (l + 31) mod 32
+            const float b[3] = {__shfl_sync(0xffffffffu, sx, (lane + 1) & 31), __shfl_sync(0xffffffffu, sy, (lane + 1) & 31),
+                                __shfl_sync(0xffffffffu, sz, (lane + 1) & 31)};
+#pragma unroll
+            for (int q = 0; q < P; ++q) {
+                fold_target(6 * q, ax[q].x); fold_target(6 * q + 1, ay[q].x); fold_target(6 * q + 2, az[q].x);
+                fold_target(6 * q + 3, ax[q].y); fold_target(6 * q + 4, ay[q].y); fold_target(6 * q + 5, az[q].y);
+            }
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                float s = turn == 0 ? 0.f : src[0][a][chunk + lane], c = turn == 0 ? 0.f : src[1][a][chunk + lane];
+                kahan_add(s, c, b[a]);
+                src[0][a][chunk + lane] = s;
+                src[1][a][chunk + lane] = c;
+            }
+            __syncthreads();   // the next turn's warp continues this chunk's sums
+        }
+        // thread j owns source j from here to its own warp's next turn 0
+        const int j = (t_begin + t) * kTileJ + tid;
+        if (j >= (row + 1) * kPairRow)
+            sources[j - (row + 1) * kPairRow] = make_float4(src[1][0][tid] - src[0][0][tid], src[1][1][tid] - src[0][1][tid],
+                                                            src[1][2][tid] - src[0][2][tid], 0.f);
+        if (tid == 0 && t + 2 < nt) {
+            fence_proxy_async_smem();
+            mbar_arrive_expect_tx(&bar[t & 1], kBytes);
+            bulk_g2s(tile[t & 1], pos + (size_t)(t_begin + t + 2) * kTileJ, kBytes, &bar[t & 1]);
+        }
+    }
+    if (abandoned) {
+        // Let the copies still in flight land before the block's shared
+        // memory is released (bounded), then report.
+        if (tid == 0) {
+            for (int q = t; q < nt && q < t + 2; ++q)
+                (void)mbar_wait_bounded(&bar[q & 1], (uint32_t)((q >> 1) & 1), kMaxPolls);
+            record_error(err, DEV_WAIT_TIMEOUT);
+        }
+        return;
+    }
+    float4* targets = part + (size_t)blockIdx.x * n_pad + (size_t)row * kPairRow;
+#pragma unroll
+    for (int k = 0; k < kPairIpt; ++k)
+        targets[k * kPairThreads + tid] = make_float4(tot[0][3 * k][tid] - tot[1][3 * k][tid],
+                                                      tot[0][3 * k + 1][tid] - tot[1][3 * k + 1][tid],
+                                                      tot[0][3 * k + 2][tid] - tot[1][3 * k + 2][tid], 0.f);
+}
+
 // K7: fold the partials of all source ranges (fixed order), apply G, add the
 // pending initial forces, store the acceleration and, when update != 0,
 // kick-drift: v += a dt; x += v dt / scale, both Kahan-compensated
@@ -206,8 +397,27 @@ __device__ __forceinline__ float3 fold_partials(const float4* __restrict__ part,
 
 // kFoldLanes consecutive threads fold one body's partials: lane j takes
 // splits j, j + kFoldLanes, ... (compensated, in that order), and the lanes'
-// corrected sums are added by a butterfly (every lane gets the same total).
+// sums are added by a butterfly (every lane gets the same total).
 constexpr int kFoldLanes = 8;
+
+// Sum over the fold's lanes of (s - c), the same in every lane: added pairwise
+// with the rounding error of each sum carried in the low part (Knuth's
+// two-sum), so that the total is rounded once.
+__device__ __forceinline__ float butterfly_total(float s, float c) {
+    float hi = s, lo = -c;
+#pragma unroll
+    for (int o = 1; o < kFoldLanes; o <<= 1) {
+        const float b = __shfl_xor_sync(0xffffffffu, hi, o);
+        const float bl = __shfl_xor_sync(0xffffffffu, lo, o);
+        const float t = __fadd_rn(hi, b);
+        const float u = __fsub_rn(t, hi);
+        // the sum's error is exact, so either side of the exchange finds the same
+        const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(t, u)), __fsub_rn(b, u));
+        lo = __fadd_rn(__fadd_rn(lo, bl), e);
+        hi = t;
+    }
+    return __fadd_rn(hi, lo);
+}
 
 __device__ __forceinline__ float3 fold_partials_lanes(const float4* __restrict__ part, int splits, int n_pad, int i,
                                                       int j) {
@@ -220,17 +430,65 @@ __device__ __forceinline__ float3 fold_partials_lanes(const float4* __restrict__
         kahan_add(az, kz, p.z);
         qx += c.x; qy += c.y; qz += c.z;
     }
-    float3 f = make_float3(ax - (kx + qx), ay - (ky + qy), az - (kz + qz));
-#pragma unroll
-    for (int o = 1; o < kFoldLanes; o <<= 1) {
-        f.x += __shfl_xor_sync(0xffffffffu, f.x, o);
-        f.y += __shfl_xor_sync(0xffffffffu, f.y, o);
-        f.z += __shfl_xor_sync(0xffffffffu, f.z, o);
-    }
-    return f;
+    return make_float3(butterfly_total(ax, kx + qx), butterfly_total(ay, ky + qy), butterfly_total(az, kz + qz));
 }
 
-__global__ void k_direct_reduce_update(const float4* __restrict__ part, int splits, int n, int n_pad, float G,
+// The same for k_direct_pairs' partials of rows [row0, row0 + rows): body i's
+// target partials when its row is among them, and its entry as a source of
+// each of those rows before its own.
+struct PairFold {
+    int units, row0, rows;
+};
+
+__device__ __forceinline__ float3 fold_pairs_lanes(const float4* __restrict__ part, const PairFold& pf, int n_pad, int i,
+                                                   int j) {
+    float ax = 0.f, ay = 0.f, az = 0.f, kx = 0.f, ky = 0.f, kz = 0.f;
+    const int row = i / kPairRow, last = pf.row0 + pf.rows;
+    auto add = [&](const float4 p) {
+        kahan_add(ax, kx, p.x);
+        kahan_add(ay, ky, p.y);
+        kahan_add(az, kz, p.z);
+    };
+    if (row >= pf.row0 && row < last) {
+        const int tiles = n_pad / kTileJ - row * kPairRowTiles, per = pair_unit_tiles(tiles, pf.units);
+        const int used = (tiles + per - 1) / per;
+#pragma unroll 4
+        for (int u = j; u < used; u += kFoldLanes) add(part[(size_t)u * n_pad + i]);
+    }
+    const float4* sources = part + (size_t)pf.units * n_pad;
+    const int end = min(row, last);
+#pragma unroll 4
+    for (int r = pf.row0 + j; r < end; r += kFoldLanes)
+        add(sources[pair_source_base(r, pf.row0, n_pad) + (size_t)(i - (r + 1) * kPairRow)]);
+    return make_float3(butterfly_total(ax, kx), butterfly_total(ay, ky), butterfly_total(az, kz));
+}
+
+// Folds the partials of one of several launches of k_direct_pairs into the
+// bodies' running (sum, compensation); the first launch starts them.
+__global__ void k_pairs_carry(const float4* __restrict__ part, PairFold pf, int n_pad, int first,
+                              float4* __restrict__ carry, const int* __restrict__ err) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = t / kFoldLanes, j = t % kFoldLanes;
+    if (i >= n_pad || *err != 0) return;
+    const float3 f = fold_pairs_lanes(part, pf, n_pad, i, j);
+    if (j != 0) return;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f), c = s;
+    if (!first) {
+        s = carry[i];
+        c = carry[n_pad + i];
+    }
+    kahan_add(s.x, c.x, f.x);
+    kahan_add(s.y, c.y, f.y);
+    kahan_add(s.z, c.z, f.z);
+    carry[i] = s;
+    carry[n_pad + i] = c;
+}
+
+// PAIRS: the partials are k_direct_pairs' (carry: the earlier launches' sums,
+// when there were several), else k_direct_force's.
+template <bool PAIRS>
+__global__ void k_direct_reduce_update(const float4* __restrict__ part, int splits, PairFold pf,
+                                       const float4* __restrict__ carry, int n, int n_pad, float G,
                                        const float4* __restrict__ finit, float4* __restrict__ acc,
                                        float4* __restrict__ pos, float4* __restrict__ posc,
                                        float4* __restrict__ vel, float4* __restrict__ velc, float dt,
@@ -241,8 +499,15 @@ __global__ void k_direct_reduce_update(const float4* __restrict__ part, int spli
     const int i = t / kFoldLanes, j = t % kFoldLanes;
     // whole groups of lanes leave together (n_pad bodies, a multiple of the block)
     if (i >= n_pad || *err != 0) return;
-    const float3 f = fold_partials_lanes(part, splits, n_pad, i, j);
+    float3 f = PAIRS ? fold_pairs_lanes(part, pf, n_pad, i, j) : fold_partials_lanes(part, splits, n_pad, i, j);
     if (i >= n || j != 0) return;
+    if (PAIRS && carry) {
+        float4 s = carry[i], c = carry[n_pad + i];
+        kahan_add(s.x, c.x, f.x);
+        kahan_add(s.y, c.y, f.y);
+        kahan_add(s.z, c.z, f.z);
+        f = make_float3(s.x - c.x, s.y - c.y, s.z - c.z);
+    }
     float3 a = make_float3(G * f.x, G * f.y, G * f.z);
     if (finit) {
         const float4 f = finit[i];
@@ -360,59 +625,127 @@ static DirectTuning default_tuning(size_t n_pad) {
     return t;
 }
 
-cudaError_t direct_force_update(nb_sim* sim, float dt, bool update) {
-    DirectTuning t = sim->tune;
-    if (!sim->tune_set) {
-        t = default_tuning(sim->n_pad);
-        t.splits = sim->tune.splits;
-    }
-    if (t.block <= 0 || t.ipt <= 0) t = default_tuning(sim->n_pad);
-    // A tuning whose target block does not divide the padded size falls back.
-    if (sim->n_pad % (size_t)(t.block * t.ipt) != 0) t = default_tuning(sim->n_pad);
-    const int splits = direct_splits(sim, t, sim->n_pad);
-    const size_t need = (size_t)splits * 2 * sim->n_pad;
-    if (need > sim->part_cap) {
-        dev_free(sim->part, sim->stream);
-        sim->part = nullptr;
-        sim->part_cap = 0;
-        cudaError_t e = dev_alloc(&sim->part, need * sizeof(float4));
-        if (e != cudaSuccess) return e;
-        sim->part_cap = need;
-    }
-    const int ntiles = (int)(sim->n_pad / kTileJ);
-    const int tps = (ntiles + splits - 1) / splits;
-    dim3 grid((unsigned)(sim->n_pad / (size_t)(t.block * t.ipt)), (unsigned)splits);
-    const float S = (float)sim->prm.softening2;
-    const bool comp = !(sim->prm.flags & NB_FLAG_NO_COMPENSATION);
-    bool ok;
-    {
-    PhaseScope ps(sim, 0);
-    if (sim->prm.law == NB_LAW_PLUMMER)
-        ok = comp ? launch_force_law<NB_LAW_PLUMMER, true>(t.block, t.ipt, grid, sim->stream, sim->pos,
-                                                          (int)sim->n_pad, tps, ntiles, splits, S, sim->part,
-                                                          sim->d_err, sim->wait_polls, sim->d_mmax, sim->heavy)
-                  : launch_force_law<NB_LAW_PLUMMER, false>(t.block, t.ipt, grid, sim->stream, sim->pos,
-                                                           (int)sim->n_pad, tps, ntiles, splits, S, sim->part,
-                                                           sim->d_err, sim->wait_polls, sim->d_mmax, sim->heavy);
-    else
-        ok = comp ? launch_force_law<NB_LAW_REFERENCE, true>(t.block, t.ipt, grid, sim->stream, sim->pos,
-                                                            (int)sim->n_pad, tps, ntiles, splits, S, sim->part,
-                                                            sim->d_err, sim->wait_polls, sim->d_mmax, sim->heavy)
-                  : launch_force_law<NB_LAW_REFERENCE, false>(t.block, t.ipt, grid, sim->stream, sim->pos,
-                                                             (int)sim->n_pad, tps, ntiles, splits, S, sim->part,
-                                                             sim->d_err, sim->wait_polls, sim->d_mmax, sim->heavy);
-    }
-    if (!ok) return cudaErrorInvalidConfiguration;
-    cudaError_t e = cudaGetLastError();
+static cudaError_t reserve_part(nb_sim* sim, size_t need) {
+    if (need <= sim->part_cap) return cudaSuccess;
+    dev_free(sim->part, sim->stream);
+    sim->part = nullptr;
+    sim->part_cap = 0;
+    cudaError_t e = dev_alloc(&sim->part, need * sizeof(float4));
     if (e != cudaSuccess) return e;
+    sim->part_cap = need;
+    return cudaSuccess;
+}
+
+// Units the first row of k_direct_pairs is cut into (later rows have fewer
+// source tiles and so shorter units, which keeps the end of the launch short):
+// about 24 units of work an SM, from one tile a unit for small states, where a
+// whole state is 3 to 30 tiles an SM, to dozens.  More units would only add
+// partials to write and fold.
+static int pair_units(const nb_sim* sim, int rows, int ntiles) {
+    const long long work = (long long)rows * ntiles - (long long)kPairRowTiles * rows * (rows - 1) / 2;
+    const long long per = std::max<long long>(1, work / (24ll * std::max(1, sim->sm_count)));
+    return std::min(ntiles, (int)std::max<long long>(8, std::min<long long>(128, (ntiles + per - 1) / per)));
+}
+
+// k_direct_pairs over all rows, as many rows a launch as keep the source
+// partials within kPairSourceBytes, folded into the carry between launches.
+// The last launch's partials are left for the reduction (*pf, *carry).
+constexpr size_t kPairSourceBytes = (size_t)1 << 30;
+constexpr size_t kPairMin = 10240;
+
+static cudaError_t launch_pairs(nb_sim* sim, PairFold* pf, const float4** carry) {
+    const int n_pad = (int)sim->n_pad, rows = n_pad / kPairRow, ntiles = n_pad / kTileJ;
+    const int units = pair_units(sim, rows, ntiles);
+    const size_t cap = kPairSourceBytes / sizeof(float4);
+    auto rows_from = [&](int row0) {   // rows of the launch that starts at row0
+        int r = 1;
+        while (row0 + r < rows && pair_source_base(row0 + r + 1, row0, n_pad) <= cap) ++r;
+        return r;
+    };
+    const bool several = rows_from(0) < rows;
+    size_t most = 0;
+    for (int r0 = 0; r0 < rows; r0 += rows_from(r0)) most = std::max(most, pair_source_base(r0 + rows_from(r0), r0, n_pad));
+    const size_t base = (size_t)units * n_pad;
+    cudaError_t e = reserve_part(sim, base + most + (several ? (size_t)2 * n_pad : 0));
+    if (e != cudaSuccess) return e;
+    float4* sums = several ? sim->part + base + most : nullptr;
+    const float S = (float)sim->prm.softening2;
+    const bool plummer = sim->prm.law == NB_LAW_PLUMMER;
+    for (int r0 = 0, count; r0 < rows; r0 += count) {
+        count = rows_from(r0);
+        const dim3 grid((unsigned)units, (unsigned)count);
+#define NB_PAIRS(L, H)                                                                                            \
+    k_direct_pairs<L, H><<<grid, kPairThreads, 0, sim->stream>>>(sim->pos, n_pad, r0, units, S, sim->part, sim->d_err, \
+                                                                 sim->wait_polls, sim->d_mmax)
+        if (plummer) { if (sim->heavy) NB_PAIRS(NB_LAW_PLUMMER, true); else NB_PAIRS(NB_LAW_PLUMMER, false); }
+        else { if (sim->heavy) NB_PAIRS(NB_LAW_REFERENCE, true); else NB_PAIRS(NB_LAW_REFERENCE, false); }
+#undef NB_PAIRS
+        *pf = PairFold{units, r0, count};
+        if (r0 + count < rows) {
+            k_pairs_carry<<<(unsigned)(sim->n_pad * kFoldLanes / 256), 256, 0, sim->stream>>>(sim->part, *pf, n_pad,
+                                                                                              r0 == 0 ? 1 : 0, sums,
+                                                                                              sim->d_err);
+            sim->prof.launches += 2;   // this pair of launches; the last one is the phase's own
+        }
+    }
+    *carry = sums;
+    return cudaGetLastError();
+}
+
+cudaError_t direct_force_update(nb_sim* sim, float dt, bool update) {
+    const bool comp = !(sim->prm.flags & NB_FLAG_NO_COMPENSATION);
+    // Each pair once from kPairMin padded bodies on: a step took 49 us against
+    // 70 at 10,000 bodies and 46 against 45 at 8,000, where a row's eight own
+    // tiles (both directions evaluated) and a unit's one-tile life cost what
+    // the shared roots save.  A handle whose launch was tuned, and
+    // uncompensated sums, keep k_direct_force.
+    const bool pairs = comp && !sim->tune_set && sim->n_pad >= kPairMin;
+    int splits = 0;
+    PairFold pf{};
+    const float4* carry = nullptr;
+    if (pairs) {
+        PhaseScope ps(sim, 0);
+        cudaError_t e = launch_pairs(sim, &pf, &carry);
+        if (e != cudaSuccess) return e;
+    } else {
+        DirectTuning t = sim->tune;
+        if (!sim->tune_set) {
+            t = default_tuning(sim->n_pad);
+            t.splits = sim->tune.splits;
+        }
+        if (t.block <= 0 || t.ipt <= 0) t = default_tuning(sim->n_pad);
+        // A tuning whose target block does not divide the padded size falls back.
+        if (sim->n_pad % (size_t)(t.block * t.ipt) != 0) t = default_tuning(sim->n_pad);
+        splits = direct_splits(sim, t, sim->n_pad);
+        cudaError_t e = reserve_part(sim, (size_t)splits * 2 * sim->n_pad);
+        if (e != cudaSuccess) return e;
+        const int ntiles = (int)(sim->n_pad / kTileJ);
+        const int tps = (ntiles + splits - 1) / splits;
+        dim3 grid((unsigned)(sim->n_pad / (size_t)(t.block * t.ipt)), (unsigned)splits);
+        const float S = (float)sim->prm.softening2;
+        bool ok;
+        PhaseScope ps(sim, 0);
+#define NB_FORCE(L, C)                                                                                               \
+    ok = launch_force_law<L, C>(t.block, t.ipt, grid, sim->stream, sim->pos, (int)sim->n_pad, tps, ntiles, splits, S, \
+                                sim->part, sim->d_err, sim->wait_polls, sim->d_mmax, sim->heavy)
+        if (sim->prm.law == NB_LAW_PLUMMER) { if (comp) NB_FORCE(NB_LAW_PLUMMER, true); else NB_FORCE(NB_LAW_PLUMMER, false); }
+        else { if (comp) NB_FORCE(NB_LAW_REFERENCE, true); else NB_FORCE(NB_LAW_REFERENCE, false); }
+#undef NB_FORCE
+        if (!ok) return cudaErrorInvalidConfiguration;
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
     const int n = (int)sim->n;
     const float inv_scale = (float)(1.0 / sim->prm.pos_scale);
     PhaseScope ps(sim, 1);
     static_assert(kPad % (256 / kFoldLanes) == 0, "the fold's blocks cover whole padded bodies");
-    k_direct_reduce_update<<<(unsigned)(sim->n_pad * kFoldLanes / 256), 256, 0, sim->stream>>>(
-        sim->part, splits, n, (int)sim->n_pad, (float)sim->prm.G, sim->finit_pending ? sim->finit : nullptr,
-        sim->acc, sim->pos, sim->posc, sim->vel, sim->velc, dt, inv_scale, update ? 1 : 0, comp ? 1 : 0,
-        update ? sim->render : nullptr, sim->rcolour, sim->rscale, sim->d_err);
+#define NB_REDUCE(PAIRS)                                                                                             \
+    k_direct_reduce_update<PAIRS><<<(unsigned)(sim->n_pad * kFoldLanes / 256), 256, 0, sim->stream>>>(               \
+        sim->part, splits, pf, carry, n, (int)sim->n_pad, (float)sim->prm.G, sim->finit_pending ? sim->finit : nullptr, \
+        sim->acc, sim->pos, sim->posc, sim->vel, sim->velc, dt, inv_scale, update ? 1 : 0, comp ? 1 : 0,             \
+        update ? sim->render : nullptr, sim->rcolour, sim->rscale, sim->d_err)
+    if (pairs) NB_REDUCE(true); else NB_REDUCE(false);
+#undef NB_REDUCE
     sim->finit_pending = false;
     const double nn = (double)sim->n;
     sim->inter_last = (uint64_t)(nn * (nn - 1.0));

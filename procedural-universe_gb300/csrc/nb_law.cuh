@@ -81,4 +81,23 @@ __device__ __forceinline__ void interact_x2(float2 jx, float2 jy, float2 jz, flo
     az = __ffma2_rn(w, dz, az);
 }
 
+// The law's factor without a mass, for two pairs at once: the force on either
+// body of a pair is the other's mass times it times the separation.
+template <int LAW>
+__device__ __forceinline__ float2 pair_factor_x2(float2 dx, float2 dy, float2 dz, float2 S2, float2 T2) {
+    if (LAW == NB_LAW_REFERENCE) {
+        float2 r2 = __fmul2_rn(dx, dx);
+        r2 = __ffma2_rn(dy, dy, r2);
+        r2 = __ffma2_rn(dz, dz, r2);
+        const float2 s = __fadd2_rn(r2, S2);
+        const float2 t = __ffma2_rn(__fmul2_rn(r2, s), s, T2);
+        return make_float2(rsqrt_approx(t.x), rsqrt_approx(t.y));
+    }
+    float2 q = __ffma2_rn(dx, dx, S2);
+    q = __ffma2_rn(dy, dy, q);
+    q = __ffma2_rn(dz, dz, q);
+    const float2 inv = make_float2(rsqrt_approx(q.x), rsqrt_approx(q.y));
+    return __fmul2_rn(inv, __fmul2_rn(inv, inv));
+}
+
 }  // namespace nb

@@ -250,3 +250,40 @@ def test_full_size_config3_properties():
         s.step(1e-3, 1)
         e1 = s.diagnostics(0.5e-3)["total"]
         assert abs(e1 - e0) < 1e-4 * abs(e0), (e0, e1)
+
+
+@pytest.mark.parametrize("law", [nb.LAW_REFERENCE, nb.LAW_PLUMMER])
+@pytest.mark.parametrize("n", [8193, 10240, 10241, 14337, 20001, 380000])
+def test_each_pair_once_matches_fp64(n, law):
+    """Sizes from the first that takes each pair once, at row and tile edges,
+    and one whose source partials need two launches; uneven masses (some
+    zero), coincident bodies in one row and across rows.  A term carries a few
+    units of 2^-24 and the sums are compensated: 5e-7 bounds their total."""
+    pm, v = nb.seed_plummer(31, n)
+    rng = np.random.default_rng(n)
+    pm[:, 3] *= rng.uniform(0.01, 2.0, n).astype(np.float32)
+    pm[rng.integers(0, n, 50), 3] = 0.0
+    pm[5, :3] = pm[6, :3]
+    pm[7, :3] = pm[n - 1, :3]
+    pm[n - 2, :3] = pm[n // 2, :3]
+    t = np.unique(np.concatenate([[5, 6, 7, n // 2, n - 2, n - 1], np.linspace(0, n - 1, 1500).astype(np.int64)]))
+    with direct_sim(law=law) as s:
+        s.init_soa(pm, v)
+        F = s.compute_forces()[t]
+        F64 = s.fp64_forces(t)
+        again = s.compute_forces()[t]
+    assert np.isfinite(F).all()
+    assert O.rel_l2(F, F64) < 5e-7
+    np.testing.assert_array_equal(F, again)
+
+
+def test_each_pair_once_with_heavy_masses():
+    """The reference's own masses (1e20 to 1e30): the raised self-pair guard."""
+    rec = nb.seed_reference(nb.SEEDER_RANDOM, 33, 12000)
+    with direct_sim(G=6.674e-11, softening2=10.0) as s:
+        s.init(rec)
+        F = s.compute_forces()
+        t = np.arange(0, 12000, 7)
+        F64 = s.fp64_forces(t)
+    assert np.isfinite(F).all()
+    assert O.rel_l2(F[t], F64) < 5e-7
