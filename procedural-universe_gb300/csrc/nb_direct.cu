@@ -178,12 +178,11 @@ __global__ void __launch_bounds__(BLOCK) k_direct_force(const float4* __restrict
 // deterministic.  Tiles of the row's own block take part as sources only: all
 // their ordered pairs are evaluated from the target side.
 //
-// Targets are folded into compensated totals every 32 sources as in
-// k_direct_force (the totals live in shared memory, registers hold the running
-// sums), sources every kPairGroup = 4 steps (16 terms in each packed half) into
+// Targets are folded into compensated totals every FOLD sources (the totals
+// live in shared memory, registers hold the running sums), sources every kPairGroup = 4 steps (16 terms in each packed half) into
 // a second running sum and once a chunk into the totals.  A unit
 // writes its targets' totals, and for each tile behind the row the sources':
-// part holds [units][n_pad] target partials, then for each row of the launch
+// part holds kPairRow target partials per unit, then for each row of the launch
 // one entry per body behind it.
 // Bound by the FP32 pipe (77-79% of its cycles; three-operand packed
 // instructions leave the rest).  Three blocks an SM at 156 registers: four
@@ -197,8 +196,15 @@ constexpr int kPairRowTiles = kPairRow / kTileJ;
 static_assert(kPairThreads == kTileJ, "one thread per source of a tile");
 static_assert(kPad % kPairRow == 0, "padded states hold whole rows");
 
-// Tiles per unit of a row that has `tiles` source tiles, cut into at most `units`.
-__host__ __device__ __forceinline__ int pair_unit_tiles(int tiles, int units) { return (tiles + units - 1) / units; }
+// Units of the rows [row0, row) of a state, `per` tiles a unit (1, 2, 4 or a
+// multiple of 8): row q has (rows - q) * kPairRowTiles source tiles.
+__host__ __device__ __forceinline__ int pair_units_before(int row, int row0, int rows, int per) {
+    const int a = rows - row0, k = row - row0;
+    if (per <= kPairRowTiles) return kPairRowTiles / per * (a * k - k * (k - 1) / 2);
+    const int m = per / kPairRowTiles;   // sum of ceil(i / m) over a - k < i <= a
+    const int qa = a / m, qb = (a - k) / m;
+    return m * (qa * (qa + 1) - qb * (qb + 1)) / 2 + (a % m) * (qa + 1) - ((a - k) % m) * (qb + 1);
+}
 
 // Source entries of the rows before `row` in a launch that starts at row0.
 __host__ __device__ __forceinline__ size_t pair_source_base(int row, int row0, int n_pad) {
@@ -206,20 +212,26 @@ __host__ __device__ __forceinline__ size_t pair_source_base(int row, int row0, i
     return r * first - (size_t)kPairRow * (r * (r - (r > 0 ? 1 : 0)) / 2);
 }
 
-template <int LAW, bool HEAVY>
+template <int LAW, bool HEAVY, int FOLD>
 __global__ void __launch_bounds__(kPairThreads, 3) k_direct_pairs(const float4* __restrict__ pos, int n_pad, int row0,
-                                                                  int units, float S, float4* __restrict__ part,
+                                                                  int nrows, int per, float S,
+                                                                  float4* __restrict__ part,
                                                                   int* __restrict__ err, uint32_t polls,
                                                                   const unsigned* __restrict__ mmax) {
     __shared__ __align__(128) float4 tile[2][kTileJ];
     __shared__ float tot[2][3 * kPairIpt][kPairThreads];   // targets: sums, compensations
     __shared__ float src[2][3][kTileJ];                    // the tile's sources: sums, compensations
     __shared__ __align__(8) uint64_t bar[2];
-    const int row = row0 + blockIdx.y, ntiles = n_pad / kTileJ;
-    const int per = pair_unit_tiles(ntiles - row * kPairRowTiles, units);
-    const int t_begin = row * kPairRowTiles + blockIdx.x * per;
+    // one block per unit and none empty: blocks that leave at once would still
+    // take part in the first placement and leave some SMs with a unit more
+    const int rows = n_pad / kPairRow, ntiles = n_pad / kTileJ, unit = blockIdx.x;
+    int row = row0;
+    for (int end = row0 + nrows; end - row > 1;) {   // the last row whose units start at or before this one
+        const int mid = (row + end) / 2;
+        if (pair_units_before(mid, row0, rows, per) <= unit) row = mid; else end = mid;
+    }
+    const int t_begin = row * kPairRowTiles + (unit - pair_units_before(row, row0, rows, per)) * per;
     const int nt = min(ntiles, t_begin + per) - t_begin;
-    if (nt <= 0) return;   // the whole block
     const float tiny = HEAVY ? self_pair_tiny(mmax) : kTiny;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int P = kPairIpt / 2;
@@ -251,7 +263,7 @@ __global__ void __launch_bounds__(kPairThreads, 3) k_direct_pairs(const float4* 
             bulk_g2s(tile[q], pos + (size_t)(t_begin + q) * kTileJ, kBytes, &bar[q]);
         }
     }
-    float4* sources = part + (size_t)units * n_pad + pair_source_base(row, row0, n_pad);
+    float4* sources = part + (size_t)gridDim.x * kPairRow + pair_source_base(row, row0, n_pad);
     auto fold_target = [&](int k, float x) {
         float s = tot[0][k][tid], c = tot[1][k][tid];
         kahan_add(s, c, x);
@@ -267,52 +279,55 @@ __global__ void __launch_bounds__(kPairThreads, 3) k_direct_pairs(const float4* 
 #pragma unroll 1
         for (int turn = 0; turn < kTurns; ++turn) {
             const int chunk = ((warp + turn) & (kTurns - 1)) * 32;
-            float2 ax[P], ay[P], az[P];
             float sx = 0.f, sy = 0.f, sz = 0.f;   // the travelling source's sums over whole groups of steps
-#pragma unroll
-            for (int q = 0; q < P; ++q) ax[q] = ay[q] = az[q] = z2;
 #pragma unroll 1
-            for (int g = 0; g < 32; g += kPairGroup) {
-                float2 bx = z2, by = z2, bz = z2;
+            for (int h = 0; h < 32; h += FOLD) {
+                float2 ax[P], ay[P], az[P];
 #pragma unroll
-                for (int u = 0; u < kPairGroup; ++u) {
-                    const float4 pj = tj[chunk + ((lane + g + u) & 31)];
-                    const float2 jx = make_float2(pj.x, pj.x), jy = make_float2(pj.y, pj.y);
-                    const float2 jz = make_float2(pj.z, pj.z), jm = make_float2(pj.w, pj.w);
+                for (int q = 0; q < P; ++q) ax[q] = ay[q] = az[q] = z2;
+#pragma unroll 1
+                for (int g = h; g < h + FOLD; g += kPairGroup) {
+                    float2 bx = z2, by = z2, bz = z2;
 #pragma unroll
-                    for (int q = 0; q < P; ++q) {
-                        const float2 dx = __fadd2_rn(jx, nx[q]), dy = __fadd2_rn(jy, ny[q]), dz = __fadd2_rn(jz, nz[q]);
-                        const float2 w = pair_factor_x2<LAW>(dx, dy, dz, S2, T2);
-                        const float2 wi = __fmul2_rn(jm, w), wj = __fmul2_rn(mi[q], w);
-                        ax[q] = __ffma2_rn(wi, dx, ax[q]);
-                        ay[q] = __ffma2_rn(wi, dy, ay[q]);
-                        az[q] = __ffma2_rn(wi, dz, az[q]);
-                        bx = __ffma2_rn(wj, dx, bx);
-                        by = __ffma2_rn(wj, dy, by);
-                        bz = __ffma2_rn(wj, dz, bz);
+                    for (int u = 0; u < kPairGroup; ++u) {
+                        const float4 pj = tj[chunk + ((lane + g + u) & 31)];
+                        const float2 jx = make_float2(pj.x, pj.x), jy = make_float2(pj.y, pj.y);
+                        const float2 jz = make_float2(pj.z, pj.z), jm = make_float2(pj.w, pj.w);
+#pragma unroll
+                        for (int q = 0; q < P; ++q) {
+                            const float2 dx = __fadd2_rn(jx, nx[q]), dy = __fadd2_rn(jy, ny[q]), dz = __fadd2_rn(jz, nz[q]);
+                            const float2 w = pair_factor_x2<LAW>(dx, dy, dz, S2, T2);
+                            const float2 wi = __fmul2_rn(jm, w), wj = __fmul2_rn(mi[q], w);
+                            ax[q] = __ffma2_rn(wi, dx, ax[q]);
+                            ay[q] = __ffma2_rn(wi, dy, ay[q]);
+                            az[q] = __ffma2_rn(wi, dz, az[q]);
+                            bx = __ffma2_rn(wj, dx, bx);
+                            by = __ffma2_rn(wj, dy, by);
+                            bz = __ffma2_rn(wj, dz, bz);
+                        }
+                        if (u + 1 < kPairGroup) {
+                            const int next = (lane + 1) & 31;
+                            bx.x = __shfl_sync(0xffffffffu, bx.x, next); bx.y = __shfl_sync(0xffffffffu, bx.y, next);
+                            by.x = __shfl_sync(0xffffffffu, by.x, next); by.y = __shfl_sync(0xffffffffu, by.y, next);
+                            bz.x = __shfl_sync(0xffffffffu, bz.x, next); bz.y = __shfl_sync(0xffffffffu, bz.y, next);
+                        }
                     }
-                    if (u + 1 < kPairGroup) {
-                        const int next = (lane + 1) & 31;
-                        bx.x = __shfl_sync(0xffffffffu, bx.x, next); bx.y = __shfl_sync(0xffffffffu, bx.y, next);
-                        by.x = __shfl_sync(0xffffffffu, by.x, next); by.y = __shfl_sync(0xffffffffu, by.y, next);
-                        bz.x = __shfl_sync(0xffffffffu, bz.x, next); bz.y = __shfl_sync(0xffffffffu, bz.y, next);
-                    }
+                    // this lane holds source (lane + g + kPairGroup - 1): its earlier groups' sums were left
+                    // kPairGroup lanes on
+                    const int from = (lane + kPairGroup) & 31;
+                    sx = __shfl_sync(0xffffffffu, sx, from) + (bx.x + bx.y);
+                    sy = __shfl_sync(0xffffffffu, sy, from) + (by.x + by.y);
+                    sz = __shfl_sync(0xffffffffu, sz, from) + (bz.x + bz.y);
                 }
-                // this lane holds source (lane + g + kPairGroup - 1): its earlier groups' sums were left
-                // kPairGroup lanes on
-                const int from = (lane + kPairGroup) & 31;
-                sx = __shfl_sync(0xffffffffu, sx, from) + (bx.x + bx.y);
-                sy = __shfl_sync(0xffffffffu, sy, from) + (by.x + by.y);
-                sz = __shfl_sync(0xffffffffu, sz, from) + (bz.x + bz.y);
+#pragma unroll
+                for (int q = 0; q < P; ++q) {
+                    fold_target(6 * q, ax[q].x); fold_target(6 * q + 1, ay[q].x); fold_target(6 * q + 2, az[q].x);
+                    fold_target(6 * q + 3, ax[q].y); fold_target(6 * q + 4, ay[q].y); fold_target(6 * q + 5, az[q].y);
+                }
             }
             // lane l now holds source (l + 31) mod 32
             const float b[3] = {__shfl_sync(0xffffffffu, sx, (lane + 1) & 31), __shfl_sync(0xffffffffu, sy, (lane + 1) & 31),
                                 __shfl_sync(0xffffffffu, sz, (lane + 1) & 31)};
-#pragma unroll
-            for (int q = 0; q < P; ++q) {
-                fold_target(6 * q, ax[q].x); fold_target(6 * q + 1, ay[q].x); fold_target(6 * q + 2, az[q].x);
-                fold_target(6 * q + 3, ax[q].y); fold_target(6 * q + 4, ay[q].y); fold_target(6 * q + 5, az[q].y);
-            }
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 float s = turn == 0 ? 0.f : src[0][a][chunk + lane], c = turn == 0 ? 0.f : src[1][a][chunk + lane];
@@ -343,7 +358,7 @@ __global__ void __launch_bounds__(kPairThreads, 3) k_direct_pairs(const float4* 
         }
         return;
     }
-    float4* targets = part + (size_t)blockIdx.x * n_pad + (size_t)row * kPairRow;
+    float4* targets = part + (size_t)unit * kPairRow;
 #pragma unroll
     for (int k = 0; k < kPairIpt; ++k)
         targets[k * kPairThreads + tid] = make_float4(tot[0][3 * k][tid] - tot[1][3 * k][tid],
@@ -368,58 +383,43 @@ __device__ __forceinline__ void write_vertex(nb_render_vertex* rv, const float4*
 }
 
 // Body i's force from its source-split partials ([split][n_pad] sums, then
-// [split][n_pad] compensations): compensated sum of the sums in split order,
-// less the compensations.  The partials of 16 splits are loaded before they
-// are added (in the same order), so that their loads overlap.
-__device__ __forceinline__ float3 fold_partials(const float4* __restrict__ part, int splits, int n_pad, int i) {
-    float ax = 0.f, ay = 0.f, az = 0.f, kx = 0.f, ky = 0.f, kz = 0.f, qx = 0.f, qy = 0.f, qz = 0.f;
-    auto add = [&](const float4 p, const float4 c) {
-        kahan_add(ax, kx, p.x);
-        kahan_add(ay, ky, p.y);
-        kahan_add(az, kz, p.z);
-        qx += c.x; qy += c.y; qz += c.z;
-    };
-    constexpr int kBatch = 16;
-    int s = 0;
-    for (; s + kBatch <= splits; s += kBatch) {
-        float4 p[kBatch], c[kBatch];
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u) {
-            p[u] = part[(size_t)(s + u) * n_pad + i];
-            c[u] = part[(size_t)(splits + s + u) * n_pad + i];
-        }
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u) add(p[u], c[u]);
-    }
-    for (; s < splits; ++s) add(part[(size_t)s * n_pad + i], part[(size_t)(splits + s) * n_pad + i]);
-    return make_float3(ax - (kx + qx), ay - (ky + qy), az - (kz + qz));
-}
-
+// [split][n_pad] compensations).
 // kFoldLanes consecutive threads fold one body's partials: lane j takes
 // splits j, j + kFoldLanes, ... (compensated, in that order), and the lanes'
 // sums are added by a butterfly (every lane gets the same total).
 constexpr int kFoldLanes = 8;
 
+// Knuth's two-sum: s + b as a rounded sum and its exact error, whichever is larger.
+__device__ __forceinline__ float two_sum(float s, float b, float& err) {
+    const float t = __fadd_rn(s, b), u = __fsub_rn(t, s);
+    err = __fadd_rn(__fsub_rn(s, __fsub_rn(t, u)), __fsub_rn(b, u));
+    return t;
+}
+
 // Sum over the fold's lanes of (s - c), the same in every lane: added pairwise
-// with the rounding error of each sum carried in the low part (Knuth's
-// two-sum), so that the total is rounded once.
-__device__ __forceinline__ float butterfly_total(float s, float c) {
+// with the rounding error of each sum carried in the low part; the total is hi + lo, hi its rounding to a few units.
+struct HiLo {
+    float hi, lo;
+    __device__ __forceinline__ float rounded() const { return __fadd_rn(hi, lo); }
+};
+struct HiLo3 {
+    HiLo x, y, z;
+};
+
+__device__ __forceinline__ HiLo butterfly_total(float s, float c) {
     float hi = s, lo = -c;
 #pragma unroll
     for (int o = 1; o < kFoldLanes; o <<= 1) {
         const float b = __shfl_xor_sync(0xffffffffu, hi, o);
         const float bl = __shfl_xor_sync(0xffffffffu, lo, o);
-        const float t = __fadd_rn(hi, b);
-        const float u = __fsub_rn(t, hi);
-        // the sum's error is exact, so either side of the exchange finds the same
-        const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(t, u)), __fsub_rn(b, u));
+        float e;   // the sum's error is exact, so either side of the exchange finds the same
+        hi = two_sum(hi, b, e);
         lo = __fadd_rn(__fadd_rn(lo, bl), e);
-        hi = t;
     }
-    return __fadd_rn(hi, lo);
+    return HiLo{hi, lo};
 }
 
-__device__ __forceinline__ float3 fold_partials_lanes(const float4* __restrict__ part, int splits, int n_pad, int i,
+__device__ __forceinline__ HiLo3 fold_partials_lanes(const float4* __restrict__ part, int splits, int n_pad, int i,
                                                       int j) {
     float ax = 0.f, ay = 0.f, az = 0.f, kx = 0.f, ky = 0.f, kz = 0.f, qx = 0.f, qy = 0.f, qz = 0.f;
     for (int s = j; s < splits; s += kFoldLanes) {
@@ -430,58 +430,73 @@ __device__ __forceinline__ float3 fold_partials_lanes(const float4* __restrict__
         kahan_add(az, kz, p.z);
         qx += c.x; qy += c.y; qz += c.z;
     }
-    return make_float3(butterfly_total(ax, kx + qx), butterfly_total(ay, ky + qy), butterfly_total(az, kz + qz));
+    return HiLo3{butterfly_total(ax, kx + qx), butterfly_total(ay, ky + qy), butterfly_total(az, kz + qz)};
 }
 
 // The same for k_direct_pairs' partials of rows [row0, row0 + rows): body i's
 // target partials when its row is among them, and its entry as a source of
 // each of those rows before its own.
 struct PairFold {
-    int units, row0, rows;
+    int per, row0, rows;   // tiles a unit, first row, rows
 };
 
-__device__ __forceinline__ float3 fold_pairs_lanes(const float4* __restrict__ part, const PairFold& pf, int n_pad, int i,
+__device__ __forceinline__ HiLo3 fold_pairs_lanes(const float4* __restrict__ part, const PairFold& pf, int n_pad, int i,
                                                    int j) {
     float ax = 0.f, ay = 0.f, az = 0.f, kx = 0.f, ky = 0.f, kz = 0.f;
-    const int row = i / kPairRow, last = pf.row0 + pf.rows;
+    const int row = i / kPairRow, last = pf.row0 + pf.rows, all = n_pad / kPairRow;
     auto add = [&](const float4 p) {
         kahan_add(ax, kx, p.x);
         kahan_add(ay, ky, p.y);
         kahan_add(az, kz, p.z);
     };
     if (row >= pf.row0 && row < last) {
-        const int tiles = n_pad / kTileJ - row * kPairRowTiles, per = pair_unit_tiles(tiles, pf.units);
-        const int used = (tiles + per - 1) / per;
+        const int first = pair_units_before(row, pf.row0, all, pf.per);
+        const int used = pair_units_before(row + 1, pf.row0, all, pf.per) - first;
+        const float4* targets = part + (size_t)first * kPairRow + (i - row * kPairRow);
 #pragma unroll 4
-        for (int u = j; u < used; u += kFoldLanes) add(part[(size_t)u * n_pad + i]);
+        for (int u = j; u < used; u += kFoldLanes) add(targets[(size_t)u * kPairRow]);
     }
-    const float4* sources = part + (size_t)pf.units * n_pad;
+    const float4* sources = part + (size_t)pair_units_before(last, pf.row0, all, pf.per) * kPairRow;
     const int end = min(row, last);
 #pragma unroll 4
     for (int r = pf.row0 + j; r < end; r += kFoldLanes)
         add(sources[pair_source_base(r, pf.row0, n_pad) + (size_t)(i - (r + 1) * kPairRow)]);
-    return make_float3(butterfly_total(ax, kx), butterfly_total(ay, ky), butterfly_total(az, kz));
+    return HiLo3{butterfly_total(ax, kx), butterfly_total(ay, ky), butterfly_total(az, kz)};
+}
+
+// Adds a fold's total to a running (sum, low part); either may be the larger,
+// which a Kahan addition does not allow for.
+__device__ __forceinline__ void add_total(float& s, float& low, const HiLo& f) {
+    float e;
+    s = two_sum(s, f.hi, e);
+    low += e + f.lo;
 }
 
 // Folds the partials of one of several launches of k_direct_pairs into the
-// bodies' running (sum, compensation); the first launch starts them.
+// bodies' running (sum, low part); the first launch starts them.
 __global__ void k_pairs_carry(const float4* __restrict__ part, PairFold pf, int n_pad, int first,
                               float4* __restrict__ carry, const int* __restrict__ err) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = t / kFoldLanes, j = t % kFoldLanes;
     if (i >= n_pad || *err != 0) return;
-    const float3 f = fold_pairs_lanes(part, pf, n_pad, i, j);
+    const HiLo3 f = fold_pairs_lanes(part, pf, n_pad, i, j);
     if (j != 0) return;
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f), c = s;
     if (!first) {
         s = carry[i];
         c = carry[n_pad + i];
     }
-    kahan_add(s.x, c.x, f.x);
-    kahan_add(s.y, c.y, f.y);
-    kahan_add(s.z, c.z, f.z);
+    add_total(s.x, c.x, f.x); add_total(s.y, c.y, f.y); add_total(s.z, c.z, f.z);
     carry[i] = s;
     carry[n_pad + i] = c;
+}
+
+// The last launch's fold f plus what the earlier ones left in the carry (if any).
+__device__ __forceinline__ float3 with_carry(const HiLo3& f, const float4* __restrict__ carry, int n_pad, int i) {
+    if (!carry) return make_float3(f.x.rounded(), f.y.rounded(), f.z.rounded());
+    float4 s = carry[i], c = carry[n_pad + i];
+    add_total(s.x, c.x, f.x); add_total(s.y, c.y, f.y); add_total(s.z, c.z, f.z);
+    return make_float3(s.x + c.x, s.y + c.y, s.z + c.z);
 }
 
 // PAIRS: the partials are k_direct_pairs' (carry: the earlier launches' sums,
@@ -499,15 +514,9 @@ __global__ void k_direct_reduce_update(const float4* __restrict__ part, int spli
     const int i = t / kFoldLanes, j = t % kFoldLanes;
     // whole groups of lanes leave together (n_pad bodies, a multiple of the block)
     if (i >= n_pad || *err != 0) return;
-    float3 f = PAIRS ? fold_pairs_lanes(part, pf, n_pad, i, j) : fold_partials_lanes(part, splits, n_pad, i, j);
+    const HiLo3 total = PAIRS ? fold_pairs_lanes(part, pf, n_pad, i, j) : fold_partials_lanes(part, splits, n_pad, i, j);
     if (i >= n || j != 0) return;
-    if (PAIRS && carry) {
-        float4 s = carry[i], c = carry[n_pad + i];
-        kahan_add(s.x, c.x, f.x);
-        kahan_add(s.y, c.y, f.y);
-        kahan_add(s.z, c.z, f.z);
-        f = make_float3(s.x - c.x, s.y - c.y, s.z - c.z);
-    }
+    const float3 f = with_carry(total, carry, n_pad, i);
     float3 a = make_float3(G * f.x, G * f.y, G * f.z);
     if (finit) {
         const float4 f = finit[i];
@@ -636,59 +645,101 @@ static cudaError_t reserve_part(nb_sim* sim, size_t need) {
     return cudaSuccess;
 }
 
-// Units the first row of k_direct_pairs is cut into (later rows have fewer
-// source tiles and so shorter units, which keeps the end of the launch short):
-// about 24 units of work an SM, from one tile a unit for small states, where a
-// whole state is 3 to 30 tiles an SM, to dozens.  More units would only add
-// partials to write and fold.
-static int pair_units(const nb_sim* sim, int rows, int ntiles) {
-    const long long work = (long long)rows * ntiles - (long long)kPairRowTiles * rows * (rows - 1) / 2;
-    const long long per = std::max<long long>(1, work / (24ll * std::max(1, sim->sm_count)));
-    return std::min(ntiles, (int)std::max<long long>(8, std::min<long long>(128, (ntiles + per - 1) / per)));
+static size_t pair_entries(const PairFold& p, int n_pad) {
+    return (size_t)pair_units_before(p.row0 + p.rows, p.row0, n_pad / kPairRow, p.per) * kPairRow +
+           pair_source_base(p.row0 + p.rows, p.row0, n_pad);
 }
 
-// k_direct_pairs over all rows, as many rows a launch as keep the source
-// partials within kPairSourceBytes, folded into the carry between launches.
-// The last launch's partials are left for the reduction (*pf, *carry).
-constexpr size_t kPairSourceBytes = (size_t)1 << 30;
-constexpr size_t kPairMin = 10240;
+// The launch of k_direct_pairs that starts at row0, within cap entries of
+// partials: tiles a unit and rows.  The length of a launch is estimated in
+// tiles of one SM's time from the units of the fullest SM, three resident at a
+// time (fewer take nearly as long: a block alone is a chain of latencies), 0.15
+// tiles a unit for its start and end, 0.3 units for the uneven end of the
+// launch and two tiles a launch; rows left over count at the same rate.  all_rows: the partials are roomy, and only
+// launches of as many rows as fit are compared.
+constexpr int kPairBlocksPerSm = 3;
 
-static cudaError_t launch_pairs(nb_sim* sim, PairFold* pf, const float4** carry) {
-    const int n_pad = (int)sim->n_pad, rows = n_pad / kPairRow, ntiles = n_pad / kTileJ;
-    const int units = pair_units(sim, rows, ntiles);
-    const size_t cap = kPairSourceBytes / sizeof(float4);
-    auto rows_from = [&](int row0) {   // rows of the launch that starts at row0
-        int r = 1;
-        while (row0 + r < rows && pair_source_base(row0 + r + 1, row0, n_pad) <= cap) ++r;
-        return r;
-    };
-    const bool several = rows_from(0) < rows;
-    size_t most = 0;
-    for (int r0 = 0; r0 < rows; r0 += rows_from(r0)) most = std::max(most, pair_source_base(r0 + rows_from(r0), r0, n_pad));
-    const size_t base = (size_t)units * n_pad;
-    cudaError_t e = reserve_part(sim, base + most + (several ? (size_t)2 * n_pad : 0));
-    if (e != cudaSuccess) return e;
-    float4* sums = several ? sim->part + base + most : nullptr;
-    const float S = (float)sim->prm.softening2;
-    const bool plummer = sim->prm.law == NB_LAW_PLUMMER;
-    for (int r0 = 0, count; r0 < rows; r0 += count) {
-        count = rows_from(r0);
-        const dim3 grid((unsigned)units, (unsigned)count);
-#define NB_PAIRS(L, H)                                                                                            \
-    k_direct_pairs<L, H><<<grid, kPairThreads, 0, sim->stream>>>(sim->pos, n_pad, r0, units, S, sim->part, sim->d_err, \
-                                                                 sim->wait_polls, sim->d_mmax)
-        if (plummer) { if (sim->heavy) NB_PAIRS(NB_LAW_PLUMMER, true); else NB_PAIRS(NB_LAW_PLUMMER, false); }
-        else { if (sim->heavy) NB_PAIRS(NB_LAW_REFERENCE, true); else NB_PAIRS(NB_LAW_REFERENCE, false); }
-#undef NB_PAIRS
-        *pf = PairFold{units, r0, count};
-        if (r0 + count < rows) {
-            k_pairs_carry<<<(unsigned)(sim->n_pad * kFoldLanes / 256), 256, 0, sim->stream>>>(sim->part, *pf, n_pad,
-                                                                                              r0 == 0 ? 1 : 0, sums,
-                                                                                              sim->d_err);
-            sim->prof.launches += 2;   // this pair of launches; the last one is the phase's own
+static PairFold pair_plan(int sm_count, int n_pad, int row0, size_t cap, bool all_rows) {
+    const int rows = n_pad / kPairRow, sms = std::max(1, sm_count);
+    const int pers[] = {1, 2, 4, 8, 16, 24, 32, 48, 64};
+    const double tail[kPairBlocksPerSm] = {0.0, 2.2, 2.6};
+    PairFold best{kPairRowTiles, row0, 1};
+    double best_time = 0.0;
+    bool any = false;
+    const int left = rows - row0;
+    for (int per : pers) {
+        for (int r = left; r >= 1; --r) {
+            const PairFold p{per, row0, r};
+            if (pair_entries(p, n_pad) > cap) continue;
+            const int units = pair_units_before(row0 + r, row0, rows, per), k = (units + sms - 1) / sms;
+            const double work = (double)r * left - 0.5 * r * (r - 1), all = 0.5 * left * (left + 1.0);
+            const double time = ((k / kPairBlocksPerSm * kPairBlocksPerSm + tail[k % kPairBlocksPerSm]) * (per + 0.15) +
+                                 0.3 * per + 2.0) * (all / work);
+            if (!any || time < best_time) {
+                any = true;
+                best_time = time;
+                best = p;
+            }
+            if (all_rows) break;
         }
     }
-    *carry = sums;
+    return best;
+}
+
+// k_direct_pairs over all rows in launches within cap entries of part, folded
+// into the carry between launches.  The last launch's partials are left for the
+// reduction (*last; *carry is null when it was the only one).  Returns the
+// launches made.
+template <bool HEAVY, int FOLD>
+static int launch_pairs(int sm_count, int law, cudaStream_t st, const float4* pos, int n_pad, float S, float4* part,
+                        size_t cap, bool all_rows, float4* carry_buf, int* err, uint32_t polls, const unsigned* mmax, PairFold* last,
+                        const float4** carry) {
+    const int rows = n_pad / kPairRow;
+    int made = 0;
+    *carry = nullptr;
+    for (int r0 = 0; r0 < rows;) {
+        const PairFold p = pair_plan(sm_count, n_pad, r0, cap, all_rows);
+        const unsigned grid = (unsigned)pair_units_before(r0 + p.rows, r0, rows, p.per);
+        if (law == NB_LAW_PLUMMER)
+            k_direct_pairs<NB_LAW_PLUMMER, HEAVY, FOLD><<<grid, kPairThreads, 0, st>>>(pos, n_pad, r0, p.rows, p.per, S, part, err,
+                                                                                 polls, mmax);
+        else
+            k_direct_pairs<NB_LAW_REFERENCE, HEAVY, FOLD><<<grid, kPairThreads, 0, st>>>(pos, n_pad, r0, p.rows, p.per, S, part, err,
+                                                                                   polls, mmax);
+        ++made;
+        *last = p;
+        if (r0 + p.rows < rows) {
+            k_pairs_carry<<<(unsigned)((size_t)n_pad * kFoldLanes / 256), 256, 0, st>>>(part, p, n_pad, r0 == 0 ? 1 : 0,
+                                                                                       carry_buf, err);
+            ++made;
+            *carry = carry_buf;
+        }
+        r0 += p.rows;
+    }
+    return made;
+}
+
+// Entries of partials a handle's k_direct_pairs launch may use (1 GiB): one
+// launch up to about 360,000 bodies.
+constexpr size_t kPairCap = ((size_t)1 << 30) / sizeof(float4);
+constexpr size_t kPairMin = 10240;
+
+static cudaError_t force_pairs(nb_sim* sim, PairFold* last, const float4** carry) {
+    const int n_pad = (int)sim->n_pad, rows = n_pad / kPairRow;
+    size_t most = 0;
+    int launches = 0;
+    for (int r0 = 0; r0 < rows; ++launches) {
+        const PairFold p = pair_plan(sim->sm_count, n_pad, r0, kPairCap, true);
+        most = std::max(most, pair_entries(p, n_pad));
+        r0 += p.rows;
+    }
+    cudaError_t e = reserve_part(sim, most + (launches > 1 ? (size_t)2 * n_pad : 0));
+    if (e != cudaSuccess) return e;
+    const float S = (float)sim->prm.softening2;
+    auto go = sim->heavy ? launch_pairs<true, kFold> : launch_pairs<false, kFold>;
+    const int made = go(sim->sm_count, sim->prm.law, sim->stream, sim->pos, n_pad, S, sim->part, kPairCap, true,
+                        sim->part + most, sim->d_err, sim->wait_polls, sim->d_mmax, last, carry);
+    sim->prof.launches += (uint64_t)(made - 1);   // the phase counts one
     return cudaGetLastError();
 }
 
@@ -705,7 +756,7 @@ cudaError_t direct_force_update(nb_sim* sim, float dt, bool update) {
     const float4* carry = nullptr;
     if (pairs) {
         PhaseScope ps(sim, 0);
-        cudaError_t e = launch_pairs(sim, &pf, &carry);
+        cudaError_t e = force_pairs(sim, &pf, &carry);
         if (e != cudaSuccess) return e;
     } else {
         DirectTuning t = sim->tune;
@@ -804,12 +855,17 @@ __global__ void k_noalloc_stage(const float4* __restrict__ in, int n, int n_pad,
 
 // Folds the partials like k_direct_reduce_update; a force kernel whose bounded
 // wait ran out poisons the output with NaN, since nothing is read back.
-__global__ void k_noalloc_reduce(const float4* __restrict__ part, int splits, int n, int n_pad, float G,
+template <bool PAIRS>
+__global__ void k_noalloc_reduce(const float4* __restrict__ part, int splits, PairFold pf,
+                                 const float4* __restrict__ carry, int n, int n_pad, float G,
                                  float4* __restrict__ acc) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float3 f = fold_partials(part, splits, n_pad, i);
-    float4 a = make_float4(G * f.x, G * f.y, G * f.z, 0.f);
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = t / kFoldLanes, j = t % kFoldLanes;
+    if (i >= n_pad) return;   // whole groups of lanes (the padded size is a multiple of the block's bodies)
+    const HiLo3 f = PAIRS ? fold_pairs_lanes(part, pf, n_pad, i, j) : fold_partials_lanes(part, splits, n_pad, i, j);
+    if (i >= n || j != 0) return;
+    const float3 s = with_carry(f, carry, n_pad, i);
+    float4 a = make_float4(G * s.x, G * s.y, G * s.z, 0.f);
     if (g_noalloc_err != 0) a = make_float4(NAN, NAN, NAN, NAN);
     acc[i] = a;
     if (i == 0) g_noalloc_mmax = 0u;
@@ -863,24 +919,50 @@ extern "C" int nb_direct_accel_noalloc(const float* pos_mass4, size_t n, float* 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const size_t n_pad = pad_up(n, kPad);
     const int ntiles = (int)(n_pad / kTileJ);
-    int splits = std::min(kNoAllocMaxSplits, ntiles);
-    const int tps = (ntiles + splits - 1) / splits;
-    splits = (ntiles + tps - 1) / tps;
     float4* pos = scratch;
     float4* part = scratch + n_pad;
+    const float S = (float)softening2;
     k_noalloc_stage<<<(unsigned)((n_pad + 255) / 256), 256, 0, st>>>(reinterpret_cast<const float4*>(pos_mass4),
                                                                     (int)n, (int)n_pad, pos);
-    const int block = 128, ipt = n_pad >= 16384 ? 2 : 1;
-    dim3 grid((unsigned)(n_pad / (size_t)(block * ipt)), (unsigned)splits);
-    const float S = (float)softening2;
-    bool ok = law == NB_LAW_PLUMMER
-                  ? launch_force_law<NB_LAW_PLUMMER, true>(block, ipt, grid, st, pos, (int)n_pad, tps, ntiles, splits,
-                                                          S, part, err, kMaxPolls, mmax, true)
-                  : launch_force_law<NB_LAW_REFERENCE, true>(block, ipt, grid, st, pos, (int)n_pad, tps, ntiles,
-                                                            splits, S, part, err, kMaxPolls, mmax, true);
-    if (!ok) return NB_EINVAL;
-    k_noalloc_reduce<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(part, splits, (int)n, (int)n_pad, (float)G,
-                                                                 reinterpret_cast<float4*>(accel4));
+    PairFold pf{};
+    const float4* carry = nullptr;
+    int splits = 0;
+    const bool pairs = n_pad >= kPairMin;
+    if (pairs) {
+        // Each pair once, as for a handle, in as many launches as the fixed array
+        // asks for (six at 65,536 bodies; two entries a body hold their running
+        // sums).  Folding targets every 16 sources instead of 32 costs 4% and
+        // keeps the error at or below that of the one-direction kernel, whose
+        // fold here rounded less than the handle's did.  GB300: 50,001 bodies
+        // 1257 -> 946 us, 65,536 2004 -> 1530, 20,000 260 -> 191, 10,000 86 -> 54.
+        int sms = 0;
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+            cudaGetLastError();
+            return NB_ECUDA;
+        }
+        const size_t cap = kNoAllocScratch - 3 * n_pad;
+        launch_pairs<true, kFold / 2>(sms, law, st, pos, (int)n_pad, S, part, cap, false, part + cap, err, kMaxPolls, mmax, &pf, &carry);
+    } else {
+        splits = std::min(kNoAllocMaxSplits, ntiles);
+        const int tps = (ntiles + splits - 1) / splits;
+        splits = (ntiles + tps - 1) / tps;
+        const int block = 128, ipt = 1;   // default_tuning's shape below 16,384 bodies
+        dim3 grid((unsigned)(n_pad / (size_t)(block * ipt)), (unsigned)splits);
+        const bool ok =
+            law == NB_LAW_PLUMMER
+                ? launch_force_law<NB_LAW_PLUMMER, true>(block, ipt, grid, st, pos, (int)n_pad, tps, ntiles, splits, S,
+                                                        part, err, kMaxPolls, mmax, true)
+                : launch_force_law<NB_LAW_REFERENCE, true>(block, ipt, grid, st, pos, (int)n_pad, tps, ntiles, splits, S,
+                                                          part, err, kMaxPolls, mmax, true);
+        if (!ok) return NB_EINVAL;
+    }
+    const unsigned rblocks = (unsigned)(n_pad * kFoldLanes / 256);
+    if (pairs)
+        k_noalloc_reduce<true><<<rblocks, 256, 0, st>>>(part, splits, pf, carry, (int)n, (int)n_pad, (float)G,
+                                                        reinterpret_cast<float4*>(accel4));
+    else
+        k_noalloc_reduce<false><<<rblocks, 256, 0, st>>>(part, splits, pf, carry, (int)n, (int)n_pad, (float)G,
+                                                         reinterpret_cast<float4*>(accel4));
     if (cudaGetLastError() != cudaSuccess) return NB_ECUDA;
     return NB_OK;
 }
