@@ -262,8 +262,8 @@ int  nb_probe_fp32x2_peak(int device, double* tflops);
 typedef struct nb_batch nb_batch;
 typedef struct nb_tuning {
     int direct_block;     /* threads per block of the direct-sum kernel (64, 128, 256) */
-    int direct_ipt;       /* target bodies per thread (1, 2; block * ipt <= 256)       */
-    int direct_jtile;     /* source bodies per work unit (multiple of 128)             */
+    int direct_ipt;       /* target bodies per thread, in fours (1, 2; block * ipt <= 256) */
+    int direct_jtile;     /* source bodies of four work units (multiple of 128)        */
     int leaf_size;        /* bodies per Barnes-Hut leaf bucket (1..64)                  */
     int traverse_block;   /* threads per block of the traversal kernel (128)           */
 } nb_tuning;

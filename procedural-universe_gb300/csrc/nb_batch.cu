@@ -64,9 +64,9 @@ struct nb_batch {
     size_t qcap = 0;
     // direct-sum tables
     int32_t* body_dgal = nullptr;
-    int4* dgal = nullptr;
+    DirGal* dgal = nullptr;
     int4* units = nullptr;
-    int32_t* unit_comp = nullptr;
+    int32_t* unit_src = nullptr;
     int nunits = 0;
     float4* part = nullptr;
     size_t part_cap = 0;
@@ -115,32 +115,56 @@ bool tuning_valid(const nb_tuning& t) {
            t.leaf_size <= 64 && t.traverse_block == 128;
 }
 
-// Work units of the direct-sum galaxies for the current tuning.
+// Work units of the direct-sum galaxies for the current tuning: rows of 128 *
+// direct_ipt target bodies against runs of source bodies (k_batch_direct).
+// Rows and chunks that hold only padding are left out; a member's units, and so
+// its results, do not depend on the other members.  Longest units first, so that
+// the launch ends evenly.
 int plan_units(nb_batch* b) {
-    std::vector<int4> units, dg(b->ndgal);
-    std::vector<int32_t> ucomp;
-    const int tb = b->tune.direct_block * b->tune.direct_ipt;
-    const int utiles = b->tune.direct_jtile / kDirTile;
+    struct Unit {
+        int4 u;
+        int32_t src;
+    };
+    std::vector<Unit> list;
+    std::vector<DirGal> dg(b->ndgal);
+    const int row = 128 * b->tune.direct_ipt, row_chunks = row / kDirChunk;
     size_t part_base = 0;
     for (const auto& g : b->gal) {
         if (g.bh) continue;
-        const int ntiles = (int)(g.n_pad / kDirTile);
-        const int splits = (ntiles + utiles - 1) / utiles;
-        dg[g.idx] = make_int4((int)g.off, (int)g.n_pad, splits, (int)part_base);
-        const int comp = splits * (int)g.n_pad;
-        for (int blk = 0; blk < (int)(g.n_pad / tb); ++blk)
-            for (int s = 0; s < splits; ++s) {
-                const int t0 = s * utiles;
-                const int nt = std::min(utiles, ntiles - t0);
-                units.push_back(make_int4((int)g.off + blk * tb, (int)(g.off / kDirTile) + t0, nt,
-                                          (int)part_base + s * (int)g.n_pad + blk * tb));
-                ucomp.push_back(comp);
+        const int n_pad = (int)g.n_pad, sources = (int)pad_up(g.n, kDirChunk);
+        const bool once = n_pad <= kDirOnceMax;
+        // chunks a unit: a quarter of the tile where units are cut finely enough to end
+        // evenly, the whole tile for large members, whose partials grow with its inverse
+        const int L = std::min(1024, b->tune.direct_jtile / (once ? 4 * kDirChunk : kDirChunk));
+        const int splits = (sources / kDirChunk + L - 1) / L;
+        const size_t rows = (size_t)n_pad / row;
+        const size_t entries = (size_t)splits * n_pad + (once ? rows * n_pad - (size_t)row * rows * (rows + 1) / 2 : 0);
+        if (part_base + entries > (size_t)INT32_MAX) return bfail(b, NB_ENOMEM, "direct-sum partials exceed 2^31 entries");
+        dg[g.idx] = DirGal{(int)g.off, n_pad, row, L * kDirChunk, (int)part_base, splits, once ? 1 : 0, sources};
+        size_t entry = part_base + (size_t)splits * n_pad;   // row r's source partials
+        for (int r = 0; (size_t)r * row < g.n; ++r) {
+            const int t0 = (int)g.off + r * row, s0 = once ? r * row : 0;
+            const int chunks = (sources - s0) / kDirChunk;
+            for (int c = 0, s = 0; c < chunks; c += L, ++s) {
+                const int k = std::min(L, chunks - c);
+                const int own = once ? std::max(0, std::min(k, row_chunks - c)) : k;
+                list.push_back(Unit{make_int4(t0, (int)g.off + s0 + c * kDirChunk, k | (own << 16),
+                                              (int)part_base + s * n_pad + r * row),
+                                    (int32_t)((long long)entry - (t0 + row))});
             }
-        part_base += 2 * (size_t)splits * g.n_pad;
+            if (once) entry += (size_t)std::max(0, n_pad - (r + 1) * row);
+        }
+        part_base += entries;
     }
-    if (part_base > (size_t)INT32_MAX) return bfail(b, NB_ENOMEM, "direct-sum partials exceed 2^31 entries");
+    std::stable_sort(list.begin(), list.end(), [](const Unit& a, const Unit& c) { return (a.u.z & 0xffff) > (c.u.z & 0xffff); });
+    std::vector<int4> units(list.size());
+    std::vector<int32_t> usrc(list.size());
+    for (size_t k = 0; k < list.size(); ++k) {
+        units[k] = list[k].u;
+        usrc[k] = list[k].src;
+    }
     NB_BCUDA(b, upload(&b->units, units, b->core->stream));
-    NB_BCUDA(b, upload(&b->unit_comp, ucomp, b->core->stream));
+    NB_BCUDA(b, upload(&b->unit_src, usrc, b->core->stream));
     NB_BCUDA(b, upload(&b->dgal, dg, b->core->stream));
     b->nunits = (int)units.size();
     if (part_base > b->part_cap) {
@@ -154,18 +178,16 @@ int plan_units(nb_batch* b) {
     return NB_OK;
 }
 
-template <int LAW>
-bool launch_direct_t(nb_batch* b, int grid, cudaStream_t st, float S) {
-    const int blk = b->tune.direct_block, ipt = b->tune.direct_ipt;
-#define NB_BD(B, I)                                                                                           \
-    if (blk == B && ipt == I) {                                                                               \
-        k_batch_direct<LAW, B, I><<<grid, B, 0, st>>>(b->core->pos, b->units, b->unit_comp, b->nunits,         \
-                                                      b->next_unit, S, b->core->d_mmax, b->part);             \
-        return true;                                                                                          \
-    }
-    NB_BD(64, 1) NB_BD(64, 2) NB_BD(128, 1) NB_BD(128, 2) NB_BD(256, 1)
-#undef NB_BD
-    return false;
+// The direct members' force kernel: as many warps as the GPU holds, at most one
+// a unit.
+template <int LAW, int IPT>
+void launch_direct(nb_batch* b, cudaStream_t st, float S) {
+    const int threads = b->tune.direct_block, warps = threads / 32;
+    int occ = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_direct<LAW, IPT>, threads, 0);
+    const int grid = std::max(1, std::min((b->nunits + warps - 1) / warps, b->core->sm_count * std::max(1, occ)));
+    k_batch_direct<LAW, IPT><<<grid, threads, 0, st>>>(b->core->pos, b->units, b->unit_src, b->nunits, b->next_unit, S,
+                                                       b->core->d_mmax, b->part);
 }
 
 // One step (update) or one force evaluation (no update) of every galaxy,
@@ -231,16 +253,17 @@ int enqueue_step(nb_batch* b, float dt, bool update, bool tree_only = false) {
     if (b->ndgal > 0) {
         PhaseScope ps(c, NB_PHASE_DIRECT_FORCE, 2);
         if (b->n_bh == 0) NB_BCUDA(b, cudaMemsetAsync(b->next_unit, 0, sizeof(int), st));   // else cleared with the counters
-        int occ = 1;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_direct<NB_LAW_REFERENCE, 128, 1>,
-                                                      b->tune.direct_block, 0);
-        const int grid = std::max(1, std::min(b->nunits, c->sm_count * std::max(1, occ)));
-        const bool ok = b->base.law == NB_LAW_PLUMMER ? launch_direct_t<NB_LAW_PLUMMER>(b, grid, st, S)
-                                                      : launch_direct_t<NB_LAW_REFERENCE>(b, grid, st, S);
-        if (!ok) return bfail(b, NB_EINVAL, "unsupported direct tuning");
-        const int cnt = (int)(b->n_total - b->dir_begin);
-        k_batch_direct_reduce<<<(cnt + 255) / 256, 256, 0, st>>>(b->body_dgal, b->dgal, (int)b->dir_begin, cnt, G,
-                                                                b->part, c->acc);
+        const bool wide = b->tune.direct_ipt == 2;
+        if (b->base.law == NB_LAW_PLUMMER) {
+            if (wide) launch_direct<NB_LAW_PLUMMER, 8>(b, st, S);
+            else launch_direct<NB_LAW_PLUMMER, 4>(b, st, S);
+        } else {
+            if (wide) launch_direct<NB_LAW_REFERENCE, 8>(b, st, S);
+            else launch_direct<NB_LAW_REFERENCE, 4>(b, st, S);
+        }
+        const int cnt = (int)(b->n_total - b->dir_begin);   // a multiple of 256
+        k_batch_direct_reduce<<<cnt / 256 * kFoldLanes, 256, 0, st>>>(b->body_dgal, b->dgal, (int)b->dir_begin, cnt, G,
+                                                                     b->part, c->acc);
         NB_BCUDA(b, cudaGetLastError());
     }
     if (update) {
@@ -476,7 +499,7 @@ int nb_batch_destroy(nb_batch* b) {
         if (b->exec) cudaGraphExecDestroy(b->exec);
         void* ptrs[] = {b->body_slot, b->gal_range, b->gal_box, b->gal_root, b->slot_start, b->groups, b->group_ctr,
                         b->box_bits, b->cell_rec, b->body_dgal, b->dgal, b->units,
-                        b->unit_comp, b->part, b->next_unit, b->held};
+                        b->unit_src, b->part, b->next_unit, b->held};
         for (void* p : ptrs) dev_free(p, b->core ? b->core->stream : nullptr);
         if (b->core) nb_destroy(b->core);
         delete b;

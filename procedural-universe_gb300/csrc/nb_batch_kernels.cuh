@@ -23,9 +23,10 @@
 //    cells far from the group go into the group's local expansion instead.
 //    This is a performance form whose parity is the force error against the
 //    FP64 direct sum (<= 1e-3), not the reference's per-body opening rule.
-//  * Direct-sum members are padded to multiples of 256 bodies; a persistent
-//    kernel takes (galaxy, target block, source range) units from a table
-//    through an atomic counter, and a second kernel folds the partials.
+//  * Direct-sum members are padded to multiples of 256 bodies; the warps of a
+//    persistent kernel take (galaxy, target rows, source range) units from a
+//    table through an atomic counter, each pair of bodies once, and a second
+//    kernel folds the partials.
 #pragma once
 
 #include <type_traits>
@@ -44,7 +45,8 @@ constexpr int kStackCellLimit = 1 << 27;   // a stack entry packs a first-child 
 constexpr int kGMultiTop = kGStack - 155 - 32;   // stack height up to which a walk step takes several cells
 constexpr int kGCells = 64;             // accepted-cell list, per warp
 constexpr int kGBodies = 192;           // gathered leaf-bucket bodies, per warp
-constexpr int kDirTile = 128;           // sources per shared tile of the batched direct kernel
+constexpr int kDirChunk = 32;           // sources a warp of the batched direct kernel holds at a time
+constexpr int kDirOnceMax = 8192;       // padded bodies up to which a direct member takes each pair once
 // far-field defaults of the group traversal (rules in nb_batch.cu's nb_batch)
 constexpr double kFarEta = 0.2;         // geometric rule: group half-diagonal / distance
 constexpr double kFarAlpha = 1e-4;      // relative rule: truncation estimate / (|a|_min / G)
@@ -848,87 +850,179 @@ __global__ void __launch_bounds__(kGWarps * 32, 5) k_group_traverse(
 }
 
 // ---- batched direct sum --------------------------------------------------------
-// unit = (first target body, first source tile, source tiles, index of the
-// target's sum partial); the compensation partial follows at +comp_offset of
-// the unit's galaxy, kept in unit_comp.
-template <int LAW, int BLOCK, int IPT>
-__global__ void __launch_bounds__(BLOCK) k_batch_direct(const float4* __restrict__ pos, const int4* __restrict__ units,
-                                                        const int32_t* __restrict__ unit_comp, int nunits,
-                                                        int* __restrict__ next_unit, float S,
-                                                        const unsigned* __restrict__ mmax,
-                                                        float4* __restrict__ part) {
-    __shared__ float4 tile[kDirTile];
-    const float tiny = self_pair_tiny(mmax);
-    __shared__ int cur;
-    static_assert(kDirTile % BLOCK == 0 || BLOCK % kDirTile == 0, "tile/block");
-    while (true) {
-        __syncthreads();
-        if (threadIdx.x == 0) cur = atomicAdd(next_unit, 1);
-        __syncthreads();
-        const int u = cur;
-        if (u >= nunits) return;
-        const int4 un = units[u];
-        float xi[IPT], yi[IPT], zi[IPT], sx[IPT], sy[IPT], sz[IPT], cx[IPT], cy[IPT], cz[IPT];
+// A unit is a row of 32 * IPT target bodies, IPT a lane in registers (packed
+// FP32x2), against a run of 32-source chunks: (first target body, first source
+// body, chunks | chunks evaluated from the target side only << 16, entry of the
+// target partials); unit_src is the entry of body 0 among the row's source
+// partials.  Sources behind the row are evaluated once for both bodies, 17
+// FP32 operations for two interactions instead of 26: lane l takes source
+// (l + r) mod 32 at step r, and the sources' sums travel with them by shuffle
+// (as in k_direct_pairs, here within one warp).  The row's own bodies, and all
+// sources of a member of more than kDirOnceMax padded bodies (whose source
+// partials would grow with its square), are evaluated from the target side.
+//
+// Bound by the FP32 pipe.  Warps share nothing, so that no barrier waits for
+// the slowest; the next chunk and the next unit are fetched while the current
+// chunk is evaluated.  GB300, 200 members of 256-4096 bodies: force
+// kernel 387 -> 237 us and the fold 8 -> 44 us (ncu, cold caches; it now reads a
+// partial per row and body), a step 399 -> 281 us; FMA pipe 63% busy, the rest
+// is the shuffles and reads that four targets a lane carry (eight: 268 us a
+// step, but small members then fill fewer rows).
+template <int LAW, int IPT, bool BOTH>
+__device__ __forceinline__ void direct_chunk(const float4* src, int lane, const float2* nx, const float2* ny,
+                                             const float2* nz, const float2* mi, float2 S2, float2 T2, float* sum,
+                                             float* comp, float3& out) {
+    constexpr int P = IPT / 2, kGroup = 4;
+    const float2 z2 = make_float2(0.f, 0.f);
+    float2 ax[P], ay[P], az[P];
 #pragma unroll
-        for (int k = 0; k < IPT; ++k) {
-            const float4 q = pos[un.x + k * BLOCK + threadIdx.x];
-            xi[k] = q.x; yi[k] = q.y; zi[k] = q.z;
-            sx[k] = sy[k] = sz[k] = cx[k] = cy[k] = cz[k] = 0.f;
-        }
-        for (int t = 0; t < un.z; ++t) {
-            __syncthreads();
-            for (int j = threadIdx.x; j < kDirTile; j += BLOCK) tile[j] = pos[(size_t)(un.y + t) * kDirTile + j];
-            __syncthreads();
+    for (int q = 0; q < P; ++q) ax[q] = ay[q] = az[q] = z2;
+    float sx = 0.f, sy = 0.f, sz = 0.f;
 #pragma unroll 1
-            for (int f = 0; f < kDirTile; f += kFold) {
-                float tx[IPT], ty[IPT], tz[IPT];
+    for (int g = 0; g < kDirChunk; g += kGroup) {
+        float2 bx = z2, by = z2, bz = z2;
 #pragma unroll
-                for (int k = 0; k < IPT; ++k) tx[k] = ty[k] = tz[k] = 0.f;
-#pragma unroll 4
-                for (int j = 0; j < kFold; ++j) {
-                    const float4 pj = tile[f + j];
+        for (int u = 0; u < kGroup; ++u) {
+            const float4 pj = src[(lane + g + u) & 31];
+            const float2 jx = make_float2(pj.x, pj.x), jy = make_float2(pj.y, pj.y);
+            const float2 jz = make_float2(pj.z, pj.z), jm = make_float2(pj.w, pj.w);
 #pragma unroll
-                    for (int k = 0; k < IPT; ++k)
-                        interact<LAW>(pj, xi[k], yi[k], zi[k], S, tiny, tx[k], ty[k], tz[k]);
-                }
-#pragma unroll
-                for (int k = 0; k < IPT; ++k) {
-                    kahan_add(sx[k], cx[k], tx[k]);
-                    kahan_add(sy[k], cy[k], ty[k]);
-                    kahan_add(sz[k], cz[k], tz[k]);
+            for (int q = 0; q < P; ++q) {
+                const float2 dx = __fadd2_rn(jx, nx[q]), dy = __fadd2_rn(jy, ny[q]), dz = __fadd2_rn(jz, nz[q]);
+                const float2 w = pair_factor_x2<LAW>(dx, dy, dz, S2, T2);
+                const float2 wi = __fmul2_rn(jm, w);
+                ax[q] = __ffma2_rn(wi, dx, ax[q]);
+                ay[q] = __ffma2_rn(wi, dy, ay[q]);
+                az[q] = __ffma2_rn(wi, dz, az[q]);
+                if (BOTH) {
+                    const float2 wj = __fmul2_rn(mi[q], w);
+                    bx = __ffma2_rn(wj, dx, bx);
+                    by = __ffma2_rn(wj, dy, by);
+                    bz = __ffma2_rn(wj, dz, bz);
                 }
             }
+            if (BOTH && u + 1 < kGroup) {
+                const int next = (lane + 1) & 31;
+                bx.x = __shfl_sync(0xffffffffu, bx.x, next); bx.y = __shfl_sync(0xffffffffu, bx.y, next);
+                by.x = __shfl_sync(0xffffffffu, by.x, next); by.y = __shfl_sync(0xffffffffu, by.y, next);
+                bz.x = __shfl_sync(0xffffffffu, bz.x, next); bz.y = __shfl_sync(0xffffffffu, bz.y, next);
+            }
         }
-        const int co = unit_comp[u];
+        if (BOTH) {   // the source's earlier groups were left kGroup lanes on
+            const int from = (lane + kGroup) & 31;
+            sx = __shfl_sync(0xffffffffu, sx, from) + (bx.x + bx.y);
+            sy = __shfl_sync(0xffffffffu, sy, from) + (by.x + by.y);
+            sz = __shfl_sync(0xffffffffu, sz, from) + (bz.x + bz.y);
+        }
+    }
 #pragma unroll
-        for (int k = 0; k < IPT; ++k) {
-            const int d = k * BLOCK + threadIdx.x;
-            part[(size_t)un.w + d] = make_float4(sx[k], sy[k], sz[k], 0.f);
-            part[(size_t)un.w + co + d] = make_float4(cx[k], cy[k], cz[k], 0.f);
-        }
+    for (int q = 0; q < P; ++q) {
+        kahan_add(sum[6 * q], comp[6 * q], ax[q].x);
+        kahan_add(sum[6 * q + 1], comp[6 * q + 1], ay[q].x);
+        kahan_add(sum[6 * q + 2], comp[6 * q + 2], az[q].x);
+        kahan_add(sum[6 * q + 3], comp[6 * q + 3], ax[q].y);
+        kahan_add(sum[6 * q + 4], comp[6 * q + 4], ay[q].y);
+        kahan_add(sum[6 * q + 5], comp[6 * q + 5], az[q].y);
+    }
+    if (BOTH) {   // lane l holds source (l + 31) mod 32
+        const int own = (lane + 1) & 31;
+        out = make_float3(-__shfl_sync(0xffffffffu, sx, own), -__shfl_sync(0xffffffffu, sy, own),
+                          -__shfl_sync(0xffffffffu, sz, own));
     }
 }
 
-// folds the partials of direct-sum body i (global index begin + i) into acc.
-__global__ void k_batch_direct_reduce(const int32_t* __restrict__ body_dgal, const int4* __restrict__ dgal /* off, n_pad, splits, part_base */,
-                                      int begin, int count, float G, const float4* __restrict__ part,
-                                      float4* __restrict__ acc) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const int g = body_dgal[i];
-    if (g < 0) return;   // padding body
-    const int4 d = dgal[g];
-    const int local = begin + i - d.x;
-    float ax = 0.f, ay = 0.f, az = 0.f, kx = 0.f, ky = 0.f, kz = 0.f, qx = 0.f, qy = 0.f, qz = 0.f;
-    for (int s = 0; s < d.z; ++s) {
-        const float4 p = part[(size_t)d.w + (size_t)s * d.y + local];
-        const float4 c = part[(size_t)d.w + (size_t)(d.z + s) * d.y + local];
-        kahan_add(ax, kx, p.x);
-        kahan_add(ay, ky, p.y);
-        kahan_add(az, kz, p.z);
-        qx += c.x; qy += c.y; qz += c.z;
+constexpr int kDirWarps = 8;   // most warps per block
+template <int LAW, int IPT>
+__global__ void __launch_bounds__(kDirWarps * 32, IPT == 4 ? 2 : 1) k_batch_direct(
+    const float4* __restrict__ pos, const int4* __restrict__ units, const int32_t* __restrict__ unit_src, int nunits,
+    int* __restrict__ next_unit, float S, const unsigned* __restrict__ mmax, float4* __restrict__ part) {
+    __shared__ float4 src[kDirWarps][2][kDirChunk];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float tiny = self_pair_tiny(mmax);
+    const float2 S2 = make_float2(S, S), T2 = make_float2(tiny, tiny);
+    constexpr int P = IPT / 2;
+    int u = 0;
+    if (lane == 0) u = atomicAdd(next_unit, 1);
+    u = __shfl_sync(0xffffffffu, u, 0);
+    while (u < nunits) {
+        const int4 un = units[u];
+        const int src0 = unit_src[u], chunks = un.z & 0xffff, own = un.z >> 16;
+        int after = 0;
+        if (lane == 0) after = atomicAdd(next_unit, 1);
+        float2 nx[P], ny[P], nz[P], mi[P];
+        float sum[3 * IPT], comp[3 * IPT];
+#pragma unroll
+        for (int q = 0; q < P; ++q) {
+            const float4 a = pos[un.x + (2 * q) * 32 + lane], b = pos[un.x + (2 * q + 1) * 32 + lane];
+            nx[q] = make_float2(-a.x, -b.x);
+            ny[q] = make_float2(-a.y, -b.y);
+            nz[q] = make_float2(-a.z, -b.z);
+            mi[q] = make_float2(a.w, b.w);
+        }
+#pragma unroll
+        for (int k = 0; k < 3 * IPT; ++k) sum[k] = comp[k] = 0.f;
+        float4 cur = pos[un.y + lane];
+        for (int c = 0; c < chunks; ++c) {
+            float4* buf = src[warp][c & 1];
+            buf[lane] = cur;
+            __syncwarp();   // also: every lane is done with the chunk that this buffer held
+            if (c + 1 < chunks) cur = pos[un.y + (c + 1) * kDirChunk + lane];
+            float3 f;
+            if (c < own) {
+                direct_chunk<LAW, IPT, false>(buf, lane, nx, ny, nz, mi, S2, T2, sum, comp, f);
+            } else {
+                direct_chunk<LAW, IPT, true>(buf, lane, nx, ny, nz, mi, S2, T2, sum, comp, f);
+                part[(long long)src0 + un.y + c * kDirChunk + lane] = make_float4(f.x, f.y, f.z, 0.f);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < IPT; ++k)
+            part[(size_t)un.w + k * 32 + lane] =
+                make_float4(sum[3 * k] - comp[3 * k], sum[3 * k + 1] - comp[3 * k + 1], sum[3 * k + 2] - comp[3 * k + 2], 0.f);
+        u = __shfl_sync(0xffffffffu, after, 0);
+        __syncwarp();   // the next unit's first chunk may take the buffer read last
     }
-    acc[begin + i] = make_float4(G * (ax - (kx + qx)), G * (ay - (ky + qy)), G * (az - (kz + qz)), 0.f);
+}
+
+// A direct-sum member's partials: [splits][n_pad] for its bodies as targets
+// (only the first ones of a row that its sources fill), then, where each pair
+// is taken once, for each row one entry per body behind it.
+struct DirGal {
+    int off, n_pad, row, split;   // first body, padded bodies, bodies a row, source bodies a unit
+    int base, splits, once, sources;   // first entry, splits, each pair once?, source bodies (to a whole chunk)
+};
+
+// Folds the partials of direct-sum body i (global index begin + i) into acc:
+// kFoldLanes consecutive threads a body, in a fixed order.
+__global__ void k_batch_direct_reduce(const int32_t* __restrict__ body_dgal, const DirGal* __restrict__ dgal, int begin,
+                                      int count, float G, const float4* __restrict__ part, float4* __restrict__ acc) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = t / kFoldLanes, j = t % kFoldLanes;
+    if (i >= count) return;   // whole groups of lanes; count is a multiple of a block's bodies
+    const int g = body_dgal[i];
+    float ax = 0.f, ay = 0.f, az = 0.f, kx = 0.f, ky = 0.f, kz = 0.f;
+    if (g >= 0) {   // not a padding body
+        const DirGal d = dgal[g];
+        const int local = begin + i - d.off, row = local / d.row;
+        auto add = [&](const float4 p) {
+            kahan_add(ax, kx, p.x);
+            kahan_add(ay, ky, p.y);
+            kahan_add(az, kz, p.z);
+        };
+        const int behind = d.sources - (d.once ? row * d.row : 0);
+        const int used = (behind + d.split - 1) / d.split;
+#pragma unroll 4
+        for (int s = j; s < used; s += kFoldLanes) add(part[(size_t)d.base + (size_t)s * d.n_pad + local]);
+        if (d.once) {
+            const float4* src = part + (size_t)d.base + (size_t)d.splits * d.n_pad;
+#pragma unroll 4
+            for (int r = j; r < row; r += kFoldLanes)
+                add(src[(size_t)r * d.n_pad - (size_t)d.row * r * (r + 1) / 2 + (local - (r + 1) * d.row)]);
+        }
+    }
+    const HiLo x = butterfly_total(ax, kx), y = butterfly_total(ay, ky), z = butterfly_total(az, kz);
+    if (g >= 0 && j == 0)
+        acc[begin + i] = make_float4(G * x.rounded(), G * y.rounded(), G * z.rounded(), 0.f);
 }
 
 }  // namespace nb

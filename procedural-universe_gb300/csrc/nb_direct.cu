@@ -387,38 +387,6 @@ __device__ __forceinline__ void write_vertex(nb_render_vertex* rv, const float4*
 // kFoldLanes consecutive threads fold one body's partials: lane j takes
 // splits j, j + kFoldLanes, ... (compensated, in that order), and the lanes'
 // sums are added by a butterfly (every lane gets the same total).
-constexpr int kFoldLanes = 8;
-
-// Knuth's two-sum: s + b as a rounded sum and its exact error, whichever is larger.
-__device__ __forceinline__ float two_sum(float s, float b, float& err) {
-    const float t = __fadd_rn(s, b), u = __fsub_rn(t, s);
-    err = __fadd_rn(__fsub_rn(s, __fsub_rn(t, u)), __fsub_rn(b, u));
-    return t;
-}
-
-// Sum over the fold's lanes of (s - c), the same in every lane: added pairwise
-// with the rounding error of each sum carried in the low part; the total is hi + lo, hi its rounding to a few units.
-struct HiLo {
-    float hi, lo;
-    __device__ __forceinline__ float rounded() const { return __fadd_rn(hi, lo); }
-};
-struct HiLo3 {
-    HiLo x, y, z;
-};
-
-__device__ __forceinline__ HiLo butterfly_total(float s, float c) {
-    float hi = s, lo = -c;
-#pragma unroll
-    for (int o = 1; o < kFoldLanes; o <<= 1) {
-        const float b = __shfl_xor_sync(0xffffffffu, hi, o);
-        const float bl = __shfl_xor_sync(0xffffffffu, lo, o);
-        float e;   // the sum's error is exact, so either side of the exchange finds the same
-        hi = two_sum(hi, b, e);
-        lo = __fadd_rn(__fadd_rn(lo, bl), e);
-    }
-    return HiLo{hi, lo};
-}
-
 __device__ __forceinline__ HiLo3 fold_partials_lanes(const float4* __restrict__ part, int splits, int n_pad, int i,
                                                       int j) {
     float ax = 0.f, ay = 0.f, az = 0.f, kx = 0.f, ky = 0.f, kz = 0.f, qx = 0.f, qy = 0.f, qz = 0.f;

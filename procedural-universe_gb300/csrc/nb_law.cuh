@@ -100,4 +100,37 @@ __device__ __forceinline__ float2 pair_factor_x2(float2 dx, float2 dy, float2 dz
     return __fmul2_rn(inv, __fmul2_rn(inv, inv));
 }
 
+// Consecutive threads that fold one body's partials together.
+constexpr int kFoldLanes = 8;
+
+// Knuth's two-sum: s + b as a rounded sum and its exact error, whichever is larger.
+__device__ __forceinline__ float two_sum(float s, float b, float& err) {
+    const float t = __fadd_rn(s, b), u = __fsub_rn(t, s);
+    err = __fadd_rn(__fsub_rn(s, __fsub_rn(t, u)), __fsub_rn(b, u));
+    return t;
+}
+
+// Sum over the fold's lanes of (s - c), the same in every lane: added pairwise
+// with the rounding error of each sum carried in the low part; the total is hi + lo, hi its rounding to a few units.
+struct HiLo {
+    float hi, lo;
+    __device__ __forceinline__ float rounded() const { return __fadd_rn(hi, lo); }
+};
+struct HiLo3 {
+    HiLo x, y, z;
+};
+
+__device__ __forceinline__ HiLo butterfly_total(float s, float c) {
+    float hi = s, lo = -c;
+#pragma unroll
+    for (int o = 1; o < kFoldLanes; o <<= 1) {
+        const float b = __shfl_xor_sync(0xffffffffu, hi, o);
+        const float bl = __shfl_xor_sync(0xffffffffu, lo, o);
+        float e;   // the sum's error is exact, so either side of the exchange finds the same
+        hi = two_sum(hi, b, e);
+        lo = __fadd_rn(__fadd_rn(lo, bl), e);
+    }
+    return HiLo{hi, lo};
+}
+
 }  // namespace nb

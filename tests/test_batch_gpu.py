@@ -267,3 +267,38 @@ def test_octree_outgrowing_its_arrays_is_resized_and_steps_rerun():
                 pb, vb = b.read(g)
                 np.testing.assert_array_equal(pa, pb)
                 np.testing.assert_array_equal(va, vb)
+
+
+@pytest.mark.parametrize("law", [nb.LAW_REFERENCE, nb.LAW_PLUMMER])
+@pytest.mark.parametrize("tune", [{}, dict(direct_ipt=2), dict(direct_block=64, direct_jtile=128),
+                                  dict(direct_block=256, direct_jtile=4096)])
+def test_direct_members_match_fp64_at_row_and_chunk_edges(law, tune):
+    """Members at the edges of source chunks, target rows and padding, the
+    largest that takes each pair once and the first beyond it; uneven masses,
+    a coincident pair.  A term carries a few units of 2^-24 and the sums are
+    compensated: 5e-7 bounds their total."""
+    sizes = [1, 2, 31, 33, 127, 129, 255, 257, 513, 1000, 4097, 8192, 8193]
+    gals = []
+    for k, n in enumerate(sizes):
+        pm, v = nb.seed_plummer(50 + k, max(n, 2))
+        pm, v = pm[:n].copy(), v[:n].copy()
+        pm[:, 3] *= np.random.default_rng(n).uniform(0.01, 2.0, n).astype(np.float32)
+        if n > 200:
+            pm[5, :3] = pm[n - 1, :3]
+        gals.append((pm, v))
+    b = nb.NBodyBatch(bh_threshold=1 << 20, softening2=EPS2, law=law)
+    with b:
+        for pm, v in gals:
+            b.add(pm, v)
+        if tune:
+            b.set_tuning(**tune)
+        b.commit()
+        for g, (pm, v) in enumerate(gals):
+            F = b.forces(g)
+            with nb.NBodySim(kind=nb.SIM_BRUTE_FORCE, softening2=EPS2, law=law) as s:
+                s.init_soa(pm, v)
+                F64 = s.fp64_forces(np.arange(pm.shape[0], dtype=np.int32))
+            if pm.shape[0] == 1:
+                assert not F.any()
+            else:
+                assert O.rel_l2(F, F64) < 5e-7, (pm.shape[0], O.rel_l2(F, F64))
