@@ -72,6 +72,11 @@ struct nb_batch {
     size_t part_cap = 0;
     int* next_unit = nullptr;
     uint64_t direct_pairs = 0;
+    // whole-batch transfers of many galaxies: runs of bodies and the dense copy of
+    // one state array, made on the first such transfer and kept
+    int4* move_runs = nullptr;
+    int nmove = 0;
+    float4* move_buf = nullptr;
     // steps whose octree did not fit its arrays leave the state unchanged and
     // count here; the wait resizes the tree and runs them again
     int* held = nullptr;
@@ -499,7 +504,7 @@ int nb_batch_destroy(nb_batch* b) {
         if (b->exec) cudaGraphExecDestroy(b->exec);
         void* ptrs[] = {b->body_slot, b->gal_range, b->gal_box, b->gal_root, b->slot_start, b->groups, b->group_ctr,
                         b->box_bits, b->cell_rec, b->body_dgal, b->dgal, b->units,
-                        b->unit_src, b->part, b->next_unit, b->held};
+                        b->unit_src, b->part, b->next_unit, b->held, b->move_runs, b->move_buf};
         for (void* p : ptrs) dev_free(p, b->core ? b->core->stream : nullptr);
         if (b->core) nb_destroy(b->core);
         delete b;
@@ -947,6 +952,33 @@ int nb_batch_autotune(nb_batch* b, float dt, int trial_steps) {
 }  // extern "C"
 
 // ---- whole-batch state transfer (the reference-facing end-to-end path) -----
+namespace {
+
+// Whether a whole-batch transfer goes through the dense copy: many galaxies,
+// and room for it (else one copy a galaxy).
+constexpr size_t kMoveMinGalaxies = 8;
+bool dense_transfer(nb_batch* b) {
+    if (b->gal.size() < kMoveMinGalaxies) return false;
+    if (b->move_buf) return true;
+    std::vector<int4> runs;
+    size_t dense = 0;
+    for (const auto& g : b->gal) {
+        for (size_t c = 0; c < g.n; c += kMoveChunk)
+            runs.push_back(make_int4((int)(g.off + c), (int)(dense + c), (int)std::min<size_t>(kMoveChunk, g.n - c), 0));
+        dense += g.n;
+    }
+    if (upload(&b->move_runs, runs, b->core->stream) != cudaSuccess ||
+        dev_alloc(&b->move_buf, dense * sizeof(float4)) != cudaSuccess) {
+        cudaGetLastError();
+        b->move_buf = nullptr;
+        return false;
+    }
+    b->nmove = (int)runs.size();
+    return true;
+}
+
+}  // namespace
+
 extern "C" {
 
 // Uploads the state of every galaxy (galaxies in index order, concatenated:
@@ -957,18 +989,27 @@ int nb_batch_write_state(nb_batch* b, const float* pos_mass4, const float* vel4)
         if (!b->committed) return bfail(b, NB_EBADSTATE, "nb_batch_commit first");
         cudaSetDevice(b->core->dev);
         nb_sim* c = b->core;
-        size_t src = 0;
-        for (const auto& g : b->gal) {
-            NB_BCUDA(b, cudaMemcpyAsync(c->pos + g.off, pos_mass4 + 4 * src, g.n * 16, cudaMemcpyHostToDevice, c->stream));
-            NB_BCUDA(b, cudaMemcpyAsync(c->vel + g.off, vel4 + 4 * src, g.n * 16, cudaMemcpyHostToDevice, c->stream));
-            NB_BCUDA(b, cudaMemsetAsync(c->posc + g.off, 0, g.n * 16, c->stream));
-            NB_BCUDA(b, cudaMemsetAsync(c->velc + g.off, 0, g.n * 16, c->stream));
-            src += g.n;
+        if (dense_transfer(b)) {
+            const float* host[2] = {pos_mass4, vel4};
+            float4* state[2] = {c->pos, c->vel};
+            for (int k = 0; k < 2; ++k) {
+                NB_BCUDA(b, cudaMemcpyAsync(b->move_buf, host[k], b->n_real * 16, cudaMemcpyHostToDevice, c->stream));
+                k_move_state<false><<<b->nmove, 256, 0, c->stream>>>(b->move_runs, state[k], b->move_buf);
+                NB_BCUDA(b, cudaGetLastError());
+            }
+        } else {
+            size_t src = 0;
+            for (const auto& g : b->gal) {
+                NB_BCUDA(b, cudaMemcpyAsync(c->pos + g.off, pos_mass4 + 4 * src, g.n * 16, cudaMemcpyHostToDevice, c->stream));
+                NB_BCUDA(b, cudaMemcpyAsync(c->vel + g.off, vel4 + 4 * src, g.n * 16, cudaMemcpyHostToDevice, c->stream));
+                src += g.n;
+            }
         }
         // accelerations belong to the previous state: the next evaluation takes
         // the far field's geometric rule, as after a commit
         NB_BCUDA(b, cudaMemsetAsync(c->acc, 0, c->n_pad * sizeof(float4), c->stream));
-        // validated (reported by the next wait) and the largest mass recorded
+        // validated (reported by the next wait), the compensation terms cleared and
+        // the largest mass recorded
         const int rc = sim_rescan_state(c);
         if (rc) return bfail(b, rc, nb_last_error(c));
         return NB_OK;
@@ -985,12 +1026,22 @@ int nb_batch_read_state(nb_batch* b, float* pos_mass4, float* vel4) {
         if (!b->committed) return bfail(b, NB_EBADSTATE, "nb_batch_commit first");
         cudaSetDevice(b->core->dev);
         nb_sim* c = b->core;
-        size_t dst = 0;
-        for (const auto& g : b->gal) {
-            NB_BCUDA(b, cudaMemcpyAsync(pos_mass4 + 4 * dst, c->pos + g.off, g.n * 16, cudaMemcpyDeviceToHost, c->stream));
-            if (vel4)
-                NB_BCUDA(b, cudaMemcpyAsync(vel4 + 4 * dst, c->vel + g.off, g.n * 16, cudaMemcpyDeviceToHost, c->stream));
-            dst += g.n;
+        if (dense_transfer(b)) {
+            float* host[2] = {pos_mass4, vel4};
+            float4* state[2] = {c->pos, c->vel};
+            for (int k = 0; k < (vel4 ? 2 : 1); ++k) {
+                k_move_state<true><<<b->nmove, 256, 0, c->stream>>>(b->move_runs, state[k], b->move_buf);
+                NB_BCUDA(b, cudaGetLastError());
+                NB_BCUDA(b, cudaMemcpyAsync(host[k], b->move_buf, b->n_real * 16, cudaMemcpyDeviceToHost, c->stream));
+            }
+        } else {
+            size_t dst = 0;
+            for (const auto& g : b->gal) {
+                NB_BCUDA(b, cudaMemcpyAsync(pos_mass4 + 4 * dst, c->pos + g.off, g.n * 16, cudaMemcpyDeviceToHost, c->stream));
+                if (vel4)
+                    NB_BCUDA(b, cudaMemcpyAsync(vel4 + 4 * dst, c->vel + g.off, g.n * 16, cudaMemcpyDeviceToHost, c->stream));
+                dst += g.n;
+            }
         }
         NB_BCUDA(b, cudaStreamSynchronize(c->stream));
         return NB_OK;

@@ -63,6 +63,22 @@ __global__ void k_fill_tables(const int4* __restrict__ runs, int32_t* __restrict
     for (int i = threadIdx.x; i < r.y; i += blockDim.x) out[r.x + i] = r.z;
 }
 
+// ---- whole-batch state transfer ----------------------------------------------
+// The galaxies' bodies between the batch's arrays and one dense array in galaxy
+// order, a run of at most kMoveChunk bodies a block: run = (first body in the
+// arrays, first in the dense order, bodies, 0).  One copy each way then replaces
+// one a galaxy, about 2 us each: reading 200 small galaxies back took 790 us.
+constexpr int kMoveChunk = 2048;
+template <bool GATHER>
+__global__ void __launch_bounds__(256) k_move_state(const int4* __restrict__ runs, float4* __restrict__ state,
+                                                    float4* __restrict__ dense) {
+    const int4 r = runs[blockIdx.x];
+    for (int i = threadIdx.x; i < r.z; i += blockDim.x) {
+        if (GATHER) dense[r.y + i] = state[r.x + i];
+        else state[r.x + i] = dense[r.y + i];
+    }
+}
+
 // ---- bounding cube of each Barnes-Hut galaxy ------------------------------
 // Min/max are exact and order-free, so chunks of kBoxChunk bodies reduce in
 // parallel into per-galaxy words with atomics on an order-preserving integer

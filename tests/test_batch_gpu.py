@@ -302,3 +302,38 @@ def test_direct_members_match_fp64_at_row_and_chunk_edges(law, tune):
                 assert not F.any()
             else:
                 assert O.rel_l2(F, F64) < 5e-7, (pm.shape[0], O.rel_l2(F, F64))
+
+
+@pytest.mark.parametrize("count", [7, 8, 11])
+def test_whole_batch_transfer_of_few_and_many_galaxies(count):
+    """Below and from the number of galaxies that go through one dense copy:
+    what is written is read back, galaxy by galaxy and whole, and a batch
+    stepped from a written state equals one committed with it."""
+    sizes = [2, 257, 2048, 2049, 9000, 300, 8192, 5000, 1, 20001, 4097][:count]
+    a_gals = [nb.seed_plummer(70 + k, max(n, 2)) for k, n in enumerate(sizes)]
+    b_gals = [nb.seed_disk(90 + k, max(n, 3)) for k, n in enumerate(sizes)]
+    a_gals = [(p[:n].copy(), w[:n].copy()) for (p, w), n in zip(a_gals, sizes)]
+    b_gals = [(p[:n].copy(), w[:n].copy()) for (p, w), n in zip(b_gals, sizes)]
+    with make_batch(a_gals) as a, make_batch(b_gals) as b:
+        a.step(1e-3, 1)
+        pm = np.concatenate([p for p, _ in b_gals])
+        vel = np.concatenate([w for _, w in b_gals])
+        a.write_state(pm, vel)
+        rp, rv = np.empty_like(pm), np.empty_like(vel)
+        a.read_state(rp, rv)
+        np.testing.assert_array_equal(rp, pm)
+        np.testing.assert_array_equal(rv, vel)
+        a.step(1e-3, 2)
+        b.step(1e-3, 2)
+        a.read_state(rp, rv)
+        off = 0
+        for g, n in enumerate(sizes):
+            pa, va = a.read(g)
+            pb, vb = b.read(g)
+            np.testing.assert_array_equal(pa, pb)
+            np.testing.assert_array_equal(va, vb)
+            np.testing.assert_array_equal(rp[off:off + n], pa)
+            off += n
+        only_pos = np.empty_like(pm)
+        a.read_state(only_pos)
+        np.testing.assert_array_equal(only_pos, rp)
