@@ -825,14 +825,16 @@ int nb_diagnostics(nb_sim* s, float half_kick_dt, nb_diag* out) {
             int rc = force_pass(s, 0.f, false);   // acceleration at the current positions
             if (rc) return rc;
         }
-        double* d_o = nullptr;
-        double h[16] = {0};
-        NB_CUDA(s, cudaMallocAsync(&d_o, 16 * sizeof(double), s->stream));
+        // the result goes through the handle's kept staging: an allocation a call
+        // mapped and unmapped memory, about 100 us
+        double* d_o = static_cast<double*>(device_stage(s, 12 * sizeof(double)));
+        double* h = static_cast<double*>(host_stage(s, 12 * sizeof(double)));
+        if (!d_o || !h) return fail(s, NB_ENOMEM, "staging allocation failed");
         cudaError_t e = fp64_diagnostics_ex(s, half_kick_dt, half_kick_dt != 0.f, true, d_o);
         if (e == cudaSuccess) e = cudaMemcpyAsync(h, d_o, 12 * sizeof(double), cudaMemcpyDeviceToHost, s->stream);
-        cudaFreeAsync(d_o, s->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
         if (e != cudaSuccess) return cuda_fail(s, e, "nb_diagnostics");
+        const int rc = check_device_error(s);   // waits for the copies
+        if (rc == NB_ECUDA) return rc;
         out->kinetic = h[0];
         out->potential = h[11];
         out->total = h[0] + h[11];
@@ -840,7 +842,7 @@ int nb_diagnostics(nb_sim* s, float half_kick_dt, nb_diag* out) {
         out->angular_momentum[0] = h[4]; out->angular_momentum[1] = h[5]; out->angular_momentum[2] = h[6];
         out->mass = h[7];
         for (int k = 0; k < 3; ++k) out->centre_of_mass[k] = h[7] != 0.0 ? h[8 + k] / h[7] : 0.0;
-        return check_device_error(s);
+        return rc;
     } catch (...) {   // no exception crosses the C-ABI: host allocation failed
         return NB_ENOMEM;
     }

@@ -287,3 +287,26 @@ def test_each_pair_once_with_heavy_masses():
         F64 = s.fp64_forces(t)
     assert np.isfinite(F).all()
     assert O.rel_l2(F[t], F64) < 5e-7
+
+
+@pytest.mark.parametrize("law", [nb.LAW_REFERENCE, nb.LAW_PLUMMER])
+@pytest.mark.parametrize("n", [1, 2, 255, 257, 2048, 2049, 10241])
+def test_potential_counts_every_pair_once(n, law):
+    """At the edges of blocks and padding, with uneven masses and a coincident
+    pair.  A term carries a few units of 2^-24, 64 of them are summed in FP32:
+    1e-6 bounds the sum."""
+    pm, v = nb.seed_disk(61, max(n, 2))
+    pm, v = pm[:n].copy(), v[:n].copy()
+    pm[:, 3] *= np.random.default_rng(n).uniform(0.01, 2.0, n).astype(np.float32)
+    if n > 2:
+        pm[1, :3] = pm[n - 1, :3]
+    with direct_sim(law=law) as s:
+        s.init_soa(pm, v)
+        d = s.diagnostics()
+    x, m = pm[:, :3].astype(np.float64), pm[:, 3].astype(np.float64)
+    eps, U = 0.01, 0.0
+    for i in range(n - 1):
+        r = np.sqrt(((x[i + 1:] - x[i]) ** 2).sum(1))
+        U -= m[i] * (m[i + 1:] * (np.arctan2(eps, r) / eps if law == 0 else 1 / np.sqrt(r * r + eps * eps))).sum()
+    assert d["potential"] == pytest.approx(U, rel=1e-6, abs=0.0)
+    assert d["mass"] == pytest.approx(m.sum(), rel=1e-12)
