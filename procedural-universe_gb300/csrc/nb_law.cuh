@@ -100,6 +100,16 @@ __device__ __forceinline__ float2 pair_factor_x2(float2 dx, float2 dy, float2 dz
     return __fmul2_rn(inv, __fmul2_rn(inv, inv));
 }
 
+// kahan_add of two sums at once in packed instructions (the same roundings);
+// nc holds the negated compensations: the represented values are s + nc.
+__device__ __forceinline__ void kahan_add_x2(float2& s, float2& nc, float2 x) {
+    const float2 minus = make_float2(-1.f, -1.f);
+    const float2 y = __fadd2_rn(x, nc);
+    const float2 t = __fadd2_rn(s, y);
+    nc = __ffma2_rn(__ffma2_rn(s, minus, t), minus, y);   // y - (t - s), each product exact
+    s = t;
+}
+
 // Consecutive threads that fold one body's partials together.
 constexpr int kFoldLanes = 8;
 

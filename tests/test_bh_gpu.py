@@ -293,3 +293,26 @@ def test_launches_per_step():
         s.synchronize()
         nb.lib().nb_launch_count(s.handle, ctypes.byref(b))
     assert (b.value - a.value) / 3 <= 20
+
+
+@pytest.mark.parametrize("n", [63, 64, 65, 129, 4097, 48640, 48641, 81088, 81089])
+def test_shared_groups_decide_like_the_oracle(n):
+    """Sizes at which a traversal group is walked by four warps, by two or by
+    one, and at group edges, with a depth-cap bucket and bodies outside the
+    root: the oracle's forces, and its decisions (interaction count) where no
+    depth-cap bucket holds bodies that differ, which the two count apart."""
+    pm, v = nb.seed_collision(45, n)
+    pm[n // 3:n // 3 + 5, :3] = pm[7, :3]
+    pm[1, 0] = 5000.0
+    rec = nb.records_from_soa(pm, v)
+    t = O.OracleTree(rec)
+    with bh_sim(theta=0.6) as s:
+        s.init(rec)
+        F = s.compute_forces()
+        inter = s.last_interactions()
+        again = s.compute_forces()
+        deeper = s.tree_stats()["deeper_buckets"]
+    Fo, inter_o = t.forces(G=1.0, S=0.005 ** 2, theta=0.6)
+    assert inter == inter_o or deeper > 0
+    assert O.rel_l2(F, Fo) < 1e-5
+    np.testing.assert_array_equal(F, again)
