@@ -81,6 +81,7 @@ struct TreeBuffers {
     // host view of the last build
     int n_in = 0, n_int = 0, n_cells = 0, final_buf = 0;
     bool trivial = false;                    // < 2 bodies in the tree: all forces zero
+    bool curve = false;                      // bodies sorted along the Hilbert curve, not by octant path
 };
 
 // Tree counters (TreeBuffers::counters)
@@ -214,7 +215,9 @@ cudaError_t fp64_diagnostics_ex(nb_sim* sim, float half_dt, bool with_acc, bool 
 // ---- Barnes-Hut (nb_tree.cu, nb_traverse.cu) ----
 cudaError_t tree_reserve(nb_sim* sim);
 void tree_free(nb_sim* sim);
-cudaError_t tree_build(nb_sim* sim);
+// export_order: bodies sorted by their octant paths, as the nb_tree_* calls
+// export them (a force pass may sort them along the Hilbert curve: same tree).
+cudaError_t tree_build(nb_sim* sim, bool export_order = false);
 cudaError_t tree_forces(nb_sim* sim);
 cudaError_t tree_sizes(nb_sim* sim, int32_t* cells, int32_t* internal);
 float theta_float(double theta);   // smallest float >= theta

@@ -119,8 +119,8 @@ int tfail(nb_sim* s, int code, const std::string& msg) {
 
 int ensure_tree(nb_sim* s) {
     if (s->n == 0) return tfail(s, NB_EBADSTATE, "no particles");
-    if (!s->tree_valid) {
-        cudaError_t e = tree_build(s);
+    if (!s->tree_valid || s->tree.curve) {
+        cudaError_t e = tree_build(s, true);
         if (e != cudaSuccess) return tfail(s, NB_ECUDA, std::string("tree_build: ") + cudaGetErrorString(e));
     }
     return nb_synchronize(s);

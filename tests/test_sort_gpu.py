@@ -49,3 +49,20 @@ def test_keys_and_order(n, spread):
         np.testing.assert_array_equal(depth, want_depth)
         if (want_depth > 0).sum() >= 2:
             np.testing.assert_array_equal(s.tree_order(), np.argsort(want, kind="stable"))
+
+
+def test_exported_order_after_a_force_pass():
+    """A force pass sorts the bodies along the Hilbert curve; the exported
+    order, nodes and statistics are still those of the octant paths."""
+    pm, v = nb.seed_disk(5, 20000)
+    with nb.NBodySim(kind=nb.SIM_BARNES_HUT, theta=0.5) as s, nb.NBodySim(kind=nb.SIM_BARNES_HUT, theta=0.5) as t:
+        s.init_soa(pm, v)
+        t.init_soa(pm, v)
+        F = s.compute_forces()
+        nodes, order, stats = s.tree_nodes(), s.tree_order(), s.tree_stats()
+        np.testing.assert_array_equal(nodes, t.tree_nodes())
+        np.testing.assert_array_equal(order, t.tree_order())
+        assert stats == t.tree_stats()
+        keys, _ = s.tree_keys()
+        np.testing.assert_array_equal(order, np.argsort(keys, kind="stable"))
+        np.testing.assert_array_equal(F, s.compute_forces())
