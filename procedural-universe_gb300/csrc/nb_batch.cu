@@ -58,7 +58,7 @@ struct nb_batch {
     int32_t* slot_start = nullptr;
     int4* groups = nullptr;          // traversal groups, rebuilt on the device every step
     int group_cap = 0;
-    int* group_ctr = nullptr;        // [0] groups emitted, [1] next group to traverse
+    int* group_ctr = nullptr;        // GroupList's counters
     unsigned* box_bits = nullptr;    // 6 ordered words per galaxy: min xyz, max xyz
     CellRec* cell_rec = nullptr;    // per cell: centre of mass, walk record, quadrupole (nb_cellrec.cuh)
     size_t qcap = 0;
@@ -219,6 +219,7 @@ int enqueue_step(nb_batch* b, float dt, bool update, bool tree_only = false) {
         NB_BCUDA(b, tree_batch_keys(c, c->pos, b->body_slot, n, b->box_bits, b->nslot, b->gal_box));
         NB_BCUDA(b, tree_build_graph(c, c->pos, n, kBatchDepth, tree_only, b->cell_rec));
         if (tree_only) return NB_OK;
+        const GroupList groups{b->groups, b->group_cap, b->group_ctr};
         {
             PhaseScope ps(c, NB_PHASE_MASS, 3);
             k_batch_moments<<<(unsigned)((t.int_cap + 127) / 128), 128, 0, st>>>(
@@ -229,7 +230,7 @@ int enqueue_step(nb_batch* b, float dt, bool update, bool tree_only = false) {
                                                                  (int)t.cell_cap, b->gal_root, c->d_err);
             k_batch_groups<<<(unsigned)((t.int_cap + 255) / 256), 256, 0, st>>>(
                 (int)t.int_cap, t.counters, t.int_cell, b->cell_rec,
-                t.vals[0], b->body_slot, (int)t.cell_cap, n, b->groups, b->group_cap, b->group_ctr, c->d_err);
+                t.vals[0], b->body_slot, (int)t.cell_cap, n, groups, c->d_err);
         }
         {
             PhaseScope ps(c, NB_PHASE_TRAVERSE);
@@ -244,7 +245,7 @@ int enqueue_step(nb_batch* b, float dt, bool update, bool tree_only = false) {
             const int blocks = std::max(1, std::min(max_blocks, c->sm_count * std::max(1, occ)));
 #define NB_GT(L)                                                                                                  \
     k_group_traverse<L><<<blocks, kGWarps * 32, 0, st>>>(                                                         \
-        b->groups, b->group_ctr, b->group_cap, b->group_ctr + 1, t.spos, t.vals[0], b->cell_rec, b->gal_box,      \
+        groups, t.spos, t.vals[0], b->cell_rec, b->gal_box,                                                       \
         b->gal_root, b->nslot,                                                                                    \
         (int)t.cell_cap, n, (int)t.int_cap, b->tune.leaf_size, th * th, S, G, (float)(b->far_eta * b->far_eta),   \
         (float)(b->far_alpha / b->base.G), (float)(b->far_cap * b->far_cap),                                      \
@@ -685,7 +686,7 @@ int nb_batch_commit(nb_batch* b) {
             // groups are disjoint and non-empty: at most one per body
             b->group_cap = (int)b->n_bh;
             NB_BCUDA(b, dev_alloc(&b->groups, b->n_bh * sizeof(int4)));
-            NB_BCUDA(b, dev_alloc(&b->group_ctr, 2 * sizeof(int)));
+            NB_BCUDA(b, dev_alloc(&b->group_ctr, kGroupCounters * sizeof(int)));
         }
         b->h_pos.clear();
         b->h_vel.clear();
@@ -856,9 +857,9 @@ int nb_batch_tree_stats(nb_batch* b, int64_t* stats4) {
         int32_t h[TC_COUNT];
         int rc = read_tree_counts(b, h);
         if (rc) return rc;
-        int ctr[2] = {0, 0};
+        int ctr[kGroupCounters] = {};
         NB_BCUDA(b, cudaMemcpy(ctr, b->group_ctr, sizeof(ctr), cudaMemcpyDeviceToHost));
-        stats4[0] = ctr[0];
+        stats4[0] = ctr[0] + ctr[2];
         stats4[1] = h[TC_NINT];
         stats4[2] = (int64_t)h[TC_NINT] + h[TC_NLEAF];
         stats4[3] = (int64_t)b->n_bh;

@@ -3,16 +3,16 @@
 // Many independent galaxies are stepped together, one launch per phase:
 //  * Barnes-Hut members (n >= threshold) are stored first, contiguously.  Each
 //    gets a tight bounding cube; a body's key is its galaxy slot (21 bits, the
-//    top 7 octal levels) followed by a 42-bit Morton code in its cube (14
-//    levels), so ONE radix sort and ONE topology build make a forest whose
+//    top 7 octal levels) followed by a 42-bit code of its octants in its cube
+//    (14 levels, sorted in Hilbert order), so ONE radix sort and ONE topology build make a forest whose
 //    level-7 nodes are the galaxy roots.
 //  * The mass pass adds traceless quadrupole moments (parallel-axis rule
 //    bottom-up); a cell's centre of mass, walk record and quadrupole form one
 //    64-byte record (nb_cellrec.cuh).  Traversal groups are
-//    taken from the tree itself: the largest subtrees of at most kGroupMax
-//    bodies whose cell is at most 1/16 of the galaxy cube, consecutive small
-//    siblings packed together, oversized depth-cap buckets cut into chunks --
-//    so a group is spatially compact and its bounding box small.  A warp
+//    taken from the tree itself: runs of at most kGroupMax bodies of the
+//    largest subtrees of at most kGroupCut bodies whose cell is at most 1/16
+//    of the galaxy cube, the bodies in Hilbert order -- so a group is
+//    spatially compact and its bounding box small.  A warp
 //    takes groups from a device queue (two bodies per lane; one for groups of
 //    at most 32 bodies, so that half-empty warps do no idle work), opens a
 //    cell when the cell side exceeds theta times the distance from the cell's
@@ -38,7 +38,9 @@ namespace nb {
 
 constexpr int kGWarps = 4;              // warps per traversal block
 constexpr int kGroupMax = 64;           // bodies per traversal group (two per lane)
-constexpr int kGroupMinDepth = 4;       // a group cell lies >= 4 levels below its galaxy root
+constexpr int kGroupCut = 512;          // most bodies of a cell that is cut into groups
+constexpr int kGroupMinDepth = 4;       // such a cell lies >= 4 levels below its galaxy root
+constexpr int kGroupFirstDepth = 7;     // groups of cells up to this depth are walked first
 constexpr int kBoxChunk = 2048;         // bodies per block of the bounding-box pass (8 a thread)
 constexpr int kGStack = 512;            // cells waiting to be opened, per warp (<= 32 pushed per step)
 constexpr int kStackCellLimit = 1 << 27;   // a stack entry packs a first-child index below this with 4 bits
@@ -96,7 +98,7 @@ __global__ void k_gal_box_init(unsigned* __restrict__ bits, int nslot, int32_t* 
     for (int j = i; j < counter_words; j += gridDim.x * blockDim.x) counters[j] = j == TC_NIN ? n_in : 0;
     if (i == 0) {
         *interactions = 0ull;
-        group_ctr[0] = group_ctr[1] = 0;
+        group_ctr[0] = group_ctr[1] = group_ctr[2] = 0;
         if (next_unit) *next_unit = 0;
     }
 }
@@ -284,42 +286,74 @@ __global__ void k_batch_roots(const int32_t* __restrict__ slot_start, int nslot,
 }
 
 // ---- traversal groups from the tree --------------------------------------------
-// One thread per internal node at or below the galaxy roots.  A node that
-// cannot be a group itself emits its children that can (packing consecutive
-// ones, children being contiguous in sorted order, when the node is deep
-// enough), emits a body that sits high in the tree on its own and cuts a
-// larger depth-cap bucket into chunks; internal children that cannot be
-// groups are handled by their own threads.  Every body lands in exactly one
-// group: the first groupable cell on its path from the galaxy root, or its
-// leaf.
-__device__ __forceinline__ void emit_group(int first, int count, const int32_t* sorder, const int32_t* body_slot,
-                                           int nbodies, int4* groups, int cap, int* n_groups, int* err) {
+// One thread per internal node at or below the galaxy roots.  A cell of at most
+// kGroupCut bodies that lies deep enough (groupable) is cut into runs of at most
+// kGroupMax bodies of nearly equal length, which are compact because bodies are
+// sorted along the Hilbert curve; groupable children that follow one another on
+// the curve are cut together when their parent is deep enough.  A node that is
+// not groupable handles its groupable children, emits a body that sits high in
+// the tree on its own and cuts a larger depth-cap bucket; its other children are
+// handled by their own threads.  Every body lands in exactly one group: a run of
+// the first groupable cell on its path from the galaxy root, or its leaf.
+// Before, a group was a whole cell of at most 64 bodies or consecutive siblings
+// packed to 64 in Morton order, which left 33% of the traversal's slots empty at
+// 1M bodies (14% now): a step 3.34 -> 2.95 ms there, 1.25 -> 1.14 ms at 300,000.
+// The group boxes are no larger, and the force error falls (2.6e-4 -> 2.5e-4 and,
+// with the relative far field, 5.4e-4 -> 4.9e-4 at 1M).
+// Groups of the cells up to kGroupFirstDepth levels below their galaxy's root go
+// to the front of the list and are walked first, the others fill it from the
+// back: the longest walks are those of wide groups next to a dense region, and
+// one that starts last holds the whole launch.
+struct GroupList {
+    int4* list;
+    int cap;
+    int* ctr;   // [0] groups at the front, [1] next group to walk, [2] groups at the back
+};
+constexpr int kGroupCounters = 3;
+
+__device__ __forceinline__ void emit_group(int first, int count, bool front, const int32_t* sorder,
+                                           const int32_t* body_slot, int nbodies, const GroupList& g, int* err) {
     if (count <= 0) return;
     if (first < 0 || first + count > nbodies) {
         record_error(err, DEV_TREE_OVERFLOW);
         return;
     }
-    const int idx = atomicAdd(n_groups, 1);
-    if (idx >= cap) {
+    const int idx = atomicAdd(&g.ctr[front ? 0 : 2], 1);
+    if (idx >= g.cap) {   // groups are disjoint and not empty: at most one a body
         record_error(err, DEV_TREE_OVERFLOW);
         return;
     }
-    groups[idx] = make_int4(body_slot[sorder[first]], first, count, 0);
+    g.list[front ? idx : g.cap - 1 - idx] = make_int4(body_slot[sorder[first]], first, count, 0);
 }
 
-// A cell can be a group when it holds at most kGroupMax bodies and lies at
-// least kGroupMinDepth levels below its galaxy's root (side <= cube / 16): a
-// few bodies spread over a large, sparse cell would give one group a box the
-// size of the galaxy and a list of ~10^5 entries (a tail that held one warp
-// for milliseconds); such cells are split further instead.
+// A cell can be cut into groups when it lies at least kGroupMinDepth levels below
+// its galaxy's root (side <= cube / 16): a few bodies spread over a large,
+// sparse cell would give one group a box the size of the galaxy and a list of
+// ~10^5 entries (a tail that held one warp for milliseconds); such cells are
+// split further instead.  For the same reason a cell at that depth is cut only
+// when it makes one group, and twice as many bodies are allowed every two levels
+// deeper, up to kGroupCut (doubling at every level left long walks at the end:
+// 1.29 ms a step at 300,000 bodies; up to 512 everywhere 1.67 ms).
 __device__ __forceinline__ bool groupable(int level, int count) {
-    return count <= kGroupMax && level >= kSlotLevels + kGroupMinDepth;
+    const int depth = level - kSlotLevels - kGroupMinDepth;
+    return depth >= 0 && count <= min(kGroupCut, kGroupMax << min(depth / 2, 8));
 }
 
-__global__ void k_batch_groups(int int_cap, const int32_t* __restrict__ counters, const int32_t* __restrict__ int_cell,
-                               const CellRec* __restrict__ rec, const int32_t* __restrict__ sorder,
-                               const int32_t* __restrict__ body_slot, int n_cells, int nbodies,
-                               int4* __restrict__ groups, int cap, int* __restrict__ n_groups, int* __restrict__ err) {
+__device__ __forceinline__ void emit_runs(int first, int count, bool front, const int32_t* sorder,
+                                          const int32_t* body_slot, int nbodies, const GroupList& g, int* err) {
+    const int runs = (count + kGroupMax - 1) / kGroupMax;
+    for (int r = 0; r < runs; ++r) {
+        const int o = (int)((long long)count * r / runs), e = (int)((long long)count * (r + 1) / runs);
+        emit_group(first + o, e - o, front, sorder, body_slot, nbodies, g, err);
+    }
+}
+
+__global__ void __launch_bounds__(256) k_batch_groups(int int_cap, const int32_t* __restrict__ counters,
+                                                      const int32_t* __restrict__ int_cell,
+                                                      const CellRec* __restrict__ rec,
+                                                      const int32_t* __restrict__ sorder,
+                                                      const int32_t* __restrict__ body_slot, int n_cells, int nbodies,
+                                                      GroupList groups, int* __restrict__ err) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     // a held step emits no groups, so the traversal after it has no work
     if (!tree_fits(counters, int_cap, n_cells)) return;
@@ -333,43 +367,56 @@ __global__ void k_batch_groups(int int_cap, const int32_t* __restrict__ counters
     const int level = wr.w >> 8;
     const int cnt = wr.y;
     if (level < kSlotLevels) return;
-    if (groupable(level, cnt)) return;   // its parent groups it
+    if (groupable(level, cnt)) return;   // its parent cuts it
     const int F = wr.x, nch = (wr.w >> 4) & 15;
     if (F < 1 || nch > 8 || F + nch > n_cells) {
         record_error(err, DEV_TREE_OVERFLOW);
         return;
     }
-    // siblings are packed only below a cell small enough to be a group itself
+    // children are cut together only below a cell small enough itself
     const bool pack = level >= kSlotLevels + kGroupMinDepth;
-    int run_first = -1, run_cnt = 0;
-    for (int j = 0; j < nch; ++j) {
-        const int ch = F + j;
-        const int4 cw = rec[ch].walk;
-        const int kind = cw.w & 15;
-        const int cc = cw.y;
-        const int cf = cw.z;
-        if (!groupable(cw.w >> 8, cc)) {
-            emit_group(run_first, run_cnt, sorder, body_slot, nbodies, groups, cap, n_groups, err);
-            run_first = -1;
-            run_cnt = 0;
-            if (kind != BK_INTERNAL)   // a body high in the tree, or an oversized depth-cap bucket
-                for (int o = 0; o < cc; o += kGroupMax)
-                    emit_group(cf + o, min(kGroupMax, cc - o), sorder, body_slot, nbodies, groups, cap, n_groups, err);
-            continue;                  // an internal child groups its own children
+    const bool front = level < kSlotLevels + kGroupFirstDepth;   // the children's level is one more
+    int first[8], count[8], kind[8];
+    bool can[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        first[j] = 0x7fffffff;
+        count[j] = kind[j] = 0;
+        can[j] = false;
+        if (j < nch) {
+            const int4 cw = rec[F + j].walk;
+            kind[j] = cw.w & 15;
+            count[j] = cw.y;
+            first[j] = cw.z;
+            can[j] = groupable(cw.w >> 8, cw.y);
         }
-        if (!pack) {
-            emit_group(cf, cc, sorder, body_slot, nbodies, groups, cap, n_groups, err);
+    }
+    int run_first = -1, run_cnt = 0, last = -1;
+    for (int it = 0; it < nch; ++it) {   // the children along the curve
+        int cf = 0x7fffffff, cc = 0, ck = 0;
+        bool cg = false;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (first[j] > last && first[j] < cf) {
+                cf = first[j];
+                cc = count[j];
+                ck = kind[j];
+                cg = can[j];
+            }
+        last = cf;
+        if (cg && pack) {
+            if (run_first < 0) run_first = cf;
+            run_cnt += cc;
             continue;
         }
-        if (run_cnt + cc > kGroupMax) {
-            emit_group(run_first, run_cnt, sorder, body_slot, nbodies, groups, cap, n_groups, err);
-            run_first = -1;
-            run_cnt = 0;
-        }
-        if (run_first < 0) run_first = cf;
-        run_cnt += cc;
+        if (run_cnt) emit_runs(run_first, run_cnt, front, sorder, body_slot, nbodies, groups, err);
+        run_first = -1;
+        run_cnt = 0;
+        // a groupable child of a cell high in the tree, a body high in the tree or a
+        // larger depth-cap bucket; another internal child cuts its own children
+        if (cg || ck != BK_INTERNAL) emit_runs(cf, cc, front, sorder, body_slot, nbodies, groups, err);
     }
-    emit_group(run_first, run_cnt, sorder, body_slot, nbodies, groups, cap, n_groups, err);
+    if (run_cnt) emit_runs(run_first, run_cnt, front, sorder, body_slot, nbodies, groups, err);
 }
 
 // Interactions of one target (negated coordinates duplicated in both halves
@@ -546,7 +593,7 @@ __device__ __forceinline__ void far_eval(const FarField& f, float x, float y, fl
 // Persistent: each warp takes groups from the queue until it is empty.
 template <int LAW>
 __global__ void __launch_bounds__(kGWarps * 32, 5) k_group_traverse(
-    const int4* __restrict__ groups, const int* __restrict__ n_groups_dev, int group_cap, int* __restrict__ next_group,
+    GroupList groups,
     const float4* __restrict__ spos, const int32_t* __restrict__ sorder, const CellRec* __restrict__ rec,
     const float4* __restrict__ gal_box, const int32_t* __restrict__ gal_root, int nslot, int n_cells, int nbodies,
     int max_pops, int leaf_size, float theta2, float S, float G, float far2, float far_rel, float far_cap2,
@@ -560,17 +607,17 @@ __global__ void __launch_bounds__(kGWarps * 32, 5) k_group_traverse(
     __shared__ int rinc[kGWarps][32], rfst[kGWarps][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
-    const int ngroups = min(*n_groups_dev, group_cap);
     const float2 S2 = make_float2(S, S);
     const float tiny = self_pair_tiny(mmax);   // a leaf's bodies include the target itself
     const float2 T2 = make_float2(tiny, tiny);
     unsigned long long total = 0;
     for (;;) {
     int gi = 0;
-    if (lane == 0) gi = atomicAdd(next_group, 1);
+    if (lane == 0) gi = atomicAdd(&groups.ctr[1], 1);
     gi = __shfl_sync(0xffffffffu, gi, 0);
-    if (gi >= ngroups) break;
-    const int4 grp = groups[gi];   // (slot, first sorted position, count, 0)
+    const int nfront = min(groups.ctr[0], groups.cap);   // read again for each group: two registers less
+    if (gi >= nfront + min(groups.ctr[2], groups.cap - nfront)) break;
+    const int4 grp = groups.list[gi < nfront ? gi : groups.cap - 1 - (gi - nfront)];   // (slot, first sorted position, count, 0)
     if (grp.x < 0 || grp.x >= nslot || grp.y < 0 || grp.z < 1 || grp.z > kGroupMax || grp.y + grp.z > nbodies) {
         if (lane == 0) record_error(err, DEV_TREE_OVERFLOW);
         continue;

@@ -1,7 +1,7 @@
 // nb_hilbert.cuh -- octant paths in Hilbert order (shared by the octree's keys
 // and the gather after their sort).
 //
-// The plain traversal walks the tree for 64 bodies that are consecutive in the
+// The traversals walk the tree for up to 64 bodies that are consecutive in the
 // sorted order.  In Morton order a run of 64 often jumps between cells that do
 // not touch, which widens its bounding box; along the Hilbert curve consecutive
 // cells share a face.  The map below rewrites a path of 3-bit octants digit by
@@ -63,9 +63,10 @@ __device__ __forceinline__ void load_hilbert(uint32_t* sh, bool inverse) {
         sh[threadIdx.x] = inverse ? c_hilbert.inverse[threadIdx.x] : c_hilbert.forward[threadIdx.x];
 }
 
-// Rewrites the D digits of a path by the table.
+// Rewrites the last D digits of a path by the table, the ones before them as
+// they are (the batched forest's galaxy slot).
 __device__ __forceinline__ uint64_t hilbert_map(uint64_t path, int D, const uint32_t* table) {
-    uint64_t out = 0;
+    uint64_t out = path >> (3 * D);
     uint32_t state = 0;
     for (int shift = 3 * (D - 1); shift >= 0; shift -= 3) {
         const uint32_t l = (uint32_t)(path >> shift) & 7u;

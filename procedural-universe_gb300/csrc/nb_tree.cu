@@ -459,13 +459,14 @@ __device__ void node_bounds(uint64_t code, int level, float half, float3& lo, fl
 }
 
 // Positions in sorted order; brings the sort result to buffer 0 when the
-// device plan left it in buffer 1 (no host read of the plan).  With curve, keys
-// that were sorted along the Hilbert curve become octant paths again.
+// device plan left it in buffer 1 (no host read of the plan).  With curve, the
+// last `curve` digits of the keys, sorted along the Hilbert curve, become octants
+// again.
 __global__ void __launch_bounds__(256) k_gather_final(const float4* __restrict__ pos, uint64_t* __restrict__ k0,
                                                       const uint64_t* __restrict__ k1, int32_t* __restrict__ v0,
                                                       const int32_t* __restrict__ v1, int n,
                                                       const int32_t* __restrict__ plan, float4* __restrict__ spos,
-                                                      bool curve, int D) {
+                                                      int curve) {
     __shared__ uint32_t table[2 * kHilbertStates];
     if (curve) {   // uniform
         load_hilbert(table, true);
@@ -477,7 +478,7 @@ __global__ void __launch_bounds__(256) k_gather_final(const float4* __restrict__
     const int v = from1 ? v1[s] : v0[s];
     if (curve) {
         const uint64_t key = from1 ? k1[s] : k0[s];
-        k0[s] = key == ~0ull ? key : hilbert_map(key, D, table);
+        k0[s] = key == ~0ull ? key : hilbert_map(key, curve, table);
     } else if (from1) {
         k0[s] = k1[s];
     }
@@ -936,7 +937,8 @@ __global__ void __launch_bounds__(128) k_mass(int n_int, const int32_t* __restri
 }
 
 // ------------------------------------------------- batched forest keys ----
-// Keys of the batched form's Barnes-Hut bodies [0, n) (nb_morton.cuh), with
+// Keys of the batched form's Barnes-Hut bodies [0, n) (nb_morton.cuh, the
+// position's digits in Hilbert order), with
 // the radix sort's histograms and the look-back status cleared,
 // kSortThreads * items keys a block; the first threads also write each galaxy's cube for the
 // traversal.  Pad entries [n, tiles * kSortTile) get key ~0.
@@ -945,6 +947,7 @@ __global__ void __launch_bounds__(kSortThreads) k_batch_keys_hist(
     int nslot, float4* __restrict__ gal_box, uint64_t* __restrict__ keys, int32_t* __restrict__ vals,
     int32_t* __restrict__ depth, uint32_t* __restrict__ ghist, unsigned long long* __restrict__ sort_status,
     int ntiles, unsigned long long* __restrict__ pos_status, int items, int key_blocks) {
+    __shared__ uint32_t table[2 * kHilbertStates];
     __shared__ uint32_t h[kPasses][256];
     __shared__ unsigned long long sh_groups[2 * kKeyGroups];
     const int g = blockIdx.x * kSortThreads + threadIdx.x;
@@ -952,6 +955,7 @@ __global__ void __launch_bounds__(kSortThreads) k_batch_keys_hist(
     if ((int)blockIdx.x >= key_blocks) return;   // blocks past the keys only write galaxy cubes (block-uniform)
     for (int i = threadIdx.x; i < kPasses * 256; i += kSortThreads) (&h[0][0])[i] = 0;
     if (threadIdx.x < 2 * kKeyGroups) sh_groups[threadIdx.x] = 0ull;
+    load_hilbert(table, false);
     zero_tile_status(sort_status, ntiles, pos_status, key_blocks);
     __syncthreads();
     for (int it = 0; it < items; ++it) {
@@ -960,7 +964,7 @@ __global__ void __launch_bounds__(kSortThreads) k_batch_keys_hist(
         uint64_t key = ~0ull;
         if (i < n) {
             const int slot = body_slot[i];
-            key = forest_key(pos[i], slot, gal_cube(box_bits, slot));
+            key = hilbert_map(forest_key(pos[i], slot, gal_cube(box_bits, slot)), kMortonLevels, table);
             depth[i] = kBatchDepth;
         }
         keys[i] = key;
@@ -1138,7 +1142,7 @@ cudaError_t tree_build(nb_sim* sim, bool export_order) {
     {
         PhaseScope ps(sim, NB_PHASE_TOPOLOGY, 2);
         k_gather_final<<<(n + 255) / 256, 256, 0, st>>>(sim->pos, t.keys[0], t.keys[1], t.vals[0], t.vals[1], n,
-                                                        t.plan, t.spos, curve, sim->prm.max_depth);
+                                                        t.plan, t.spos, curve ? sim->prm.max_depth : 0);
         t.final_buf = 0;
         TopoView tv = topo_view(sim);
         k_positions_scan<<<ntiles, kPosThreads, 0, st>>>(tv, t.spos, t.pos_nint, t.leaf_level, t.leaf_count,
@@ -1262,7 +1266,7 @@ cudaError_t tree_build_graph(nb_sim* sim, const float4* pos, int n, int D, bool 
     const int ptiles = (icap + kSortTile - 1) / kSortTile;
     PhaseScope ps(sim, NB_PHASE_TOPOLOGY, 6);
     k_gather_final<<<(n + 255) / 256, 256, 0, st>>>(pos, t.keys[0], t.keys[1], t.vals[0], t.vals[1], n, t.plan,
-                                                    t.spos, false, D);
+                                                    t.spos, kMortonLevels);
     // this scan also clears the internal-node hash table for the emission
     k_positions_scan<<<ntiles, kPosThreads, 0, st>>>(tv, t.spos, t.pos_nint, t.leaf_level, t.leaf_count, t.counters,
                                                       t.pos_status, ntiles, counts_only ? nullptr : t.hkeys,
