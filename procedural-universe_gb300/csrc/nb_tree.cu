@@ -15,7 +15,8 @@
 //  * K3: stable LSD radix sort of (key, body) pairs, 8 passes of 8 bits, one
 //    launch per pass: the digit histograms of all passes come with the keys,
 //    and each pass ranks, finds its tile's offsets by decoupled look-back and
-//    scatters in one kernel (the scatter ranks digits with warp match_any).
+//    scatters in one kernel (digits are ranked by warp ballots); small states
+//    are sorted whole by one block.
 //    Passes whose digit is the same for every key are skipped on the device.
 //  * K4: the reference tree splits a node when a second body arrives and
 //    creates all 8 children, so its internal nodes are exactly the key
@@ -49,7 +50,6 @@
 namespace nb {
 
 constexpr int kSortThreads = 256;
-constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kSortItems = 16;
 constexpr int kSortTile = kSortThreads * kSortItems;   // 4096 keys per tile
 // a radix pass ranks a tile with more threads and fewer keys each (more warps
@@ -289,10 +289,78 @@ __global__ void __launch_bounds__(256) k_sort_plan(const uint32_t* __restrict__ 
     }
 }
 
+// The lanes of the warp that hold the same 8-bit digit: eight ballots.  (One
+// __match_any_sync goes through the warp's distinct values one by one: a pass
+// over one tile of random digits took 13 us with it, 6.5 us over equal ones.)
+__device__ __forceinline__ uint32_t same_digit(uint32_t d) {
+    uint32_t peers = 0xffffffffu;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const bool set = (d >> b) & 1u;
+        const uint32_t m = __ballot_sync(0xffffffffu, set);
+        peers &= set ? m : ~m;
+    }
+    return peers;
+}
+
+// Stable ranks of a warp's keys (in the order it, lane) among its keys of the
+// same digit, each given to put(item, rank); hist (zero before) receives the warp's digit counts.
+template <int ITEMS, class Put>
+__device__ __forceinline__ void rank_keys(const uint64_t (&k)[ITEMS], int shift, uint16_t* hist, Put put) {
+    const uint32_t lt = lanemask_lt();
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int it = 0; it < ITEMS; ++it) {
+        const uint32_t d = (uint32_t)(k[it] >> shift) & 255u;
+        const uint32_t peers = same_digit(d);
+        const uint32_t b = hist[d];
+        put(it, b + __popc(peers & lt));
+        __syncwarp();
+        if (lane == 31 - __clz(peers)) hist[d] = (uint16_t)(b + __popc(peers));
+        __syncwarp();
+    }
+}
+
+// Turns the warps' digit counts into each warp's first place among the block's
+// keys of the digit; returns, in threads 0..255, the block's keys of digit
+// threadIdx.x.  Every thread of the block calls it: a warp takes 32 digits of
+// WARPS / SHARE rows (no bank conflicts), SHARE warps a digit.
+template <int THREADS>
+__device__ __forceinline__ uint32_t warp_places(uint16_t (*whist)[256], uint32_t (*count)[256]) {
+    constexpr int WARPS = THREADS / 32, SHARE = THREADS / 256, EACH = WARPS / SHARE;
+    const int d = threadIdx.x & 255, q = threadIdx.x >> 8;
+    uint32_t c[EACH], sum = 0;
+#pragma unroll
+    for (int w = 0; w < EACH; ++w) {
+        c[w] = whist[q * EACH + w][d];
+        sum += c[w];
+    }
+    count[q][d] = sum;
+    __syncthreads();
+    uint32_t run = 0, all = 0;
+#pragma unroll
+    for (int o = 0; o < SHARE; ++o) {
+        const uint32_t t = count[o][d];
+        all += t;
+        if (o < q) run += t;
+    }
+#pragma unroll
+    for (int w = 0; w < EACH; ++w) {
+        whist[q * EACH + w][d] = (uint16_t)run;
+        run += c[w];
+    }
+    return threadIdx.x < 256 ? all : 0u;
+}
+
 // One pass of the stable LSD sort in one launch (the one-sweep scheme,
 // Adinets and Merrill 2022): a tile ranks its keys by the pass's digit
-// (warp match_any, warps in order: stable), publishes its digit counts and
-// finds where earlier tiles put theirs by decoupled look-back, then scatters.
+// (warps in order: stable), publishes its digit counts and finds where earlier
+// tiles put theirs by decoupled look-back.  The keys, then the indices, go
+// through shared memory in the tile's order, so that neighbouring threads
+// write neighbouring words: the sort of 2^20 keys took 141 us with match_any
+// and a direct scatter, takes 119 (eight passes at 24 bytes a key: 28 us of
+// copying; the rest is the latency of load, rank, look-back and scatter in
+// about one wave of tiles).
 __global__ void __launch_bounds__(kPassThreads, 2) k_sort_pass(uint64_t* __restrict__ k0, uint64_t* __restrict__ k1,
                                                             int32_t* __restrict__ v0, int32_t* __restrict__ v1,
                                                             int ntiles, const int32_t* __restrict__ plan, int pass,
@@ -305,13 +373,13 @@ __global__ void __launch_bounds__(kPassThreads, 2) k_sort_pass(uint64_t* __restr
     uint64_t* kd = src ? k0 : k1;
     const int32_t* vs = src ? v1 : v0;
     int32_t* vd = src ? v0 : v1;
-    __shared__ uint32_t whist[kPassWarps][256];
-    __shared__ int32_t gbase[256];
-    __shared__ int sh_tile;
+    __shared__ __align__(16) uint64_t stage[kSortTile];
+    __shared__ __align__(16) uint16_t whist[kPassWarps][256];
+    __shared__ uint32_t count[kPassThreads / 256][256];
+    __shared__ int32_t start[256], shift_to[256];   // the tile's first key of a digit; its place less that
+    __shared__ int sh_warp[33], sh_tile;
     const int tile = lb_tile_index(tile_ctr, &sh_tile);
     if (tile >= ntiles) return;   // cannot happen with one block per tile; kept as a guard
-    for (int i = threadIdx.x; i < kPassWarps * 256; i += kPassThreads) (&whist[0][0])[i] = 0;
-    __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int shift = 8 * pass;
     const int base = tile * kSortTile + warp * (32 * kPassItems) + lane;
@@ -323,46 +391,134 @@ __global__ void __launch_bounds__(kPassThreads, 2) k_sort_pass(uint64_t* __restr
         k[it] = ks[base + it * 32];
         v[it] = vs[base + it * 32];
     }
-    const uint32_t lt = lanemask_lt();
-#pragma unroll
-    for (int it = 0; it < kPassItems; ++it) {
-        const uint32_t d = (uint32_t)(k[it] >> shift) & 255u;
-        const uint32_t peers = __match_any_sync(0xffffffffu, d);
-        const uint32_t b = whist[warp][d];
-        r[it] = b + __popc(peers & lt);
-        __syncwarp();
-        if (lane == 31 - __clz(peers)) whist[warp][d] = b + __popc(peers);
-        __syncwarp();
-    }
+    for (int i = threadIdx.x; i < kPassWarps * 256 / 8; i += kPassThreads)
+        reinterpret_cast<uint4*>(&whist[0][0])[i] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
+    rank_keys<kPassItems>(k, shift, whist[warp], [&](int it, uint32_t rank) { r[it] = rank; });
+    __syncthreads();
+    const uint32_t mine = warp_places<kPassThreads>(whist, count);
+    uint32_t excl = 0;
     if (threadIdx.x < 256) {   // one thread per digit
         const int d = threadIdx.x;
-        uint32_t run = 0;
-#pragma unroll
-        for (int w = 0; w < kPassWarps; ++w) {
-            const uint32_t c = whist[w][d];
-            whist[w][d] = run;
-            run += c;
-        }
         unsigned long long* st = status + (size_t)tile * 256 + d;
-        uint32_t excl = 0;
         if (tile == 0) {
-            lb_publish(st, 2u, run);
+            lb_publish(st, 2u, mine);
         } else {
-            lb_publish(st, 1u, run);
+            lb_publish(st, 1u, mine);
             excl = lb_exclusive(status + d, tile, 256, err);
-            lb_publish(st, 2u, excl + run);
+            lb_publish(st, 2u, excl + mine);
         }
-        gbase[d] = dig_off[pass * 256 + d] + (int)excl;
+    }
+    int total;
+    const int first = block_excl_scan((int)mine, sh_warp, &total);   // threads past the digits add nothing
+    if (threadIdx.x < 256) {
+        start[threadIdx.x] = first;
+        shift_to[threadIdx.x] = dig_off[pass * 256 + threadIdx.x] + (int)excl - first;
     }
     __syncthreads();
+    int place[kPassItems];
 #pragma unroll
     for (int it = 0; it < kPassItems; ++it) {
         const uint32_t d = (uint32_t)(k[it] >> shift) & 255u;
-        const int dst = gbase[d] + (int)whist[warp][d] + (int)r[it];
-        kd[dst] = k[it];
-        vd[dst] = v[it];
+        place[it] = start[d] + (int)whist[warp][d] + (int)r[it];
+        stage[place[it]] = k[it];
     }
+    __syncthreads();
+    int dst[kPassItems];
+#pragma unroll
+    for (int it = 0; it < kPassItems; ++it) {
+        const int j = it * kPassThreads + threadIdx.x;
+        const uint64_t key = stage[j];
+        dst[it] = shift_to[(uint32_t)(key >> shift) & 255u] + j;
+        kd[dst[it]] = key;
+    }
+    __syncthreads();
+    int32_t* vstage = reinterpret_cast<int32_t*>(stage);
+#pragma unroll
+    for (int it = 0; it < kPassItems; ++it) vstage[place[it]] = v[it];
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < kPassItems; ++it) vd[dst[it]] = vstage[it * kPassThreads + threadIdx.x];
+}
+
+// The whole sort of at most 1024 * ITEMS keys in one block: every pass ranks
+// the keys in registers and reorders them in shared memory, where the plan and
+// one launch per pass cost 58 to 70 us however few the keys: 27 to 35 us for
+// 4000 keys, 46 for 7000 (58).  Three tiles (12 keys a thread, which spill)
+// took 78 against 66 and four 98 against 63: those stay with the passes.  The
+// keys end in buffer 0.
+constexpr int kOneThreads = 1024, kOneWarps = kOneThreads / 32;
+template <int ITEMS>
+constexpr size_t one_block_bytes() {
+    return (size_t)kOneThreads * ITEMS * 10 + (size_t)kOneWarps * 256 * 2;
+}
+template <int ITEMS>
+__global__ void __launch_bounds__(kOneThreads) k_sort_block(uint64_t* __restrict__ keys, int32_t* __restrict__ vals,
+                                                            const uint32_t* __restrict__ ghist,
+                                                            int32_t* __restrict__ plan) {
+    constexpr int N = kOneThreads * ITEMS;
+    extern __shared__ __align__(16) unsigned char sm[];
+    uint64_t* sk = reinterpret_cast<uint64_t*>(sm);
+    uint16_t* sv = reinterpret_cast<uint16_t*>(sk + N);
+    uint16_t (*whist)[256] = reinterpret_cast<uint16_t (*)[256]>(sv + N);
+    __shared__ uint32_t count[kOneThreads / 256][256];
+    __shared__ int32_t start[256];
+    __shared__ int sh_warp[33], triv[kPasses];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int base = warp * (32 * ITEMS) + lane;
+    if (warp < kPasses) {   // the passes to skip, as in k_sort_plan
+        const uint4* bins = reinterpret_cast<const uint4*>(ghist + warp * 256) + 2 * lane;
+        const uint4 a = bins[0], b = bins[1];
+        const unsigned long long* gb = group_bits(const_cast<uint32_t*>(ghist));
+        const unsigned long long v = lane < kKeyGroups ? gb[lane] & gb[kKeyGroups + lane] : 0ull;
+        const unsigned long long var = ((unsigned long long)__reduce_or_sync(0xffffffffu, (uint32_t)(v >> 32)) << 32) |
+                                       __reduce_or_sync(0xffffffffu, (uint32_t)v);
+        const uint32_t n = (uint32_t)N;
+        const bool all = a.x == n || a.y == n || a.z == n || a.w == n || b.x == n || b.y == n || b.z == n || b.w == n;
+        const bool one = __any_sync(0xffffffffu, all);
+        if (lane == 0) triv[warp] = one || (warp < kPasses - 1 && ((var >> (8 * warp)) & 255ull) == 0ull);
+    }
+    uint64_t k[ITEMS];
+    uint32_t rv[ITEMS];   // a key's index (low half: at most 2^14) and its rank
+#pragma unroll
+    for (int it = 0; it < ITEMS; ++it) {
+        k[it] = keys[base + it * 32];
+        rv[it] = (uint32_t)(base + it * 32);   // the keys come in input order
+    }
+    __syncthreads();
+    for (int pass = 0; pass < kPasses; ++pass) {
+        if (triv[pass]) continue;   // block-uniform
+        const int shift = 8 * pass;
+        for (int i = threadIdx.x; i < kOneWarps * 256 / 8; i += kOneThreads)
+            reinterpret_cast<uint4*>(&whist[0][0])[i] = make_uint4(0u, 0u, 0u, 0u);
+        __syncthreads();
+        rank_keys<ITEMS>(k, shift, whist[warp], [&](int it, uint32_t r) { rv[it] |= r << 16; });
+        __syncthreads();
+        const uint32_t mine = warp_places<kOneThreads>(whist, count);
+        int total;
+        const int first = block_excl_scan((int)mine, sh_warp, &total);
+        if (threadIdx.x < 256) start[threadIdx.x] = first;
+        __syncthreads();
+#pragma unroll
+        for (int it = 0; it < ITEMS; ++it) {
+            const uint32_t d = (uint32_t)(k[it] >> shift) & 255u;
+            const int p = start[d] + (int)whist[warp][d] + (int)(rv[it] >> 16);
+            sk[p] = k[it];
+            sv[p] = (uint16_t)rv[it];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int it = 0; it < ITEMS; ++it) {
+            k[it] = sk[base + it * 32];
+            rv[it] = sv[base + it * 32];
+        }
+    }
+#pragma unroll
+    for (int it = 0; it < ITEMS; ++it) {
+        keys[base + it * 32] = k[it];
+        vals[base + it * 32] = (int32_t)rv[it];
+    }
+    if (threadIdx.x == 0) plan[16] = 0;
 }
 
 // --------------------------------------------------------- K4 topology ----
@@ -1106,12 +1262,27 @@ static cudaError_t launch_keys(nb_sim* sim, size_t nk, bool curve) {
     return cudaGetLastError();
 }
 
-// The radix sort of t.keys[0] / t.vals[0] (histograms already made): the
-// device plan, then one launch per pass.
+template <int ITEMS>
+static cudaError_t launch_sort_block(TreeBuffers& t, cudaStream_t st) {
+    // (set on each call: cheap, and right for every device)
+    const cudaError_t e = cudaFuncSetAttribute(k_sort_block<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)one_block_bytes<ITEMS>());
+    if (e != cudaSuccess) return e;
+    k_sort_block<ITEMS><<<1, kOneThreads, one_block_bytes<ITEMS>(), st>>>(t.keys[0], t.vals[0], t.ghist, t.plan);
+    return cudaGetLastError();
+}
+
+// The radix sort of t.keys[0] / t.vals[0] (histograms already made): in one
+// block up to two tiles, else the device plan, then one launch per pass.
 static cudaError_t launch_sort(nb_sim* sim, size_t nk) {
     TreeBuffers& t = sim->tree;
     const int ntiles = (int)(nk / kSortTile);
     cudaStream_t st = sim->stream;
+    static_assert(kSortTile == 4 * kOneThreads, "a tile is four keys a thread");
+    if (ntiles <= 2) {
+        PhaseScope ps(sim, NB_PHASE_SORT);
+        return ntiles == 1 ? launch_sort_block<4>(t, st) : launch_sort_block<8>(t, st);
+    }
     PhaseScope ps(sim, NB_PHASE_SORT, 1 + kPasses);
     k_sort_plan<<<1, 256, 0, st>>>(t.ghist, (int)nk, t.plan, t.dig_off);
     for (int p = 0; p < kPasses; ++p)
