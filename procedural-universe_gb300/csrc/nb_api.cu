@@ -129,48 +129,82 @@ __global__ void k_pack_writeback(const float4* __restrict__ pos, const float4* _
 }
 
 // nb_write_back straight into the caller's records (host memory the GPU can
-// address).  A warp rewrites its 32 records as one contiguous run of 4-byte
-// words, so that every store is coalesced into whole cache lines over the
-// chip-to-chip link: the words of Position (0-2), Velocity (12-17) and Forces
-// (18-23) get the new values, all other words (colours, padding, mass) are
-// read back and stored unchanged.
+// address).  A warp rewrites its 32 records as one contiguous run, so that
+// every store is coalesced into whole cache lines over the chip-to-chip link:
+// Position, Velocity and Forces get the new values, all other words (colours,
+// padding, mass) are read back and stored unchanged.  Bound by the link: its
+// latency for few records, its rate for many.  So a warp has its whole run of
+// loads in flight before its first store (16 bytes a load where the records
+// are aligned to that), the fields are set in shared memory between, and the
+// error word goes to the host beside the records, with no copy of its own.
+// Word by word, each load behind the store before it, and a copy: 52 us for
+// 1000 records, 51 for 4000, 103 for 100003, 897 for 2^20 (pageable records);
+// this: 15, 17, 88 and 721 us.  Two blocks an SM keep the link's reads busy and
+// spread the runs in time, so that reads and stores overlap: with all runs in
+// flight at once 100003 records took 111 us and 262144 took 236, with two 197.
 constexpr int kRecWords = (int)(sizeof(nb_particle) / 4);   // 26
 static_assert(sizeof(nb_particle) == 104, "reference record layout");
+constexpr int kWbWarps = 2;                       // warps a block
+constexpr int kWbPerSm = 2;                       // blocks an SM
+constexpr int kWbVecs = 32 * kRecWords / 4;       // 16-byte words of a full run
 
-__global__ void __launch_bounds__(256) k_writeback_records(const float4* __restrict__ pos,
-                                                           const float4* __restrict__ vel,
-                                                           const float4* __restrict__ velc,
-                                                           const float4* __restrict__ acc, int n, int zero_forces,
-                                                           uint32_t* __restrict__ out_words) {
-    const int lane = threadIdx.x & 31;
-    const long long base = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32;
-    if (base >= n) return;
-    const int nrec = (int)min(32LL, (long long)n - base);
-    uint32_t* w0 = out_words + base * kRecWords;
-    for (int w = lane; w < nrec * kRecWords; w += 32) {
-        const long long r = base + w / kRecWords;
-        const int o = w % kRecWords;
-        uint32_t val;
-        if (o < 3) {
-            const float4 p = pos[r];
-            val = __float_as_uint(o == 0 ? p.x : (o == 1 ? p.y : p.z));
-        } else if (o >= 12 && o < 24) {
-            const int c = ((o - 12) >> 1) % 3;
-            double d;
-            if (o < 18) {
-                const float4 v = vel[r], vc = velc[r];
-                d = c == 0 ? (double)v.x - (double)vc.x : (c == 1 ? (double)v.y - (double)vc.y : (double)v.z - (double)vc.z);
-            } else {
-                const float4 a = acc[r];
-                const double m = pos[r].w;
-                d = zero_forces ? 0.0 : m * (double)(c == 0 ? a.x : (c == 1 ? a.y : a.z));
-            }
-            const unsigned long long bits = (unsigned long long)__double_as_longlong(d);
-            val = (o & 1) ? (uint32_t)(bits >> 32) : (uint32_t)bits;   // little-endian halves
+__global__ void __launch_bounds__(32 * kWbWarps) k_writeback_records(
+    const float4* __restrict__ pos, const float4* __restrict__ vel, const float4* __restrict__ velc,
+    const float4* __restrict__ acc, int n, int zero_forces, uint32_t* __restrict__ out_words,
+    const int* __restrict__ d_err, int* __restrict__ h_err) {
+    __shared__ uint4 run4[kWbWarps][kWbVecs];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *h_err = *d_err;
+    uint32_t* run = reinterpret_cast<uint32_t*>(run4[warp]);
+    const bool aligned = (reinterpret_cast<uintptr_t>(out_words) & 15) == 0;   // a run is 3328 bytes
+    const long long step = (long long)gridDim.x * kWbWarps * 32;
+    for (long long base = ((long long)blockIdx.x * kWbWarps + warp) * 32; base < n; base += step) {
+        const int nrec = (int)min(32LL, (long long)n - base), nwords = nrec * kRecWords;
+        uint32_t* w0 = out_words + base * kRecWords;
+        const bool wide = nrec == 32 && aligned;   // else word by word
+        float4 p, v, vc, a;
+        if (wide) {
+            constexpr int PER = (kWbVecs + 31) / 32;
+            const uint4* in = reinterpret_cast<const uint4*>(w0);
+            uint4 q[PER];
+#pragma unroll
+            for (int k = 0; k < PER; ++k)
+                if (lane + 32 * k < kWbVecs) q[k] = in[lane + 32 * k];
+            p = pos[base + lane]; v = vel[base + lane]; vc = velc[base + lane]; a = acc[base + lane];
+#pragma unroll
+            for (int k = 0; k < PER; ++k)
+                if (lane + 32 * k < kWbVecs) run4[warp][lane + 32 * k] = q[k];
         } else {
-            val = w0[w];
+            uint32_t q[kRecWords];
+#pragma unroll
+            for (int k = 0; k < kRecWords; ++k)
+                if (lane + 32 * k < nwords) q[k] = w0[lane + 32 * k];
+            if (lane < nrec) { p = pos[base + lane]; v = vel[base + lane]; vc = velc[base + lane]; a = acc[base + lane]; }
+#pragma unroll
+            for (int k = 0; k < kRecWords; ++k)
+                if (lane + 32 * k < nwords) run[lane + 32 * k] = q[k];
         }
-        w0[w] = val;
+        __syncwarp();
+        if (lane < nrec) {
+            float* f = reinterpret_cast<float*>(run + lane * kRecWords);
+            f[0] = p.x; f[1] = p.y; f[2] = p.z;
+            double* d = reinterpret_cast<double*>(f + 12);   // byte 48 of a 104-byte record: aligned
+            const double m = p.w;
+            d[0] = (double)v.x - (double)vc.x;
+            d[1] = (double)v.y - (double)vc.y;
+            d[2] = (double)v.z - (double)vc.z;
+            d[3] = zero_forces ? 0.0 : m * (double)a.x;
+            d[4] = zero_forces ? 0.0 : m * (double)a.y;
+            d[5] = zero_forces ? 0.0 : m * (double)a.z;
+        }
+        __syncwarp();
+        if (wide) {
+            uint4* out = reinterpret_cast<uint4*>(w0);
+            for (int j = lane; j < kWbVecs; j += 32) out[j] = run4[warp][j];
+        } else {
+            for (int j = lane; j < nwords; j += 32) w0[j] = run[j];
+        }
+        __syncwarp();
     }
 }
 
@@ -711,10 +745,11 @@ int nb_write_back(nb_sim* s, nb_particle* particles, size_t n) {
         cudaSetDevice(s->dev);
         const int zero = (s->prm.kind != NB_SIM_BARNES_HUT) && !s->forces_fresh;
         if (host_direct(s) && ((uintptr_t)particles & 3) == 0) {
-            k_writeback_records<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(
-                s->pos, s->vel, s->velc, s->acc, (int)n, zero, reinterpret_cast<uint32_t*>(particles));
+            const size_t blocks = (n + 32 * kWbWarps - 1) / (32 * kWbWarps);
+            k_writeback_records<<<(unsigned)std::min(blocks, (size_t)kWbPerSm * (size_t)s->sm_count), 32 * kWbWarps, 0,
+                                  s->stream>>>(s->pos, s->vel, s->velc, s->acc, (int)n, zero,
+                                               reinterpret_cast<uint32_t*>(particles), s->d_err, s->h_err);
             cudaError_t e = cudaGetLastError();
-            if (e == cudaSuccess) e = cudaMemcpyAsync(s->h_err, s->d_err, sizeof(int), cudaMemcpyDeviceToHost, s->stream);
             if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
             if (e != cudaSuccess) return cuda_fail(s, e, "nb_write_back");
             return decode_device_error(s);
