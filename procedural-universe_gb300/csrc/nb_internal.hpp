@@ -98,6 +98,7 @@ enum : int {
     TC_TILE_POS = 8,
     TC_TILE_POPC = 9,
     TC_TILE_SORT = 10,   // one per radix pass
+    TC_DONE_POS = 18,    // tiles of the positions scan that are done
 };
 constexpr int kCounterWords = 32;   // counters before the radix histograms in the same buffer
 

@@ -672,7 +672,8 @@ __device__ __forceinline__ void position_nodes(const TopoView& tv, const float4*
 // Per tile of kSortTile sorted positions: the nodes starting there, and the
 // exclusive prefix of their internal-node counts by single-pass scan (pos_nint;
 // the total goes to counters[TC_NINT]).  With hk_zero, the threads also clear
-// the internal-node hash table for the emission that follows.
+// the internal-node hash table for the emission that follows.  With
+// host_counters (pinned), the last tile to finish sends the counters there.
 //
 // A thread takes every kPosThreads-th position (neighbouring threads read and
 // write neighbouring words), and the counts go through shared memory to the
@@ -688,12 +689,14 @@ __global__ void __launch_bounds__(kPosThreads) k_positions_scan(TopoView tv, con
                                                                 int32_t* __restrict__ leaf_count,
                                                                 int32_t* __restrict__ counters,
                                                                 unsigned long long* __restrict__ status, int ntiles,
-                                                                uint64_t* __restrict__ hk_zero, int hk_n,
+                                                                uint64_t* __restrict__ hk_zero, size_t hk_n,
+                                                                int32_t* __restrict__ host_counters,
                                                                 int* __restrict__ err) {
     __shared__ int sh_warp[33], sh_off, sh_tile, sh_leaf, sh_deeper;
     __shared__ __align__(16) int sh_nint[kSortTile];
     if (hk_zero)
-        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < hk_n; i += gridDim.x * blockDim.x) hk_zero[i] = 0ull;
+        for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < hk_n; i += (size_t)gridDim.x * blockDim.x)
+            hk_zero[i] = 0ull;
     if (threadIdx.x == 0) sh_leaf = sh_deeper = 0;
     const int tile = lb_tile_index(&counters[TC_TILE_POS], &sh_tile);
     tv.n_in = counters[TC_NIN];
@@ -734,6 +737,14 @@ __global__ void __launch_bounds__(kPosThreads) k_positions_scan(TopoView tv, con
     for (int k = 0; k < kPosItems; ++k) {
         const int j = k * kPosThreads + threadIdx.x, s = tile * kSortTile + j;
         if (s < tv.n_total) pos_nint[s] = sh_nint[j];
+    }
+    // (thread 0 made this tile's additions to the counters)
+    if (host_counters && threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&counters[TC_DONE_POS], 1) == ntiles - 1) {
+            __threadfence();
+            for (int k = 0; k < TC_COUNT; ++k) host_counters[k] = __ldcg(counters + k);
+        }
     }
 }
 
@@ -1316,9 +1327,13 @@ cudaError_t tree_build(nb_sim* sim, bool export_order) {
                                                         t.plan, t.spos, curve ? sim->prm.max_depth : 0);
         t.final_buf = 0;
         TopoView tv = topo_view(sim);
+        // The scan clears the hash table as it stands and sends the counters to the
+        // host itself: a copy before the wait and a memset behind it
+        // took 5 us more of the phase at 4000 bodies (52 now), 8 at 2^20 (192).
         k_positions_scan<<<ntiles, kPosThreads, 0, st>>>(tv, t.spos, t.pos_nint, t.leaf_level, t.leaf_count,
-                                                          t.counters, t.pos_status, ntiles, nullptr, 0, sim->d_err);
-        NB_TRY(cudaMemcpyAsync(t.h_counters, t.counters, TC_COUNT * 4, cudaMemcpyDeviceToHost, st));
+                                                          t.counters, t.pos_status, ntiles, t.hkeys, t.hash_cap,
+                                                          t.h_counters, sim->d_err);
+        NB_TRY(cudaGetLastError());
         NB_TRY(cudaStreamSynchronize(st));
     }
     t.n_in = t.h_counters[TC_NIN];
@@ -1327,14 +1342,15 @@ cudaError_t tree_build(nb_sim* sim, bool export_order) {
     t.trivial = (n < 2) || (t.n_in < 2 && t.n_int == 0) || t.n_in == 0;
     t.curve = curve;
     if (t.trivial) return cudaSuccess;
+    const size_t cleared = t.hash_cap;
     NB_TRY(reserve_nodes(sim, (size_t)t.n_int, (size_t)t.n_cells));
+    if (t.hash_cap != cleared) NB_TRY(cudaMemsetAsync(t.hkeys, 0, t.hash_cap * 8, st));   // grew
     TopoView tv = topo_view(sim);
     const int ni = t.n_int;
     const float tf = theta_float(sim->prm.theta);
     const uint32_t hmask = (uint32_t)(t.hash_cap - 1);
     {
         PhaseScope ps(sim, NB_PHASE_TOPOLOGY, 4);
-        NB_TRY(cudaMemsetAsync(t.hkeys, 0, t.hash_cap * 8, st));
         const int nbk = (t.n_in + kEmitBlock - 1) / kEmitBlock;
         const int ib = (ni + kEmitBlock - 1) / kEmitBlock;
         const int ptiles = (ni + kSortTile - 1) / kSortTile;
@@ -1441,7 +1457,7 @@ cudaError_t tree_build_graph(nb_sim* sim, const float4* pos, int n, int D, bool 
     // this scan also clears the internal-node hash table for the emission
     k_positions_scan<<<ntiles, kPosThreads, 0, st>>>(tv, t.spos, t.pos_nint, t.leaf_level, t.leaf_count, t.counters,
                                                       t.pos_status, ntiles, counts_only ? nullptr : t.hkeys,
-                                                      (int)t.hash_cap, sim->d_err);
+                                                      t.hash_cap, nullptr, sim->d_err);
     if (counts_only) return cudaGetLastError();   // the node counts are in counters[TC_NINT], [TC_NLEAF]
     k_emit<<<nbk, kEmitBlock, 0, st>>>(tv, t.pos_nint, t.int_level, t.int_first, t.int_code, t.hkeys, t.hvals, hmask,
                                       t.int_mask, t.int_nint, t.int_pending, t.counters, t.popc_status, ptiles);
