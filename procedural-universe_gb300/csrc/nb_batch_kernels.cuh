@@ -47,7 +47,6 @@ constexpr int kStackCellLimit = 1 << 27;   // a stack entry packs a first-child 
 constexpr int kGMultiTop = kGStack - 155 - 32;   // stack height up to which a walk step takes several cells
 constexpr int kGCells = 64;             // accepted-cell list, per warp
 constexpr int kGBodies = 192;           // gathered leaf-bucket bodies, per warp
-constexpr int kDirChunk = 32;           // sources a warp of the batched direct kernel holds at a time
 constexpr int kDirOnceMax = 8192;       // padded bodies up to which a direct member takes each pair once
 // far-field defaults of the group traversal (rules in nb_batch.cu's nb_batch)
 constexpr double kFarEta = 0.2;         // geometric rule: group half-diagonal / distance
@@ -922,7 +921,8 @@ __global__ void __launch_bounds__(kGWarps * 32, 5) k_group_traverse(
 // (l + r) mod 32 at step r, and the sources' sums travel with them by shuffle
 // (as in k_direct_pairs, here within one warp).  The row's own bodies, and all
 // sources of a member of more than kDirOnceMax padded bodies (whose source
-// partials would grow with its square), are evaluated from the target side.
+// partials would grow with its square), are evaluated from the target side
+// (direct_chunk).
 //
 // Bound by the FP32 pipe.  Warps share nothing, so that no barrier waits for
 // the slowest; the next chunk and the next unit are fetched while the current
@@ -931,69 +931,6 @@ __global__ void __launch_bounds__(kGWarps * 32, 5) k_group_traverse(
 // partial per row and body), a step 399 -> 281 us; FMA pipe 63% busy, the rest
 // is the shuffles and reads that four targets a lane carry (eight: 268 us a
 // step, but small members then fill fewer rows).
-template <int LAW, int IPT, bool BOTH>
-__device__ __forceinline__ void direct_chunk(const float4* src, int lane, const float2* nx, const float2* ny,
-                                             const float2* nz, const float2* mi, float2 S2, float2 T2, float* sum,
-                                             float* comp, float3& out) {
-    constexpr int P = IPT / 2, kGroup = 4;
-    const float2 z2 = make_float2(0.f, 0.f);
-    float2 ax[P], ay[P], az[P];
-#pragma unroll
-    for (int q = 0; q < P; ++q) ax[q] = ay[q] = az[q] = z2;
-    float sx = 0.f, sy = 0.f, sz = 0.f;
-#pragma unroll 1
-    for (int g = 0; g < kDirChunk; g += kGroup) {
-        float2 bx = z2, by = z2, bz = z2;
-#pragma unroll
-        for (int u = 0; u < kGroup; ++u) {
-            const float4 pj = src[(lane + g + u) & 31];
-            const float2 jx = make_float2(pj.x, pj.x), jy = make_float2(pj.y, pj.y);
-            const float2 jz = make_float2(pj.z, pj.z), jm = make_float2(pj.w, pj.w);
-#pragma unroll
-            for (int q = 0; q < P; ++q) {
-                const float2 dx = __fadd2_rn(jx, nx[q]), dy = __fadd2_rn(jy, ny[q]), dz = __fadd2_rn(jz, nz[q]);
-                const float2 w = pair_factor_x2<LAW>(dx, dy, dz, S2, T2);
-                const float2 wi = __fmul2_rn(jm, w);
-                ax[q] = __ffma2_rn(wi, dx, ax[q]);
-                ay[q] = __ffma2_rn(wi, dy, ay[q]);
-                az[q] = __ffma2_rn(wi, dz, az[q]);
-                if (BOTH) {
-                    const float2 wj = __fmul2_rn(mi[q], w);
-                    bx = __ffma2_rn(wj, dx, bx);
-                    by = __ffma2_rn(wj, dy, by);
-                    bz = __ffma2_rn(wj, dz, bz);
-                }
-            }
-            if (BOTH && u + 1 < kGroup) {
-                const int next = (lane + 1) & 31;
-                bx.x = __shfl_sync(0xffffffffu, bx.x, next); bx.y = __shfl_sync(0xffffffffu, bx.y, next);
-                by.x = __shfl_sync(0xffffffffu, by.x, next); by.y = __shfl_sync(0xffffffffu, by.y, next);
-                bz.x = __shfl_sync(0xffffffffu, bz.x, next); bz.y = __shfl_sync(0xffffffffu, bz.y, next);
-            }
-        }
-        if (BOTH) {   // the source's earlier groups were left kGroup lanes on
-            const int from = (lane + kGroup) & 31;
-            sx = __shfl_sync(0xffffffffu, sx, from) + (bx.x + bx.y);
-            sy = __shfl_sync(0xffffffffu, sy, from) + (by.x + by.y);
-            sz = __shfl_sync(0xffffffffu, sz, from) + (bz.x + bz.y);
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < P; ++q) {
-        kahan_add(sum[6 * q], comp[6 * q], ax[q].x);
-        kahan_add(sum[6 * q + 1], comp[6 * q + 1], ay[q].x);
-        kahan_add(sum[6 * q + 2], comp[6 * q + 2], az[q].x);
-        kahan_add(sum[6 * q + 3], comp[6 * q + 3], ax[q].y);
-        kahan_add(sum[6 * q + 4], comp[6 * q + 4], ay[q].y);
-        kahan_add(sum[6 * q + 5], comp[6 * q + 5], az[q].y);
-    }
-    if (BOTH) {   // lane l holds source (l + 31) mod 32
-        const int own = (lane + 1) & 31;
-        out = make_float3(-__shfl_sync(0xffffffffu, sx, own), -__shfl_sync(0xffffffffu, sy, own),
-                          -__shfl_sync(0xffffffffu, sz, own));
-    }
-}
-
 constexpr int kDirWarps = 8;   // most warps per block
 template <int LAW, int IPT>
 __global__ void __launch_bounds__(kDirWarps * 32, IPT == 4 ? 2 : 1) k_batch_direct(

@@ -123,4 +123,28 @@ __device__ __forceinline__ void record_error(int* err, int code) {
     if (err) atomicCAS(err, 0, code);
 }
 
+// Programmatic dependent launch.  A kernel launched by launch_after may start
+// once every block of the kernel before it in the stream has ended, before that
+// one's completion has been seen to; it calls wait_for_previous before its
+// first access to global memory, which returns when that kernel (and so, where
+// that one waited too, all work before it) has completed.  What the earlier
+// kernel wrote is then read by ordinary loads through pointers that are not
+// __restrict__: it was not read-only for this kernel's whole life, and a load
+// that the compiler takes for one of read-only memory could move before the wait.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 }  // namespace nb

@@ -366,6 +366,82 @@ __global__ void __launch_bounds__(kPairThreads, 3) k_direct_pairs(const float4* 
                                                       tot[0][3 * k + 2][tid] - tot[1][3 * k + 2][tid], 0.f);
 }
 
+// K1 for small states: each pair once, by single warps.  A unit is a row of 128
+// target bodies (four a lane) against up to L chunks of 32 sources behind it
+// (direct_chunk; the row's own four chunks from the target side only), so that
+// a few thousand bodies give a thousand warps of a few microseconds.  Bound by
+// the FP32 pipe at a few warps a scheduler, and below some 2000 bodies by the
+// latency of two dependent launches.  Those are programmatic dependent launches
+// (nb_common.cuh), and a block is one warp, so that the units spread evenly.
+// A step, with k_direct_force before: 1000 bodies 11.3 -> 6.7 us, 2048 12.3 ->
+// 7.5, 4096 19.5 -> 12.5, 8192 45 -> 30; with ordinary launches 12.4, 12.4, 17.5
+// and 37.  Early triggers (griddepcontrol.launch_dependents) gave nothing more, and
+// in the update let the next step's warps gather on the SMs that emptied first
+// (5000 bodies 32 us instead of 19).  Error against FP64 at 4096: 5.5e-8 (5.8e-8)
+constexpr int kRowIpt = 4, kRowBodies = 32 * kRowIpt, kRowChunks = kRowBodies / kDirChunk;
+struct RowPlan {
+    int chunks, rows, per;   // source chunks, rows, chunks a unit (1, 2 or 4)
+    __host__ __device__ int first_row_units() const { return (chunks + per - 1) / per; }
+    // units of the rows before row r: row r has kRowChunks / per fewer than row r - 1
+    __host__ __device__ int units_before(int r) const { return r * first_row_units() - (kRowChunks / per) * (r * (r - 1) / 2); }
+    __host__ __device__ int row_units(int r) const { return first_row_units() - (kRowChunks / per) * r; }
+};
+
+// Entry of body (r + 1) * kRowBodies among row r's source partials (they follow
+// the target partials, [units of a row][n_pad]).
+__host__ __device__ inline size_t row_source_base(const RowPlan& p, int r, int n_pad) {
+    return (size_t)p.first_row_units() * n_pad + (size_t)r * n_pad - (size_t)kRowBodies * (r * (r + 1) / 2);
+}
+
+template <int LAW>
+__global__ void __launch_bounds__(32) k_direct_rows(const float4* pos, int n_pad, RowPlan plan, float S,
+                                                                const unsigned* mmax, float4* part) {
+    __shared__ float4 src[2][kDirChunk];
+    const int lane = threadIdx.x, u = blockIdx.x;
+    int row = -1;   // the last row whose units start at or before u
+    for (int r0 = 0; r0 < plan.rows; r0 += 32)
+        row += __popc(__ballot_sync(0xffffffffu, r0 + lane < plan.rows && plan.units_before(r0 + lane) <= u));
+    const int s = u - plan.units_before(row);
+    const int c0 = row * kRowChunks + s * plan.per, c1 = min(plan.chunks, c0 + plan.per);
+    const int own = (row + 1) * kRowChunks;   // chunks before this one are the row's own
+    wait_for_previous();
+    const float tiny = mmax ? self_pair_tiny(mmax) : kTiny;
+    const float2 S2 = make_float2(S, S), T2 = make_float2(tiny, tiny);
+    constexpr int P = kRowIpt / 2;
+    const int t0 = row * kRowBodies + lane;
+    float2 nx[P], ny[P], nz[P], mi[P];
+    float sum[3 * kRowIpt], comp[3 * kRowIpt];
+    float4 cur = pos[c0 * kDirChunk + lane];
+#pragma unroll
+    for (int q = 0; q < P; ++q) {
+        const float4 a = pos[t0 + (2 * q) * 32], b = pos[t0 + (2 * q + 1) * 32];
+        nx[q] = make_float2(-a.x, -b.x);
+        ny[q] = make_float2(-a.y, -b.y);
+        nz[q] = make_float2(-a.z, -b.z);
+        mi[q] = make_float2(a.w, b.w);
+    }
+#pragma unroll
+    for (int k = 0; k < 3 * kRowIpt; ++k) sum[k] = comp[k] = 0.f;
+    float4* sources = part + row_source_base(plan, row, n_pad);
+    for (int c = c0; c < c1; ++c) {
+        float4* buf = src[c & 1];
+        buf[lane] = cur;
+        __syncwarp();   // also: every lane is done with the chunk that this buffer held
+        if (c + 1 < c1) cur = pos[(c + 1) * kDirChunk + lane];
+        float3 f;
+        if (c < own) {
+            direct_chunk<LAW, kRowIpt, false>(buf, lane, nx, ny, nz, mi, S2, T2, sum, comp, f);
+        } else {
+            direct_chunk<LAW, kRowIpt, true>(buf, lane, nx, ny, nz, mi, S2, T2, sum, comp, f);
+            sources[(c - own) * kDirChunk + lane] = make_float4(f.x, f.y, f.z, 0.f);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kRowIpt; ++k)
+        part[(size_t)s * n_pad + t0 + k * 32] =
+            make_float4(sum[3 * k] - comp[3 * k], sum[3 * k + 1] - comp[3 * k + 1], sum[3 * k + 2] - comp[3 * k + 2], 0.f);
+}
+
 // K7: fold the partials of all source ranges (fixed order), apply G, add the
 // pending initial forces, store the acceleration and, when update != 0,
 // kick-drift: v += a dt; x += v dt / scale, both Kahan-compensated
@@ -467,16 +543,54 @@ __device__ __forceinline__ float3 with_carry(const HiLo3& f, const float4* __res
     return make_float3(s.x + c.x, s.y + c.y, s.z + c.z);
 }
 
+// What an update reads and writes (K7).
+struct UpdateArgs {
+    float G, dt, inv_scale;
+    int update, comp;
+    const float4* finit;
+    float4 *acc, *pos, *posc, *vel, *velc;
+    nb_render_vertex* rv;
+    const float4* rcol;
+    float rscale;
+};
+
+struct BodyState {
+    float4 v, vc, x, xc;
+    __device__ __forceinline__ void read(const UpdateArgs& u, int i) { v = u.vel[i]; vc = u.velc[i]; x = u.pos[i]; xc = u.posc[i]; }
+};
+
+__device__ __forceinline__ void finish_body(const UpdateArgs& u, int i, const float3 f, BodyState b) {
+    float3 a = make_float3(u.G * f.x, u.G * f.y, u.G * f.z);
+    if (u.finit) {
+        const float4 f0 = u.finit[i];
+        a.x += f0.x; a.y += f0.y; a.z += f0.z;
+    }
+    u.acc[i] = make_float4(a.x, a.y, a.z, 0.f);
+    if (!u.update) return;
+    float4 &v = b.v, &vc = b.vc, &x = b.x, &xc = b.xc;
+    if (u.comp) {
+        kahan_add(v.x, vc.x, a.x * u.dt);
+        kahan_add(v.y, vc.y, a.y * u.dt);
+        kahan_add(v.z, vc.z, a.z * u.dt);
+        kahan_add(x.x, xc.x, ((v.x - vc.x) * u.dt) * u.inv_scale);
+        kahan_add(x.y, xc.y, ((v.y - vc.y) * u.dt) * u.inv_scale);
+        kahan_add(x.z, xc.z, ((v.z - vc.z) * u.dt) * u.inv_scale);
+        u.velc[i] = vc;
+        u.posc[i] = xc;
+    } else {
+        v.x += a.x * u.dt; v.y += a.y * u.dt; v.z += a.z * u.dt;
+        x.x += (v.x * u.dt) * u.inv_scale; x.y += (v.y * u.dt) * u.inv_scale; x.z += (v.z * u.dt) * u.inv_scale;
+    }
+    u.vel[i] = v;
+    u.pos[i] = x;
+    if (u.rv) write_vertex(u.rv, u.rcol, u.rscale, i, x);
+}
+
 // PAIRS: the partials are k_direct_pairs' (carry: the earlier launches' sums,
 // when there were several), else k_direct_force's.
 template <bool PAIRS>
 __global__ void k_direct_reduce_update(const float4* __restrict__ part, int splits, PairFold pf,
-                                       const float4* __restrict__ carry, int n, int n_pad, float G,
-                                       const float4* __restrict__ finit, float4* __restrict__ acc,
-                                       float4* __restrict__ pos, float4* __restrict__ posc,
-                                       float4* __restrict__ vel, float4* __restrict__ velc, float dt,
-                                       float inv_scale, int update, int comp, nb_render_vertex* __restrict__ rv,
-                                       const float4* __restrict__ rcol, float rscale,
+                                       const float4* __restrict__ carry, int n, int n_pad, UpdateArgs u,
                                        const int* __restrict__ err) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = t / kFoldLanes, j = t % kFoldLanes;
@@ -484,31 +598,60 @@ __global__ void k_direct_reduce_update(const float4* __restrict__ part, int spli
     if (i >= n_pad || *err != 0) return;
     const HiLo3 total = PAIRS ? fold_pairs_lanes(part, pf, n_pad, i, j) : fold_partials_lanes(part, splits, n_pad, i, j);
     if (i >= n || j != 0) return;
-    const float3 f = with_carry(total, carry, n_pad, i);
-    float3 a = make_float3(G * f.x, G * f.y, G * f.z);
-    if (finit) {
-        const float4 f = finit[i];
-        a.x += f.x; a.y += f.y; a.z += f.z;
+    BodyState b;
+    b.read(u, i);
+    finish_body(u, i, with_carry(total, carry, n_pad, i), b);
+}
+
+// The fold of k_direct_rows' partials: a block's warps share 32 bodies, warp j
+// taking every kRowFold-th partial of them (neighbouring bodies' entries lie
+// together), and the first warp adds the warps' sums in order.  Returns the
+// force in the first warp's threads.
+constexpr int kRowFold = 8;
+__device__ __forceinline__ float3 fold_rows(const float4* part, const RowPlan& plan, int n_pad, int i, int j,
+                                            float (*sums)[6][32]) {
+    float ax = 0.f, ay = 0.f, az = 0.f, kx = 0.f, ky = 0.f, kz = 0.f;
+    const int row = i / kRowBodies, lane = threadIdx.x & 31;   // one row a block
+    auto add = [&](const float4 p) {
+        kahan_add(ax, kx, p.x);
+        kahan_add(ay, ky, p.y);
+        kahan_add(az, kz, p.z);
+    };
+    const int used = plan.row_units(row);
+#pragma unroll 4
+    for (int s = j; s < used; s += kRowFold) add(part[(size_t)s * n_pad + i]);
+#pragma unroll 4
+    for (int r = j; r < row; r += kRowFold) add(part[row_source_base(plan, r, n_pad) + (i - (r + 1) * kRowBodies)]);
+    sums[j][0][lane] = ax; sums[j][1][lane] = ay; sums[j][2][lane] = az;
+    sums[j][3][lane] = kx; sums[j][4][lane] = ky; sums[j][5][lane] = kz;
+    __syncthreads();
+    float r[3] = {0.f, 0.f, 0.f};
+    if (j == 0) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            float hi = sums[0][d][lane], lo = -sums[0][3 + d][lane];
+#pragma unroll
+            for (int w = 1; w < kRowFold; ++w) {
+                float e;
+                hi = two_sum(hi, sums[w][d][lane], e);
+                lo += e - sums[w][3 + d][lane];
+            }
+            r[d] = hi + lo;
+        }
     }
-    acc[i] = make_float4(a.x, a.y, a.z, 0.f);
-    if (!update) return;
-    float4 v = vel[i], vc = velc[i], x = pos[i], xc = posc[i];
-    if (comp) {
-        kahan_add(v.x, vc.x, a.x * dt);
-        kahan_add(v.y, vc.y, a.y * dt);
-        kahan_add(v.z, vc.z, a.z * dt);
-        kahan_add(x.x, xc.x, ((v.x - vc.x) * dt) * inv_scale);
-        kahan_add(x.y, xc.y, ((v.y - vc.y) * dt) * inv_scale);
-        kahan_add(x.z, xc.z, ((v.z - vc.z) * dt) * inv_scale);
-        velc[i] = vc;
-        posc[i] = xc;
-    } else {
-        v.x += a.x * dt; v.y += a.y * dt; v.z += a.z * dt;
-        x.x += (v.x * dt) * inv_scale; x.y += (v.y * dt) * inv_scale; x.z += (v.z * dt) * inv_scale;
-    }
-    vel[i] = v;
-    pos[i] = x;
-    if (rv) write_vertex(rv, rcol, rscale, i, x);
+    return make_float3(r[0], r[1], r[2]);
+}
+
+__global__ void __launch_bounds__(32 * kRowFold) k_direct_rows_update(const float4* part, RowPlan plan, int n, int n_pad,
+                                                                      UpdateArgs u, const int* err) {
+    __shared__ float sums[kRowFold][6][32];
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31), j = threadIdx.x >> 5;
+    wait_for_previous();
+    const int failed = *err;
+    BodyState b;
+    if (j == 0) b.read(u, i);   // in flight beside the partials (i < n_pad)
+    const float3 f = fold_rows(part, plan, n_pad, i, j, sums);
+    if (j == 0 && i < n && failed == 0) finish_body(u, i, f, b);
 }
 
 // Kick-drift from a stored acceleration (Barnes-Hut path,
@@ -690,7 +833,31 @@ static int launch_pairs(int sm_count, int law, cudaStream_t st, const float4* po
 // Entries of partials a handle's k_direct_pairs launch may use (1 GiB): one
 // launch up to about 360,000 bodies.
 constexpr size_t kPairCap = ((size_t)1 << 30) / sizeof(float4);
-constexpr size_t kPairMin = 10240;
+// Padded bodies up to which single warps take the pairs (k_direct_rows), for a
+// handle and in the allocation-free call, whose fixed array holds no more rows'
+// partials.  A step of 8192 bodies takes 30 us by warps, of 10000 44 (k_direct_pairs
+// 49), of 16384 95 (109), of 20480 146 (154), of 24000 199 (202): past that the
+// row partials' own cost grows with the square of the bodies.
+constexpr size_t kRowMax = 20480, kRowMaxNoAlloc = 8192;
+
+// The units of k_direct_rows within cap entries of partials.
+static size_t row_entries(const RowPlan& p, int n_pad) { return row_source_base(p, p.rows, n_pad); }
+
+static RowPlan row_plan(int n, int n_pad, size_t cap) {
+    RowPlan p;
+    p.chunks = (n + kDirChunk - 1) / kDirChunk;
+    p.rows = (n + kRowBodies - 1) / kRowBodies;
+    p.per = p.chunks <= 64 ? 1 : p.chunks <= 256 ? 2 : 4;
+    if (row_entries(p, n_pad) > cap) p.per = 4;
+    return p;
+}
+
+static cudaError_t launch_rows(const RowPlan& p, int law, cudaStream_t st, const float4* pos, int n_pad, float S,
+                        const unsigned* mmax, float4* part) {
+    const unsigned grid = (unsigned)p.units_before(p.rows);
+    return launch_after(law == NB_LAW_PLUMMER ? k_direct_rows<NB_LAW_PLUMMER> : k_direct_rows<NB_LAW_REFERENCE>, grid,
+                        32, st, pos, n_pad, p, S, mmax, part);
+}
 
 static cudaError_t force_pairs(nb_sim* sim, PairFold* last, const float4** carry) {
     const int n_pad = (int)sim->n_pad, rows = n_pad / kPairRow;
@@ -713,18 +880,24 @@ static cudaError_t force_pairs(nb_sim* sim, PairFold* last, const float4** carry
 
 cudaError_t direct_force_update(nb_sim* sim, float dt, bool update) {
     const bool comp = !(sim->prm.flags & NB_FLAG_NO_COMPENSATION);
-    // Each pair once from kPairMin padded bodies on: a step took 49 us against
-    // 70 at 10,000 bodies and 46 against 45 at 8,000, where a row's eight own
-    // tiles (both directions evaluated) and a unit's one-tile life cost what
-    // the shared roots save.  A handle whose launch was tuned, and
-    // uncompensated sums, keep k_direct_force.
-    const bool pairs = comp && !sim->tune_set && sim->n_pad >= kPairMin;
+    // Each pair once.  A handle whose launch was tuned, and uncompensated sums,
+    // keep k_direct_force.
+    const bool once = comp && !sim->tune_set, by_rows = once && sim->n_pad <= kRowMax, pairs = once && !by_rows;
+    RowPlan rp{};
     int splits = 0;
     PairFold pf{};
     const float4* carry = nullptr;
     if (pairs) {
         PhaseScope ps(sim, 0);
         cudaError_t e = force_pairs(sim, &pf, &carry);
+        if (e != cudaSuccess) return e;
+    } else if (by_rows) {
+        rp = row_plan((int)sim->n, (int)sim->n_pad, kPairCap);
+        cudaError_t e = reserve_part(sim, row_entries(rp, (int)sim->n_pad));
+        if (e != cudaSuccess) return e;
+        PhaseScope ps(sim, 0);
+        e = launch_rows(rp, sim->prm.law, sim->stream, sim->pos, (int)sim->n_pad, (float)sim->prm.softening2,
+                        sim->heavy ? sim->d_mmax : nullptr, sim->part);
         if (e != cudaSuccess) return e;
     } else {
         DirectTuning t = sim->tune;
@@ -755,19 +928,21 @@ cudaError_t direct_force_update(nb_sim* sim, float dt, bool update) {
         if (e != cudaSuccess) return e;
     }
     const int n = (int)sim->n;
-    const float inv_scale = (float)(1.0 / sim->prm.pos_scale);
-    PhaseScope ps(sim, 1);
-    static_assert(kPad % (256 / kFoldLanes) == 0, "the fold's blocks cover whole padded bodies");
-#define NB_REDUCE(PAIRS)                                                                                             \
-    k_direct_reduce_update<PAIRS><<<(unsigned)(sim->n_pad * kFoldLanes / 256), 256, 0, sim->stream>>>(               \
-        sim->part, splits, pf, carry, n, (int)sim->n_pad, (float)sim->prm.G, sim->finit_pending ? sim->finit : nullptr, \
-        sim->acc, sim->pos, sim->posc, sim->vel, sim->velc, dt, inv_scale, update ? 1 : 0, comp ? 1 : 0,             \
-        update ? sim->render : nullptr, sim->rcolour, sim->rscale, sim->d_err)
-    if (pairs) NB_REDUCE(true); else NB_REDUCE(false);
-#undef NB_REDUCE
+    const UpdateArgs ua{(float)sim->prm.G, dt, (float)(1.0 / sim->prm.pos_scale), update ? 1 : 0, comp ? 1 : 0,
+                        sim->finit_pending ? sim->finit : nullptr, sim->acc, sim->pos, sim->posc, sim->vel, sim->velc,
+                        update ? sim->render : nullptr, sim->rcolour, sim->rscale};
     sim->finit_pending = false;
     const double nn = (double)sim->n;
     sim->inter_last = (uint64_t)(nn * (nn - 1.0));
+    PhaseScope ps(sim, 1);
+    static_assert(kPad % (256 / kFoldLanes) == 0 && kPad % 32 == 0, "the fold's blocks cover whole padded bodies");
+    const unsigned rblocks = (unsigned)(sim->n_pad * kFoldLanes / 256);
+    if (pairs)
+        k_direct_reduce_update<true><<<rblocks, 256, 0, sim->stream>>>(sim->part, splits, pf, carry, n, (int)sim->n_pad, ua, sim->d_err);
+    else if (by_rows)
+        return launch_after(k_direct_rows_update, (unsigned)((n + 31) / 32), 32 * kRowFold, sim->stream, sim->part, rp, n, (int)sim->n_pad, ua, sim->d_err);
+    else
+        k_direct_reduce_update<false><<<rblocks, 256, 0, sim->stream>>>(sim->part, splits, pf, carry, n, (int)sim->n_pad, ua, sim->d_err);
     return cudaGetLastError();
 }
 
@@ -799,9 +974,10 @@ cudaError_t kick_drift(nb_sim* sim, float dt, const int32_t* hold, int int_cap, 
 
 namespace nb {
 
-constexpr int kNoAllocMaxSplits = 8;
-// padded copy of the input + (sum, compensation) partials of up to 8 source ranges
-constexpr size_t kNoAllocScratch = (size_t)NB_NOALLOC_MAX_BODIES * (1 + 2 * kNoAllocMaxSplits);
+// padded copy of the input + 16 entries of partials a body at the most bodies
+constexpr size_t kNoAllocScratch = (size_t)NB_NOALLOC_MAX_BODIES * 17;
+static_assert((kRowMaxNoAlloc / (4 * kDirChunk) + kRowMaxNoAlloc / kRowBodies / 2 + 1) * kRowMaxNoAlloc <= kNoAllocScratch,
+              "the array holds the rows' partials at four chunks a unit");
 static __device__ __align__(256) float4 g_noalloc_scratch[kNoAllocScratch];   // 17.8 MB
 static __device__ int g_noalloc_err;
 // float bits of the call's largest |mass| (the force law's self-pair guard);
@@ -823,19 +999,28 @@ __global__ void k_noalloc_stage(const float4* __restrict__ in, int n, int n_pad,
 
 // Folds the partials like k_direct_reduce_update; a force kernel whose bounded
 // wait ran out poisons the output with NaN, since nothing is read back.
-template <bool PAIRS>
-__global__ void k_noalloc_reduce(const float4* __restrict__ part, int splits, PairFold pf,
-                                 const float4* __restrict__ carry, int n, int n_pad, float G,
-                                 float4* __restrict__ acc) {
+__global__ void k_noalloc_reduce(const float4* __restrict__ part, PairFold pf, const float4* __restrict__ carry, int n,
+                                 int n_pad, float G, float4* __restrict__ acc) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = t / kFoldLanes, j = t % kFoldLanes;
     if (i >= n_pad) return;   // whole groups of lanes (the padded size is a multiple of the block's bodies)
-    const HiLo3 f = PAIRS ? fold_pairs_lanes(part, pf, n_pad, i, j) : fold_partials_lanes(part, splits, n_pad, i, j);
+    const HiLo3 f = fold_pairs_lanes(part, pf, n_pad, i, j);
     if (i >= n || j != 0) return;
     const float3 s = with_carry(f, carry, n_pad, i);
     float4 a = make_float4(G * s.x, G * s.y, G * s.z, 0.f);
     if (g_noalloc_err != 0) a = make_float4(NAN, NAN, NAN, NAN);
     acc[i] = a;
+    if (i == 0) g_noalloc_mmax = 0u;
+}
+
+// The same for k_direct_rows (which has no wait to run out).
+__global__ void __launch_bounds__(32 * kRowFold) k_noalloc_rows(const float4* part, RowPlan plan, int n, int n_pad,
+                                                                float G, float4* acc) {
+    __shared__ float sums[kRowFold][6][32];
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31), j = threadIdx.x >> 5;
+    const float3 s = fold_rows(part, plan, n_pad, i, j, sums);
+    if (i >= n || j != 0) return;
+    acc[i] = make_float4(G * s.x, G * s.y, G * s.z, 0.f);
     if (i == 0) g_noalloc_mmax = 0u;
 }
 
@@ -886,17 +1071,19 @@ extern "C" int nb_direct_accel_noalloc(const float* pos_mass4, size_t n, float* 
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const size_t n_pad = pad_up(n, kPad);
-    const int ntiles = (int)(n_pad / kTileJ);
     float4* pos = scratch;
     float4* part = scratch + n_pad;
     const float S = (float)softening2;
     k_noalloc_stage<<<(unsigned)((n_pad + 255) / 256), 256, 0, st>>>(reinterpret_cast<const float4*>(pos_mass4),
                                                                     (int)n, (int)n_pad, pos);
-    PairFold pf{};
-    const float4* carry = nullptr;
-    int splits = 0;
-    const bool pairs = n_pad >= kPairMin;
-    if (pairs) {
+    float4* acc = reinterpret_cast<float4*>(accel4);
+    if (n_pad <= kRowMaxNoAlloc) {
+        const RowPlan rp = row_plan((int)n, (int)n_pad, kNoAllocScratch - n_pad);
+        if (launch_rows(rp, law, st, pos, (int)n_pad, S, mmax, part) != cudaSuccess) return NB_ECUDA;
+        k_noalloc_rows<<<(unsigned)((n + 31) / 32), 32 * kRowFold, 0, st>>>(part, rp, (int)n, (int)n_pad, (float)G, acc);
+    } else {
+        PairFold pf{};
+        const float4* carry = nullptr;
         // Each pair once, as for a handle, in as many launches as the fixed array
         // asks for (six at 65,536 bodies; two entries a body hold their running
         // sums).  Folding targets every 16 sources instead of 32 costs 4% and
@@ -910,27 +1097,9 @@ extern "C" int nb_direct_accel_noalloc(const float* pos_mass4, size_t n, float* 
         }
         const size_t cap = kNoAllocScratch - 3 * n_pad;
         launch_pairs<true, kFold / 2>(sms, law, st, pos, (int)n_pad, S, part, cap, false, part + cap, err, kMaxPolls, mmax, &pf, &carry);
-    } else {
-        splits = std::min(kNoAllocMaxSplits, ntiles);
-        const int tps = (ntiles + splits - 1) / splits;
-        splits = (ntiles + tps - 1) / tps;
-        const int block = 128, ipt = 1;   // default_tuning's shape below 16,384 bodies
-        dim3 grid((unsigned)(n_pad / (size_t)(block * ipt)), (unsigned)splits);
-        const bool ok =
-            law == NB_LAW_PLUMMER
-                ? launch_force_law<NB_LAW_PLUMMER, true>(block, ipt, grid, st, pos, (int)n_pad, tps, ntiles, splits, S,
-                                                        part, err, kMaxPolls, mmax, true)
-                : launch_force_law<NB_LAW_REFERENCE, true>(block, ipt, grid, st, pos, (int)n_pad, tps, ntiles, splits, S,
-                                                          part, err, kMaxPolls, mmax, true);
-        if (!ok) return NB_EINVAL;
+        k_noalloc_reduce<<<(unsigned)(n_pad * kFoldLanes / 256), 256, 0, st>>>(part, pf, carry, (int)n, (int)n_pad,
+                                                                              (float)G, acc);
     }
-    const unsigned rblocks = (unsigned)(n_pad * kFoldLanes / 256);
-    if (pairs)
-        k_noalloc_reduce<true><<<rblocks, 256, 0, st>>>(part, splits, pf, carry, (int)n, (int)n_pad, (float)G,
-                                                        reinterpret_cast<float4*>(accel4));
-    else
-        k_noalloc_reduce<false><<<rblocks, 256, 0, st>>>(part, splits, pf, carry, (int)n, (int)n_pad, (float)G,
-                                                         reinterpret_cast<float4*>(accel4));
     if (cudaGetLastError() != cudaSuccess) return NB_ECUDA;
     return NB_OK;
 }

@@ -22,7 +22,7 @@ constexpr float kTiny = 1e-30f;
 
 // tiny for a state whose largest |mass| has the float bits *mmax_bits: the
 // self pair's factor m / sqrt(tiny) stays <= 1e36 (1e-30 for masses <= 1e21).
-__device__ __forceinline__ float self_pair_tiny(const unsigned* __restrict__ mmax_bits) {
+__device__ __forceinline__ float self_pair_tiny(const unsigned* mmax_bits) {
     const float q = __uint_as_float(*mmax_bits) * 1e-36f;
     return fmaxf(kTiny, q * q);
 }
@@ -141,6 +141,78 @@ __device__ __forceinline__ HiLo butterfly_total(float s, float c) {
         lo = __fadd_rn(__fadd_rn(lo, bl), e);
     }
     return HiLo{hi, lo};
+}
+
+// One warp's evaluation of a chunk of 32 sources (in shared memory) against its
+// 32 * IPT targets (IPT a lane in registers, negated coordinates nx, ny, nz and
+// masses mi, packed in pairs).  BOTH: each pair serves both bodies, 17 FP32
+// operations for two interactions instead of 26: lane l takes source
+// (l + r) mod 32 at step r, and the sources' sums travel with them by shuffle;
+// lane l receives source l's sum in out.  Else only the targets' side.  The
+// chunk's target sums are added to the compensated sum (x, y, z of target k at
+// 3 k, comp negated).
+constexpr int kDirChunk = 32;
+template <int LAW, int IPT, bool BOTH>
+__device__ __forceinline__ void direct_chunk(const float4* src, int lane, const float2* nx, const float2* ny,
+                                             const float2* nz, const float2* mi, float2 S2, float2 T2, float* sum,
+                                             float* comp, float3& out) {
+    constexpr int P = IPT / 2, kGroup = 4;
+    const float2 z2 = make_float2(0.f, 0.f);
+    float2 ax[P], ay[P], az[P];
+#pragma unroll
+    for (int q = 0; q < P; ++q) ax[q] = ay[q] = az[q] = z2;
+    float sx = 0.f, sy = 0.f, sz = 0.f;
+#pragma unroll 1
+    for (int g = 0; g < kDirChunk; g += kGroup) {
+        float2 bx = z2, by = z2, bz = z2;
+#pragma unroll
+        for (int u = 0; u < kGroup; ++u) {
+            const float4 pj = src[(lane + g + u) & 31];
+            const float2 jx = make_float2(pj.x, pj.x), jy = make_float2(pj.y, pj.y);
+            const float2 jz = make_float2(pj.z, pj.z), jm = make_float2(pj.w, pj.w);
+#pragma unroll
+            for (int q = 0; q < P; ++q) {
+                const float2 dx = __fadd2_rn(jx, nx[q]), dy = __fadd2_rn(jy, ny[q]), dz = __fadd2_rn(jz, nz[q]);
+                const float2 w = pair_factor_x2<LAW>(dx, dy, dz, S2, T2);
+                const float2 wi = __fmul2_rn(jm, w);
+                ax[q] = __ffma2_rn(wi, dx, ax[q]);
+                ay[q] = __ffma2_rn(wi, dy, ay[q]);
+                az[q] = __ffma2_rn(wi, dz, az[q]);
+                if (BOTH) {
+                    const float2 wj = __fmul2_rn(mi[q], w);
+                    bx = __ffma2_rn(wj, dx, bx);
+                    by = __ffma2_rn(wj, dy, by);
+                    bz = __ffma2_rn(wj, dz, bz);
+                }
+            }
+            if (BOTH && u + 1 < kGroup) {
+                const int next = (lane + 1) & 31;
+                bx.x = __shfl_sync(0xffffffffu, bx.x, next); bx.y = __shfl_sync(0xffffffffu, bx.y, next);
+                by.x = __shfl_sync(0xffffffffu, by.x, next); by.y = __shfl_sync(0xffffffffu, by.y, next);
+                bz.x = __shfl_sync(0xffffffffu, bz.x, next); bz.y = __shfl_sync(0xffffffffu, bz.y, next);
+            }
+        }
+        if (BOTH) {   // the source's earlier groups were left kGroup lanes on
+            const int from = (lane + kGroup) & 31;
+            sx = __shfl_sync(0xffffffffu, sx, from) + (bx.x + bx.y);
+            sy = __shfl_sync(0xffffffffu, sy, from) + (by.x + by.y);
+            sz = __shfl_sync(0xffffffffu, sz, from) + (bz.x + bz.y);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < P; ++q) {
+        kahan_add(sum[6 * q], comp[6 * q], ax[q].x);
+        kahan_add(sum[6 * q + 1], comp[6 * q + 1], ay[q].x);
+        kahan_add(sum[6 * q + 2], comp[6 * q + 2], az[q].x);
+        kahan_add(sum[6 * q + 3], comp[6 * q + 3], ax[q].y);
+        kahan_add(sum[6 * q + 4], comp[6 * q + 4], ay[q].y);
+        kahan_add(sum[6 * q + 5], comp[6 * q + 5], az[q].y);
+    }
+    if (BOTH) {   // lane l holds source (l + 31) mod 32
+        const int own = (lane + 1) & 31;
+        out = make_float3(-__shfl_sync(0xffffffffu, sx, own), -__shfl_sync(0xffffffffu, sy, own),
+                          -__shfl_sync(0xffffffffu, sz, own));
+    }
 }
 
 }  // namespace nb

@@ -337,3 +337,39 @@ def test_records_written_in_place(n, offset):
         got.append(out)
     for f in ("position", "velocity", "forces"):
         assert got[0][f].tobytes() == got[1][f].tobytes(), f
+
+
+@pytest.mark.parametrize("law", [nb.LAW_REFERENCE, nb.LAW_PLUMMER])
+@pytest.mark.parametrize("n", [2, 33, 127, 129, 2048, 2049, 4097, 8191, 16383, 20480, 20481])
+def test_pairs_by_single_warps(n, law):
+    """At the edges of chunks, rows, chunks a unit and of the range; uneven
+    masses.  A term carries a few units of 2^-24 and the sums are compensated:
+    5e-7 bounds their total."""
+    pm, v = nb.seed_plummer(31, n)
+    pm[:, 3] *= np.random.default_rng(n).uniform(0.01, 2.0, n).astype(np.float32)
+    if n > 100:
+        pm[5, :3] = pm[6, :3]
+        pm[7, :3] = pm[n - 1, :3]
+        pm[n // 2, 3] = 0.0
+    with direct_sim(law=law) as s:
+        s.init_soa(pm, v)
+        F, F64 = s.compute_forces(), s.fp64_forces(np.arange(n))
+    assert np.isfinite(F).all()
+    assert O.rel_l2(F, F64) < 5e-7
+
+
+@pytest.mark.parametrize("n", [100, 1000, 5000])
+def test_steps_of_small_states_follow_each_other(n):
+    """Each launch waits for the one before: 200 queued steps are those of 200
+    calls with a synchronisation behind each, byte for byte."""
+    pm, v = nb.seed_plummer(8, n)
+    out = []
+    for chunk in (200, 1):
+        with direct_sim() as s:
+            s.init_soa(pm, v)
+            for _ in range(200 // chunk):
+                s.step(1e-3, chunk)
+                s.synchronize()
+            out.append(s.read_state())
+    for a, b in zip(*out):
+        assert a.tobytes() == b.tobytes()
