@@ -134,10 +134,11 @@ __device__ __forceinline__ void record_error(int* err, int code) {
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <class... P, class... A>
-cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t shared, cudaStream_t st, A... args) {
     cudaLaunchConfig_t c{};
     c.gridDim = grid;
     c.blockDim = block;
+    c.dynamicSmemBytes = shared;
     c.stream = st;
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;

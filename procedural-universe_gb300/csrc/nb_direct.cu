@@ -656,11 +656,12 @@ __global__ void __launch_bounds__(32 * kRowFold) k_direct_rows_update(const floa
 
 // Kick-drift from a stored acceleration (Barnes-Hut path,
 // src/Sim/BarnesHut.cpp:81-95).
-__global__ void k_kick_drift(const float4* __restrict__ acc, int n, float4* __restrict__ pos,
-                             float4* __restrict__ posc, float4* __restrict__ vel, float4* __restrict__ velc,
-                             float dt, float inv_scale, int comp, nb_render_vertex* __restrict__ rv,
-                             const float4* __restrict__ rcol, float rscale, const int32_t* __restrict__ hold,
-                             int int_cap, int cell_cap, int* __restrict__ held) {
+__global__ void k_kick_drift(const float4* acc, int n, float4* pos,
+                             float4* posc, float4* vel, float4* velc,
+                             float dt, float inv_scale, int comp, nb_render_vertex* rv,
+                             const float4* rcol, float rscale, const int32_t* hold,
+                             int int_cap, int cell_cap, int* held) {
+    wait_for_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     if (hold && !tree_fits(hold, int_cap, cell_cap)) {   // the step is held: the state stays as it was
@@ -856,7 +857,7 @@ static cudaError_t launch_rows(const RowPlan& p, int law, cudaStream_t st, const
                         const unsigned* mmax, float4* part) {
     const unsigned grid = (unsigned)p.units_before(p.rows);
     return launch_after(law == NB_LAW_PLUMMER ? k_direct_rows<NB_LAW_PLUMMER> : k_direct_rows<NB_LAW_REFERENCE>, grid,
-                        32, st, pos, n_pad, p, S, mmax, part);
+                        32, 0, st, pos, n_pad, p, S, mmax, part);
 }
 
 static cudaError_t force_pairs(nb_sim* sim, PairFold* last, const float4** carry) {
@@ -940,7 +941,8 @@ cudaError_t direct_force_update(nb_sim* sim, float dt, bool update) {
     if (pairs)
         k_direct_reduce_update<true><<<rblocks, 256, 0, sim->stream>>>(sim->part, splits, pf, carry, n, (int)sim->n_pad, ua, sim->d_err);
     else if (by_rows)
-        return launch_after(k_direct_rows_update, (unsigned)((n + 31) / 32), 32 * kRowFold, sim->stream, sim->part, rp, n, (int)sim->n_pad, ua, sim->d_err);
+        return launch_after(k_direct_rows_update, (unsigned)((n + 31) / 32), 32 * kRowFold, 0, sim->stream,
+                            sim->part, rp, n, (int)sim->n_pad, ua, sim->d_err);
     else
         k_direct_reduce_update<false><<<rblocks, 256, 0, sim->stream>>>(sim->part, splits, pf, carry, n, (int)sim->n_pad, ua, sim->d_err);
     return cudaGetLastError();
@@ -950,11 +952,9 @@ cudaError_t kick_drift(nb_sim* sim, float dt, const int32_t* hold, int int_cap, 
     const int n = (int)sim->n;
     const bool comp = !(sim->prm.flags & NB_FLAG_NO_COMPENSATION);
     PhaseScope ps(sim, 7);
-    k_kick_drift<<<(n + 255) / 256, 256, 0, sim->stream>>>(sim->acc, n, sim->pos, sim->posc, sim->vel, sim->velc,
-                                                           dt, (float)(1.0 / sim->prm.pos_scale), comp ? 1 : 0,
-                                                           sim->render, sim->rcolour, sim->rscale, hold, int_cap,
-                                                           cell_cap, held);
-    return cudaGetLastError();
+    return launch_after(k_kick_drift, (n + 255) / 256, 256, 0, sim->stream, sim->acc, n, sim->pos, sim->posc,
+                        sim->vel, sim->velc, dt, (float)(1.0 / sim->prm.pos_scale), comp ? 1 : 0, sim->render,
+                        sim->rcolour, sim->rscale, hold, int_cap, cell_cap, held);
 }
 
 }  // namespace nb

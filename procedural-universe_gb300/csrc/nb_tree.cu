@@ -244,8 +244,9 @@ __global__ void __launch_bounds__(kSortThreads) k_keys_hist(const float4* __rest
 // One warp per pass, eight digits a lane: 8.3 -> 4 us against eight block scans
 // one after the other (ncu).
 static_assert(kPasses * 32 == 256, "one warp per pass");
-__global__ void __launch_bounds__(256) k_sort_plan(const uint32_t* __restrict__ ghist, int nk,
-                                                   int32_t* __restrict__ plan, int32_t* __restrict__ dig_off) {
+__global__ void __launch_bounds__(256) k_sort_plan(const uint32_t* ghist, int nk,
+                                                   int32_t* plan, int32_t* dig_off) {
+    wait_for_previous();
     __shared__ int triv[kPasses];
     const int p = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint4* bins = reinterpret_cast<const uint4*>(ghist + p * 256) + 2 * lane;
@@ -358,15 +359,16 @@ __device__ __forceinline__ uint32_t warp_places(uint16_t (*whist)[256], uint32_t
 // tiles put theirs by decoupled look-back.  The keys, then the indices, go
 // through shared memory in the tile's order, so that neighbouring threads
 // write neighbouring words: the sort of 2^20 keys took 141 us with match_any
-// and a direct scatter, takes 119 (eight passes at 24 bytes a key: 28 us of
+// and a direct scatter, takes 98 (eight passes at 24 bytes a key: 28 us of
 // copying; the rest is the latency of load, rank, look-back and scatter in
 // about one wave of tiles).
-__global__ void __launch_bounds__(kPassThreads, 2) k_sort_pass(uint64_t* __restrict__ k0, uint64_t* __restrict__ k1,
-                                                            int32_t* __restrict__ v0, int32_t* __restrict__ v1,
-                                                            int ntiles, const int32_t* __restrict__ plan, int pass,
-                                                            const int32_t* __restrict__ dig_off,
-                                                            unsigned long long* __restrict__ status,
-                                                            int* __restrict__ tile_ctr, int* __restrict__ err) {
+__global__ void __launch_bounds__(kPassThreads, 2) k_sort_pass(uint64_t* k0, uint64_t* k1,
+                                                            int32_t* v0, int32_t* v1,
+                                                            int ntiles, const int32_t* plan, int pass,
+                                                            const int32_t* dig_off,
+                                                            unsigned long long* status,
+                                                            int* tile_ctr, int* err) {
+    wait_for_previous();
     if (plan[pass]) return;
     const int src = plan[8 + pass];
     const uint64_t* ks = src ? k1 : k0;
@@ -453,9 +455,10 @@ constexpr size_t one_block_bytes() {
     return (size_t)kOneThreads * ITEMS * 10 + (size_t)kOneWarps * 256 * 2;
 }
 template <int ITEMS>
-__global__ void __launch_bounds__(kOneThreads) k_sort_block(uint64_t* __restrict__ keys, int32_t* __restrict__ vals,
-                                                            const uint32_t* __restrict__ ghist,
-                                                            int32_t* __restrict__ plan) {
+__global__ void __launch_bounds__(kOneThreads) k_sort_block(uint64_t* keys, int32_t* vals,
+                                                            const uint32_t* ghist,
+                                                            int32_t* plan) {
+    wait_for_previous();
     constexpr int N = kOneThreads * ITEMS;
     extern __shared__ __align__(16) unsigned char sm[];
     uint64_t* sk = reinterpret_cast<uint64_t*>(sm);
@@ -618,11 +621,12 @@ __device__ void node_bounds(uint64_t code, int level, float half, float3& lo, fl
 // device plan left it in buffer 1 (no host read of the plan).  With curve, the
 // last `curve` digits of the keys, sorted along the Hilbert curve, become octants
 // again.
-__global__ void __launch_bounds__(256) k_gather_final(const float4* __restrict__ pos, uint64_t* __restrict__ k0,
-                                                      const uint64_t* __restrict__ k1, int32_t* __restrict__ v0,
-                                                      const int32_t* __restrict__ v1, int n,
-                                                      const int32_t* __restrict__ plan, float4* __restrict__ spos,
+__global__ void __launch_bounds__(256) k_gather_final(const float4* pos, uint64_t* k0,
+                                                      const uint64_t* k1, int32_t* v0,
+                                                      const int32_t* v1, int n,
+                                                      const int32_t* plan, float4* spos,
                                                       int curve) {
+    wait_for_previous();
     __shared__ uint32_t table[2 * kHilbertStates];
     if (curve) {   // uniform
         load_hilbert(table, true);
@@ -683,15 +687,16 @@ __device__ __forceinline__ void position_nodes(const TopoView& tv, const float4*
 constexpr int kPosThreads = 1024;
 constexpr int kPosItems = kSortTile / kPosThreads;
 static_assert(kPosItems == 4, "the scan's counts are read as one int4 a thread");
-__global__ void __launch_bounds__(kPosThreads) k_positions_scan(TopoView tv, const float4* __restrict__ spos,
-                                                                int32_t* __restrict__ pos_nint,
-                                                                int32_t* __restrict__ leaf_level,
-                                                                int32_t* __restrict__ leaf_count,
-                                                                int32_t* __restrict__ counters,
-                                                                unsigned long long* __restrict__ status, int ntiles,
-                                                                uint64_t* __restrict__ hk_zero, size_t hk_n,
-                                                                int32_t* __restrict__ host_counters,
-                                                                int* __restrict__ err) {
+__global__ void __launch_bounds__(kPosThreads) k_positions_scan(TopoView tv, const float4* spos,
+                                                                int32_t* pos_nint,
+                                                                int32_t* leaf_level,
+                                                                int32_t* leaf_count,
+                                                                int32_t* counters,
+                                                                unsigned long long* status, int ntiles,
+                                                                uint64_t* hk_zero, size_t hk_n,
+                                                                int32_t* host_counters,
+                                                                int* err) {
+    wait_for_previous();
     __shared__ int sh_warp[33], sh_off, sh_tile, sh_leaf, sh_deeper;
     __shared__ __align__(16) int sh_nint[kSortTile];
     if (hk_zero)
@@ -751,12 +756,13 @@ __global__ void __launch_bounds__(kPosThreads) k_positions_scan(TopoView tv, con
 // Emits the internal nodes starting at each sorted position (level, first
 // body, code, hash entry) and clears their child mask and counters, and the
 // look-back status of the child-count scan.
-__global__ void k_emit(TopoView tv, const int32_t* __restrict__ int_base, int32_t* __restrict__ int_level,
-                       int32_t* __restrict__ int_first, uint64_t* __restrict__ int_code, uint64_t* __restrict__ hk,
-                       int32_t* __restrict__ hv, uint32_t hmask, uint32_t* __restrict__ int_mask,
-                       int32_t* __restrict__ int_nint, int32_t* __restrict__ int_pending,
-                       int32_t* __restrict__ counters, unsigned long long* __restrict__ popc_status,
+__global__ void k_emit(TopoView tv, const int32_t* int_base, int32_t* int_level,
+                       int32_t* int_first, uint64_t* int_code, uint64_t* hk,
+                       int32_t* hv, uint32_t hmask, uint32_t* int_mask,
+                       int32_t* int_nint, int32_t* int_pending,
+                       int32_t* counters, unsigned long long* popc_status,
                        int popc_tiles) {
+    wait_for_previous();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     for (int i = s; i < popc_tiles; i += gridDim.x * blockDim.x) popc_status[i] = 0ull;   // for k_popc_scan
     if (s >= tv.n_in) return;
@@ -827,13 +833,14 @@ __device__ __forceinline__ void link_leaf(int s, const TopoView& tv, const int32
 // Every node's parent and the parents' child masks: blocks [0, int_blocks)
 // link internal nodes, the rest link the leaf starting at each position.
 // n_int_dev (graph builds) bounds the internal nodes by the device count.
-__global__ void k_link(const int32_t* __restrict__ int_level, const int32_t* __restrict__ int_first,
-                       const uint64_t* __restrict__ int_code, TopoView tv, int n_int,
-                       const int32_t* __restrict__ n_int_dev, int int_blocks, const int32_t* __restrict__ int_base,
-                       const int32_t* __restrict__ leaf_level, const uint64_t* __restrict__ hk,
-                       const int32_t* __restrict__ hv, uint32_t hmask, int32_t* __restrict__ int_parent,
-                       int32_t* __restrict__ leaf_parent, uint32_t* __restrict__ int_mask,
-                       int32_t* __restrict__ int_nint, int32_t* __restrict__ counters) {
+__global__ void k_link(const int32_t* int_level, const int32_t* int_first,
+                       const uint64_t* int_code, TopoView tv, int n_int,
+                       const int32_t* n_int_dev, int int_blocks, const int32_t* int_base,
+                       const int32_t* leaf_level, const uint64_t* hk,
+                       const int32_t* hv, uint32_t hmask, int32_t* int_parent,
+                       int32_t* leaf_parent, uint32_t* int_mask,
+                       int32_t* int_nint, int32_t* counters) {
+    wait_for_previous();
     tv.read_gaps(counters);
     if ((int)blockIdx.x < int_blocks) {
         const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -849,11 +856,12 @@ __global__ void k_link(const int32_t* __restrict__ int_level, const int32_t* __r
 // int_block[k] = non-empty children of internal nodes before k (their first
 // child cell, less one), by single-pass scan over tiles of kSortTile nodes
 // (the layout of k_positions_scan).
-__global__ void __launch_bounds__(kPosThreads) k_popc_scan(const uint32_t* __restrict__ mask, int n_int,
-                                                            const int32_t* __restrict__ n_int_dev,
-                                                            int32_t* __restrict__ out, int32_t* __restrict__ counters,
-                                                            unsigned long long* __restrict__ status, int ntiles,
-                                                            int* __restrict__ err) {
+__global__ void __launch_bounds__(kPosThreads) k_popc_scan(const uint32_t* mask, int n_int,
+                                                            const int32_t* n_int_dev,
+                                                            int32_t* out, int32_t* counters,
+                                                            unsigned long long* status, int ntiles,
+                                                            int* err) {
+    wait_for_previous();
     __shared__ int sh_warp[33], sh_off, sh_tile;
     const int tile = lb_tile_index(&counters[TC_TILE_POPC], &sh_tile);
     const int ni = n_int_dev ? min(*n_int_dev, n_int) : n_int;
@@ -988,15 +996,16 @@ __device__ __forceinline__ void place_leaf(int s, const TopoView& tv, const int3
 // (bounds, thresholds, mass and centre of mass of its body or bucket).  With
 // rec (the batched form) an internal node only gets its cell and a leaf its
 // 64-byte record.
-__global__ void k_place(const int32_t* __restrict__ int_level, const uint64_t* __restrict__ int_code,
-                        const int32_t* __restrict__ int_parent, const uint32_t* __restrict__ int_mask,
-                        const int32_t* __restrict__ int_block, int n_int, const int32_t* __restrict__ n_int_dev,
-                        int int_blocks, TopoView tv, const int32_t* __restrict__ leaf_level,
-                        const int32_t* __restrict__ leaf_count, const int32_t* __restrict__ leaf_parent,
-                        const float4* __restrict__ spos, float half, float theta_f, int32_t* __restrict__ int_cell,
-                        float4* __restrict__ cell_com, double* __restrict__ cell_mass,
-                        int32_t* __restrict__ cell_count, int4* __restrict__ cell_meta, float4* __restrict__ cell_lo,
-                        float4* __restrict__ cell_hi, uint64_t* __restrict__ cell_code, CellRec* __restrict__ rec) {
+__global__ void k_place(const int32_t* int_level, const uint64_t* int_code,
+                        const int32_t* int_parent, const uint32_t* int_mask,
+                        const int32_t* int_block, int n_int, const int32_t* n_int_dev,
+                        int int_blocks, TopoView tv, const int32_t* leaf_level,
+                        const int32_t* leaf_count, const int32_t* leaf_parent,
+                        const float4* spos, float half, float theta_f, int32_t* int_cell,
+                        float4* cell_com, double* cell_mass,
+                        int32_t* cell_count, int4* cell_meta, float4* cell_lo,
+                        float4* cell_hi, uint64_t* cell_code, CellRec* rec) {
+    wait_for_previous();
     if ((int)blockIdx.x < int_blocks) {
         const int k = blockIdx.x * blockDim.x + threadIdx.x;
         const int ni = n_int_dev ? min(*n_int_dev, n_int) : n_int;
@@ -1062,13 +1071,14 @@ __device__ __forceinline__ NodeMass sum_children(int F, int nch, const float4* c
     return m;
 }
 
-__global__ void __launch_bounds__(128) k_mass(int n_int, const int32_t* __restrict__ int_parent,
-                                              const int32_t* __restrict__ int_nint, int32_t* __restrict__ int_pending,
-                                              const int32_t* __restrict__ int_cell,
-                                              const int32_t* __restrict__ int_block,
-                                              const uint32_t* __restrict__ int_mask, float4* __restrict__ cell_com,
-                                              double* __restrict__ cell_mass, int32_t* __restrict__ cell_count,
+__global__ void __launch_bounds__(128) k_mass(int n_int, const int32_t* int_parent,
+                                              const int32_t* int_nint, int32_t* int_pending,
+                                              const int32_t* int_cell,
+                                              const int32_t* int_block,
+                                              const uint32_t* int_mask, float4* cell_com,
+                                              double* cell_mass, int32_t* cell_count,
                                               int dropped) {
+    wait_for_previous();
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n_int || int_nint[k] != 0) return;
     int cell = int_cell[k], parent = k > 0 ? int_parent[k] : 0;
@@ -1279,7 +1289,8 @@ static cudaError_t launch_sort_block(TreeBuffers& t, cudaStream_t st) {
     const cudaError_t e = cudaFuncSetAttribute(k_sort_block<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)one_block_bytes<ITEMS>());
     if (e != cudaSuccess) return e;
-    k_sort_block<ITEMS><<<1, kOneThreads, one_block_bytes<ITEMS>(), st>>>(t.keys[0], t.vals[0], t.ghist, t.plan);
+    NB_TRY(launch_after(k_sort_block<ITEMS>, 1, kOneThreads, one_block_bytes<ITEMS>(), st, t.keys[0], t.vals[0],
+                        t.ghist, t.plan));
     return cudaGetLastError();
 }
 
@@ -1295,11 +1306,11 @@ static cudaError_t launch_sort(nb_sim* sim, size_t nk) {
         return ntiles == 1 ? launch_sort_block<4>(t, st) : launch_sort_block<8>(t, st);
     }
     PhaseScope ps(sim, NB_PHASE_SORT, 1 + kPasses);
-    k_sort_plan<<<1, 256, 0, st>>>(t.ghist, (int)nk, t.plan, t.dig_off);
+    NB_TRY(launch_after(k_sort_plan, 1, 256, 0, st, t.ghist, (int)nk, t.plan, t.dig_off));
     for (int p = 0; p < kPasses; ++p)
-        k_sort_pass<<<ntiles, kPassThreads, 0, st>>>(t.keys[0], t.keys[1], t.vals[0], t.vals[1], ntiles, t.plan, p,
-                                                     t.dig_off, t.sort_status + (size_t)p * ntiles * 256,
-                                                     t.counters + TC_TILE_SORT + p, sim->d_err);
+        NB_TRY(launch_after(k_sort_pass, ntiles, kPassThreads, 0, st, t.keys[0], t.keys[1], t.vals[0], t.vals[1],
+                            ntiles, t.plan, p, t.dig_off, t.sort_status + (size_t)p * ntiles * 256,
+                            t.counters + TC_TILE_SORT + p, sim->d_err));
     return cudaGetLastError();
 }
 
@@ -1316,6 +1327,10 @@ cudaError_t tree_build(nb_sim* sim, bool export_order) {
     const int ntiles = (int)(nk / kSortTile);
     NB_TRY(tree_reserve(sim));
     cudaStream_t st = sim->stream;
+    // Every launch up to the traversal is a programmatic dependent launch
+    // (nb_common.cuh): up to 17 dependent kernels of 3 to 40 us each, whose gaps
+    // added up.  A step of 4000 bodies 155 -> 143 us, of 100,003 639 -> 600, of 2^20
+    // 3552 -> 3514.
     NB_TRY(launch_keys(sim, nk, curve));
     NB_TRY(launch_sort(sim, nk));
     // The sort result's buffer is decided on the device (passes with a constant
@@ -1323,16 +1338,16 @@ cudaError_t tree_build(nb_sim* sim, bool export_order) {
     // buffer 1, so no host read is needed here.
     {
         PhaseScope ps(sim, NB_PHASE_TOPOLOGY, 2);
-        k_gather_final<<<(n + 255) / 256, 256, 0, st>>>(sim->pos, t.keys[0], t.keys[1], t.vals[0], t.vals[1], n,
-                                                        t.plan, t.spos, curve ? sim->prm.max_depth : 0);
+        NB_TRY(launch_after(k_gather_final, (n + 255) / 256, 256, 0, st, sim->pos, t.keys[0], t.keys[1], t.vals[0],
+                            t.vals[1], n, t.plan, t.spos, curve ? sim->prm.max_depth : 0));
         t.final_buf = 0;
         TopoView tv = topo_view(sim);
         // The scan clears the hash table as it stands and sends the counters to the
         // host itself: a copy before the wait and a memset behind it
         // took 5 us more of the phase at 4000 bodies (52 now), 8 at 2^20 (192).
-        k_positions_scan<<<ntiles, kPosThreads, 0, st>>>(tv, t.spos, t.pos_nint, t.leaf_level, t.leaf_count,
-                                                          t.counters, t.pos_status, ntiles, t.hkeys, t.hash_cap,
-                                                          t.h_counters, sim->d_err);
+        NB_TRY(launch_after(k_positions_scan, ntiles, kPosThreads, 0, st, tv, t.spos, t.pos_nint, t.leaf_level,
+                            t.leaf_count, t.counters, t.pos_status, ntiles, t.hkeys, t.hash_cap, t.h_counters,
+                            sim->d_err));
         NB_TRY(cudaGetLastError());
         NB_TRY(cudaStreamSynchronize(st));
     }
@@ -1354,25 +1369,25 @@ cudaError_t tree_build(nb_sim* sim, bool export_order) {
         const int nbk = (t.n_in + kEmitBlock - 1) / kEmitBlock;
         const int ib = (ni + kEmitBlock - 1) / kEmitBlock;
         const int ptiles = (ni + kSortTile - 1) / kSortTile;
-        k_emit<<<nbk, kEmitBlock, 0, st>>>(tv, t.pos_nint, t.int_level, t.int_first, t.int_code, t.hkeys, t.hvals,
-                                          hmask, t.int_mask, t.int_nint, t.int_pending, t.counters, t.popc_status,
-                                          ptiles);
-        k_link<<<ib + nbk, kEmitBlock, 0, st>>>(t.int_level, t.int_first, t.int_code, tv, ni, nullptr, ib, t.pos_nint,
-                                               t.leaf_level, t.hkeys, t.hvals, hmask, t.int_parent, t.leaf_parent,
-                                               t.int_mask, t.int_nint, t.counters);
-        k_popc_scan<<<ptiles, kPosThreads, 0, st>>>(t.int_mask, ni, nullptr, t.int_block, t.counters,
-                                                     t.popc_status, ptiles, sim->d_err);
-        k_place<<<ib + nbk, kEmitBlock, 0, st>>>(t.int_level, t.int_code, t.int_parent, t.int_mask, t.int_block, ni,
-                                                nullptr, ib, tv, t.leaf_level, t.leaf_count, t.leaf_parent, t.spos,
-                                                sim->prm.bounds_half, tf, t.int_cell, t.cell_com, t.cell_mass,
-                                                t.cell_count, t.cell_meta, t.cell_lo, t.cell_hi, t.cell_code,
-                                                nullptr);
+        NB_TRY(launch_after(k_emit, nbk, kEmitBlock, 0, st, tv, t.pos_nint, t.int_level, t.int_first, t.int_code,
+                            t.hkeys, t.hvals, hmask, t.int_mask, t.int_nint, t.int_pending, t.counters,
+                            t.popc_status, ptiles));
+        NB_TRY(launch_after(k_link, ib + nbk, kEmitBlock, 0, st, t.int_level, t.int_first, t.int_code, tv, ni,
+                            nullptr, ib, t.pos_nint, t.leaf_level, t.hkeys, t.hvals, hmask, t.int_parent,
+                            t.leaf_parent, t.int_mask, t.int_nint, t.counters));
+        NB_TRY(launch_after(k_popc_scan, ptiles, kPosThreads, 0, st, t.int_mask, ni, nullptr, t.int_block,
+                            t.counters, t.popc_status, ptiles, sim->d_err));
+        NB_TRY(launch_after(k_place, ib + nbk, kEmitBlock, 0, st, t.int_level, t.int_code, t.int_parent, t.int_mask,
+                            t.int_block, ni, nullptr, ib, tv, t.leaf_level, t.leaf_count, t.leaf_parent, t.spos,
+                            sim->prm.bounds_half, tf, t.int_cell, t.cell_com, t.cell_mass, t.cell_count,
+                            t.cell_meta, t.cell_lo, t.cell_hi, t.cell_code, nullptr));
         NB_TRY(cudaGetLastError());
     }
     {
         PhaseScope ps(sim, NB_PHASE_MASS);
-        k_mass<<<(ni + 127) / 128, 128, 0, st>>>(ni, t.int_parent, t.int_nint, t.int_pending, t.int_cell, t.int_block,
-                                                t.int_mask, t.cell_com, t.cell_mass, t.cell_count, n - t.n_in);
+        NB_TRY(launch_after(k_mass, (ni + 127) / 128, 128, 0, st, ni, t.int_parent, t.int_nint, t.int_pending,
+                            t.int_cell, t.int_block, t.int_mask, t.cell_com, t.cell_mass, t.cell_count,
+                            n - t.n_in));
         NB_TRY(cudaGetLastError());
     }
     sim->tree_valid = true;
@@ -1452,24 +1467,25 @@ cudaError_t tree_build_graph(nb_sim* sim, const float4* pos, int n, int D, bool 
     const int ib = (icap + kEmitBlock - 1) / kEmitBlock;
     const int ptiles = (icap + kSortTile - 1) / kSortTile;
     PhaseScope ps(sim, NB_PHASE_TOPOLOGY, 6);
-    k_gather_final<<<(n + 255) / 256, 256, 0, st>>>(pos, t.keys[0], t.keys[1], t.vals[0], t.vals[1], n, t.plan,
-                                                    t.spos, kMortonLevels);
+    NB_TRY(launch_after(k_gather_final, (n + 255) / 256, 256, 0, st, pos, t.keys[0], t.keys[1], t.vals[0],
+                        t.vals[1], n, t.plan, t.spos, kMortonLevels));
     // this scan also clears the internal-node hash table for the emission
-    k_positions_scan<<<ntiles, kPosThreads, 0, st>>>(tv, t.spos, t.pos_nint, t.leaf_level, t.leaf_count, t.counters,
-                                                      t.pos_status, ntiles, counts_only ? nullptr : t.hkeys,
-                                                      t.hash_cap, nullptr, sim->d_err);
+    NB_TRY(launch_after(k_positions_scan, ntiles, kPosThreads, 0, st, tv, t.spos, t.pos_nint, t.leaf_level,
+                        t.leaf_count, t.counters, t.pos_status, ntiles, counts_only ? nullptr : t.hkeys, t.hash_cap,
+                        nullptr, sim->d_err));
     if (counts_only) return cudaGetLastError();   // the node counts are in counters[TC_NINT], [TC_NLEAF]
-    k_emit<<<nbk, kEmitBlock, 0, st>>>(tv, t.pos_nint, t.int_level, t.int_first, t.int_code, t.hkeys, t.hvals, hmask,
-                                      t.int_mask, t.int_nint, t.int_pending, t.counters, t.popc_status, ptiles);
-    k_link<<<ib + nbk, kEmitBlock, 0, st>>>(t.int_level, t.int_first, t.int_code, tv, icap, t.counters + TC_NINT, ib,
-                                           t.pos_nint, t.leaf_level, t.hkeys, t.hvals, hmask, t.int_parent,
-                                           t.leaf_parent, t.int_mask, t.int_nint, t.counters);
-    k_popc_scan<<<ptiles, kPosThreads, 0, st>>>(t.int_mask, icap, t.counters + TC_NINT, t.int_block, t.counters,
-                                                 t.popc_status, ptiles, sim->d_err);
-    k_place<<<ib + nbk, kEmitBlock, 0, st>>>(t.int_level, t.int_code, t.int_parent, t.int_mask, t.int_block, icap,
-                                            t.counters + TC_NINT, ib, tv, t.leaf_level, t.leaf_count, t.leaf_parent,
-                                            t.spos, sim->prm.bounds_half, 1.0f, t.int_cell, t.cell_com, t.cell_mass,
-                                            t.cell_count, t.cell_meta, t.cell_lo, t.cell_hi, t.cell_code, rec);
+    NB_TRY(launch_after(k_emit, nbk, kEmitBlock, 0, st, tv, t.pos_nint, t.int_level, t.int_first, t.int_code,
+                        t.hkeys, t.hvals, hmask, t.int_mask, t.int_nint, t.int_pending, t.counters, t.popc_status,
+                        ptiles));
+    NB_TRY(launch_after(k_link, ib + nbk, kEmitBlock, 0, st, t.int_level, t.int_first, t.int_code, tv, icap,
+                        t.counters + TC_NINT, ib, t.pos_nint, t.leaf_level, t.hkeys, t.hvals, hmask, t.int_parent,
+                        t.leaf_parent, t.int_mask, t.int_nint, t.counters));
+    NB_TRY(launch_after(k_popc_scan, ptiles, kPosThreads, 0, st, t.int_mask, icap, t.counters + TC_NINT,
+                        t.int_block, t.counters, t.popc_status, ptiles, sim->d_err));
+    NB_TRY(launch_after(k_place, ib + nbk, kEmitBlock, 0, st, t.int_level, t.int_code, t.int_parent, t.int_mask,
+                        t.int_block, icap, t.counters + TC_NINT, ib, tv, t.leaf_level, t.leaf_count, t.leaf_parent,
+                        t.spos, sim->prm.bounds_half, 1.0f, t.int_cell, t.cell_com, t.cell_mass, t.cell_count,
+                        t.cell_meta, t.cell_lo, t.cell_hi, t.cell_code, rec));
     return cudaGetLastError();
 }
 

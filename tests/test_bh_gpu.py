@@ -316,3 +316,20 @@ def test_shared_groups_decide_like_the_oracle(n):
     assert inter == inter_o or deeper > 0
     assert O.rel_l2(F, Fo) < 1e-5
     np.testing.assert_array_equal(F, again)
+
+
+@pytest.mark.parametrize("n", [1000, 8000, 60000])
+def test_steps_follow_each_other(n):
+    """Each launch waits for the one before: 30 queued steps are those of 30
+    calls with a synchronisation behind each, byte for byte."""
+    pm, v = nb.seed_plummer(8, n)
+    out = []
+    for chunk in (30, 1):
+        with bh_sim(theta=0.7) as s:
+            s.init_soa(pm, v)
+            for _ in range(30 // chunk):
+                s.step(1e-3, chunk)
+                s.synchronize()
+            out.append(s.read_state())
+    for a, b in zip(*out):
+        assert a.tobytes() == b.tobytes()
