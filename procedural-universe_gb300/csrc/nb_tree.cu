@@ -443,23 +443,17 @@ __global__ void __launch_bounds__(kPassThreads, 2) k_sort_pass(uint64_t* k0, uin
     for (int it = 0; it < kPassItems; ++it) vd[dst[it]] = vstage[it * kPassThreads + threadIdx.x];
 }
 
-// The whole sort of at most 1024 * ITEMS keys in one block: every pass ranks
-// the keys in registers and reorders them in shared memory, where the plan and
-// one launch per pass cost 58 to 70 us however few the keys: 27 to 35 us for
-// 4000 keys, 46 for 7000 (58).  Three tiles (12 keys a thread, which spill)
-// took 78 against 66 and four 98 against 63: those stay with the passes.  The
+// The whole sort of one tile's keys in one block: every pass ranks the keys in
+// registers and reorders them in shared memory, where the plan and one launch per
+// pass cost 40 to 50 us however few the keys: 27 to 36 us for 4000 keys.  (Two
+// tiles so took 46 us against 44, with four keys more a thread to keep.)  The
 // keys end in buffer 0.
-constexpr int kOneThreads = 1024, kOneWarps = kOneThreads / 32;
-template <int ITEMS>
-constexpr size_t one_block_bytes() {
-    return (size_t)kOneThreads * ITEMS * 10 + (size_t)kOneWarps * 256 * 2;
-}
-template <int ITEMS>
-__global__ void __launch_bounds__(kOneThreads) k_sort_block(uint64_t* keys, int32_t* vals,
-                                                            const uint32_t* ghist,
+constexpr int kOneThreads = 1024, kOneWarps = kOneThreads / 32, kOneItems = kSortTile / kOneThreads;
+constexpr size_t kOneBytes = (size_t)kSortTile * 10 + (size_t)kOneWarps * 256 * 2;   // keys, indices, histograms
+__global__ void __launch_bounds__(kOneThreads) k_sort_block(uint64_t* keys, int32_t* vals, const uint32_t* ghist,
                                                             int32_t* plan) {
     wait_for_previous();
-    constexpr int N = kOneThreads * ITEMS;
+    constexpr int N = kSortTile, ITEMS = kOneItems;
     extern __shared__ __align__(16) unsigned char sm[];
     uint64_t* sk = reinterpret_cast<uint64_t*>(sm);
     uint16_t* sv = reinterpret_cast<uint16_t*>(sk + N);
@@ -1283,27 +1277,25 @@ static cudaError_t launch_keys(nb_sim* sim, size_t nk, bool curve) {
     return cudaGetLastError();
 }
 
-template <int ITEMS>
 static cudaError_t launch_sort_block(TreeBuffers& t, cudaStream_t st) {
     // (set on each call: cheap, and right for every device)
-    const cudaError_t e = cudaFuncSetAttribute(k_sort_block<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)one_block_bytes<ITEMS>());
+    const cudaError_t e = cudaFuncSetAttribute(k_sort_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)kOneBytes);
     if (e != cudaSuccess) return e;
-    NB_TRY(launch_after(k_sort_block<ITEMS>, 1, kOneThreads, one_block_bytes<ITEMS>(), st, t.keys[0], t.vals[0],
+    NB_TRY(launch_after(k_sort_block, 1, kOneThreads, kOneBytes, st, t.keys[0], t.vals[0],
                         t.ghist, t.plan));
     return cudaGetLastError();
 }
 
-// The radix sort of t.keys[0] / t.vals[0] (histograms already made): in one
-// block up to two tiles, else the device plan, then one launch per pass.
+// The radix sort of t.keys[0] / t.vals[0] (histograms already made): one tile
+// in one block, else the device plan, then one launch per pass.
 static cudaError_t launch_sort(nb_sim* sim, size_t nk) {
     TreeBuffers& t = sim->tree;
     const int ntiles = (int)(nk / kSortTile);
     cudaStream_t st = sim->stream;
-    static_assert(kSortTile == 4 * kOneThreads, "a tile is four keys a thread");
-    if (ntiles <= 2) {
+    if (ntiles == 1) {
         PhaseScope ps(sim, NB_PHASE_SORT);
-        return ntiles == 1 ? launch_sort_block<4>(t, st) : launch_sort_block<8>(t, st);
+        return launch_sort_block(t, st);
     }
     PhaseScope ps(sim, NB_PHASE_SORT, 1 + kPasses);
     NB_TRY(launch_after(k_sort_plan, 1, 256, 0, st, t.ghist, (int)nk, t.plan, t.dig_off));
