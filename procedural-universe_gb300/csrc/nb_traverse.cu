@@ -78,12 +78,13 @@ cudaError_t tree_forces(nb_sim* sim) {
     const float S = (float)sim->prm.softening2;
     const float G = (float)sim->prm.G;
     PhaseScope ps(sim, NB_PHASE_TRAVERSE);
-    // Warps that share a group: as many as keep the GPU's resident warps (20 an
-    // SM) busy.  A shared walk repeats its first steps and parts unevenly, so it
-    // pays only while warps are missing: 30,000 bodies 318 us alone, 271 by two,
-    // 197 by four; 80,000 428, 386, 552; 100,003 435, 540, 653.
-    const long long groups = (n + kTravBodies - 1) / kTravBodies, slots = 20ll * std::max(1, sim->sm_count);
-    const int share = groups * 4 <= slots ? 4 : groups * 2 <= slots * 5 / 6 ? 2 : 1;
+    // Warps that share a group: as many as keep the GPU's resident warps busy (16 an
+    // SM for these kernels, and a few groups more in a second wave).  A shared walk
+    // repeats its first steps and parts unevenly, so it pays only while warps are
+    // missing: 40,000 bodies 249 us by four, 259 by two; 47,000 364 and 323; 80,000
+    // 376 to 452 by two (two models), 412 to 417 alone; 100,003 552 and 440.
+    const long long groups = (n + kTravBodies - 1) / kTravBodies, slots = 33ll * std::max(1, sim->sm_count) / 2;
+    const int share = groups * 4 <= slots ? 4 : groups * 2 <= slots ? 2 : 1;
     const int per_block = kTravWarps / share;
     const unsigned blocks = (unsigned)((groups + per_block - 1) / per_block);
 #define NB_TRAV(L, K)                                                                                          \
