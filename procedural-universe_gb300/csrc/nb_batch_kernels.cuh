@@ -508,9 +508,11 @@ struct FarField {
     float v[kFarTerms];
 };
 
-// Adds one cell's terms to a lane's partial sums (term k at f[k * stride]).
+// Adds one cell's terms to a lane's partial sums in shared memory, four terms a
+// 16-byte word (term 4 k + c is component c of f[k * stride]): a quarter of the
+// loads and stores of single terms.
 template <int LAW>
-__device__ __forceinline__ void far_add(float* f, int stride, const float4 cm, const float4 q1, const float4 q2,
+__device__ __forceinline__ void far_add(float4* f, int stride, const float4 cm, const float4 q1, const float4 q2,
                                         float Xx, float Xy, float Xz, float S) {
     const float dx = cm.x - Xx, dy = cm.y - Xy, dz = cm.z - Xz;
     const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
@@ -530,37 +532,46 @@ __device__ __forceinline__ void far_add(float* f, int stride, const float4 cm, c
     const float qz = fmaf(q2.y, dx, fmaf(q2.z, dy, q1.z * dz));
     const float sq = fmaf(dx, qx, fmaf(dy, qy, dz * qz));   // d.Q.d
     const float c7 = 2.5f * sq * ir7;
-    f[0 * stride] += fmaf(w + c7, dx, -qx * ir5);
-    f[1 * stride] += fmaf(w + c7, dy, -qy * ir5);
-    f[2 * stride] += fmaf(w + c7, dz, -qz * ir5);
+    float4 t;
+    auto T = [&](int k, float x) {
+        switch (k & 3) {   // k is a constant
+            case 0: t = f[(k >> 2) * stride]; t.x += x; break;
+            case 1: t.y += x; break;
+            case 2: t.z += x; break;
+            default: t.w += x; f[(k >> 2) * stride] = t;
+        }
+    };
+    T(0, fmaf(w + c7, dx, -qx * ir5));
+    T(1, fmaf(w + c7, dy, -qy * ir5));
+    T(2, fmaf(w + c7, dz, -qz * ir5));
     const float m3 = 3.f * m * ir5, m1 = m * ir3;
     const float t5 = 5.f * ir7, g9 = 17.5f * sq * ir7 * ir2, dg = m1 + c7;   // c7 = 5/2 s / r^7
-    f[3 * stride] += fmaf(m3 * dx, dx, -dg) + fmaf(q1.x, ir5, dx * fmaf(g9, dx, -2.f * t5 * qx));   // J xx
-    f[4 * stride] += fmaf(m3 * dy, dy, -dg) + fmaf(q1.y, ir5, dy * fmaf(g9, dy, -2.f * t5 * qy));   // J yy
-    f[5 * stride] += fmaf(m3 * dx + g9 * dx, dy, fmaf(q2.x, ir5, -t5 * fmaf(qx, dy, qy * dx)));     // J xy
-    f[6 * stride] += fmaf(m3 * dx + g9 * dx, dz, fmaf(q2.y, ir5, -t5 * fmaf(qx, dz, qz * dx)));     // J xz
-    f[7 * stride] += fmaf(m3 * dy + g9 * dy, dz, fmaf(q2.z, ir5, -t5 * fmaf(qy, dz, qz * dy)));     // J yz
+    T(3, fmaf(m3 * dx, dx, -dg) + fmaf(q1.x, ir5, dx * fmaf(g9, dx, -2.f * t5 * qx)));   // J xx
+    T(4, fmaf(m3 * dy, dy, -dg) + fmaf(q1.y, ir5, dy * fmaf(g9, dy, -2.f * t5 * qy)));   // J yy
+    T(5, fmaf(m3 * dx + g9 * dx, dy, fmaf(q2.x, ir5, -t5 * fmaf(qx, dy, qy * dx))));     // J xy
+    T(6, fmaf(m3 * dx + g9 * dx, dz, fmaf(q2.y, ir5, -t5 * fmaf(qx, dz, qz * dx))));     // J xz
+    T(7, fmaf(m3 * dy + g9 * dy, dz, fmaf(q2.z, ir5, -t5 * fmaf(qy, dz, qz * dy))));     // J yz
     const float m15 = 15.f * m * ir7;
     const float tx = m15 * dx, ty = m15 * dy;
-    f[8 * stride] += dx * fmaf(tx, dx, -3.f * m3);    // H xxx = 15 m dx^3 / r^7 - 9 m dx / r^5
-    f[9 * stride] += dy * fmaf(ty, dy, -3.f * m3);    // H yyy
-    f[10 * stride] += dy * fmaf(tx, dx, -m3);         // H xxy
-    f[11 * stride] += dz * fmaf(tx, dx, -m3);         // H xxz
-    f[12 * stride] += dx * fmaf(ty, dy, -m3);         // H xyy
-    f[13 * stride] += dz * fmaf(ty, dy, -m3);         // H yyz
-    f[14 * stride] += tx * dy * dz;                   // H xyz
+    T(8, dx * fmaf(tx, dx, -3.f * m3));    // H xxx = 15 m dx^3 / r^7 - 9 m dx / r^5
+    T(9, dy * fmaf(ty, dy, -3.f * m3));    // H yyy
+    T(10, dy * fmaf(tx, dx, -m3));         // H xxy
+    T(11, dz * fmaf(tx, dx, -m3));         // H xxz
+    T(12, dx * fmaf(ty, dy, -m3));         // H xyy
+    T(13, dz * fmaf(ty, dy, -m3));         // H yyz
+    T(14, tx * dy * dz);                   // H xyz
     const float a9 = 105.f * m * ir7 * ir2;           // 105 m / r^9
     const float x2 = dx * dx, y2 = dy * dy;
     const float ax2 = a9 * x2, ay2 = a9 * y2;
-    f[15 * stride] += fmaf(x2, ax2 - 6.f * m15, 3.f * m3);          // T xxxx
-    f[16 * stride] += fmaf(y2, ay2 - 6.f * m15, 3.f * m3);          // T yyyy
-    f[17 * stride] += fmaf(ax2, y2, fmaf(-m15, x2 + y2, m3));        // T xxyy
-    f[18 * stride] += dx * dy * (ax2 - 3.f * m15);                  // T xxxy
-    f[19 * stride] += dx * dy * (ay2 - 3.f * m15);                  // T xyyy
-    f[20 * stride] += dx * dz * (ax2 - 3.f * m15);                  // T xxxz
-    f[21 * stride] += dx * dz * (ay2 - m15);                        // T xyyz
-    f[22 * stride] += dy * dz * (ax2 - m15);                        // T xxyz
-    f[23 * stride] += dy * dz * (ay2 - 3.f * m15);                  // T yyyz
+    T(15, fmaf(x2, ax2 - 6.f * m15, 3.f * m3));          // T xxxx
+    T(16, fmaf(y2, ay2 - 6.f * m15, 3.f * m3));          // T yyyy
+    T(17, fmaf(ax2, y2, fmaf(-m15, x2 + y2, m3)));        // T xxyy
+    T(18, dx * dy * (ax2 - 3.f * m15));                  // T xxxy
+    T(19, dx * dy * (ay2 - 3.f * m15));                  // T xyyy
+    T(20, dx * dz * (ax2 - 3.f * m15));                  // T xxxz
+    T(21, dx * dz * (ay2 - m15));                        // T xyyz
+    T(22, dy * dz * (ax2 - m15));                        // T xxyz
+    T(23, dy * dz * (ay2 - 3.f * m15));                  // T yyyz
 }
 
 // A + J y + 1/2 H(y, y) + 1/6 T(y, y, y) at offset y from the expansion centre.
@@ -590,6 +601,13 @@ __device__ __forceinline__ void far_eval(const FarField& f, float x, float y, fl
 }
 
 // Persistent: each warp takes groups from the queue until it is empty.
+// Bound by instruction issue (62% of the cycles, five warps a scheduler, their
+// stalls mostly the fixed latency of dependent instructions): a group of 52
+// bodies meets 368 cells and 1917 bodies in 90 walk steps at 1,048,576 bodies, a
+// third to the bodies' evaluation and nearly half to the steps.  Four body pairs
+// an iteration, four far-field terms a shared-memory word, exact powers of two
+// for ldexpf and the gather below: 2.93 -> 2.76 ms a step there, 16 galaxies of
+// 65,536 2.78 -> 2.63, 200 of 2048 to 8192 1.64 -> 1.57.
 template <int LAW>
 __global__ void __launch_bounds__(kGWarps * 32, 5) k_group_traverse(
     GroupList groups,
@@ -602,8 +620,8 @@ __global__ void __launch_bounds__(kGWarps * 32, 5) k_group_traverse(
     __shared__ int stk[kGWarps][kGStack];
     __shared__ float4 lcl[kGWarps][kGCells / 2][5];
     __shared__ float4 lbd[kGWarps][kGBodies / 2][2];
-    __shared__ float ffs[kGWarps][kFarTerms][32];   // far-field partial sums, one column per lane
-    __shared__ int rinc[kGWarps][32], rfst[kGWarps][32];
+    __shared__ float4 ffs[kGWarps][kFarTerms / 4][32];   // far-field partial sums, one column per lane
+    __shared__ int rfst[kGWarps][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
     const float2 S2 = make_float2(S, S);
@@ -659,7 +677,7 @@ __global__ void __launch_bounds__(kGWarps * 32, 5) k_group_traverse(
         if (a2 > 0.f && a2 < INFINITY) far_thr = far_rel * sqrtf(a2);
     }
     const bool use_far = far2 > 0.f || far_rel > 0.f;
-    for (int k = 0; k < kFarTerms; ++k) ffs[w][k][lane] = 0.f;   // this lane's share of the far field
+    for (int k = 0; k < kFarTerms / 4; ++k) ffs[w][k][lane] = make_float4(0.f, 0.f, 0.f, 0.f);   // this lane's share of the far field
     // negated target coordinates, duplicated: the pair partner is the other list entry
     const float2 n0x = make_float2(-p0.x, -p0.x), n0y = make_float2(-p0.y, -p0.y), n0z = make_float2(-p0.z, -p0.z);
     const float2 n1x = make_float2(-p1.x, -p1.x), n1y = make_float2(-p1.y, -p1.y), n1z = make_float2(-p1.z, -p1.z);
@@ -714,9 +732,9 @@ __global__ void __launch_bounds__(kGWarps * 32, 5) k_group_traverse(
         auto body_loop = [&](auto both) {
             int k = 0;
 #pragma unroll 1
-            for (; k + 2 <= np; k += 2) {
+            for (; k + 4 <= np; k += 4) {
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
+                for (int u = 0; u < 4; ++u) {
                     const float4 e0 = lbd[w][k + u][0], e1 = lbd[w][k + u][1];
                     const float2 bx = make_float2(e0.x, e0.y), by = make_float2(e0.z, e0.w);
                     const float2 bz = make_float2(e1.x, e1.y), bm = make_float2(e1.z, e1.w);
@@ -741,35 +759,36 @@ __global__ void __launch_bounds__(kGWarps * 32, 5) k_group_traverse(
     };
     // Appends the bodies of this step's accepted leaf ranges (lane l: first,
     // count; count 0 for lanes without one) to the body list, all lanes
-    // copying, evaluating the list whenever it fills.
+    // copying, 32 bodies at a time, evaluating the list whenever it fills.  A
+    // body's range is the last that starts at or before it: the starts of a
+    // window as a bit mask (a binary search in the ranges' ends cost five
+    // dependent reads a body; this took 3% off the batched step).  The list is
+    // filled to its last place, so that its evaluation, four pairs at a time,
+    // has no rest but at the walk's end: flushing at the last whole window instead
+    // took all of that back.
     auto gather_ranges = [&](int first, int count) {
         int incl = count;
         for (int o = 1; o < 32; o <<= 1) {
             const int t = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += t;
         }
-        const int tot = __shfl_sync(0xffffffffu, incl, 31);
+        const int tot = __shfl_sync(0xffffffffu, incl, 31), start = incl - count;
+        const uint32_t some = __ballot_sync(0xffffffffu, count > 0);
         __syncwarp();
-        rinc[w][lane] = incl;
-        rfst[w][lane] = first;
+        if (count > 0) rfst[w][__popc(some & lt)] = first - start;
         __syncwarp();
-        for (int done = 0; done < tot;) {
+        int before = -1;   // the last range that starts before the window
+        for (int done = 0, take; done < tot; done += take) {
             if (nbd == kGBodies) flush_bodies();
-            const int take = min(kGBodies - nbd, tot - done);
-            for (int j = lane; j < take; j += 32) {
-                const int jj = done + j;
-                int lo = 0, hi = 31;   // owner: the first lane whose inclusive end exceeds jj
-                while (lo < hi) {
-                    const int mid = (lo + hi) >> 1;
-                    if (rinc[w][mid] > jj) hi = mid; else lo = mid + 1;
-                }
-                const int base = lo > 0 ? rinc[w][lo - 1] : 0;
-                put_body(lbd[w], nbd + j, spos[rfst[w][lo] + (jj - base)]);
-            }
+            take = min(min(32, kGBodies - nbd), tot - done);
+            const unsigned at = (unsigned)(start - done);
+            const uint32_t starts = __reduce_or_sync(0xffffffffu, count > 0 && at < (unsigned)take ? 1u << at : 0u);
+            if (lane < take)
+                put_body(lbd[w], nbd + lane, spos[rfst[w][before + __popc(starts & ((2u << lane) - 1u))] + done + lane]);
+            before += __popc(starts);
             nbd += take;
-            done += take;
-            __syncwarp();
         }
+        __syncwarp();
     };
 
     const int root = gal_root[grp.x];
@@ -831,7 +850,7 @@ __global__ void __launch_bounds__(kGWarps * 32, 5) k_group_traverse(
             // The group form of the reference's rule side / r < theta: r is bounded
             // below for every body of the group by the distance from the centre of
             // mass to the group's bounding box.
-            const float side = ldexpf(gb.w, kSlotLevels - (wr.w >> 8));
+            const float side = gb.w * __int_as_float((127 + kSlotLevels - (wr.w >> 8)) << 23);   // box size / 2^level   // box size / 2^level
             float d2 = 0.f;
             const float cc[3] = {ccm.x, ccm.y, ccm.z};
             for (int a = 0; a < 3; ++a) {
@@ -891,8 +910,10 @@ __global__ void __launch_bounds__(kGWarps * 32, 5) k_group_traverse(
     // the group's far field: sum the lanes' partial expansions, evaluate at each body
     if (use_far) {
         FarField ff;
+#pragma unroll
         for (int k = 0; k < kFarTerms; ++k) {
-            float x = ffs[w][k][lane];
+            const float4 t = ffs[w][k >> 2][lane];
+            float x = (k & 3) == 0 ? t.x : (k & 3) == 1 ? t.y : (k & 3) == 2 ? t.z : t.w;
             for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
             ff.v[k] = x;
         }
