@@ -85,21 +85,25 @@ cudaError_t tree_forces(nb_sim* sim) {
     // 376 to 452 by two (two models), 412 to 417 alone; 100,003 552 and 440.
     const long long groups = (n + kTravBodies - 1) / kTravBodies, slots = 33ll * std::max(1, sim->sm_count) / 2;
     const int share = groups * 4 <= slots ? 4 : groups * 2 <= slots ? 2 : 1;
+    // Alone, a warp gets 126 registers while every group still finds a place at 16
+    // warps an SM, else 96: 100,003 bodies 430 us (447 at 96), 200,000 785 (717).
+    const bool roomy = groups <= 16ll * std::max(1, sim->sm_count);
     const int per_block = kTravWarps / share;
     const unsigned blocks = (unsigned)((groups + per_block - 1) / per_block);
-#define NB_TRAV(L, K)                                                                                          \
-    k_traverse<L, K><<<blocks, kTravBlock, 0, st>>>(t.spos, t.vals[t.final_buf], n, t.cell_com, t.cell_meta,   \
-                                                    t.cell_lo, t.n_cells, t.n_int + 1, tf, S, G, sim->acc,     \
-                                                    t.interactions, sim->d_err)
-    if (sim->prm.law == NB_LAW_PLUMMER) {
-        if (share == 4) NB_TRAV(NB_LAW_PLUMMER, 4);
-        else if (share == 2) NB_TRAV(NB_LAW_PLUMMER, 2);
-        else NB_TRAV(NB_LAW_PLUMMER, 1);
-    } else {
-        if (share == 4) NB_TRAV(NB_LAW_REFERENCE, 4);
-        else if (share == 2) NB_TRAV(NB_LAW_REFERENCE, 2);
-        else NB_TRAV(NB_LAW_REFERENCE, 1);
-    }
+#define NB_TRAV(L, K, B)                                                                                       \
+    k_traverse<L, K, B><<<blocks, kTravBlock, 0, st>>>(t.spos, t.vals[t.final_buf], n, t.cell_com, t.cell_meta, \
+                                                       t.cell_lo, t.n_cells, t.n_int + 1, tf, S, G, sim->acc,  \
+                                                       t.interactions, sim->d_err)
+#define NB_TRAV_LAW(L)                         \
+    do {                                       \
+        if (share == 4) NB_TRAV(L, 4, 4);      \
+        else if (share == 2) NB_TRAV(L, 2, 4); \
+        else if (roomy) NB_TRAV(L, 1, 4);      \
+        else NB_TRAV(L, 1, 0);                 \
+    } while (0)
+    if (sim->prm.law == NB_LAW_PLUMMER) NB_TRAV_LAW(NB_LAW_PLUMMER);
+    else NB_TRAV_LAW(NB_LAW_REFERENCE);
+#undef NB_TRAV_LAW
 #undef NB_TRAV
     return cudaGetLastError();
 }

@@ -89,8 +89,11 @@ __device__ __forceinline__ void bucket_accel(const float4* __restrict__ spos, in
 constexpr int kSplitAt = 12;   // waiting entries at which a shared group's warps part
 enum : int { CL_NONE = -1, CL_SOURCE = 0, CL_OPEN = 2, CL_DECIDE = 3, CL_EMPTY = 4 };
 
-template <int LAW, int K>
-__global__ void __launch_bounds__(kTravBlock) k_traverse(const float4* __restrict__ spos,
+// BLOCKS: blocks an SM is to hold, which sets the registers (4: 126; 0, the
+// compiler's own choice: 96 and five blocks; asked for five outright it does
+// 1.5% worse at 1,048,576 bodies).
+template <int LAW, int K, int BLOCKS>
+__global__ void __launch_bounds__(kTravBlock, BLOCKS) k_traverse(const float4* __restrict__ spos,
                                                          const int32_t* __restrict__ sorder, int n,
                                                          const float4* __restrict__ cell_com,
                                                          const int4* __restrict__ cell_meta,
