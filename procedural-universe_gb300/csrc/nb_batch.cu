@@ -268,7 +268,7 @@ int enqueue_step(nb_batch* b, float dt, bool update, bool tree_only = false) {
             else launch_direct<NB_LAW_REFERENCE, 4>(b, st, S);
         }
         const int cnt = (int)(b->n_total - b->dir_begin);   // a multiple of 256
-        k_batch_direct_reduce<<<cnt / 256 * kFoldLanes, 256, 0, st>>>(b->body_dgal, b->dgal, (int)b->dir_begin, cnt, G,
+        k_batch_direct_reduce<<<cnt / 32, 32 * kFoldWarps, 0, st>>>(b->body_dgal, b->dgal, (int)b->dir_begin, G,
                                                                      b->part, c->acc);
         NB_BCUDA(b, cudaGetLastError());
     }

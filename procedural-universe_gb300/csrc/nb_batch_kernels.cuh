@@ -948,8 +948,8 @@ __global__ void __launch_bounds__(kGWarps * 32, 5) k_group_traverse(
 // Bound by the FP32 pipe.  Warps share nothing, so that no barrier waits for
 // the slowest; the next chunk and the next unit are fetched while the current
 // chunk is evaluated.  GB300, 200 members of 256-4096 bodies: force
-// kernel 387 -> 237 us and the fold 8 -> 44 us (ncu, cold caches; it now reads a
-// partial per row and body), a step 399 -> 281 us; FMA pipe 63% busy, the rest
+// kernel 387 -> 235 us and the fold 8 -> 34 us (ncu, cold caches; it now reads a
+// partial per row and body), a step 399 -> 270 us; FMA pipe 63% busy, the rest
 // is the shuffles and reads that four targets a lane carry (eight: 268 us a
 // step, but small members then fill fewer rows).
 constexpr int kDirWarps = 8;   // most warps per block
@@ -1013,13 +1013,16 @@ struct DirGal {
     int base, splits, once, sources;   // first entry, splits, each pair once?, source bodies (to a whole chunk)
 };
 
-// Folds the partials of direct-sum body i (global index begin + i) into acc:
-// kFoldLanes consecutive threads a body, in a fixed order.
-__global__ void k_batch_direct_reduce(const int32_t* __restrict__ body_dgal, const DirGal* __restrict__ dgal, int begin,
-                                      int count, float G, const float4* __restrict__ part, float4* __restrict__ acc) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = t / kFoldLanes, j = t % kFoldLanes;
-    if (i >= count) return;   // whole groups of lanes; count is a multiple of a block's bodies
+// Folds the partials of direct-sum body i (global index begin + i) into acc, in
+// a fixed order: a block's warps share 32 bodies (of one row).  With eight
+// neighbouring threads a body instead, whose reads are a row apart, the fold of 200
+// members of 256-4096 bodies took 44 us instead of 34, a step 294 instead of 283.
+__global__ void __launch_bounds__(32 * kFoldWarps) k_batch_direct_reduce(const int32_t* __restrict__ body_dgal,
+                                                                         const DirGal* __restrict__ dgal, int begin,
+                                                                         float G, const float4* __restrict__ part,
+                                                                         float4* __restrict__ acc) {
+    __shared__ float sums[kFoldWarps][6][32];
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31), j = threadIdx.x >> 5;
     const int g = body_dgal[i];
     float ax = 0.f, ay = 0.f, az = 0.f, kx = 0.f, ky = 0.f, kz = 0.f;
     if (g >= 0) {   // not a padding body
@@ -1033,17 +1036,16 @@ __global__ void k_batch_direct_reduce(const int32_t* __restrict__ body_dgal, con
         const int behind = d.sources - (d.once ? row * d.row : 0);
         const int used = (behind + d.split - 1) / d.split;
 #pragma unroll 4
-        for (int s = j; s < used; s += kFoldLanes) add(part[(size_t)d.base + (size_t)s * d.n_pad + local]);
+        for (int s = j; s < used; s += kFoldWarps) add(part[(size_t)d.base + (size_t)s * d.n_pad + local]);
         if (d.once) {
             const float4* src = part + (size_t)d.base + (size_t)d.splits * d.n_pad;
 #pragma unroll 4
-            for (int r = j; r < row; r += kFoldLanes)
+            for (int r = j; r < row; r += kFoldWarps)
                 add(src[(size_t)r * d.n_pad - (size_t)d.row * r * (r + 1) / 2 + (local - (r + 1) * d.row)]);
         }
     }
-    const HiLo x = butterfly_total(ax, kx), y = butterfly_total(ay, ky), z = butterfly_total(az, kz);
-    if (g >= 0 && j == 0)
-        acc[begin + i] = make_float4(G * x.rounded(), G * y.rounded(), G * z.rounded(), 0.f);
+    const float3 f = add_warps(sums, ax, ay, az, kx, ky, kz);
+    if (g >= 0 && j == 0) acc[begin + i] = make_float4(G * f.x, G * f.y, G * f.z, 0.f);
 }
 
 }  // namespace nb

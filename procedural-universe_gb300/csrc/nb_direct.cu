@@ -604,14 +604,12 @@ __global__ void k_direct_reduce_update(const float4* __restrict__ part, int spli
 }
 
 // The fold of k_direct_rows' partials: a block's warps share 32 bodies, warp j
-// taking every kRowFold-th partial of them (neighbouring bodies' entries lie
-// together), and the first warp adds the warps' sums in order.  Returns the
-// force in the first warp's threads.
-constexpr int kRowFold = 8;
+// taking every kFoldWarps-th partial of them.  Returns the force in the first
+// warp's threads.
 __device__ __forceinline__ float3 fold_rows(const float4* part, const RowPlan& plan, int n_pad, int i, int j,
                                             float (*sums)[6][32]) {
     float ax = 0.f, ay = 0.f, az = 0.f, kx = 0.f, ky = 0.f, kz = 0.f;
-    const int row = i / kRowBodies, lane = threadIdx.x & 31;   // one row a block
+    const int row = i / kRowBodies;   // one row a block
     auto add = [&](const float4 p) {
         kahan_add(ax, kx, p.x);
         kahan_add(ay, ky, p.y);
@@ -619,32 +617,15 @@ __device__ __forceinline__ float3 fold_rows(const float4* part, const RowPlan& p
     };
     const int used = plan.row_units(row);
 #pragma unroll 4
-    for (int s = j; s < used; s += kRowFold) add(part[(size_t)s * n_pad + i]);
+    for (int s = j; s < used; s += kFoldWarps) add(part[(size_t)s * n_pad + i]);
 #pragma unroll 4
-    for (int r = j; r < row; r += kRowFold) add(part[row_source_base(plan, r, n_pad) + (i - (r + 1) * kRowBodies)]);
-    sums[j][0][lane] = ax; sums[j][1][lane] = ay; sums[j][2][lane] = az;
-    sums[j][3][lane] = kx; sums[j][4][lane] = ky; sums[j][5][lane] = kz;
-    __syncthreads();
-    float r[3] = {0.f, 0.f, 0.f};
-    if (j == 0) {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            float hi = sums[0][d][lane], lo = -sums[0][3 + d][lane];
-#pragma unroll
-            for (int w = 1; w < kRowFold; ++w) {
-                float e;
-                hi = two_sum(hi, sums[w][d][lane], e);
-                lo += e - sums[w][3 + d][lane];
-            }
-            r[d] = hi + lo;
-        }
-    }
-    return make_float3(r[0], r[1], r[2]);
+    for (int r = j; r < row; r += kFoldWarps) add(part[row_source_base(plan, r, n_pad) + (i - (r + 1) * kRowBodies)]);
+    return add_warps(sums, ax, ay, az, kx, ky, kz);
 }
 
-__global__ void __launch_bounds__(32 * kRowFold) k_direct_rows_update(const float4* part, RowPlan plan, int n, int n_pad,
+__global__ void __launch_bounds__(32 * kFoldWarps) k_direct_rows_update(const float4* part, RowPlan plan, int n, int n_pad,
                                                                       UpdateArgs u, const int* err) {
-    __shared__ float sums[kRowFold][6][32];
+    __shared__ float sums[kFoldWarps][6][32];
     const int i = blockIdx.x * 32 + (threadIdx.x & 31), j = threadIdx.x >> 5;
     wait_for_previous();
     const int failed = *err;
@@ -941,7 +922,7 @@ cudaError_t direct_force_update(nb_sim* sim, float dt, bool update) {
     if (pairs)
         k_direct_reduce_update<true><<<rblocks, 256, 0, sim->stream>>>(sim->part, splits, pf, carry, n, (int)sim->n_pad, ua, sim->d_err);
     else if (by_rows)
-        return launch_after(k_direct_rows_update, (unsigned)((n + 31) / 32), 32 * kRowFold, 0, sim->stream,
+        return launch_after(k_direct_rows_update, (unsigned)((n + 31) / 32), 32 * kFoldWarps, 0, sim->stream,
                             sim->part, rp, n, (int)sim->n_pad, ua, sim->d_err);
     else
         k_direct_reduce_update<false><<<rblocks, 256, 0, sim->stream>>>(sim->part, splits, pf, carry, n, (int)sim->n_pad, ua, sim->d_err);
@@ -1014,9 +995,9 @@ __global__ void k_noalloc_reduce(const float4* __restrict__ part, PairFold pf, c
 }
 
 // The same for k_direct_rows (which has no wait to run out).
-__global__ void __launch_bounds__(32 * kRowFold) k_noalloc_rows(const float4* part, RowPlan plan, int n, int n_pad,
+__global__ void __launch_bounds__(32 * kFoldWarps) k_noalloc_rows(const float4* part, RowPlan plan, int n, int n_pad,
                                                                 float G, float4* acc) {
-    __shared__ float sums[kRowFold][6][32];
+    __shared__ float sums[kFoldWarps][6][32];
     const int i = blockIdx.x * 32 + (threadIdx.x & 31), j = threadIdx.x >> 5;
     const float3 s = fold_rows(part, plan, n_pad, i, j, sums);
     if (i >= n || j != 0) return;
@@ -1080,7 +1061,7 @@ extern "C" int nb_direct_accel_noalloc(const float* pos_mass4, size_t n, float* 
     if (n_pad <= kRowMaxNoAlloc) {
         const RowPlan rp = row_plan((int)n, (int)n_pad, kNoAllocScratch - n_pad);
         if (launch_rows(rp, law, st, pos, (int)n_pad, S, mmax, part) != cudaSuccess) return NB_ECUDA;
-        k_noalloc_rows<<<(unsigned)((n + 31) / 32), 32 * kRowFold, 0, st>>>(part, rp, (int)n, (int)n_pad, (float)G, acc);
+        k_noalloc_rows<<<(unsigned)((n + 31) / 32), 32 * kFoldWarps, 0, st>>>(part, rp, (int)n, (int)n_pad, (float)G, acc);
     } else {
         PairFold pf{};
         const float4* carry = nullptr;
