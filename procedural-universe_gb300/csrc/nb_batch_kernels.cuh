@@ -949,7 +949,7 @@ __global__ void __launch_bounds__(kGWarps * 32, 5) k_group_traverse(
 // the slowest; the next chunk and the next unit are fetched while the current
 // chunk is evaluated.  GB300, 200 members of 256-4096 bodies: force
 // kernel 387 -> 235 us and the fold 8 -> 34 us (ncu, cold caches; it now reads a
-// partial per row and body), a step 399 -> 270 us; FMA pipe 63% busy, the rest
+// partial per row and body), ten steps and a read 4.76 -> 2.83 ms; FMA pipe 63% busy, the rest
 // is the shuffles and reads that four targets a lane carry (eight: 268 us a
 // step, but small members then fill fewer rows).
 constexpr int kDirWarps = 8;   // most warps per block
@@ -1044,7 +1044,7 @@ __global__ void __launch_bounds__(32 * kFoldWarps) k_batch_direct_reduce(const i
                 add(src[(size_t)r * d.n_pad - (size_t)d.row * r * (r + 1) / 2 + (local - (r + 1) * d.row)]);
         }
     }
-    const float3 f = add_warps(sums, ax, ay, az, kx, ky, kz);
+    const float3 f = add_warps(sums, ax, ay, az, kx, ky, kz).rounded();
     if (g >= 0 && j == 0) acc[begin + i] = make_float4(G * f.x, G * f.y, G * f.z, 0.f);
 }
 

@@ -479,13 +479,16 @@ __device__ __forceinline__ HiLo3 fold_partials_lanes(const float4* __restrict__ 
 
 // The same for k_direct_pairs' partials of rows [row0, row0 + rows): body i's
 // target partials when its row is among them, and its entry as a source of
-// each of those rows before its own.
+// each of those rows before its own.  A block's warps share 32 bodies (of one
+// row), warp j taking every kFoldWarps-th entry; the first warp gets the totals.
+// (Eight neighbouring threads a body: 10.6 us a fold at 50,001 bodies, now 8.9;
+// the allocation-free call there 945 -> 937, a step of 262,144 20.10 -> 20.02 ms.)
 struct PairFold {
     int per, row0, rows;   // tiles a unit, first row, rows
 };
 
-__device__ __forceinline__ HiLo3 fold_pairs_lanes(const float4* __restrict__ part, const PairFold& pf, int n_pad, int i,
-                                                   int j) {
+__device__ __forceinline__ HiLo3 fold_pairs(const float4* __restrict__ part, const PairFold& pf, int n_pad, int i, int j,
+                                            float (*sums)[6][32]) {
     float ax = 0.f, ay = 0.f, az = 0.f, kx = 0.f, ky = 0.f, kz = 0.f;
     const int row = i / kPairRow, last = pf.row0 + pf.rows, all = n_pad / kPairRow;
     auto add = [&](const float4 p) {
@@ -498,14 +501,14 @@ __device__ __forceinline__ HiLo3 fold_pairs_lanes(const float4* __restrict__ par
         const int used = pair_units_before(row + 1, pf.row0, all, pf.per) - first;
         const float4* targets = part + (size_t)first * kPairRow + (i - row * kPairRow);
 #pragma unroll 4
-        for (int u = j; u < used; u += kFoldLanes) add(targets[(size_t)u * kPairRow]);
+        for (int u = j; u < used; u += kFoldWarps) add(targets[(size_t)u * kPairRow]);
     }
     const float4* sources = part + (size_t)pair_units_before(last, pf.row0, all, pf.per) * kPairRow;
     const int end = min(row, last);
 #pragma unroll 4
-    for (int r = pf.row0 + j; r < end; r += kFoldLanes)
+    for (int r = pf.row0 + j; r < end; r += kFoldWarps)
         add(sources[pair_source_base(r, pf.row0, n_pad) + (size_t)(i - (r + 1) * kPairRow)]);
-    return HiLo3{butterfly_total(ax, kx), butterfly_total(ay, ky), butterfly_total(az, kz)};
+    return add_warps(sums, ax, ay, az, kx, ky, kz);
 }
 
 // Adds a fold's total to a running (sum, low part); either may be the larger,
@@ -518,12 +521,12 @@ __device__ __forceinline__ void add_total(float& s, float& low, const HiLo& f) {
 
 // Folds the partials of one of several launches of k_direct_pairs into the
 // bodies' running (sum, low part); the first launch starts them.
-__global__ void k_pairs_carry(const float4* __restrict__ part, PairFold pf, int n_pad, int first,
+__global__ void __launch_bounds__(32 * kFoldWarps) k_pairs_carry(const float4* __restrict__ part, PairFold pf, int n_pad, int first,
                               float4* __restrict__ carry, const int* __restrict__ err) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = t / kFoldLanes, j = t % kFoldLanes;
-    if (i >= n_pad || *err != 0) return;
-    const HiLo3 f = fold_pairs_lanes(part, pf, n_pad, i, j);
+    __shared__ float sums[kFoldWarps][6][32];
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31), j = threadIdx.x >> 5;
+    if (*err != 0) return;
+    const HiLo3 f = fold_pairs(part, pf, n_pad, i, j, sums);
     if (j != 0) return;
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f), c = s;
     if (!first) {
@@ -586,17 +589,29 @@ __device__ __forceinline__ void finish_body(const UpdateArgs& u, int i, const fl
     if (u.rv) write_vertex(u.rv, u.rcol, u.rscale, i, x);
 }
 
-// PAIRS: the partials are k_direct_pairs' (carry: the earlier launches' sums,
-// when there were several), else k_direct_force's.
-template <bool PAIRS>
-__global__ void k_direct_reduce_update(const float4* __restrict__ part, int splits, PairFold pf,
-                                       const float4* __restrict__ carry, int n, int n_pad, UpdateArgs u,
+// After k_direct_force.
+__global__ void k_direct_reduce_update(const float4* __restrict__ part, int splits, int n, int n_pad, UpdateArgs u,
                                        const int* __restrict__ err) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = t / kFoldLanes, j = t % kFoldLanes;
     // whole groups of lanes leave together (n_pad bodies, a multiple of the block)
     if (i >= n_pad || *err != 0) return;
-    const HiLo3 total = PAIRS ? fold_pairs_lanes(part, pf, n_pad, i, j) : fold_partials_lanes(part, splits, n_pad, i, j);
+    const HiLo3 total = fold_partials_lanes(part, splits, n_pad, i, j);
+    if (i >= n || j != 0) return;
+    BodyState b;
+    b.read(u, i);
+    finish_body(u, i, total.rounded(), b);
+}
+
+// After k_direct_pairs (carry: the earlier launches' sums, when there were several).
+__global__ void __launch_bounds__(32 * kFoldWarps) k_direct_pairs_update(const float4* __restrict__ part, PairFold pf,
+                                                                         const float4* __restrict__ carry, int n,
+                                                                         int n_pad, UpdateArgs u,
+                                                                         const int* __restrict__ err) {
+    __shared__ float sums[kFoldWarps][6][32];
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31), j = threadIdx.x >> 5;
+    if (*err != 0) return;
+    const HiLo3 total = fold_pairs(part, pf, n_pad, i, j, sums);
     if (i >= n || j != 0) return;
     BodyState b;
     b.read(u, i);
@@ -620,7 +635,7 @@ __device__ __forceinline__ float3 fold_rows(const float4* part, const RowPlan& p
     for (int s = j; s < used; s += kFoldWarps) add(part[(size_t)s * n_pad + i]);
 #pragma unroll 4
     for (int r = j; r < row; r += kFoldWarps) add(part[row_source_base(plan, r, n_pad) + (i - (r + 1) * kRowBodies)]);
-    return add_warps(sums, ax, ay, az, kx, ky, kz);
+    return add_warps(sums, ax, ay, az, kx, ky, kz).rounded();
 }
 
 __global__ void __launch_bounds__(32 * kFoldWarps) k_direct_rows_update(const float4* part, RowPlan plan, int n, int n_pad,
@@ -802,8 +817,7 @@ static int launch_pairs(int sm_count, int law, cudaStream_t st, const float4* po
         ++made;
         *last = p;
         if (r0 + p.rows < rows) {
-            k_pairs_carry<<<(unsigned)((size_t)n_pad * kFoldLanes / 256), 256, 0, st>>>(part, p, n_pad, r0 == 0 ? 1 : 0,
-                                                                                       carry_buf, err);
+            k_pairs_carry<<<(unsigned)(n_pad / 32), 32 * kFoldWarps, 0, st>>>(part, p, n_pad, r0 == 0 ? 1 : 0, carry_buf, err);
             ++made;
             *carry = carry_buf;
         }
@@ -918,14 +932,15 @@ cudaError_t direct_force_update(nb_sim* sim, float dt, bool update) {
     sim->inter_last = (uint64_t)(nn * (nn - 1.0));
     PhaseScope ps(sim, 1);
     static_assert(kPad % (256 / kFoldLanes) == 0 && kPad % 32 == 0, "the fold's blocks cover whole padded bodies");
-    const unsigned rblocks = (unsigned)(sim->n_pad * kFoldLanes / 256);
     if (pairs)
-        k_direct_reduce_update<true><<<rblocks, 256, 0, sim->stream>>>(sim->part, splits, pf, carry, n, (int)sim->n_pad, ua, sim->d_err);
+        k_direct_pairs_update<<<(unsigned)((n + 31) / 32), 32 * kFoldWarps, 0, sim->stream>>>(
+            sim->part, pf, carry, n, (int)sim->n_pad, ua, sim->d_err);
     else if (by_rows)
         return launch_after(k_direct_rows_update, (unsigned)((n + 31) / 32), 32 * kFoldWarps, 0, sim->stream,
                             sim->part, rp, n, (int)sim->n_pad, ua, sim->d_err);
     else
-        k_direct_reduce_update<false><<<rblocks, 256, 0, sim->stream>>>(sim->part, splits, pf, carry, n, (int)sim->n_pad, ua, sim->d_err);
+        k_direct_reduce_update<<<(unsigned)(sim->n_pad * kFoldLanes / 256), 256, 0, sim->stream>>>(
+            sim->part, splits, n, (int)sim->n_pad, ua, sim->d_err);
     return cudaGetLastError();
 }
 
@@ -980,12 +995,12 @@ __global__ void k_noalloc_stage(const float4* __restrict__ in, int n, int n_pad,
 
 // Folds the partials like k_direct_reduce_update; a force kernel whose bounded
 // wait ran out poisons the output with NaN, since nothing is read back.
-__global__ void k_noalloc_reduce(const float4* __restrict__ part, PairFold pf, const float4* __restrict__ carry, int n,
-                                 int n_pad, float G, float4* __restrict__ acc) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = t / kFoldLanes, j = t % kFoldLanes;
-    if (i >= n_pad) return;   // whole groups of lanes (the padded size is a multiple of the block's bodies)
-    const HiLo3 f = fold_pairs_lanes(part, pf, n_pad, i, j);
+__global__ void __launch_bounds__(32 * kFoldWarps) k_noalloc_reduce(const float4* __restrict__ part, PairFold pf,
+                                                                    const float4* __restrict__ carry, int n, int n_pad,
+                                                                    float G, float4* __restrict__ acc) {
+    __shared__ float sums[kFoldWarps][6][32];
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31), j = threadIdx.x >> 5;
+    const HiLo3 f = fold_pairs(part, pf, n_pad, i, j, sums);
     if (i >= n || j != 0) return;
     const float3 s = with_carry(f, carry, n_pad, i);
     float4 a = make_float4(G * s.x, G * s.y, G * s.z, 0.f);
@@ -1078,8 +1093,8 @@ extern "C" int nb_direct_accel_noalloc(const float* pos_mass4, size_t n, float* 
         }
         const size_t cap = kNoAllocScratch - 3 * n_pad;
         launch_pairs<true, kFold / 2>(sms, law, st, pos, (int)n_pad, S, part, cap, false, part + cap, err, kMaxPolls, mmax, &pf, &carry);
-        k_noalloc_reduce<<<(unsigned)(n_pad * kFoldLanes / 256), 256, 0, st>>>(part, pf, carry, (int)n, (int)n_pad,
-                                                                              (float)G, acc);
+        k_noalloc_reduce<<<(unsigned)((n + 31) / 32), 32 * kFoldWarps, 0, st>>>(part, pf, carry, (int)n, (int)n_pad, (float)G,
+                                                                                acc);
     }
     if (cudaGetLastError() != cudaSuccess) return NB_ECUDA;
     return NB_OK;

@@ -128,6 +128,7 @@ struct HiLo {
 };
 struct HiLo3 {
     HiLo x, y, z;
+    __device__ __forceinline__ float3 rounded() const { return make_float3(x.rounded(), y.rounded(), z.rounded()); }
 };
 
 __device__ __forceinline__ HiLo butterfly_total(float s, float c) {
@@ -148,27 +149,26 @@ __device__ __forceinline__ HiLo butterfly_total(float s, float c) {
 // (s, c); the first warp's threads get the totals, added in the warps' order with
 // the rounding errors carried.  Every thread of the block calls it.
 constexpr int kFoldWarps = 8;
-__device__ __forceinline__ float3 add_warps(float (*sums)[6][32], float ax, float ay, float az, float kx, float ky,
+__device__ __forceinline__ HiLo3 add_warps(float (*sums)[6][32], float ax, float ay, float az, float kx, float ky,
                                             float kz) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     sums[w][0][lane] = ax; sums[w][1][lane] = ay; sums[w][2][lane] = az;
     sums[w][3][lane] = kx; sums[w][4][lane] = ky; sums[w][5][lane] = kz;
     __syncthreads();
-    float r[3] = {0.f, 0.f, 0.f};
+    HiLo r[3] = {};
     if (w == 0) {
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            float hi = sums[0][d][lane], lo = -sums[0][3 + d][lane];
+            r[d] = HiLo{sums[0][d][lane], -sums[0][3 + d][lane]};
 #pragma unroll
             for (int v = 1; v < kFoldWarps; ++v) {
                 float e;
-                hi = two_sum(hi, sums[v][d][lane], e);
-                lo += e - sums[v][3 + d][lane];
+                r[d].hi = two_sum(r[d].hi, sums[v][d][lane], e);
+                r[d].lo += e - sums[v][3 + d][lane];
             }
-            r[d] = hi + lo;
         }
     }
-    return make_float3(r[0], r[1], r[2]);
+    return HiLo3{r[0], r[1], r[2]};
 }
 
 // One warp's evaluation of a chunk of 32 sources (in shared memory) against its
