@@ -731,10 +731,6 @@ int direct_splits(const nb_sim* sim, const DirectTuning& t, size_t n_pad) {
     return (ntiles + tps - 1) / tps;
 }
 
-size_t direct_part_entries(const nb_sim* sim, const DirectTuning& t, size_t n_pad) {
-    return (size_t)direct_splits(sim, t, n_pad) * 2 * n_pad;
-}
-
 static DirectTuning default_tuning(size_t n_pad) {
     DirectTuning t;
     t.block = 128;

@@ -200,7 +200,6 @@ namespace nb {
 // the same reduction kernel also performs the kick-drift update.
 cudaError_t direct_force_update(nb_sim* sim, float dt, bool update);
 int direct_splits(const nb_sim* sim, const DirectTuning& t, size_t n_pad);
-size_t direct_part_entries(const nb_sim* sim, const DirectTuning& t, size_t n_pad);
 
 // Generic kick-drift of bodies from sim->acc (used after a Barnes-Hut force pass).
 // hold (device tree counters, optional): a step whose tree does not fit
