@@ -5,16 +5,19 @@
 // (src/Sim/BruteForceGPU.cpp:45-71).
 //
 // Layout: bodies are float4 (x, y, z, m) in HBM, padded to a multiple of
-// kPad with zero-mass bodies.  A work unit of K1 is (target block, source
-// range): BLOCK*IPT target bodies held in registers against a contiguous
-// range of source tiles.  Each 128-body source tile (2 KB) is moved from HBM
-// to shared memory by the TMA engine (cp.async.bulk) into a double buffer
-// guarded by mbarriers; every thread then reads each source body as a
-// broadcast float4.  Forces are accumulated in FP32 in groups of kFold
-// sources, and each group sum is folded into a Kahan-compensated total.
-// Each unit writes its (sum, compensation) partials; K7 folds the partials of
-// all source ranges in a fixed order (deterministic), applies G, and performs
-// the kick-drift with Kahan-compensated velocity and position.
+// kPad with zero-mass bodies.  Three force kernels:
+//   * k_direct_pairs (large states): each unordered pair once, blocks taking
+//     rows of 1024 targets against the source tiles behind them;
+//   * k_direct_rows (small states): the same by single warps, rows of 128;
+//   * k_direct_force (tuned handles, uncompensated sums): every interaction
+//     from its target's side, BLOCK * IPT targets in registers against a
+//     contiguous range of 128-body source tiles.
+// The block kernels move source tiles (2 KB) from HBM to shared memory by the
+// TMA engine (cp.async.bulk) into a double buffer guarded by mbarriers.  Forces
+// are accumulated in FP32 in groups of sources, each group's sum folded into a
+// compensated total.  K7 folds the partials in a fixed order (deterministic),
+// applies G, and performs the kick-drift with Kahan-compensated velocity and
+// position.
 //
 // Force law per source j on target i (reference law, Phys::Gravity,
 // src/Sim/Physics.hpp:25-35, S = softening2):

@@ -4,8 +4,8 @@
 // Replaces Octree::CalculateForce (src/Sim/Octree.cpp:107-145) called for
 // every body by BarnesHut::Exec (src/Sim/BarnesHut.cpp:103-110).
 //
-// A warp owns 64 consecutive bodies of the key-sorted order, two per lane
-// (spatially close, so their walks mostly coincide).  The warp shares one
+// A warp owns 64 consecutive bodies of the sorted order (along the Hilbert
+// curve), two per lane (spatially close, so their walks mostly coincide).  The warp shares one
 // node stack in shared memory; an entry is (child range of a cell, lane mask
 // per body slot): the bodies that decided to open that cell.  Popping an
 // entry, lanes 0..7 load the
@@ -23,7 +23,7 @@
 // with the cell's precomputed accept / reject thresholds; only when r^2 falls
 // between them (a 2e-5 relative band) is the exactly rounded ratio
 // float(side / sqrtf(r^2)) compared with theta_f, the smallest float >= Theta.
-// Forces are summed in FP32 per popped cell and folded into a Kahan total.
+// Forces are summed in FP32 per evaluated list and folded into a Kahan total.
 #include "nb_common.cuh"
 #include "nb_internal.hpp"
 #include "nb_law.cuh"
