@@ -227,8 +227,11 @@ __device__ __forceinline__ void finish_moments(int c, int F, int nch, int first,
 // The bound is the chain of round trips from the deepest node to its root: a
 // node's own words are read while the arrival counter is on the way, and a
 // node with one internal child needs no counter (its other children are
-// leaves, complete since the placement).
-__global__ void __launch_bounds__(128) k_batch_moments(
+// leaves, complete since the placement).  In large states it is the nodes in
+// flight: 128 registers give four blocks an SM where 137 gave three (a step of 180
+// galaxies of 8192 to 65,536 bodies 8.98 -> 8.85 ms, of 16 x 65,536 2.63 -> 2.61; 96
+// registers spill: 8.95).  Eight lanes a node, at 40 registers, took 9.02.
+__global__ void __launch_bounds__(128, 4) k_batch_moments(
     int int_cap, const int32_t* __restrict__ counters, const int32_t* __restrict__ int_parent,
     const int32_t* __restrict__ int_nint, int32_t* __restrict__ int_pending, const int32_t* __restrict__ int_cell,
     const int32_t* __restrict__ int_block, const uint32_t* __restrict__ int_mask,
