@@ -1193,6 +1193,7 @@ static cudaError_t reserve_nodes(nb_sim* sim, size_t n_int, size_t n_cells) {
     TreeBuffers& t = sim->tree;
     if (n_int > t.int_cap) {
         const size_t cap = n_int + n_int / 4 + 64;
+        t.int_cap = 0;   // until every array is there: a failed allocation is made good by the next call
         NB_TRY(grow((void**)&t.int_level, cap * 4, sim->stream));
         NB_TRY(grow((void**)&t.int_first, cap * 4, sim->stream));
         NB_TRY(grow((void**)&t.int_parent, cap * 4, sim->stream));
@@ -1205,15 +1206,16 @@ static cudaError_t reserve_nodes(nb_sim* sim, size_t n_int, size_t n_cells) {
         // internal nodes can outnumber bodies (chains of one-child nodes above
         // close pairs): the child-count scan's status is sized by them
         NB_TRY(grow((void**)&t.popc_status, ((cap + kSortTile - 1) / kSortTile) * sizeof(unsigned long long), sim->stream));
-        t.int_cap = cap;
         size_t h = 1024;
         while (h < 2 * cap) h <<= 1;
         NB_TRY(grow((void**)&t.hkeys, h * 8, sim->stream));
         NB_TRY(grow((void**)&t.hvals, h * 4, sim->stream));
         t.hash_cap = h;
+        t.int_cap = cap;
     }
     if (n_cells > t.cell_cap) {
         const size_t cap = n_cells + n_cells / 4 + 64;
+        t.cell_cap = 0;
         NB_TRY(grow((void**)&t.cell_com, cap * 16, sim->stream));
         NB_TRY(grow((void**)&t.cell_meta, cap * 16, sim->stream));
         NB_TRY(grow((void**)&t.cell_mass, cap * 8, sim->stream));
@@ -1349,9 +1351,10 @@ cudaError_t tree_build(nb_sim* sim, bool export_order) {
     t.trivial = (n < 2) || (t.n_in < 2 && t.n_int == 0) || t.n_in == 0;
     t.curve = curve;
     if (t.trivial) return cudaSuccess;
-    const size_t cleared = t.hash_cap;
+    const size_t cleared = t.int_cap;
     NB_TRY(reserve_nodes(sim, (size_t)t.n_int, (size_t)t.n_cells));
-    if (t.hash_cap != cleared) NB_TRY(cudaMemsetAsync(t.hkeys, 0, t.hash_cap * 8, st));   // grew
+    // grown arrays come with a new table, of the same size or not
+    if (t.int_cap != cleared) NB_TRY(cudaMemsetAsync(t.hkeys, 0, t.hash_cap * 8, st));
     TopoView tv = topo_view(sim);
     const int ni = t.n_int;
     const float tf = theta_float(sim->prm.theta);

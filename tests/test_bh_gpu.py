@@ -333,3 +333,23 @@ def test_steps_follow_each_other(n):
             out.append(s.read_state())
     for a, b in zip(*out):
         assert a.tobytes() == b.tobytes()
+
+
+def test_tree_arrays_growing_step_by_step():
+    """Node arrays that grow a little at a time, so that the table of internal
+    nodes is often replaced by one of the same size: each state's step is that
+    of a fresh handle, byte for byte."""
+    sizes, n = [], 300
+    while n < 6000:
+        sizes.append(n)
+        n = int(n * 1.3) + 1
+    with bh_sim(theta=0.5) as s:
+        for n in sizes:
+            pm, v = nb.seed_plummer(n, n)
+            out = []
+            for h in (s, bh_sim(theta=0.5)):
+                h.init_soa(pm, v)
+                h.step(1e-3, 2)
+                out.append(h.read_state())
+            for a, b in zip(*out):
+                assert a.tobytes() == b.tobytes(), n
