@@ -77,6 +77,7 @@ struct TreeBuffers {
     // counters (device: kCounterWords words, then ghist) and their pinned host mirror
     int32_t* counters = nullptr;
     int32_t* h_counters = nullptr;
+    cudaEvent_t counted = nullptr;          // h_counters have arrived
     unsigned long long* interactions = nullptr;
     // host view of the last build
     int n_in = 0, n_int = 0, n_cells = 0, final_buf = 0;
