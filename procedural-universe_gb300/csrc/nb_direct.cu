@@ -876,8 +876,10 @@ static cudaError_t force_pairs(nb_sim* sim, PairFold* last, const float4** carry
 cudaError_t direct_force_update(nb_sim* sim, float dt, bool update) {
     const bool comp = !(sim->prm.flags & NB_FLAG_NO_COMPENSATION);
     // Each pair once.  A handle whose launch was tuned, and uncompensated sums,
-    // keep k_direct_force.
-    const bool once = comp && !sim->tune_set, by_rows = once && sim->n_pad <= kRowMax, pairs = once && !by_rows;
+    // keep k_direct_force; so do small states whose waits were tuned
+    // (k_direct_rows has none that could run out).
+    const bool small = sim->n_pad <= kRowMax, once = comp && !sim->tune_set && !(small && sim->wait_polls != kMaxPolls);
+    const bool by_rows = once && small, pairs = once && !small;
     RowPlan rp{};
     int splits = 0;
     PairFold pf{};

@@ -373,3 +373,30 @@ def test_steps_of_small_states_follow_each_other(n):
             out.append(s.read_state())
     for a, b in zip(*out):
         assert a.tobytes() == b.tobytes()
+
+
+@pytest.mark.parametrize("n", [1000, 20000])
+def test_bounded_wait_runs_out_in_small_states(n):
+    """A handle of few bodies whose waits were lowered still reports the
+    timeout with its state unchanged, and steps on once they are restored."""
+    pm, v = nb.seed_plummer(21, n)
+    rec = nb.records_from_soa(pm, v)
+    with direct_sim() as s:
+        s.init(rec)
+        s.tune("wait_polls", 0)
+        s.step(1e-3, 1)
+        with pytest.raises(nb.NBodyError) as ei:
+            s.synchronize()
+        assert ei.value.code == nb.NB_ETIMEOUT
+        out = rec.copy()
+        s.write_back(out)
+        np.testing.assert_array_equal(out["position"], rec["position"])
+        s.tune("wait_polls", 1 << 22)
+        s.step(1e-3, 1)
+        s.write_back(out)
+    with direct_sim() as s:
+        want = rec.copy()
+        s.init(rec)
+        s.step(1e-3, 1)
+        s.write_back(want)
+    assert out.tobytes() == want.tobytes()
