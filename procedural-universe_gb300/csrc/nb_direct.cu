@@ -299,8 +299,8 @@ __global__ void __launch_bounds__(kPairThreads, 3) k_direct_pairs(const float4* 
 #pragma unroll
                         for (int q = 0; q < P; ++q) {
                             const float2 dx = __fadd2_rn(jx, nx[q]), dy = __fadd2_rn(jy, ny[q]), dz = __fadd2_rn(jz, nz[q]);
-                            const float2 w = pair_factor_x2<LAW>(dx, dy, dz, S2, T2);
-                            const float2 wi = __fmul2_rn(jm, w), wj = __fmul2_rn(mi[q], w);
+                            float2 wi, wj;
+                            pair_factors_x2<LAW>(dx, dy, dz, S2, T2, jm, mi[q], wi, wj);
                             ax[q] = __ffma2_rn(wi, dx, ax[q]);
                             ay[q] = __ffma2_rn(wi, dy, ay[q]);
                             az[q] = __ffma2_rn(wi, dz, az[q]);

@@ -81,23 +81,33 @@ __device__ __forceinline__ void interact_x2(float2 jx, float2 jy, float2 jz, flo
     az = __ffma2_rn(w, dz, az);
 }
 
-// The law's factor without a mass, for two pairs at once: the force on either
-// body of a pair is the other's mass times it times the separation.
+// The factors of the separation for both bodies of two pairs at once: wi, with
+// the mass jm of one body, is the acceleration of the other, and wj, with mi, its
+// own.  Under the Plummer law a mass enters before the cube of the inverse
+// distance is complete, as in interact_x2: the cube alone leaves FP32's range
+// beyond 4e12 length units (and with a softening below 1e-13), far inside that
+// of the factor (states in metres and kilograms, or in very small units).
 template <int LAW>
-__device__ __forceinline__ float2 pair_factor_x2(float2 dx, float2 dy, float2 dz, float2 S2, float2 T2) {
+__device__ __forceinline__ void pair_factors_x2(float2 dx, float2 dy, float2 dz, float2 S2, float2 T2, float2 jm,
+                                                float2 mi, float2& wi, float2& wj) {
     if (LAW == NB_LAW_REFERENCE) {
         float2 r2 = __fmul2_rn(dx, dx);
         r2 = __ffma2_rn(dy, dy, r2);
         r2 = __ffma2_rn(dz, dz, r2);
         const float2 s = __fadd2_rn(r2, S2);
         const float2 t = __ffma2_rn(__fmul2_rn(r2, s), s, T2);
-        return make_float2(rsqrt_approx(t.x), rsqrt_approx(t.y));
+        const float2 w = make_float2(rsqrt_approx(t.x), rsqrt_approx(t.y));
+        wi = __fmul2_rn(jm, w);
+        wj = __fmul2_rn(mi, w);
+        return;
     }
     float2 q = __ffma2_rn(dx, dx, S2);
     q = __ffma2_rn(dy, dy, q);
     q = __ffma2_rn(dz, dz, q);
     const float2 inv = make_float2(rsqrt_approx(q.x), rsqrt_approx(q.y));
-    return __fmul2_rn(inv, __fmul2_rn(inv, inv));
+    const float2 inv2 = __fmul2_rn(inv, inv);
+    wi = __fmul2_rn(__fmul2_rn(jm, inv), inv2);
+    wj = __fmul2_rn(__fmul2_rn(mi, inv), inv2);
 }
 
 // kahan_add of two sums at once in packed instructions (the same roundings);
@@ -201,13 +211,12 @@ __device__ __forceinline__ void direct_chunk(const float4* src, int lane, const 
 #pragma unroll
             for (int q = 0; q < P; ++q) {
                 const float2 dx = __fadd2_rn(jx, nx[q]), dy = __fadd2_rn(jy, ny[q]), dz = __fadd2_rn(jz, nz[q]);
-                const float2 w = pair_factor_x2<LAW>(dx, dy, dz, S2, T2);
-                const float2 wi = __fmul2_rn(jm, w);
+                float2 wi, wj;
+                pair_factors_x2<LAW>(dx, dy, dz, S2, T2, jm, mi[q], wi, wj);
                 ax[q] = __ffma2_rn(wi, dx, ax[q]);
                 ay[q] = __ffma2_rn(wi, dy, ay[q]);
                 az[q] = __ffma2_rn(wi, dz, az[q]);
                 if (BOTH) {
-                    const float2 wj = __fmul2_rn(mi[q], w);
                     bx = __ffma2_rn(wj, dx, bx);
                     by = __ffma2_rn(wj, dy, by);
                     bz = __ffma2_rn(wj, dz, bz);
