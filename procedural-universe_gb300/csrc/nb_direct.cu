@@ -29,6 +29,7 @@
 #include "nb_common.cuh"
 #include "nb_internal.hpp"
 #include "nb_law.cuh"
+#include "nb_pair_plan.hpp"
 #include <algorithm>
 #include <cmath>
 
@@ -194,29 +195,12 @@ __global__ void __launch_bounds__(BLOCK) k_direct_force(const float4* __restrict
 // force error against FP64 is k_direct_force's (2.8e-8 and 2.8e-8 at 262,144
 // bodies of the Plummer sphere, 3.5e-8 and 3.5e-8 at 20,001).
 constexpr int kPairThreads = 128, kPairIpt = 8, kPairGroup = 4;
-constexpr int kPairRow = kPairThreads * kPairIpt;
-constexpr int kPairRowTiles = kPairRow / kTileJ;
+static_assert(kPairRow == kPairThreads * kPairIpt && kPairRowTiles == kPairRow / kTileJ, "the planner's rows");
 static_assert(kPairThreads == kTileJ, "one thread per source of a tile");
 static_assert(kPad % kPairRow == 0, "padded states hold whole rows");
 
-// Units of the rows [row0, row) of a state, `per` tiles a unit (1, 2, 4 or a
-// multiple of 8): row q has (rows - q) * kPairRowTiles source tiles.
-__host__ __device__ __forceinline__ int pair_units_before(int row, int row0, int rows, int per) {
-    const int a = rows - row0, k = row - row0;
-    if (per <= kPairRowTiles) return kPairRowTiles / per * (a * k - k * (k - 1) / 2);
-    const int m = per / kPairRowTiles;   // sum of ceil(i / m) over a - k < i <= a
-    const int qa = a / m, qb = (a - k) / m;
-    return m * (qa * (qa + 1) - qb * (qb + 1)) / 2 + (a % m) * (qa + 1) - ((a - k) % m) * (qb + 1);
-}
-
-// Source entries of the rows before `row` in a launch that starts at row0.
-__host__ __device__ __forceinline__ size_t pair_source_base(int row, int row0, int n_pad) {
-    const size_t r = (size_t)(row - row0), first = (size_t)n_pad - (size_t)(row0 + 1) * kPairRow;
-    return r * first - (size_t)kPairRow * (r * (r - (r > 0 ? 1 : 0)) / 2);
-}
-
 template <int LAW, bool HEAVY, int FOLD>
-__global__ void __launch_bounds__(kPairThreads, 3) k_direct_pairs(const float4* __restrict__ pos, int n_pad, int row0,
+__global__ void __launch_bounds__(kPairThreads, kPairBlocksPerSm) k_direct_pairs(const float4* __restrict__ pos, int n_pad, int row0,
                                                                   int nrows, int per, float S,
                                                                   float4* __restrict__ part,
                                                                   int* __restrict__ err, uint32_t polls,
@@ -486,10 +470,6 @@ __device__ __forceinline__ HiLo3 fold_partials_lanes(const float4* __restrict__ 
 // row), warp j taking every kFoldWarps-th entry; the first warp gets the totals.
 // (Eight neighbouring threads a body: 10.6 us a fold at 50,001 bodies, now 8.9;
 // the allocation-free call there 945 -> 937, a step of 262,144 20.10 -> 20.02 ms.)
-struct PairFold {
-    int per, row0, rows;   // tiles a unit, first row, rows
-};
-
 __device__ __forceinline__ HiLo3 fold_pairs(const float4* __restrict__ part, const PairFold& pf, int n_pad, int i, int j,
                                             float (*sums)[6][32]) {
     float ax = 0.f, ay = 0.f, az = 0.f, kx = 0.f, ky = 0.f, kz = 0.f;
@@ -752,77 +732,40 @@ static cudaError_t reserve_part(nb_sim* sim, size_t need) {
     return cudaSuccess;
 }
 
-static size_t pair_entries(const PairFold& p, int n_pad) {
-    return (size_t)pair_units_before(p.row0 + p.rows, p.row0, n_pad / kPairRow, p.per) * kPairRow +
-           pair_source_base(p.row0 + p.rows, p.row0, n_pad);
-}
-
-// The launch of k_direct_pairs that starts at row0, within cap entries of
-// partials: tiles a unit and rows.  The length of a launch is estimated in
-// tiles of one SM's time from the units of the fullest SM, three resident at a
-// time (fewer take nearly as long: a block alone is a chain of latencies), 0.15
-// tiles a unit for its start and end, 0.3 units for the uneven end of the
-// launch and two tiles a launch; rows left over count at the same rate.  all_rows: the partials are roomy, and only
-// launches of as many rows as fit are compared.
-constexpr int kPairBlocksPerSm = 3;
-
-static PairFold pair_plan(int sm_count, int n_pad, int row0, size_t cap, bool all_rows) {
-    const int rows = n_pad / kPairRow, sms = std::max(1, sm_count);
-    const int pers[] = {1, 2, 4, 8, 16, 24, 32, 48, 64};
-    const double tail[kPairBlocksPerSm] = {0.0, 2.2, 2.6};
-    PairFold best{kPairRowTiles, row0, 1};
-    double best_time = 0.0;
-    bool any = false;
-    const int left = rows - row0;
-    for (int per : pers) {
-        for (int r = left; r >= 1; --r) {
-            const PairFold p{per, row0, r};
-            if (pair_entries(p, n_pad) > cap) continue;
-            const int units = pair_units_before(row0 + r, row0, rows, per), k = (units + sms - 1) / sms;
-            const double work = (double)r * left - 0.5 * r * (r - 1), all = 0.5 * left * (left + 1.0);
-            const double time = ((k / kPairBlocksPerSm * kPairBlocksPerSm + tail[k % kPairBlocksPerSm]) * (per + 0.15) +
-                                 0.3 * per + 2.0) * (all / work);
-            if (!any || time < best_time) {
-                any = true;
-                best_time = time;
-                best = p;
-            }
-            if (all_rows) break;
-        }
-    }
-    return best;
-}
-
 // k_direct_pairs over all rows in launches within cap entries of part, folded
 // into the carry between launches.  The last launch's partials are left for the
-// reduction (*last; *carry is null when it was the only one).  Returns the
-// launches made.
+// reduction (*last; *carry is null when it was the only one).  *made: the
+// launches.  After a launch that failed nothing is queued behind it.
 template <bool HEAVY, int FOLD>
-static int launch_pairs(int sm_count, int law, cudaStream_t st, const float4* pos, int n_pad, float S, float4* part,
-                        size_t cap, bool all_rows, float4* carry_buf, int* err, uint32_t polls, const unsigned* mmax, PairFold* last,
-                        const float4** carry) {
+static cudaError_t launch_pairs(int sm_count, int law, cudaStream_t st, const float4* pos, int n_pad, float S,
+                                float4* part, size_t cap, bool all_rows, float4* carry_buf, int* err, uint32_t polls,
+                                const unsigned* mmax, PairFold* last, const float4** carry, int* made) {
     const int rows = n_pad / kPairRow;
-    int made = 0;
+    *made = 0;
     *carry = nullptr;
     for (int r0 = 0; r0 < rows;) {
         const PairFold p = pair_plan(sm_count, n_pad, r0, cap, all_rows);
-        const unsigned grid = (unsigned)pair_units_before(r0 + p.rows, r0, rows, p.per);
+        const unsigned grid = (unsigned)pair_units(p, n_pad);
         if (law == NB_LAW_PLUMMER)
             k_direct_pairs<NB_LAW_PLUMMER, HEAVY, FOLD><<<grid, kPairThreads, 0, st>>>(pos, n_pad, r0, p.rows, p.per, S, part, err,
                                                                                  polls, mmax);
         else
             k_direct_pairs<NB_LAW_REFERENCE, HEAVY, FOLD><<<grid, kPairThreads, 0, st>>>(pos, n_pad, r0, p.rows, p.per, S, part, err,
                                                                                    polls, mmax);
-        ++made;
+        cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        ++*made;
         *last = p;
         if (r0 + p.rows < rows) {
             k_pairs_carry<<<(unsigned)(n_pad / 32), 32 * kFoldWarps, 0, st>>>(part, p, n_pad, r0 == 0 ? 1 : 0, carry_buf, err);
-            ++made;
+            e = cudaGetLastError();
+            if (e != cudaSuccess) return e;
+            ++*made;
             *carry = carry_buf;
         }
         r0 += p.rows;
     }
-    return made;
+    return cudaSuccess;
 }
 
 // Entries of partials a handle's k_direct_pairs launch may use (1 GiB): one
@@ -867,18 +810,20 @@ static cudaError_t force_pairs(nb_sim* sim, PairFold* last, const float4** carry
     if (e != cudaSuccess) return e;
     const float S = (float)sim->prm.softening2;
     auto go = sim->heavy ? launch_pairs<true, kFold> : launch_pairs<false, kFold>;
-    const int made = go(sim->sm_count, sim->prm.law, sim->stream, sim->pos, n_pad, S, sim->part, kPairCap, true,
-                        sim->part + most, sim->d_err, sim->wait_polls, sim->d_mmax, last, carry);
-    sim->prof.launches += (uint64_t)(made - 1);   // the phase counts one
-    return cudaGetLastError();
+    int made = 0;
+    e = go(sim->sm_count, sim->prm.law, sim->stream, sim->pos, n_pad, S, sim->part, kPairCap, true, sim->part + most,
+           sim->d_err, sim->wait_polls, sim->d_mmax, last, carry, &made);
+    if (made > 1) sim->prof.launches += (uint64_t)(made - 1);   // the phase counts one
+    return e;
 }
 
 cudaError_t direct_force_update(nb_sim* sim, float dt, bool update) {
     const bool comp = !(sim->prm.flags & NB_FLAG_NO_COMPENSATION);
     // Each pair once.  A handle whose launch was tuned, and uncompensated sums,
     // keep k_direct_force; so do small states whose waits were tuned
-    // (k_direct_rows has none that could run out).
-    const bool small = sim->n_pad <= kRowMax, once = comp && !sim->tune_set && !(small && sim->wait_polls != kMaxPolls);
+    // (k_direct_rows has none that could run out) and states beyond kPairMax.
+    const bool small = sim->n_pad <= kRowMax;
+    const bool once = comp && !sim->tune_set && sim->n_pad <= kPairMax && !(small && sim->wait_polls != kMaxPolls);
     const bool by_rows = once && small, pairs = once && !small;
     RowPlan rp{};
     int splits = 0;
@@ -1093,7 +1038,10 @@ extern "C" int nb_direct_accel_noalloc(const float* pos_mass4, size_t n, float* 
             return NB_ECUDA;
         }
         const size_t cap = kNoAllocScratch - 3 * n_pad;
-        launch_pairs<true, kFold / 2>(sms, law, st, pos, (int)n_pad, S, part, cap, false, part + cap, err, kMaxPolls, mmax, &pf, &carry);
+        int made = 0;
+        if (launch_pairs<true, kFold / 2>(sms, law, st, pos, (int)n_pad, S, part, cap, false, part + cap, err, kMaxPolls, mmax,
+                                          &pf, &carry, &made) != cudaSuccess)
+            return NB_ECUDA;
         k_noalloc_reduce<<<(unsigned)((n + 31) / 32), 32 * kFoldWarps, 0, st>>>(part, pf, carry, (int)n, (int)n_pad, (float)G,
                                                                                 acc);
     }
