@@ -276,6 +276,7 @@ void free_state(nb_sim* s) {
         dev_free(p, s->stream);
     s->pos = s->posc = s->vel = s->velc = s->acc = s->finit = s->part = nullptr;
     s->part_cap = 0;
+    s->pair_cap = 0;
     s->cap = 0;
     tree_free(s);
 }

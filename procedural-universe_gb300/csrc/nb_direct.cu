@@ -798,20 +798,22 @@ static cudaError_t launch_rows(const RowPlan& p, int law, cudaStream_t st, const
 }
 
 static cudaError_t force_pairs(nb_sim* sim, PairFold* last, const float4** carry) {
-    const int n_pad = (int)sim->n_pad, rows = n_pad / kPairRow;
+    const int n_pad = (int)sim->n_pad;
     size_t most = 0;
-    int launches = 0;
-    for (int r0 = 0; r0 < rows; ++launches) {
-        const PairFold p = pair_plan(sim->sm_count, n_pad, r0, kPairCap, true);
-        most = std::max(most, pair_entries(p, n_pad));
-        r0 += p.rows;
-    }
-    cudaError_t e = reserve_part(sim, most + (launches > 1 ? (size_t)2 * n_pad : 0));
+    cudaError_t e = cudaSuccess;
+    // A handle that had to make do with less keeps to it until its state is
+    // set up anew: no allocation is tried again on each step.
+    const size_t cap = pair_reserve(sim->sm_count, n_pad, sim->pair_cap ? sim->pair_cap : kPairCap, &most, [&](size_t need) {
+        e = reserve_part(sim, need);
+        if (e == cudaErrorMemoryAllocation) cudaGetLastError();   // reported here or made good, not by the next launch
+        return e != cudaErrorMemoryAllocation;
+    });
     if (e != cudaSuccess) return e;
+    if (cap != kPairCap) sim->pair_cap = cap;
     const float S = (float)sim->prm.softening2;
     auto go = sim->heavy ? launch_pairs<true, kFold> : launch_pairs<false, kFold>;
     int made = 0;
-    e = go(sim->sm_count, sim->prm.law, sim->stream, sim->pos, n_pad, S, sim->part, kPairCap, true, sim->part + most,
+    e = go(sim->sm_count, sim->prm.law, sim->stream, sim->pos, n_pad, S, sim->part, cap, true, sim->part + most,
            sim->d_err, sim->wait_polls, sim->d_mmax, last, carry, &made);
     if (made > 1) sim->prof.launches += (uint64_t)(made - 1);   // the phase counts one
     return e;
@@ -836,6 +838,11 @@ cudaError_t direct_force_update(nb_sim* sim, float dt, bool update) {
     } else if (by_rows) {
         rp = row_plan((int)sim->n, (int)sim->n_pad, kPairCap);
         cudaError_t e = reserve_part(sim, row_entries(rp, (int)sim->n_pad));
+        if (e == cudaErrorMemoryAllocation && rp.per < 4) {   // no room: longer units, fewer partials
+            cudaGetLastError();
+            rp.per = 4;
+            e = reserve_part(sim, row_entries(rp, (int)sim->n_pad));
+        }
         if (e != cudaSuccess) return e;
         PhaseScope ps(sim, 0);
         e = launch_rows(rp, sim->prm.law, sim->stream, sim->pos, (int)sim->n_pad, (float)sim->prm.softening2,

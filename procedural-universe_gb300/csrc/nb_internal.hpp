@@ -166,6 +166,7 @@ struct nb_sim {
     // direct-sum partial sums
     float4* part = nullptr;   // [splits][n_pad] sums then [splits][n_pad] compensations
     size_t part_cap = 0;      // in float4 entries
+    size_t pair_cap = 0;      // entries that k_direct_pairs may use where there was no room for its usual ones; 0: those
     nb::DirectTuning tune{};
     // Barnes-Hut
     nb::TreeBuffers tree{};

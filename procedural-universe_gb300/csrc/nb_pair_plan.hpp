@@ -93,4 +93,31 @@ inline PairFold pair_plan(int sm_count, int n_pad, int row0, size_t cap, bool al
     return best;
 }
 
+// Entries of partials that the launches of a state need within cap: the largest
+// launch's, and two a body for the sums carried over when there are several.
+inline size_t pair_scratch(int sm_count, int n_pad, size_t cap, size_t* largest) {
+    const int rows = n_pad / kPairRow;
+    int launches = 0;
+    *largest = 0;
+    for (int r0 = 0; r0 < rows; ++launches) {
+        const PairFold p = pair_plan(sm_count, n_pad, r0, cap, true);
+        *largest = std::max(*largest, pair_entries(p, n_pad));
+        r0 += p.rows;
+    }
+    return *largest + (launches > 1 ? (size_t)2 * n_pad : 0);
+}
+
+// Reserves the partials of a state's launches: within cap, or, while there is no
+// room (reserve(entries) is false), within half of it and so on down to launches
+// of single rows.  Returns the cap that the launches are to be planned with, 0
+// when there is no room at all.
+template <class Reserve>
+size_t pair_reserve(int sm_count, int n_pad, size_t cap, size_t* largest, Reserve reserve) {
+    for (;; cap /= 2) {
+        const size_t need = pair_scratch(sm_count, n_pad, cap, largest);
+        if (reserve(need)) return cap;
+        if (*largest > cap) return 0;   // single rows that do not fit cap: no smaller plan
+    }
+}
+
 }  // namespace nb
