@@ -67,10 +67,16 @@ struct nb_batch {
     DirGal* dgal = nullptr;
     int4* units = nullptr;
     int32_t* unit_src = nullptr;
-    int nunits = 0;
+    // the members' launches: each takes the units [unit, unit + units) and folds
+    // the bodies [body, body + bodies) of the direct-sum range, in the same partials
+    struct DirLaunch {
+        int unit, units, body, bodies;
+    };
+    std::vector<DirLaunch> dlaunch;
     float4* part = nullptr;
     size_t part_cap = 0;
-    int* next_unit = nullptr;
+    int* next_unit = nullptr;        // one counter a launch
+    size_t next_cap = 0;
     uint64_t direct_pairs = 0;
     // whole-batch transfers of many galaxies: runs of bodies and the dense copy of
     // one state array, made on the first such transfer and kept
@@ -120,20 +126,52 @@ bool tuning_valid(const nb_tuning& t) {
            t.leaf_size <= 64 && t.traverse_block == 128;
 }
 
+// Entries of partials that the direct members of one launch may need together
+// (1 GiB); a batch that needs more takes several launches, one after the other.
+// A pair taken once leaves a partial at either body, about 64 entries a body at
+// 8192 bodies: 129 members of that size fill this, and their 134,000 units fill
+// the GPU many times over.
+constexpr size_t kDirPartials = ((size_t)1 << 30) / sizeof(float4);
+
+// The direct members' work units, and their launches within cap entries of partials.
+struct DirPlan {
+    std::vector<int4> units;
+    std::vector<int32_t> src;
+    std::vector<DirGal> gal;
+    std::vector<nb_batch::DirLaunch> launches;
+    size_t entries = 0, largest = 0;   // of the largest launch, of the largest member
+};
+
 // Work units of the direct-sum galaxies for the current tuning: rows of 128 *
 // direct_ipt target bodies against runs of source bodies (k_batch_direct).
 // Rows and chunks that hold only padding are left out; a member's units, and so
 // its results, do not depend on the other members.  Longest units first, so that
-// the launch ends evenly.
-int plan_units(nb_batch* b) {
+// a launch ends evenly.
+int make_direct_plan(nb_batch* b, size_t cap, DirPlan* plan) {
     struct Unit {
         int4 u;
         int32_t src;
     };
     std::vector<Unit> list;
-    std::vector<DirGal> dg(b->ndgal);
+    *plan = DirPlan{};
+    plan->gal.resize(b->ndgal);
     const int row = 128 * b->tune.direct_ipt, row_chunks = row / kDirChunk;
     size_t part_base = 0;
+    int body = 0, bodies = 0;
+    auto close = [&]() {
+        std::stable_sort(list.begin(), list.end(),
+                         [](const Unit& a, const Unit& c) { return (a.u.z & 0xffff) > (c.u.z & 0xffff); });
+        plan->launches.push_back({(int)plan->units.size(), (int)list.size(), body, bodies});
+        for (const Unit& u : list) {
+            plan->units.push_back(u.u);
+            plan->src.push_back(u.src);
+        }
+        list.clear();
+        plan->entries = std::max(plan->entries, part_base);
+        body += bodies;
+        part_base = 0;
+        bodies = 0;
+    };
     for (const auto& g : b->gal) {
         if (g.bh) continue;
         const int n_pad = (int)g.n_pad, sources = (int)pad_up(g.n, kDirChunk);
@@ -144,8 +182,10 @@ int plan_units(nb_batch* b) {
         const int splits = (sources / kDirChunk + L - 1) / L;
         const size_t rows = (size_t)n_pad / row;
         const size_t entries = (size_t)splits * n_pad + (once ? rows * n_pad - (size_t)row * rows * (rows + 1) / 2 : 0);
-        if (part_base + entries > (size_t)INT32_MAX) return bfail(b, NB_ENOMEM, "direct-sum partials exceed 2^31 entries");
-        dg[g.idx] = DirGal{(int)g.off, n_pad, row, L * kDirChunk, (int)part_base, splits, once ? 1 : 0, sources};
+        if (entries > (size_t)INT32_MAX) return bfail(b, NB_ENOMEM, "a member's direct-sum partials exceed 2^31 entries");
+        plan->largest = std::max(plan->largest, entries);
+        if (bodies > 0 && part_base + entries > cap) close();
+        plan->gal[g.idx] = DirGal{(int)g.off, n_pad, row, L * kDirChunk, (int)part_base, splits, once ? 1 : 0, sources};
         size_t entry = part_base + (size_t)splits * n_pad;   // row r's source partials
         for (int r = 0; (size_t)r * row < g.n; ++r) {
             const int t0 = (int)g.off + r * row, s0 = once ? r * row : 0;
@@ -160,25 +200,43 @@ int plan_units(nb_batch* b) {
             if (once) entry += (size_t)std::max(0, n_pad - (r + 1) * row);
         }
         part_base += entries;
+        bodies += n_pad;
     }
-    std::stable_sort(list.begin(), list.end(), [](const Unit& a, const Unit& c) { return (a.u.z & 0xffff) > (c.u.z & 0xffff); });
-    std::vector<int4> units(list.size());
-    std::vector<int32_t> usrc(list.size());
-    for (size_t k = 0; k < list.size(); ++k) {
-        units[k] = list[k].u;
-        usrc[k] = list[k].src;
-    }
-    NB_BCUDA(b, upload(&b->units, units, b->core->stream));
-    NB_BCUDA(b, upload(&b->unit_src, usrc, b->core->stream));
-    NB_BCUDA(b, upload(&b->dgal, dg, b->core->stream));
-    b->nunits = (int)units.size();
-    if (part_base > b->part_cap) {
+    if (bodies > 0) close();
+    return NB_OK;
+}
+
+// Plans the direct members and reserves their partials; where there is no room,
+// within half of them and so on down to one member a launch.
+int plan_units(nb_batch* b) {
+    DirPlan plan;
+    b->dlaunch.clear();   // none until all is in place
+    for (size_t cap = kDirPartials;; cap = plan.entries / 2) {
+        const int rc = make_direct_plan(b, cap, &plan);
+        if (rc) return rc;
+        if (plan.entries <= b->part_cap) break;
         dev_free(b->part, b->core->stream);
         b->part = nullptr;
         b->part_cap = 0;
-        NB_BCUDA(b, dev_alloc(&b->part, std::max<size_t>(part_base, 1) * sizeof(float4)));
-        b->part_cap = part_base;
+        const cudaError_t e = dev_alloc(&b->part, plan.entries * sizeof(float4));
+        if (e == cudaSuccess) {
+            b->part_cap = plan.entries;
+            break;
+        }
+        if (e != cudaErrorMemoryAllocation || plan.entries <= plan.largest) NB_BCUDA(b, e);
+        cudaGetLastError();
     }
+    if (plan.launches.size() > b->next_cap) {
+        dev_free(b->next_unit, b->core->stream);
+        b->next_unit = nullptr;
+        b->next_cap = 0;
+        NB_BCUDA(b, dev_alloc(&b->next_unit, plan.launches.size() * sizeof(int)));
+        b->next_cap = plan.launches.size();
+    }
+    NB_BCUDA(b, upload(&b->units, plan.units, b->core->stream));
+    NB_BCUDA(b, upload(&b->unit_src, plan.src, b->core->stream));
+    NB_BCUDA(b, upload(&b->dgal, plan.gal, b->core->stream));
+    b->dlaunch = plan.launches;
     b->graph_dirty = true;
     return NB_OK;
 }
@@ -186,13 +244,13 @@ int plan_units(nb_batch* b) {
 // The direct members' force kernel: as many warps as the GPU holds, at most one
 // a unit.
 template <int LAW, int IPT>
-void launch_direct(nb_batch* b, cudaStream_t st, float S) {
+void launch_direct(nb_batch* b, const nb_batch::DirLaunch& d, int* next_unit, cudaStream_t st, float S) {
     const int threads = b->tune.direct_block, warps = threads / 32;
     int occ = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_direct<LAW, IPT>, threads, 0);
-    const int grid = std::max(1, std::min((b->nunits + warps - 1) / warps, b->core->sm_count * std::max(1, occ)));
-    k_batch_direct<LAW, IPT><<<grid, threads, 0, st>>>(b->core->pos, b->units, b->unit_src, b->nunits, b->next_unit, S,
-                                                       b->core->d_mmax, b->part);
+    const int grid = std::max(1, std::min((d.units + warps - 1) / warps, b->core->sm_count * std::max(1, occ)));
+    k_batch_direct<LAW, IPT><<<grid, threads, 0, st>>>(b->core->pos, b->units + d.unit, b->unit_src + d.unit, d.units,
+                                                       next_unit, S, b->core->d_mmax, b->part);
 }
 
 // One step (update) or one force evaluation (no update) of every galaxy,
@@ -212,7 +270,7 @@ int enqueue_step(nb_batch* b, float dt, bool update, bool tree_only = false) {
             const int words = std::max(6 * b->nslot, tree_counter_words());
             k_gal_box_init<<<(words + 255) / 256, 256, 0, st>>>(b->box_bits, b->nslot, t.counters,
                                                                tree_counter_words(), n, t.interactions, b->group_ctr,
-                                                               b->ndgal > 0 ? b->next_unit : nullptr);
+                                                               b->next_unit, (int)b->dlaunch.size());
             k_gal_box_chunks<<<(unsigned)((n + kBoxChunk - 1) / kBoxChunk), 256, 0, st>>>(c->pos, b->body_slot, n,
                                                                                        b->nslot, b->box_bits);
         }
@@ -257,19 +315,25 @@ int enqueue_step(nb_batch* b, float dt, bool update, bool tree_only = false) {
         NB_BCUDA(b, cudaGetLastError());
     }
     if (b->ndgal > 0) {
-        PhaseScope ps(c, NB_PHASE_DIRECT_FORCE, 2);
-        if (b->n_bh == 0) NB_BCUDA(b, cudaMemsetAsync(b->next_unit, 0, sizeof(int), st));   // else cleared with the counters
+        const int launches = (int)b->dlaunch.size();
+        if (launches == 0) return bfail(b, NB_ENOMEM, "the direct-sum members found no memory");
+        PhaseScope ps(c, NB_PHASE_DIRECT_FORCE, 2 * launches);
+        // (else cleared with the counters)
+        if (b->n_bh == 0) NB_BCUDA(b, cudaMemsetAsync(b->next_unit, 0, launches * sizeof(int), st));
         const bool wide = b->tune.direct_ipt == 2;
-        if (b->base.law == NB_LAW_PLUMMER) {
-            if (wide) launch_direct<NB_LAW_PLUMMER, 8>(b, st, S);
-            else launch_direct<NB_LAW_PLUMMER, 4>(b, st, S);
-        } else {
-            if (wide) launch_direct<NB_LAW_REFERENCE, 8>(b, st, S);
-            else launch_direct<NB_LAW_REFERENCE, 4>(b, st, S);
+        for (int k = 0; k < launches; ++k) {
+            const auto& d = b->dlaunch[k];
+            if (b->base.law == NB_LAW_PLUMMER) {
+                if (wide) launch_direct<NB_LAW_PLUMMER, 8>(b, d, b->next_unit + k, st, S);
+                else launch_direct<NB_LAW_PLUMMER, 4>(b, d, b->next_unit + k, st, S);
+            } else {
+                if (wide) launch_direct<NB_LAW_REFERENCE, 8>(b, d, b->next_unit + k, st, S);
+                else launch_direct<NB_LAW_REFERENCE, 4>(b, d, b->next_unit + k, st, S);
+            }
+            // whole members: a multiple of 256 bodies
+            k_batch_direct_reduce<<<d.bodies / 32, 32 * kFoldWarps, 0, st>>>(
+                b->body_dgal + d.body, b->dgal, (int)b->dir_begin + d.body, G, b->part, c->acc);
         }
-        const int cnt = (int)(b->n_total - b->dir_begin);   // a multiple of 256
-        k_batch_direct_reduce<<<cnt / 32, 32 * kFoldWarps, 0, st>>>(b->body_dgal, b->dgal, (int)b->dir_begin, G,
-                                                                     b->part, c->acc);
         NB_BCUDA(b, cudaGetLastError());
     }
     if (update) {
@@ -485,7 +549,7 @@ int nb_batch_create(const nb_params* base, size_t bh_threshold, double bh_theta,
         b->bh_threshold = bh_threshold;
         b->bh_theta = bh_theta;
         b->core = core;
-        if (dev_alloc(&b->next_unit, sizeof(int)) != cudaSuccess || dev_alloc(&b->held, sizeof(int)) != cudaSuccess) {
+        if (dev_alloc(&b->held, sizeof(int)) != cudaSuccess) {
             cudaGetLastError();
             nb_batch_destroy(b);
             return NB_ENOMEM;

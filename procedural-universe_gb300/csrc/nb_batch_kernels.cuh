@@ -87,19 +87,19 @@ __global__ void __launch_bounds__(256) k_move_state(const int4* __restrict__ run
 //
 // The first kernel of a batched step also clears the step's counters: the
 // tree counters and the radix histograms (TC_NIN set to the bodies in the
-// forest), the interaction count, the traversal group counters and the
-// direct-sum unit counter.
+// forest), the interaction count, the traversal group counters and the unit
+// counters of the direct-sum launches.
 __global__ void k_gal_box_init(unsigned* __restrict__ bits, int nslot, int32_t* __restrict__ counters,
                                int counter_words, int n_in, unsigned long long* __restrict__ interactions,
-                               int* __restrict__ group_ctr, int* __restrict__ next_unit) {
+                               int* __restrict__ group_ctr, int* __restrict__ next_unit, int n_next) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < 6 * nslot) bits[i] = (i % 6) < 3 ? 0xffffffffu : 0u;
     for (int j = i; j < counter_words; j += gridDim.x * blockDim.x) counters[j] = j == TC_NIN ? n_in : 0;
     if (i == 0) {
         *interactions = 0ull;
         group_ctr[0] = group_ctr[1] = group_ctr[2] = 0;
-        if (next_unit) *next_unit = 0;
     }
+    for (int j = i; j < n_next; j += gridDim.x * blockDim.x) next_unit[j] = 0;
 }
 
 __device__ __forceinline__ void box_flush(unsigned* bits, int slot, const float lo[3], const float hi[3]) {
