@@ -160,7 +160,7 @@ int make_direct_plan(nb_batch* b, size_t cap, DirPlan* plan) {
     int body = 0, bodies = 0;
     auto close = [&]() {
         std::stable_sort(list.begin(), list.end(),
-                         [](const Unit& a, const Unit& c) { return (a.u.z & 0xffff) > (c.u.z & 0xffff); });
+                         [](const Unit& a, const Unit& c) { return (a.u.z & kDirChunks) > (c.u.z & kDirChunks); });
         plan->launches.push_back({(int)plan->units.size(), (int)list.size(), body, bodies});
         for (const Unit& u : list) {
             plan->units.push_back(u.u);
@@ -181,21 +181,22 @@ int make_direct_plan(nb_batch* b, size_t cap, DirPlan* plan) {
         const int L = std::min(1024, b->tune.direct_jtile / (once ? 4 * kDirChunk : kDirChunk));
         const int splits = (sources / kDirChunk + L - 1) / L;
         const size_t rows = (size_t)n_pad / row;
-        const size_t entries = (size_t)splits * n_pad + (once ? rows * n_pad - (size_t)row * rows * (rows + 1) / 2 : 0);
+        const size_t targets = (size_t)splits * n_pad;
+        const size_t entries = targets + (once ? rows * n_pad - (size_t)row * rows * (rows + 1) / 2 : targets);
         if (entries > (size_t)INT32_MAX) return bfail(b, NB_ENOMEM, "a member's direct-sum partials exceed 2^31 entries");
         plan->largest = std::max(plan->largest, entries);
         if (bodies > 0 && part_base + entries > cap) close();
         plan->gal[g.idx] = DirGal{(int)g.off, n_pad, row, L * kDirChunk, (int)part_base, splits, once ? 1 : 0, sources};
-        size_t entry = part_base + (size_t)splits * n_pad;   // row r's source partials
+        size_t entry = part_base + targets;   // row r's source partials
         for (int r = 0; (size_t)r * row < g.n; ++r) {
             const int t0 = (int)g.off + r * row, s0 = once ? r * row : 0;
             const int chunks = (sources - s0) / kDirChunk;
             for (int c = 0, s = 0; c < chunks; c += L, ++s) {
                 const int k = std::min(L, chunks - c);
                 const int own = once ? std::max(0, std::min(k, row_chunks - c)) : k;
-                list.push_back(Unit{make_int4(t0, (int)g.off + s0 + c * kDirChunk, k | (own << 16),
+                list.push_back(Unit{make_int4(t0, (int)g.off + s0 + c * kDirChunk, k | (once ? 0 : kDirBothParts) | (own << 16),
                                               (int)part_base + s * n_pad + r * row),
-                                    (int32_t)((long long)entry - (t0 + row))});
+                                    once ? (int32_t)((long long)entry - (t0 + row)) : (int32_t)targets});
             }
             if (once) entry += (size_t)std::max(0, n_pad - (r + 1) * row);
         }

@@ -938,15 +938,19 @@ __global__ void __launch_bounds__(kGWarps * 32, 5) k_group_traverse(
 // ---- batched direct sum --------------------------------------------------------
 // A unit is a row of 32 * IPT target bodies, IPT a lane in registers (packed
 // FP32x2), against a run of 32-source chunks: (first target body, first source
-// body, chunks | chunks evaluated from the target side only << 16, entry of the
-// target partials); unit_src is the entry of body 0 among the row's source
-// partials.  Sources behind the row are evaluated once for both bodies, 17
+// body, chunks | kDirBothParts | chunks evaluated from the target side only << 16,
+// entry of the target partials); unit_src is the entry of body 0 among the row's
+// source partials, or, with kDirBothParts, the distance of the compensations from
+// the targets' sums.  Sources behind the row are evaluated once for both bodies, 17
 // FP32 operations for two interactions instead of 26: lane l takes source
 // (l + r) mod 32 at step r, and the sources' sums travel with them by shuffle
 // (as in k_direct_pairs, here within one warp).  The row's own bodies, and all
 // sources of a member of more than kDirOnceMax padded bodies (whose source
 // partials would grow with its square), are evaluated from the target side
-// (direct_chunk).
+// (direct_chunk).  Such a member's few partials keep sum and compensation apart:
+// rounded to one word they added 2% to the force error at 9000 and 16,000 bodies.
+// (Where each pair is taken once, the many partials of a body carry less: the error
+// is 4% below that of the target side with both parts.)
 //
 // Bound by the FP32 pipe.  Warps share nothing, so that no barrier waits for
 // the slowest; the next chunk and the next unit are fetched while the current
@@ -956,6 +960,7 @@ __global__ void __launch_bounds__(kGWarps * 32, 5) k_group_traverse(
 // is the shuffles and reads that four targets a lane carry (eight: 268 us a
 // step, but small members then fill fewer rows).
 constexpr int kDirWarps = 8;   // most warps per block
+constexpr int kDirChunks = 0x7fff, kDirBothParts = 0x8000;   // fields of a unit
 template <int LAW, int IPT>
 __global__ void __launch_bounds__(kDirWarps * 32, IPT == 4 ? 2 : 1) k_batch_direct(
     const float4* __restrict__ pos, const int4* __restrict__ units, const int32_t* __restrict__ unit_src, int nunits,
@@ -970,7 +975,7 @@ __global__ void __launch_bounds__(kDirWarps * 32, IPT == 4 ? 2 : 1) k_batch_dire
     u = __shfl_sync(0xffffffffu, u, 0);
     while (u < nunits) {
         const int4 un = units[u];
-        const int src0 = unit_src[u], chunks = un.z & 0xffff, own = un.z >> 16;
+        const int src0 = unit_src[u], chunks = un.z & kDirChunks, own = un.z >> 16;
         int after = 0;
         if (lane == 0) after = atomicAdd(next_unit, 1);
         float2 nx[P], ny[P], nz[P], mi[P];
@@ -999,10 +1004,19 @@ __global__ void __launch_bounds__(kDirWarps * 32, IPT == 4 ? 2 : 1) k_batch_dire
                 part[(long long)src0 + un.y + c * kDirChunk + lane] = make_float4(f.x, f.y, f.z, 0.f);
             }
         }
+        if (un.z & kDirBothParts) {
 #pragma unroll
-        for (int k = 0; k < IPT; ++k)
-            part[(size_t)un.w + k * 32 + lane] =
-                make_float4(sum[3 * k] - comp[3 * k], sum[3 * k + 1] - comp[3 * k + 1], sum[3 * k + 2] - comp[3 * k + 2], 0.f);
+            for (int k = 0; k < IPT; ++k) {
+                const size_t at = (size_t)un.w + k * 32 + lane;
+                part[at] = make_float4(sum[3 * k], sum[3 * k + 1], sum[3 * k + 2], 0.f);
+                part[at + src0] = make_float4(comp[3 * k], comp[3 * k + 1], comp[3 * k + 2], 0.f);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < IPT; ++k)
+                part[(size_t)un.w + k * 32 + lane] =
+                    make_float4(sum[3 * k] - comp[3 * k], sum[3 * k + 1] - comp[3 * k + 1], sum[3 * k + 2] - comp[3 * k + 2], 0.f);
+        }
         u = __shfl_sync(0xffffffffu, after, 0);
         __syncwarp();   // the next unit's first chunk may take the buffer read last
     }
@@ -1010,7 +1024,8 @@ __global__ void __launch_bounds__(kDirWarps * 32, IPT == 4 ? 2 : 1) k_batch_dire
 
 // A direct-sum member's partials: [splits][n_pad] for its bodies as targets
 // (only the first ones of a row that its sources fill), then, where each pair
-// is taken once, for each row one entry per body behind it.
+// is taken once, for each row one entry per body behind it, else the targets'
+// compensations, [splits][n_pad] again.
 struct DirGal {
     int off, n_pad, row, split;   // first body, padded bodies, bodies a row, source bodies a unit
     int base, splits, once, sources;   // first entry, splits, each pair once?, source bodies (to a whole chunk)
@@ -1045,6 +1060,15 @@ __global__ void __launch_bounds__(32 * kFoldWarps) k_batch_direct_reduce(const i
 #pragma unroll 4
             for (int r = j; r < row; r += kFoldWarps)
                 add(src[(size_t)r * d.n_pad - (size_t)d.row * r * (r + 1) / 2 + (local - (r + 1) * d.row)]);
+        } else {
+            const float4* low = part + (size_t)d.base + (size_t)d.splits * d.n_pad + local;
+            float qx = 0.f, qy = 0.f, qz = 0.f;
+#pragma unroll 4
+            for (int s = j; s < used; s += kFoldWarps) {
+                const float4 c = low[(size_t)s * d.n_pad];
+                qx += c.x; qy += c.y; qz += c.z;
+            }
+            kx += qx; ky += qy; kz += qz;
         }
     }
     const float3 f = add_warps(sums, ax, ay, az, kx, ky, kz).rounded();
