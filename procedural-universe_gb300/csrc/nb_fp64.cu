@@ -143,7 +143,7 @@ __device__ __forceinline__ float2 pair_potential(float2 r2, float2 eps2, float2 
 constexpr int kPotThreads = kF64Block / 2;   // two targets a thread
 constexpr int kPotGroup = 64;                // terms summed in FP32 before FP64
 template <int LAW>
-__global__ void __launch_bounds__(kPotThreads) k_diag_potential(const float4* __restrict__ pos, int nblocks, float eps,
+__global__ void __launch_bounds__(kPotThreads) k_diag_potential(const float4* __restrict__ pos, int n, int nblocks, float eps,
                                                                 float S, double* __restrict__ partial) {
     __shared__ float4 tile[kF64Block];
     __shared__ double red[kPotThreads / 32];
@@ -171,13 +171,12 @@ __global__ void __launch_bounds__(kPotThreads) k_diag_potential(const float4* __
                 const float2 dy = __fadd2_rn(make_float2(pj.y, pj.y), ny);
                 const float2 dz = __fadd2_rn(make_float2(pj.z, pj.z), nz);
                 const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-                const float2 phi = pair_potential<LAW>(r2, eps2, S2);
-                float2 m = make_float2(pj.w, pj.w);
-                if (d == 0) {   // the body itself
-                    if (g + k == tid) m.x = 0.f;
-                    if (g + k == tid + kPotThreads) m.y = 0.f;
+                float2 phi = pair_potential<LAW>(r2, eps2, S2);
+                if (d == 0) {   // the body itself (infinite where S underflows in FP32)
+                    if (g + k == tid) phi.x = 0.f;
+                    if (g + k == tid + kPotThreads) phi.y = 0.f;
                 }
-                s = __ffma2_rn(m, phi, s);
+                s = __ffma2_rn(make_float2(pj.w, pj.w), phi, s);
             }
             v0 += (double)s.x;
             v1 += (double)s.y;
@@ -186,6 +185,8 @@ __global__ void __launch_bounds__(kPotThreads) k_diag_potential(const float4* __
         u0 += weight * v0;
         u1 += weight * v1;
     }
+    if (b * kF64Block + tid >= n) u0 = 0.0;   // padding
+    if (b * kF64Block + kPotThreads + tid >= n) u1 = 0.0;
     double u = (double)p0.w * u0 + (double)p1.w * u1;
     for (int o = 16; o > 0; o >>= 1) u += __shfl_down_sync(0xffffffffu, u, o);
     if ((tid & 31) == 0) red[tid >> 5] = u;
@@ -254,9 +255,9 @@ cudaError_t fp64_diagnostics_ex(nb_sim* sim, float half_dt, bool with_acc, bool 
     if (with_potential) {
         const dim3 grid((unsigned)nblocks, (unsigned)runs);
         if (sim->prm.law == NB_LAW_PLUMMER)
-            k_diag_potential<NB_LAW_PLUMMER><<<grid, kPotThreads, 0, sim->stream>>>(sim->pos, nblocks, eps, S, potential);
+            k_diag_potential<NB_LAW_PLUMMER><<<grid, kPotThreads, 0, sim->stream>>>(sim->pos, (int)sim->n, nblocks, eps, S, potential);
         else
-            k_diag_potential<NB_LAW_REFERENCE><<<grid, kPotThreads, 0, sim->stream>>>(sim->pos, nblocks, eps, S,
+            k_diag_potential<NB_LAW_REFERENCE><<<grid, kPotThreads, 0, sim->stream>>>(sim->pos, (int)sim->n, nblocks, eps, S,
                                                                                       potential);
     }
     cudaError_t e = cudaGetLastError();
