@@ -351,15 +351,16 @@ int read_tree_counts(nb_batch* b, int32_t* h) {
 
 int reserve_tree(nb_batch* b, size_t n_int, size_t n_cells) {
     if (b->n_bh == 0) return NB_OK;
+    b->graph_dirty = true;   // also when this fails: the arrays of the captured graph may be gone
     NB_BCUDA(b, tree_reserve_graph(b->core, (int)b->n_bh, n_int, n_cells));
     const size_t cap = b->core->tree.cell_cap;
     if (cap > b->qcap) {
         dev_free(b->cell_rec, b->core->stream);
         b->cell_rec = nullptr;
+        b->qcap = 0;
         NB_BCUDA(b, dev_alloc(&b->cell_rec, cap * sizeof(CellRec)));
         b->qcap = cap;
     }
-    b->graph_dirty = true;
     return NB_OK;
 }
 

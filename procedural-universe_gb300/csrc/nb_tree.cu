@@ -43,6 +43,7 @@
 #include "nb_morton.cuh"
 #include "nb_cellrec.cuh"
 #include "nb_hilbert.cuh"
+#include "nb_tree_nodes.hpp"
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -1164,6 +1165,7 @@ static cudaError_t reserve_bodies(nb_sim* sim, size_t nk) {
     TreeBuffers& t = sim->tree;
     if (nk <= t.body_cap) return cudaSuccess;
     const size_t cap = nk;
+    t.body_cap = 0;   // until every array is there
     NB_TRY(grow((void**)&t.keys[0], cap * 8, sim->stream));
     NB_TRY(grow((void**)&t.keys[1], cap * 8, sim->stream));
     NB_TRY(grow((void**)&t.vals[0], cap * 4, sim->stream));
@@ -1192,42 +1194,8 @@ static cudaError_t reserve_bodies(nb_sim* sim, size_t nk) {
 }
 
 static cudaError_t reserve_nodes(nb_sim* sim, size_t n_int, size_t n_cells) {
-    TreeBuffers& t = sim->tree;
-    if (n_int > t.int_cap) {
-        const size_t cap = n_int + n_int / 4 + 64;
-        t.int_cap = 0;   // until every array is there: a failed allocation is made good by the next call
-        NB_TRY(grow((void**)&t.int_level, cap * 4, sim->stream));
-        NB_TRY(grow((void**)&t.int_first, cap * 4, sim->stream));
-        NB_TRY(grow((void**)&t.int_parent, cap * 4, sim->stream));
-        NB_TRY(grow((void**)&t.int_mask, cap * 4, sim->stream));
-        NB_TRY(grow((void**)&t.int_nint, cap * 4, sim->stream));
-        NB_TRY(grow((void**)&t.int_pending, cap * 4, sim->stream));
-        NB_TRY(grow((void**)&t.int_block, cap * 4, sim->stream));
-        NB_TRY(grow((void**)&t.int_cell, cap * 4, sim->stream));
-        NB_TRY(grow((void**)&t.int_code, cap * 8, sim->stream));
-        // internal nodes can outnumber bodies (chains of one-child nodes above
-        // close pairs): the child-count scan's status is sized by them
-        NB_TRY(grow((void**)&t.popc_status, ((cap + kSortTile - 1) / kSortTile) * sizeof(unsigned long long), sim->stream));
-        size_t h = 1024;
-        while (h < 2 * cap) h <<= 1;
-        NB_TRY(grow((void**)&t.hkeys, h * 8, sim->stream));
-        NB_TRY(grow((void**)&t.hvals, h * 4, sim->stream));
-        t.hash_cap = h;
-        t.int_cap = cap;
-    }
-    if (n_cells > t.cell_cap) {
-        const size_t cap = n_cells + n_cells / 4 + 64;
-        t.cell_cap = 0;
-        NB_TRY(grow((void**)&t.cell_com, cap * 16, sim->stream));
-        NB_TRY(grow((void**)&t.cell_meta, cap * 16, sim->stream));
-        NB_TRY(grow((void**)&t.cell_mass, cap * 8, sim->stream));
-        NB_TRY(grow((void**)&t.cell_count, cap * 4, sim->stream));
-        NB_TRY(grow((void**)&t.cell_lo, cap * 16, sim->stream));
-        NB_TRY(grow((void**)&t.cell_hi, cap * 16, sim->stream));
-        NB_TRY(grow((void**)&t.cell_code, cap * 8, sim->stream));
-        t.cell_cap = cap;
-    }
-    return cudaSuccess;
+    return grow_nodes(sim->tree, n_int, n_cells, (size_t)kSortTile,
+                      [sim](void** p, size_t bytes) { return grow(p, bytes, sim->stream); });
 }
 
 cudaError_t tree_reserve(nb_sim* sim) {
@@ -1354,8 +1322,8 @@ cudaError_t tree_build(nb_sim* sim, bool export_order) {
         // host itself: a copy before the wait and a memset behind it
         // took 5 us more of the phase at 4000 bodies (52 now), 8 at 2^20 (192).
         NB_TRY(launch_after(k_positions_scan, ntiles, kPosThreads, 0, st, tv, t.spos, t.pos_nint, t.leaf_level,
-                            t.leaf_count, t.counters, t.pos_status, ntiles, t.hkeys, t.hash_cap, t.h_counters,
-                            sim->d_err));
+                            t.leaf_count, t.counters, t.pos_status, ntiles, t.int_cap > 0 ? t.hkeys : nullptr, t.hash_cap,
+                            t.h_counters, sim->d_err));
         NB_TRY(cudaEventRecord(t.counted, st));
         // While the host waits for the counts, the nodes are emitted into the arrays
         // as they are; if they turn out too small, again into larger ones.
@@ -1464,6 +1432,7 @@ cudaError_t tree_build_graph(nb_sim* sim, const float4* pos, int n, int D, bool 
     const size_t nk = pad_up(std::max<size_t>((size_t)n, 1), kSortTile);
     const int ntiles = (int)(nk / kSortTile);
     cudaStream_t st = sim->stream;
+    if (!counts_only && t.int_cap == 0) return cudaErrorMemoryAllocation;   // the node arrays were not to be had
     NB_TRY(launch_sort(sim, nk));
     t.final_buf = 0;
     t.n_in = n;
