@@ -784,13 +784,13 @@ __global__ void k_emit(TopoView tv, const int32_t* int_base, int32_t* int_level,
     }
 }
 
-__device__ __forceinline__ void link_internal(int k, const int32_t* __restrict__ int_level,
-                                              const int32_t* __restrict__ int_first,
-                                              const uint64_t* __restrict__ int_code, const TopoView& tv, int ni,
-                                              const uint64_t* __restrict__ hk, const int32_t* __restrict__ hv,
-                                              uint32_t hmask, int32_t* __restrict__ int_parent,
-                                              uint32_t* __restrict__ int_mask, int32_t* __restrict__ int_nint,
-                                              int32_t* __restrict__ counters) {
+__device__ __forceinline__ void link_internal(int k, const int32_t* int_level,
+                                              const int32_t* int_first,
+                                              const uint64_t* int_code, const TopoView& tv, int ni,
+                                              const uint64_t* hk, const int32_t* hv,
+                                              uint32_t hmask, int32_t* int_parent,
+                                              uint32_t* int_mask, int32_t* int_nint,
+                                              int32_t* counters) {
     if (k >= ni || k == 0) return;
     const int l = int_level[k];
     const int s = int_first[k];
@@ -806,11 +806,11 @@ __device__ __forceinline__ void link_internal(int k, const int32_t* __restrict__
     atomicAdd(&int_nint[parent], 1);
 }
 
-__device__ __forceinline__ void link_leaf(int s, const TopoView& tv, const int32_t* __restrict__ int_base,
-                                          const int32_t* __restrict__ leaf_level, const uint64_t* __restrict__ hk,
-                                          const int32_t* __restrict__ hv, uint32_t hmask,
-                                          int32_t* __restrict__ leaf_parent, uint32_t* __restrict__ int_mask,
-                                          int32_t* __restrict__ counters) {
+__device__ __forceinline__ void link_leaf(int s, const TopoView& tv, const int32_t* int_base,
+                                          const int32_t* leaf_level, const uint64_t* hk,
+                                          const int32_t* hv, uint32_t hmask,
+                                          int32_t* leaf_parent, uint32_t* int_mask,
+                                          int32_t* counters) {
     if (s >= tv.n_in) return;
     const int lf = leaf_level[s];
     if (lf <= 0) return;
@@ -895,14 +895,14 @@ __device__ __forceinline__ int child_cell(const int32_t* int_block, const uint32
     return 1 + int_block[parent] + __popc(int_mask[parent] & ((1u << oct) - 1u));
 }
 
-__device__ __forceinline__ void place_internal(int k, const int32_t* __restrict__ int_level,
-                                               const uint64_t* __restrict__ int_code,
-                                               const int32_t* __restrict__ int_parent,
-                                               const uint32_t* __restrict__ int_mask,
-                                               const int32_t* __restrict__ int_block, int ni, int cell_cap,
-                                               float half, float theta_f, int32_t* __restrict__ int_cell,
-                                               int4* __restrict__ cell_meta, float4* __restrict__ cell_lo,
-                                               float4* __restrict__ cell_hi, uint64_t* __restrict__ cell_code,
+__device__ __forceinline__ void place_internal(int k, const int32_t* int_level,
+                                               const uint64_t* int_code,
+                                               const int32_t* int_parent,
+                                               const uint32_t* int_mask,
+                                               const int32_t* int_block, int ni, int cell_cap,
+                                               float half, float theta_f, int32_t* int_cell,
+                                               int4* cell_meta, float4* cell_lo,
+                                               float4* cell_hi, uint64_t* cell_code,
                                                bool batch) {
     if (k >= ni) return;
     const uint64_t code = int_code[k];
@@ -926,16 +926,16 @@ __device__ __forceinline__ void place_internal(int k, const int32_t* __restrict_
     cell_code[cell] = code;
 }
 
-__device__ __forceinline__ void place_leaf(int s, const TopoView& tv, const int32_t* __restrict__ leaf_level,
-                                           const int32_t* __restrict__ leaf_count,
-                                           const int32_t* __restrict__ leaf_parent,
-                                           const uint32_t* __restrict__ int_mask,
-                                           const int32_t* __restrict__ int_block, const float4* __restrict__ spos,
-                                           float half, float theta_f, float4* __restrict__ cell_com,
-                                           double* __restrict__ cell_mass, int32_t* __restrict__ cell_count,
-                                           int4* __restrict__ cell_meta, float4* __restrict__ cell_lo,
-                                           float4* __restrict__ cell_hi, uint64_t* __restrict__ cell_code,
-                                           CellRec* __restrict__ rec) {
+__device__ __forceinline__ void place_leaf(int s, const TopoView& tv, const int32_t* leaf_level,
+                                           const int32_t* leaf_count,
+                                           const int32_t* leaf_parent,
+                                           const uint32_t* int_mask,
+                                           const int32_t* int_block, const float4* spos,
+                                           float half, float theta_f, float4* cell_com,
+                                           double* cell_mass, int32_t* cell_count,
+                                           int4* cell_meta, float4* cell_lo,
+                                           float4* cell_hi, uint64_t* cell_code,
+                                           CellRec* rec) {
     if (s >= tv.n_in) return;
     const int lf = leaf_level[s];
     if (lf < 0) return;
