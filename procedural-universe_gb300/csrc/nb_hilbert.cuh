@@ -54,18 +54,14 @@ constexpr HilbertTables make_hilbert() {
 }
 
 #ifdef __CUDACC__
-__constant__ HilbertTables c_hilbert = make_hilbert();
-
-// Copies one direction's table to shared memory (divergent states would
-// serialise constant reads); the caller synchronises.
-__device__ __forceinline__ void load_hilbert(uint32_t* sh, bool inverse) {
-    if (threadIdx.x < 2 * kHilbertStates)
-        sh[threadIdx.x] = inverse ? c_hilbert.inverse[threadIdx.x] : c_hilbert.forward[threadIdx.x];
-}
+#define NB_HILBERT __host__ __device__ __forceinline__
+#else
+#define NB_HILBERT inline
+#endif
 
 // Rewrites the last D digits of a path by the table, the ones before them as
 // they are (the batched forest's galaxy slot).
-__device__ __forceinline__ uint64_t hilbert_map(uint64_t path, int D, const uint32_t* table) {
+NB_HILBERT uint64_t hilbert_map(uint64_t path, int D, const uint32_t* table) {
     uint64_t out = path >> (3 * D);
     uint32_t state = 0;
     for (int shift = 3 * (D - 1); shift >= 0; shift -= 3) {
@@ -75,6 +71,25 @@ __device__ __forceinline__ uint64_t hilbert_map(uint64_t path, int D, const uint
         state = b >> 3;
     }
     return out;
+}
+
+// The same for a path that a gap between float child bounds cut after `depth` of
+// its D digits: the rest stays zero, here as in octant order the first place of
+// the last cell that holds the body.  (Mapped as octant 0, it would fall between
+// the bodies of that cell's child 0, and the child would be emitted twice.)
+NB_HILBERT uint64_t hilbert_map_cut(uint64_t path, int depth, int D, const uint32_t* table) {
+    const int rest = 3 * (D - depth);
+    return hilbert_map(path, D, table) >> rest << rest;
+}
+
+#ifdef __CUDACC__
+__constant__ HilbertTables c_hilbert = make_hilbert();
+
+// Copies one direction's table to shared memory (divergent states would
+// serialise constant reads); the caller synchronises.
+__device__ __forceinline__ void load_hilbert(uint32_t* sh, bool inverse) {
+    if (threadIdx.x < 2 * kHilbertStates)
+        sh[threadIdx.x] = inverse ? c_hilbert.inverse[threadIdx.x] : c_hilbert.forward[threadIdx.x];
 }
 #endif
 

@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(kSortThreads) k_keys_hist(const float4* __rest
             int d;
             key = body_key(pos[i], half, D, inside, gap, d);
             depth[i] = d;
-            if (curve && inside) key = hilbert_map(key, D, table);
+            if (curve && inside) key = hilbert_map_cut(key, d, D, table);
         }
         keys[i] = key;
         count_key(key, h, sh_groups);
@@ -615,12 +615,14 @@ __device__ void node_bounds(uint64_t code, int level, float half, float3& lo, fl
 // Positions in sorted order; brings the sort result to buffer 0 when the
 // device plan left it in buffer 1 (no host read of the plan).  With curve, the
 // last `curve` digits of the keys, sorted along the Hilbert curve, become octants
-// again.
+// again, those of a path that a gap cut (counters, depth; null where there are none)
+// up to its end.
 __global__ void __launch_bounds__(256) k_gather_final(const float4* pos, uint64_t* k0,
                                                       const uint64_t* k1, int32_t* v0,
                                                       const int32_t* v1, int n,
                                                       const int32_t* plan, float4* spos,
-                                                      int curve) {
+                                                      int curve, const int32_t* counters,
+                                                      const int32_t* depth) {
     wait_for_previous();
     __shared__ uint32_t table[2 * kHilbertStates];
     if (curve) {   // uniform
@@ -633,7 +635,8 @@ __global__ void __launch_bounds__(256) k_gather_final(const float4* pos, uint64_
     const int v = from1 ? v1[s] : v0[s];
     if (curve) {
         const uint64_t key = from1 ? k1[s] : k0[s];
-        k0[s] = key == ~0ull ? key : hilbert_map(key, curve, table);
+        const int d = counters && counters[TC_GAPS] != 0 && key != ~0ull ? depth[v] : curve;
+        k0[s] = key == ~0ull ? key : hilbert_map_cut(key, d, curve, table);
     } else if (from1) {
         k0[s] = k1[s];
     }
@@ -1315,7 +1318,7 @@ cudaError_t tree_build(nb_sim* sim, bool export_order) {
     {
         PhaseScope ps(sim, NB_PHASE_TOPOLOGY, t.int_cap > 0 ? 3 : 2);
         NB_TRY(launch_after(k_gather_final, (n + 255) / 256, 256, 0, st, sim->pos, t.keys[0], t.keys[1], t.vals[0],
-                            t.vals[1], n, t.plan, t.spos, curve ? sim->prm.max_depth : 0));
+                            t.vals[1], n, t.plan, t.spos, curve ? sim->prm.max_depth : 0, t.counters, t.depth));
         t.final_buf = 0;
         TopoView tv = topo_view(sim);
         // The scan clears the hash table as it stands and sends the counters to the
@@ -1453,7 +1456,7 @@ cudaError_t tree_build_graph(nb_sim* sim, const float4* pos, int n, int D, bool 
     const int ptiles = (icap + kSortTile - 1) / kSortTile;
     PhaseScope ps(sim, NB_PHASE_TOPOLOGY, 6);
     NB_TRY(launch_after(k_gather_final, (n + 255) / 256, 256, 0, st, pos, t.keys[0], t.keys[1], t.vals[0],
-                        t.vals[1], n, t.plan, t.spos, kMortonLevels));
+                        t.vals[1], n, t.plan, t.spos, kMortonLevels, (const int32_t*)nullptr, (const int32_t*)nullptr));
     // this scan also clears the internal-node hash table for the emission
     NB_TRY(launch_after(k_positions_scan, ntiles, kPosThreads, 0, st, tv, t.spos, t.pos_nint, t.leaf_level,
                         t.leaf_count, t.counters, t.pos_status, ntiles, counts_only ? nullptr : t.hkeys, t.hash_cap,
