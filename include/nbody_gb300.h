@@ -263,7 +263,9 @@ typedef struct nb_batch nb_batch;
 typedef struct nb_tuning {
     int direct_block;     /* threads per block of the direct-sum kernel (64, 128, 256) */
     int direct_ipt;       /* target bodies per thread, in fours (1, 2; block * ipt <= 256) */
-    int direct_jtile;     /* source bodies of four work units (multiple of 128)        */
+    int direct_jtile;     /* source bodies of a work unit (multiple of 128, at most 32,768 count);
+                             members of up to 8192 bodies, padded to 256, take each pair once
+                             and a quarter of it a unit                                 */
     int leaf_size;        /* bodies per Barnes-Hut leaf bucket (1..64)                  */
     int traverse_block;   /* threads per block of the traversal kernel (128)           */
 } nb_tuning;

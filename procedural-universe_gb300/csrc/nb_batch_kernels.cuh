@@ -853,7 +853,7 @@ __global__ void __launch_bounds__(kGWarps * 32, 5) k_group_traverse(
             // The group form of the reference's rule side / r < theta: r is bounded
             // below for every body of the group by the distance from the centre of
             // mass to the group's bounding box.
-            const float side = gb.w * __int_as_float((127 + kSlotLevels - (wr.w >> 8)) << 23);   // box size / 2^level   // box size / 2^level
+            const float side = gb.w * __int_as_float((127 + kSlotLevels - (wr.w >> 8)) << 23);   // box size / 2^level
             float d2 = 0.f;
             const float cc[3] = {ccm.x, ccm.y, ccm.z};
             for (int a = 0; a < 3; ++a) {

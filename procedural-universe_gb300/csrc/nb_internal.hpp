@@ -163,8 +163,9 @@ struct nb_sim {
     size_t d_stage_bytes = 0;
     void* h_stage = nullptr;   // pinned
     size_t h_stage_bytes = 0;
-    // direct-sum partial sums
-    float4* part = nullptr;   // [splits][n_pad] sums then [splits][n_pad] compensations
+    // direct-sum partial sums: [splits][n_pad] sums then [splits][n_pad] compensations
+    // (k_direct_force), or as the pair kernels lay them out (nb_direct.cu)
+    float4* part = nullptr;
     size_t part_cap = 0;      // in float4 entries
     size_t pair_cap = 0;      // entries that k_direct_pairs may use where there was no room for its usual ones; 0: those
     nb::DirectTuning tune{};

@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(kOneThreads) k_sort_block(uint64_t* keys, int3
         if (lane == 0) triv[warp] = one || (warp < kPasses - 1 && ((var >> (8 * warp)) & 255ull) == 0ull);
     }
     uint64_t k[ITEMS];
-    uint32_t rv[ITEMS];   // a key's index (low half: at most 2^14) and its rank
+    uint32_t rv[ITEMS];   // a key's index (low half: below kSortTile) and its rank
 #pragma unroll
     for (int it = 0; it < ITEMS; ++it) {
         k[it] = keys[base + it * 32];
@@ -1306,7 +1306,7 @@ cudaError_t tree_build(nb_sim* sim, bool export_order) {
     NB_TRY(tree_reserve(sim));
     cudaStream_t st = sim->stream;
     // Every launch up to the traversal is a programmatic dependent launch
-    // (nb_common.cuh): up to 17 dependent kernels of 3 to 40 us each, whose gaps
+    // (nb_common.cuh): up to 17 dependent kernels, most of 3 to 40 us, whose gaps
     // added up.  A step of 4000 bodies 155 -> 143 us, of 100,003 639 -> 600, of 2^20
     // 3552 -> 3514.
     NB_TRY(launch_keys(sim, nk, curve));
