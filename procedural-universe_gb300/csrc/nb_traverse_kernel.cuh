@@ -86,16 +86,6 @@ __device__ __forceinline__ void bucket_accel(const float4* __restrict__ spos, in
     }
 }
 
-// The reference's float distance squared, (dx^2 + dy^2) + dz^2, every operation
-// rounded: these intrinsics are never contracted.  (The compiler contracts packed
-// products and sums, __fmul2_rn into __fadd2_rn, and the last bit of r2 then decided
-// otherwise for one body at one cell in some 2e8 decisions.  Taking the rounded r2
-// only inside the thresholds' band was 5% slower at 2^20 bodies by the registers
-// that the compiler then chose, taking it always 1%.)
-__device__ __forceinline__ float reference_r2(float dx, float dy, float dz) {
-    return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-}
-
 // Waiting entries at which a shared group's warps part: sooner, the parts are uneven,
 // later, the steps made alike are more.  A step by 6, 12 and 24: 4000 bodies 222, 195
 // and 227 us, 10,000 282, 262 and 304, 40,000 376, 365 and 372 (1000: 153, 161 and 161;
@@ -319,7 +309,7 @@ __global__ void __launch_bounds__(kTravBlock, BLOCKS) k_traverse(const float4* _
             const float2 dx = __fadd2_rn(make_float2(cm.x, cm.x), nx);
             const float2 dy = __fadd2_rn(make_float2(cm.y, cm.y), ny);
             const float2 dz = __fadd2_rn(make_float2(cm.z, cm.z), nz);
-            const float2 r2 = make_float2(reference_r2(dx.x, dy.x, dz.x), reference_r2(dx.y, dy.y, dz.y));
+            const float2 r2 = __fadd2_rn(__fadd2_rn(__fmul2_rn(dx, dx), __fmul2_rn(dy, dy)), __fmul2_rn(dz, dz));
             const float thr_acc = __int_as_float(mt.y), thr_rej = __int_as_float(mt.z);
             bool acc0 = r2.x > thr_acc, acc1 = r2.y > thr_acc;
             const bool band0 = a0 && !acc0 && !(r2.x < thr_rej), band1 = a1 && !acc1 && !(r2.y < thr_rej);
