@@ -19,7 +19,7 @@
 //     monopole (COM, TotalMass) acts, else an internal node is opened
 //     (__ballot_sync collects the lanes that open it into the pushed entry)
 //     and a depth-cap bucket acts body by body.
-// The opening test compares the float r^2 (computed as the reference does)
+// The opening test compares the float r^2 (the reference's up to its last bit)
 // with the cell's precomputed accept / reject thresholds; only when r^2 falls
 // between them (a 2e-5 relative band) is the exactly rounded ratio
 // float(side / sqrtf(r^2)) compared with theta_f, the smallest float >= Theta.
