@@ -67,15 +67,16 @@ struct nb_batch {
     DirGal* dgal = nullptr;
     int4* units = nullptr;
     int32_t* unit_src = nullptr;
-    // the members' launches: each takes the units [unit, unit + units) and folds
-    // the bodies [body, body + bodies) of the direct-sum range, in the same partials
+    // the members' launches, one after the other in the same partials: each takes the
+    // units [unit, unit + units) of members that take each pair once, then `apart` units of
+    // larger ones, and folds the bodies [body, body + bodies) of the direct-sum range
     struct DirLaunch {
-        int unit, units, body, bodies;
+        int unit, units, apart, body, bodies;
     };
     std::vector<DirLaunch> dlaunch;
     float4* part = nullptr;
     size_t part_cap = 0;
-    int* next_unit = nullptr;        // one counter a launch
+    int* next_unit = nullptr;        // two counters a launch
     size_t next_cap = 0;
     uint64_t direct_pairs = 0;
     // whole-batch transfers of many galaxies: runs of bodies and the dense copy of
@@ -152,21 +153,23 @@ int make_direct_plan(nb_batch* b, size_t cap, DirPlan* plan) {
         int4 u;
         int32_t src;
     };
-    std::vector<Unit> list;
+    std::vector<Unit> list, apart;
     *plan = DirPlan{};
     plan->gal.resize(b->ndgal);
     const int row = 128 * b->tune.direct_ipt, row_chunks = row / kDirChunk;
     size_t part_base = 0;
     int body = 0, bodies = 0;
     auto close = [&]() {
-        std::stable_sort(list.begin(), list.end(),
-                         [](const Unit& a, const Unit& c) { return (a.u.z & kDirChunks) > (c.u.z & kDirChunks); });
-        plan->launches.push_back({(int)plan->units.size(), (int)list.size(), body, bodies});
-        for (const Unit& u : list) {
-            plan->units.push_back(u.u);
-            plan->src.push_back(u.src);
+        plan->launches.push_back({(int)plan->units.size(), (int)list.size(), (int)apart.size(), body, bodies});
+        for (std::vector<Unit>* l : {&list, &apart}) {
+            std::stable_sort(l->begin(), l->end(),
+                             [](const Unit& a, const Unit& c) { return (a.u.z & 0xffff) > (c.u.z & 0xffff); });
+            for (const Unit& u : *l) {
+                plan->units.push_back(u.u);
+                plan->src.push_back(u.src);
+            }
+            l->clear();
         }
-        list.clear();
         plan->entries = std::max(plan->entries, part_base);
         body += bodies;
         part_base = 0;
@@ -194,9 +197,9 @@ int make_direct_plan(nb_batch* b, size_t cap, DirPlan* plan) {
             for (int c = 0, s = 0; c < chunks; c += L, ++s) {
                 const int k = std::min(L, chunks - c);
                 const int own = once ? std::max(0, std::min(k, row_chunks - c)) : k;
-                list.push_back(Unit{make_int4(t0, (int)g.off + s0 + c * kDirChunk, k | (once ? 0 : kDirBothParts) | (own << 16),
-                                              (int)part_base + s * n_pad + r * row),
-                                    once ? (int32_t)((long long)entry - (t0 + row)) : (int32_t)targets});
+                (once ? list : apart).push_back(Unit{make_int4(t0, (int)g.off + s0 + c * kDirChunk, k | (own << 16),
+                                                               (int)part_base + s * n_pad + r * row),
+                                                     once ? (int32_t)((long long)entry - (t0 + row)) : (int32_t)targets});
             }
             if (once) entry += (size_t)std::max(0, n_pad - (r + 1) * row);
         }
@@ -231,7 +234,7 @@ int plan_units(nb_batch* b) {
         dev_free(b->next_unit, b->core->stream);
         b->next_unit = nullptr;
         b->next_cap = 0;
-        NB_BCUDA(b, dev_alloc(&b->next_unit, plan.launches.size() * sizeof(int)));
+        NB_BCUDA(b, dev_alloc(&b->next_unit, 2 * plan.launches.size() * sizeof(int)));
         b->next_cap = plan.launches.size();
     }
     NB_BCUDA(b, upload(&b->units, plan.units, b->core->stream));
@@ -244,14 +247,21 @@ int plan_units(nb_batch* b) {
 
 // The direct members' force kernel: as many warps as the GPU holds, at most one
 // a unit.
-template <int LAW, int IPT>
-void launch_direct(nb_batch* b, const nb_batch::DirLaunch& d, int* next_unit, cudaStream_t st, float S) {
+template <int LAW, int IPT, bool APART>
+void launch_units(nb_batch* b, int unit, int units, int* next_unit, cudaStream_t st, float S) {
+    if (units == 0) return;
     const int threads = b->tune.direct_block, warps = threads / 32;
     int occ = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_direct<LAW, IPT>, threads, 0);
-    const int grid = std::max(1, std::min((d.units + warps - 1) / warps, b->core->sm_count * std::max(1, occ)));
-    k_batch_direct<LAW, IPT><<<grid, threads, 0, st>>>(b->core->pos, b->units + d.unit, b->unit_src + d.unit, d.units,
-                                                       next_unit, S, b->core->d_mmax, b->part);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_direct<LAW, IPT, APART>, threads, 0);
+    const int grid = std::max(1, std::min((units + warps - 1) / warps, b->core->sm_count * std::max(1, occ)));
+    k_batch_direct<LAW, IPT, APART><<<grid, threads, 0, st>>>(b->core->pos, b->units + unit, b->unit_src + unit, units,
+                                                              next_unit, S, b->core->d_mmax, b->part);
+}
+
+template <int LAW, int IPT>
+void launch_direct(nb_batch* b, const nb_batch::DirLaunch& d, int* next_unit, cudaStream_t st, float S) {
+    launch_units<LAW, IPT, false>(b, d.unit, d.units, next_unit, st, S);
+    launch_units<LAW, IPT, true>(b, d.unit + d.units, d.apart, next_unit + 1, st, S);
 }
 
 // One step (update) or one force evaluation (no update) of every galaxy,
@@ -271,7 +281,7 @@ int enqueue_step(nb_batch* b, float dt, bool update, bool tree_only = false) {
             const int words = std::max(6 * b->nslot, tree_counter_words());
             k_gal_box_init<<<(words + 255) / 256, 256, 0, st>>>(b->box_bits, b->nslot, t.counters,
                                                                tree_counter_words(), n, t.interactions, b->group_ctr,
-                                                               b->next_unit, (int)b->dlaunch.size());
+                                                               b->next_unit, 2 * (int)b->dlaunch.size());
             k_gal_box_chunks<<<(unsigned)((n + kBoxChunk - 1) / kBoxChunk), 256, 0, st>>>(c->pos, b->body_slot, n,
                                                                                        b->nslot, b->box_bits);
         }
@@ -318,18 +328,20 @@ int enqueue_step(nb_batch* b, float dt, bool update, bool tree_only = false) {
     if (b->ndgal > 0) {
         const int launches = (int)b->dlaunch.size();
         if (launches == 0) return bfail(b, NB_ENOMEM, "the direct-sum members found no memory");
-        PhaseScope ps(c, NB_PHASE_DIRECT_FORCE, 2 * launches);
+        int kernels = 0;
+        for (const auto& d : b->dlaunch) kernels += (d.units > 0) + (d.apart > 0) + 1;
+        PhaseScope ps(c, NB_PHASE_DIRECT_FORCE, kernels);
         // (else cleared with the counters)
-        if (b->n_bh == 0) NB_BCUDA(b, cudaMemsetAsync(b->next_unit, 0, launches * sizeof(int), st));
+        if (b->n_bh == 0) NB_BCUDA(b, cudaMemsetAsync(b->next_unit, 0, 2 * launches * sizeof(int), st));
         const bool wide = b->tune.direct_ipt == 2;
         for (int k = 0; k < launches; ++k) {
             const auto& d = b->dlaunch[k];
             if (b->base.law == NB_LAW_PLUMMER) {
-                if (wide) launch_direct<NB_LAW_PLUMMER, 8>(b, d, b->next_unit + k, st, S);
-                else launch_direct<NB_LAW_PLUMMER, 4>(b, d, b->next_unit + k, st, S);
+                if (wide) launch_direct<NB_LAW_PLUMMER, 8>(b, d, b->next_unit + 2 * k, st, S);
+                else launch_direct<NB_LAW_PLUMMER, 4>(b, d, b->next_unit + 2 * k, st, S);
             } else {
-                if (wide) launch_direct<NB_LAW_REFERENCE, 8>(b, d, b->next_unit + k, st, S);
-                else launch_direct<NB_LAW_REFERENCE, 4>(b, d, b->next_unit + k, st, S);
+                if (wide) launch_direct<NB_LAW_REFERENCE, 8>(b, d, b->next_unit + 2 * k, st, S);
+                else launch_direct<NB_LAW_REFERENCE, 4>(b, d, b->next_unit + 2 * k, st, S);
             }
             // whole members: a multiple of 256 bodies
             k_batch_direct_reduce<<<d.bodies / 32, 32 * kFoldWarps, 0, st>>>(

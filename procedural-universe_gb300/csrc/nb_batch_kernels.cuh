@@ -938,17 +938,16 @@ __global__ void __launch_bounds__(kGWarps * 32, 5) k_group_traverse(
 // ---- batched direct sum --------------------------------------------------------
 // A unit is a row of 32 * IPT target bodies, IPT a lane in registers (packed
 // FP32x2), against a run of 32-source chunks: (first target body, first source
-// body, chunks | kDirBothParts | chunks evaluated from the target side only << 16,
-// entry of the target partials); unit_src is the entry of body 0 among the row's
-// source partials, or, with kDirBothParts, the distance of the compensations from
-// the targets' sums.  Sources behind the row are evaluated once for both bodies, 17
+// body, chunks | chunks evaluated from the target side only << 16, entry of the
+// target partials); unit_src is the entry of body 0 among the row's source
+// partials, or, with APART, the distance of the compensations from the targets' sums.  Sources behind the row are evaluated once for both bodies, 17
 // FP32 operations for two interactions instead of 26: lane l takes source
 // (l + r) mod 32 at step r, and the sources' sums travel with them by shuffle
 // (as in k_direct_pairs, here within one warp).  The row's own bodies, and all
 // sources of a member of more than kDirOnceMax padded bodies (whose source
 // partials would grow with its square), are evaluated from the target side
-// (direct_chunk).  Such a member's few partials keep sum and compensation apart:
-// rounded to one word they added 2% to the force error at 9000 and 16,000 bodies.
+// (direct_chunk).  Such a member's few partials keep sum and compensation apart
+// (APART): rounded to one word they added 2% to the force error at 9000 and 16,000 bodies.
 // (Where each pair is taken once, the many partials of a body carry less: the error
 // is 4% below that of the target side with both parts.)
 //
@@ -960,8 +959,7 @@ __global__ void __launch_bounds__(kGWarps * 32, 5) k_group_traverse(
 // is the shuffles and reads that four targets a lane carry (eight: 268 us a
 // step, but small members then fill fewer rows).
 constexpr int kDirWarps = 8;   // most warps per block
-constexpr int kDirChunks = 0x7fff, kDirBothParts = 0x8000;   // fields of a unit
-template <int LAW, int IPT>
+template <int LAW, int IPT, bool APART>
 __global__ void __launch_bounds__(kDirWarps * 32, IPT == 4 ? 2 : 1) k_batch_direct(
     const float4* __restrict__ pos, const int4* __restrict__ units, const int32_t* __restrict__ unit_src, int nunits,
     int* __restrict__ next_unit, float S, const unsigned* __restrict__ mmax, float4* __restrict__ part) {
@@ -975,7 +973,7 @@ __global__ void __launch_bounds__(kDirWarps * 32, IPT == 4 ? 2 : 1) k_batch_dire
     u = __shfl_sync(0xffffffffu, u, 0);
     while (u < nunits) {
         const int4 un = units[u];
-        const int src0 = unit_src[u], chunks = un.z & kDirChunks, own = un.z >> 16;
+        const int src0 = unit_src[u], chunks = un.z & 0xffff, own = un.z >> 16;
         int after = 0;
         if (lane == 0) after = atomicAdd(next_unit, 1);
         float2 nx[P], ny[P], nz[P], mi[P];
@@ -997,14 +995,14 @@ __global__ void __launch_bounds__(kDirWarps * 32, IPT == 4 ? 2 : 1) k_batch_dire
             __syncwarp();   // also: every lane is done with the chunk that this buffer held
             if (c + 1 < chunks) cur = pos[un.y + (c + 1) * kDirChunk + lane];
             float3 f;
-            if (c < own) {
+            if (APART || c < own) {
                 direct_chunk<LAW, IPT, false>(buf, lane, nx, ny, nz, mi, S2, T2, sum, comp, f);
             } else {
                 direct_chunk<LAW, IPT, true>(buf, lane, nx, ny, nz, mi, S2, T2, sum, comp, f);
                 part[(long long)src0 + un.y + c * kDirChunk + lane] = make_float4(f.x, f.y, f.z, 0.f);
             }
         }
-        if (un.z & kDirBothParts) {
+        if (APART) {
 #pragma unroll
             for (int k = 0; k < IPT; ++k) {
                 const size_t at = (size_t)un.w + k * 32 + lane;
