@@ -276,8 +276,8 @@ def run_reference(args, name, w):
 # (dram__bytes_read.sum + dram__bytes_write.sum); the summaries under
 # profiles/ give the command and the figures.
 NCU_TRAFFIC = {
-    ("bh1m", "k_traverse"): (75.8e6, "profiles/k_traverse_bh1m.md"),
-    ("direct262k", "k_direct_pairs"): (1022.3e6, "profiles/k_direct_pairs_direct262k.md"),
+    ("bh1m", "k_traverse"): (79.5e6, "profiles/k_traverse_bh1m.md"),
+    ("direct262k", "k_direct_pairs"): (1021.5e6, "profiles/k_direct_pairs_direct262k.md"),
 }
 
 
