@@ -134,6 +134,8 @@ bool tuning_valid(const nb_tuning& t) {
 // the GPU many times over.
 constexpr size_t kDirPartials = ((size_t)1 << 30) / sizeof(float4);
 
+constexpr int kDirMaxChunks = 1024;   // chunks of the longest unit
+
 // The direct members' work units, and their launches within cap entries of partials.
 struct DirPlan {
     std::vector<int4> units;
@@ -161,12 +163,16 @@ int make_direct_plan(nb_batch* b, size_t cap, DirPlan* plan) {
     int body = 0, bodies = 0;
     auto close = [&]() {
         plan->launches.push_back({(int)plan->units.size(), (int)list.size(), (int)apart.size(), body, bodies});
-        for (std::vector<Unit>* l : {&list, &apart}) {
-            std::stable_sort(l->begin(), l->end(),
-                             [](const Unit& a, const Unit& c) { return (a.u.z & 0xffff) > (c.u.z & 0xffff); });
+        for (std::vector<Unit>* l : {&list, &apart}) {   // by chunks, the most first, else in their order
+            size_t at[kDirMaxChunks + 2] = {}, base = plan->units.size();
+            for (const Unit& u : *l) ++at[kDirMaxChunks - (u.u.z & 0xffff) + 1];
+            for (int k = 1; k <= kDirMaxChunks; ++k) at[k] += at[k - 1];
+            plan->units.resize(base + l->size());
+            plan->src.resize(base + l->size());
             for (const Unit& u : *l) {
-                plan->units.push_back(u.u);
-                plan->src.push_back(u.src);
+                const size_t k = base + at[kDirMaxChunks - (u.u.z & 0xffff)]++;
+                plan->units[k] = u.u;
+                plan->src[k] = u.src;
             }
             l->clear();
         }
@@ -181,7 +187,7 @@ int make_direct_plan(nb_batch* b, size_t cap, DirPlan* plan) {
         const bool once = n_pad <= kDirOnceMax;
         // chunks a unit: a quarter of the tile where units are cut finely enough to end
         // evenly, the whole tile for large members, whose partials grow with its inverse
-        const int L = std::min(1024, b->tune.direct_jtile / (once ? 4 * kDirChunk : kDirChunk));
+        const int L = std::min(kDirMaxChunks, b->tune.direct_jtile / (once ? 4 * kDirChunk : kDirChunk));
         const int splits = (sources / kDirChunk + L - 1) / L;
         const size_t rows = (size_t)n_pad / row;
         const size_t targets = (size_t)splits * n_pad;
